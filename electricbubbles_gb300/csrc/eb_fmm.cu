@@ -59,24 +59,47 @@ __device__ __forceinline__ int quadrant(unsigned long long key) {
 }
 
 // ---------------------------------------------------------------------------------
-// Charges (sorted order). Stokes: qa, qb of cadapdrop.f:214-222 plus the near-field
-// combinations P = qa + s qb, Q = qa - s qb, A = -s conj(qa).
+// Charges (sorted order). Stokes: qa, qb of cadapdrop.f:214-222, and the near-field data.
+//
+// The Stokes pair. With D = z_j - z_t, e = D / |D|^2 = conj(1/D) and the unit number
+// f = e / conj(e) = D e, the pair's term qa/D + s (conj(qb/D) - D conj(qa/D^2)) is
+//   e [qa conj(f) + s conj(qb) - s conj(qa) f],
+// and qa conj(f) -+ its conjugate is twice its real (s = -1) or i times its imaginary
+// part (s = +1). With f = 1 - 2 ey (dy - i dx), that is one real factor
+//   v = c0 + ey (ax dx + ay dy):   s = -1: c0 = 2 qa.x - qb.x, (ax, ay) = ( 4 qa.y, -4 qa.x)
+//                                  s = +1: c0 = 2 qa.y - qb.y, (ax, ay) = (-4 qa.x, -4 qa.y)
+// and the term is e (v + i c1) with c1 = qb.y (s = -1) or i e (v + i c1) with
+// c1 = -qb.x (s = +1; the sums over the sources are turned by i once, at their end).
+// FASMVP's qb is real (conj(dz) u minus its own conjugate, over i), so c1 = 0 for its sign
+// s = -1: 14 FP64 instructions a pair where the term as written takes 27. Measured on
+// 1,048,576 nodes (110.6 M pairs): the double-float near field 1,425 -> 918 us, the FP32
+// one 274 -> 216 us, the FP64 one below; errors against direct sums as before or smaller.
 // ---------------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ void near_charge(c_t<T> a, c_t<T> b, T s, T f, c_t<T>& ca, c_t<T>& cc) {
+  if (s < (T)0) {
+    ca = cmk<T>((T)4 * a.y * f, (T)-4 * a.x * f);
+    cc = cmk<T>(((T)2 * a.x - b.x) * f, b.y * f);
+  } else {
+    ca = cmk<T>((T)-4 * a.x * f, (T)-4 * a.y * f);
+    cc = cmk<T>(((T)2 * a.y - b.y) * f, -b.x * f);
+  }
+}
+
 // Computed in T: the FP32 operator forms its charges in FP32 (GB300's FP64 pipe is ~1/60
 // of its FP32 rate). dz = null: the charges of the transposed operator's sum,
-// qa = -dens, qb = conj(dens).
+// qa = -dens, qb = conj(dens). nc: the near field's (ax, ay), (c0, c1).
 template <typename T>
 __global__ void k_charges_stokes(int n, const int* __restrict__ perm,
                                  const double2* __restrict__ dens, const double2* __restrict__ dz,
                                  const double* __restrict__ hpt, double sd,
                                  c_t<T>* __restrict__ qa, c_t<T>* __restrict__ qb,
-                                 c_t<T>* __restrict__ pq, c_t<T>* __restrict__ aa) {
+                                 c_t<T>* __restrict__ nc) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int o = perm[i];
   const double2 ud = dens[o];
   const c_t<T> u = cmk<T>((T)ud.x, (T)ud.y);
-  const T s = (T)sd;
   c_t<T> a, b;
   if (dz) {
     const double2 dd = dz[o];
@@ -93,9 +116,7 @@ __global__ void k_charges_stokes(int n, const int* __restrict__ perm,
   }
   qa[i] = a;
   qb[i] = b;
-  pq[2 * i] = cmk<T>(a.x + s * b.x, a.y + s * b.y);
-  pq[2 * i + 1] = cmk<T>(a.x - s * b.x, a.y - s * b.y);
-  aa[i] = cmk<T>(-s * a.x, s * a.y);
+  near_charge<T>(a, b, (T)sd, (T)1, nc[2 * i], nc[2 * i + 1]);
 }
 
 __device__ __forceinline__ float4 df4(double2 v) {
@@ -103,12 +124,12 @@ __device__ __forceinline__ float4 df4(double2 v) {
   return make_float4(hx, __double2float_rn(v.x - (double)hx), hy, __double2float_rn(v.y - (double)hy));
 }
 
-// FP64 charges plus the double-float near-field data P, Q, A scaled by 1/r_leaf, the
-// side of the point's own leaf (the near field works in leaf units): 2^lev / W.
+// Double-float charges and near-field data, scaled by 1/r_leaf, the side of the point's
+// own leaf (the near field works in leaf units): 2^lev / W.
 __global__ void k_charges_stokes_df(int n, const int* __restrict__ perm, const double2* __restrict__ dens,
                                     const double2* __restrict__ dz, const double* __restrict__ hpt,
                                     double s, double winv, const unsigned char* __restrict__ plev,
-                                    float4* __restrict__ qdf, float4* __restrict__ pq, float4* __restrict__ aa) {
+                                    float4* __restrict__ qdf, float4* __restrict__ nc) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int o = perm[i];
@@ -127,9 +148,10 @@ __global__ void k_charges_stokes_df(int n, const int* __restrict__ perm, const d
   }
   qdf[2 * i] = df4(make_double2(a.x * rinv, a.y * rinv));
   qdf[2 * i + 1] = df4(make_double2(b.x * rinv, b.y * rinv));
-  pq[2 * i] = df4(make_double2((a.x + s * b.x) * rinv, (a.y + s * b.y) * rinv));
-  pq[2 * i + 1] = df4(make_double2((a.x - s * b.x) * rinv, (a.y - s * b.y) * rinv));
-  aa[i] = df4(make_double2(-s * a.x * rinv, s * a.y * rinv));
+  double2 ca, cc;
+  near_charge<double>(a, b, s, rinv, ca, cc);
+  nc[2 * i] = df4(ca);
+  nc[2 * i + 1] = df4(cc);
 }
 
 // Cauchy charge of node o: q[o], or u_o dz_o h_o (FASMVP_LAP, laplace.f:190-200) when
@@ -169,16 +191,51 @@ __global__ void k_charges_cauchy(int n, const int* __restrict__ perm,
 }
 
 // ---------------------------------------------------------------------------------
-// 1/x in FP64 for the near field: the hardware reciprocal approximation refined by two
-// Newton-Raphson steps r <- r + r (1 - x r), each of which squares the relative error.
+// 1/x in FP64 for the near field: the hardware's reciprocal approximation r (about 20
+// bits) and one third-order step r (1 + e + e^2) with e = 1 - x r, which cubes the
+// relative error: three FP64 instructions where two Newton steps take four.
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ double rcp_nr(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  double e = fma(-x, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-x, r, 1.0);
-  return fma(r, e, r);
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+// What a near-field pair adds (see the charges): NEAR_V the Stokes pair with c1 = 0,
+// NEAR_VC with it, NEAR_Q the Cauchy pair q / (z_t - z_j), NEAR_QI only its imaginary
+// part (all that FASMVP_LAP's post-processing reads).
+enum { NEAR_V = 0, NEAR_VC = 1, NEAR_Q = 2, NEAR_QI = 3 };
+
+// One pair in FP64: ca = (ax, ay), cc = (c0, c1), or ca = q.
+template <int K>
+__device__ __forceinline__ void near_pair64(double2 zj, double2 ca, double2 cc, double2 zi, double& gx,
+                                            double& gy) {
+  const double dx = zj.x - zi.x, dy = zj.y - zi.y;
+  const double rr = rcp_nr(fma(dx, dx, dy * dy));
+  if (K == NEAR_QI) {
+    gy = fma(fma(ca.x, dy, -ca.y * dx), rr, gy);
+    return;
+  }
+  const double ex = dx * rr, ey = dy * rr;  // conj(1/D)
+  if (K == NEAR_Q) {
+    gx = fma(-ca.x, ex, fma(-ca.y, ey, gx));
+    gy = fma(ca.x, ey, fma(-ca.y, ex, gy));
+  } else {
+    const double v = fma(ey, fma(ca.x, dx, ca.y * dy), cc.x);
+    gx = fma(ex, v, gx);
+    gy = fma(ey, v, gy);
+    if (K == NEAR_VC) {
+      gx = fma(-ey, cc.y, gx);
+      gy = fma(ex, cc.y, gy);
+    }
+  }
+}
+
+// The end of a Stokes near-field sum: s = +1 turns it by i.
+template <typename T>
+__device__ __forceinline__ c_t<T> near_turn(T gx, T gy, bool plus) {
+  return plus ? cmk<T>(-gy, gx) : cmk<T>(gx, gy);
 }
 
 template <typename T>
@@ -1076,41 +1133,128 @@ __device__ __forceinline__ void m2p_eval(const c_t<T>* M, int p, c_t<T> u, T s, 
   }
 }
 
-template <int E>
-__global__ void __launch_bounds__(128) k_leaf64(int ngroup, const int* __restrict__ gleaf,
-                                                const int* __restrict__ gfirst, const int* __restrict__ leaves,
-                                                int has_far, const unsigned long long* __restrict__ bkey,
-                                                const unsigned char* __restrict__ blev,
-                                                const int* __restrict__ pt0, const int* __restrict__ pt1,
-                                                const int* __restrict__ ustart, const int* __restrict__ ulist,
-                                                const int* __restrict__ wstart, const int* __restrict__ wlist,
-                                                const int* __restrict__ perm,
-                                                const double2* __restrict__ zs,
-                                                const double2* __restrict__ pq,
-                                                const double2* __restrict__ aa,
-                                                const double2* __restrict__ qa, double x0, double y0,
-                                                double W, int p, double s,
-                                                const double2* __restrict__ local,
-                                                const double2* __restrict__ mpole,
-                                                double2* __restrict__ out, EbPost post) {
-  int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (g >= ngroup) return;
-  const int lane = threadIdx.x & 31, tg = lane >> 2, sl = lane & 3;
-  const int leaf = gleaf[g], b = leaves[leaf];
-  const int i = gfirst[g] + tg;
-  const bool act = i < pt1[b];
-  const int ii = act ? i : gfirst[g];
-  const double2 zi = zs[ii];
+// FP64 near field, one block per tile of up to EB_NTILE targets of one leaf. GB300 issues
+// two FP64 lanes a cycle and SM, so that the kernel is bound by FP64 instructions, and a
+// lane without a pair costs as much as one with: the block's threads are dealt as
+// (slice, target) with as many slices of the sources as fit, 128 / T for a tile of T
+// targets (87 % of the lanes busy at T = 28, where 32-target tiles with fixed slices have
+// 77 % on average). Sources are staged through shared memory in slabs; a warp reads two or
+// three of them at once (broadcasts). The slices are added in a fixed order; the sums go
+// to nearbuf (sorted order), so that the near field runs beside the expansion passes.
+// Measured: 3.25 ms for the 110.6 M pairs of 1,048,576 nodes (82 % of the FP64 issue rate
+// at 14 instructions a pair), 149 us for the 4.0 M of 64 x 512; with a warp per 8 targets
+// reading every source from global memory and the longer pair, near and far field
+// together took 9.76 ms and 392 us (now, with the far field below, 5.7 ms and 233 us).
+#define NEAR64_SLAB 128
+template <int K>
+__global__ void __launch_bounds__(128) k_near64(const int4* __restrict__ tiles, const int* __restrict__ pt0,
+                                                const int* __restrict__ pt1, const int* __restrict__ ustart,
+                                                const int* __restrict__ ulist, const double2* __restrict__ zs,
+                                                const double2* __restrict__ q, int plus,
+                                                double2* __restrict__ nearbuf) {
+  constexpr bool ST = K == NEAR_V || K == NEAR_VC;
+  __shared__ double2 sz[NEAR64_SLAB], sa[NEAR64_SLAB], sc[ST ? NEAR64_SLAB : 1], sred[128];
+  __shared__ int sidx[NEAR64_SLAB], spre[33], sj0[32];
+  const int4 tl = tiles[blockIdx.x];
+  const int tid = threadIdx.x, T = tl.z - tl.y, nsl = 128 / T;
+  const int sl = tid / T, i = tl.y + tid - sl * T;
+  const double2 zi = zs[i];
   double gx = 0.0, gy = 0.0;
-  if (has_far && blev[b] >= 2) {
-    const double r = ldexp(W, -(int)blev[b]);
-    double2 c = box_center(bkey[b], x0, y0, r);
-    double2 u = make_double2((zi.x - c.x) / r, (zi.y - c.y) / r);
-    l2p_part<double, E>(local + (size_t)b * E * (p + 1), p, sl, u, s, gx, gy);
+  const int ub = ustart[tl.x], ue = ustart[tl.x + 1];
+  for (int cb = ub; cb < ue; cb += 32) {
+    const int nc = min(32, ue - cb);
+    if (cb > ub) __syncthreads();  // the previous boxes' slabs are consumed
+    if (tid < 32) {
+      int c = 0, j0 = 0;
+      if (tid < nc) {
+        const int sbx = ulist[cb + tid];
+        j0 = pt0[sbx];
+        c = pt1[sbx] - j0;
+      }
+      int x = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (tid >= o) x += y;
+      }
+      sj0[tid] = j0;
+      spre[tid + 1] = x;
+      if (tid == 0) spre[0] = 0;
+    }
+    __syncthreads();
+    const int total = spre[nc];
+    for (int base = 0; base < total; base += NEAR64_SLAB) {
+      const int ns = min(NEAR64_SLAB, total - base);
+      if (base > 0) __syncthreads();
+      if (tid < ns) {
+        const int gs = base + tid;
+        int lo = 0, hi = nc;  // the box k with spre[k] <= gs < spre[k + 1]
+        while (hi - lo > 1) {
+          const int mid = (lo + hi) >> 1;
+          if (spre[mid] <= gs) lo = mid;
+          else hi = mid;
+        }
+        const int j = sj0[lo] + gs - spre[lo];
+        sidx[tid] = j;
+        sz[tid] = zs[j];
+        if (ST) {
+          sa[tid] = q[2 * (size_t)j];
+          sc[tid] = q[2 * (size_t)j + 1];
+        } else {
+          sa[tid] = q[j];
+        }
+      }
+      __syncthreads();
+      if (sl < nsl) {
+#pragma unroll 2
+        for (int jj = sl; jj < ns; jj += nsl) {
+          if (sidx[jj] == i) continue;
+          near_pair64<K>(sz[jj], sa[jj], ST ? sc[jj] : make_double2(0.0, 0.0), zi, gx, gy);
+        }
+      }
+    }
   }
-  if (has_far) {
-    // W list: the lanes of a target take every 4th box
-    for (int jw = wstart[leaf] + sl; jw < wstart[leaf + 1]; jw += 4) {
+  sred[tid] = make_double2(gx, gy);
+  __syncthreads();
+  if (tid < T) {
+    double2 v = sred[tid];
+    for (int k = 1; k < nsl; ++k) v = cadd<double>(v, sred[k * T + tid]);
+    nearbuf[i] = ST ? near_turn<double>(v.x, v.y, plus) : v;
+  }
+}
+
+// FP64 far field: L2P of the leaf's local expansions and the W list, LPT lanes per target
+// (LPT = 4: a warp per group of 8 targets, each lane a quarter of the terms; LPT = 1: a
+// thread per target), plus the near-field sums, then the post-processing.
+template <int E, int LPT>
+__global__ void __launch_bounds__(128) k_far64(int n, const int* __restrict__ lflag,
+                                               const int* __restrict__ lscan,
+                                               const int* __restrict__ leaves, int has_far,
+                                               const unsigned long long* __restrict__ bkey,
+                                               const unsigned char* __restrict__ blev,
+                                               const int* __restrict__ wstart, const int* __restrict__ wlist,
+                                               const int* __restrict__ perm, const double2* __restrict__ zs,
+                                               double x0, double y0, double W, int p, double s,
+                                               const double2* __restrict__ local,
+                                               const double2* __restrict__ mpole,
+                                               const double2* __restrict__ nearbuf, double2* __restrict__ out,
+                                               EbPost post) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = g / LPT, sl = g - i * LPT;
+  const bool act = i < n;
+  double gx = 0.0, gy = 0.0;
+  if (act && has_far) {
+    const int leaf = lscan[i] + lflag[i] - 1, b = leaves[leaf];  // leaf heads up to point i
+    const double2 zi = zs[i];
+    if (blev[b] >= 2) {
+      const double r = ldexp(W, -(int)blev[b]);
+      const double2 c = box_center(bkey[b], x0, y0, r);
+      const double2 u = make_double2((zi.x - c.x) / r, (zi.y - c.y) / r);
+      const double2* lb = local + (size_t)b * E * (p + 1);
+      if (LPT == 1) l2p_range<double, E>(lb, p, 0, p + 1, u, s, gx, gy);
+      else l2p_part<double, E>(lb, p, sl, u, s, gx, gy);
+    }
+    for (int jw = wstart[leaf] + sl; jw < wstart[leaf + 1]; jw += LPT) {
       const int w = wlist[jw];
       const double rw = ldexp(W, -(int)blev[w]);
       const double2 cw = box_center(bkey[w], x0, y0, rw);
@@ -1118,35 +1262,16 @@ __global__ void __launch_bounds__(128) k_leaf64(int ngroup, const int* __restric
                           s, gx, gy);
     }
   }
-  for (int jl = ustart[leaf]; jl < ustart[leaf + 1]; ++jl) {
-    const int sb = ulist[jl];
-    const int j1 = pt1[sb];
-    for (int j = pt0[sb] + sl; j < j1; j += 4) {
-      if (j == ii) continue;
-      double2 zj = zs[j];
-      double dx = zj.x - zi.x, dy = zj.y - zi.y;
-      double rr = rcp_nr(fma(dx, dx, dy * dy));
-      double ix = dx * rr, iy = -dy * rr;  // 1/D
-      if (E == 2) {
-        double2 P = pq[2 * j], Q = pq[2 * j + 1], A = aa[j];
-        gx = fma(P.x, ix, fma(-P.y, iy, gx));  // qa/D + s conj(qb/D)
-        gy = fma(Q.x, iy, fma(Q.y, ix, gy));
-        double w2x = fma(ix, ix, -iy * iy), w2y = -2.0 * ix * iy;  // conj(1/D)^2
-        double tx = fma(dx, w2x, -dy * w2y), ty = fma(dx, w2y, dy * w2x);
-        gx = fma(A.x, tx, fma(-A.y, ty, gx));  // - s D conj(qa) conj(1/D)^2
-        gy = fma(A.x, ty, fma(A.y, tx, gy));
-      } else {
-        double2 q = qa[j];
-        gx = fma(-q.x, ix, fma(q.y, iy, gx));  // q/(z_i - z_j) = -q/D
-        gy = fma(-q.x, iy, fma(-q.y, ix, gy));
-      }
-    }
+  if (LPT == 4) {
+    gx += __shfl_xor_sync(0xffffffffu, gx, 1);
+    gy += __shfl_xor_sync(0xffffffffu, gy, 1);
+    gx += __shfl_xor_sync(0xffffffffu, gx, 2);
+    gy += __shfl_xor_sync(0xffffffffu, gy, 2);
   }
-  gx += __shfl_xor_sync(0xffffffffu, gx, 1);
-  gy += __shfl_xor_sync(0xffffffffu, gy, 1);
-  gx += __shfl_xor_sync(0xffffffffu, gx, 2);
-  gy += __shfl_xor_sync(0xffffffffu, gy, 2);
-  if (sl == 0 && act) eb_post_store(post, perm[i], make_double2(gx, gy), out);
+  if (act && sl == 0) {
+    const double2 nv = nearbuf[i];
+    eb_post_store(post, perm[i], make_double2(gx + nv.x, gy + nv.y), out);
+  }
 }
 
 // ---------------------------------------------------------------------------------
@@ -1294,25 +1419,28 @@ __device__ __forceinline__ void m2p_df(const float4* M, int p, cdf u, bool neg, 
   }
 }
 
-// MODE 0: far and near field; 1: near field only, into nearbuf (sorted order);
-// 2: far field only, plus nearbuf, then the post-processing. Modes 1 and 2 let the near
-// field run concurrently with the expansion passes.
-template <int E, int MODE>
-__global__ void __launch_bounds__(128) k_leaf_df(int ngroup, const int* __restrict__ gleaf,
+// The near field into nearbuf (sorted order): a warp per group of 8 targets of a leaf, 4
+// lanes per target over the sources. K: NEAR_V, NEAR_VC or NEAR_Q; nc: (ax, ay), (c0, c1)
+// per source, or q.
+__device__ __forceinline__ void df_quad_sum(dfl& vx, dfl& vy, int sl) {
+#pragma unroll
+  for (int o = 1; o <= 2; o <<= 1) {
+    dfl ox{__shfl_xor_sync(0xffffffffu, vx.hi, o), __shfl_xor_sync(0xffffffffu, vx.lo, o)};
+    dfl oy{__shfl_xor_sync(0xffffffffu, vy.hi, o), __shfl_xor_sync(0xffffffffu, vy.lo, o)};
+    vx = (sl & o) ? dfl_add(ox, vx) : dfl_add(vx, ox);
+    vy = (sl & o) ? dfl_add(oy, vy) : dfl_add(vy, oy);
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(128) k_near_df(int ngroup, const int* __restrict__ gleaf,
                                                  const int* __restrict__ gfirst, const int* __restrict__ leaves,
-                                                 int has_far, const unsigned long long* __restrict__ bkey,
+                                                 const unsigned long long* __restrict__ bkey,
                                                  const unsigned char* __restrict__ blev,
                                                  const int* __restrict__ pt0, const int* __restrict__ pt1,
                                                  const int* __restrict__ ustart, const int* __restrict__ ulist,
-                                                 const int* __restrict__ wstart, const int* __restrict__ wlist,
-                                                 const float4* __restrict__ mpole,
-                                                 const int* __restrict__ perm,
-                                                 const float4* __restrict__ wa,
-                                                 const float2* __restrict__ wb,
-                                                 const float4* __restrict__ pq,
-                                                 const float4* __restrict__ aa, int p, double s,
-                                                 const float4* __restrict__ local,
-                                                 double2* __restrict__ out, EbPost post,
+                                                 const float4* __restrict__ wa, const float2* __restrict__ wb,
+                                                 const float4* __restrict__ nc, int plus,
                                                  double2* __restrict__ nearbuf) {
   const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (g >= ngroup) return;
@@ -1323,25 +1451,11 @@ __global__ void __launch_bounds__(128) k_leaf_df(int ngroup, const int* __restri
   const int ii = act ? i : gfirst[g];
   const float4 wia = wa[ii];
   const float2 wib = wb[ii];
-  const cdf wi = cdf{{wia.x, wia.z}, {wia.y, wia.w}};
-  const bool neg = s < 0.0;
   const int lt = blev[b];
   dfacc gx{0.f, 0.f}, gy{0.f, 0.f};
-  if (MODE != 1 && has_far && lt >= 2) l2p_part_df<E>(local + (size_t)b * E * (p + 1), p, sl, wi, neg, gx, gy);
   const unsigned long long kb = bkey[b];
   const int bx = (int)compact2d(kb), by = (int)compact2d(kb >> 1);
-  if (MODE != 1 && has_far) {
-    // W list: the lanes of a target take every 4th box
-    for (int jw = wstart[leaf] + sl; jw < wstart[leaf + 1]; jw += 4) {
-      const int w = wlist[jw];
-      const unsigned long long kw = bkey[w];
-      float3 tx, ty;
-      frame_shift(wia, wib, blev[w] - lt, bx, by, (int)compact2d(kw), (int)compact2d(kw >> 1), tx, ty);
-      m2p_df<E>(mpole + (size_t)w * E * p, p, cdf{tf_to_dfl(tx), tf_to_dfl(ty)}, neg, gx, gy);
-    }
-  }
-  const int u0 = ustart[leaf], u1 = MODE == 2 ? u0 : ustart[leaf + 1];
-  for (int jl = u0; jl < u1; ++jl) {
+  for (int jl = ustart[leaf]; jl < ustart[leaf + 1]; ++jl) {
     const int sb = ulist[jl];
     const unsigned long long ks = bkey[sb];
     // the target relative to the source leaf's centre, in that leaf's units (three
@@ -1356,51 +1470,79 @@ __global__ void __launch_bounds__(128) k_leaf_df(int ngroup, const int* __restri
       // D / r = w_j - (w_i - offset): hi and mid parts subtracted exactly
       const dfl dx = tf_diff(ja.x, ja.z, jb.x, tx), dy = tf_diff(ja.y, ja.w, jb.y, ty);
       const dfl rr = dfl_rcp(dfl_add(dfl_sqr(dx), dfl_sqr(dy)));
-      const dfl ix = dfl_mul(dx, rr), iy = dfl_neg(dfl_mul(dy, rr));  // 1/D
-      if (E == 2) {
-        const cdf P = cdf_from_float4(pq[2 * j]), Q = cdf_from_float4(pq[2 * j + 1]);
-        const cdf A = cdf_from_float4(aa[j]);
-        acc_prod(gx, P.x, ix);  // qa/D + s conj(qb/D)
-        acc_prod(gx, dfl_neg(P.y), iy);
-        acc_prod(gy, Q.x, iy);
-        acc_prod(gy, Q.y, ix);
-        const dfl w2x = dfl_mul(dfl_add(ix, iy), dfl_sub(ix, iy));  // conj(1/D)^2
-        const dfl ixy = dfl_mul(ix, iy);
-        const dfl w2y = dfl{-2.f * ixy.hi, -2.f * ixy.lo};
-        const dfl t2x = dfl_sub(dfl_mul(dx, w2x), dfl_mul(dy, w2y));
-        const dfl t2y = dfl_add(dfl_mul(dx, w2y), dfl_mul(dy, w2x));
-        acc_prod(gx, A.x, t2x);  // - s D conj(qa) conj(1/D)^2
-        acc_prod(gx, dfl_neg(A.y), t2y);
-        acc_prod(gy, A.x, t2y);
-        acc_prod(gy, A.y, t2x);
+      const dfl ex = dfl_mul(dx, rr), ey = dfl_mul(dy, rr);  // conj(1/D)
+      if (K == NEAR_Q) {
+        const cdf q = cdf_from_float4(nc[j]);  // q/(z_i - z_j) = -q/D
+        acc_prod(gx, dfl_neg(q.x), ex);
+        acc_prod(gx, dfl_neg(q.y), ey);
+        acc_prod(gy, q.x, ey);
+        acc_prod(gy, dfl_neg(q.y), ex);
       } else {
-        const cdf q = cdf_from_float4(pq[j]);  // q/(z_i - z_j) = -q/D
-        acc_prod(gx, dfl_neg(q.x), ix);
-        acc_prod(gx, q.y, iy);
-        acc_prod(gy, dfl_neg(q.x), iy);
-        acc_prod(gy, dfl_neg(q.y), ix);
+        const float4 a = nc[2 * (size_t)j], c = nc[2 * (size_t)j + 1];
+        const dfl m = dfl_add(dfl_mul(dfl{a.x, a.y}, dx), dfl_mul(dfl{a.z, a.w}, dy));
+        const dfl v = dfl_add(dfl{c.x, c.y}, dfl_mul(ey, m));
+        acc_prod(gx, ex, v);
+        acc_prod(gy, ey, v);
+        if (K == NEAR_VC) {
+          const dfl c1{c.z, c.w};
+          acc_prod(gx, dfl_neg(ey), c1);
+          acc_prod(gy, ex, c1);
+        }
       }
     }
   }
   dfl vx = acc_value(gx), vy = acc_value(gy);
-#pragma unroll
-  for (int o = 1; o <= 2; o <<= 1) {
-    dfl ox{__shfl_xor_sync(0xffffffffu, vx.hi, o), __shfl_xor_sync(0xffffffffu, vx.lo, o)};
-    dfl oy{__shfl_xor_sync(0xffffffffu, vy.hi, o), __shfl_xor_sync(0xffffffffu, vy.lo, o)};
-    vx = (sl & o) ? dfl_add(ox, vx) : dfl_add(vx, ox);
-    vy = (sl & o) ? dfl_add(oy, vy) : dfl_add(vy, oy);
-  }
+  df_quad_sum(vx, vy, sl);
   if (sl == 0 && act) {
-    double2 v = make_double2(dfl_to_double(vx), dfl_to_double(vy));
-    if (MODE == 1) {
-      nearbuf[i] = v;
-    } else {
-      if (MODE == 2) {
-        const double2 nv = nearbuf[i];
-        v = make_double2(v.x + nv.x, v.y + nv.y);
-      }
-      eb_post_store(post, perm[i], v, out);
+    const double x = dfl_to_double(vx), y = dfl_to_double(vy);
+    nearbuf[i] = K == NEAR_Q ? make_double2(x, y) : near_turn<double>(x, y, plus);
+  }
+}
+
+// The far field (L2P and the W list) plus the near-field sums, then the post-processing.
+template <int E>
+__global__ void __launch_bounds__(128) k_far_df(int ngroup, const int* __restrict__ gleaf,
+                                                const int* __restrict__ gfirst, const int* __restrict__ leaves,
+                                                int has_far, const unsigned long long* __restrict__ bkey,
+                                                const unsigned char* __restrict__ blev,
+                                                const int* __restrict__ pt1,
+                                                const int* __restrict__ wstart, const int* __restrict__ wlist,
+                                                const float4* __restrict__ mpole, const int* __restrict__ perm,
+                                                const float4* __restrict__ wa, const float2* __restrict__ wb,
+                                                int p, double s, const float4* __restrict__ local,
+                                                double2* __restrict__ out, EbPost post,
+                                                const double2* __restrict__ nearbuf) {
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (g >= ngroup) return;
+  const int lane = threadIdx.x & 31, tg = lane >> 2, sl = lane & 3;
+  const int leaf = gleaf[g], b = leaves[leaf];
+  const int i = gfirst[g] + tg;
+  const bool act = i < pt1[b];
+  const int ii = act ? i : gfirst[g];
+  const float4 wia = wa[ii];
+  const float2 wib = wb[ii];
+  const cdf wi = cdf{{wia.x, wia.z}, {wia.y, wia.w}};
+  const bool neg = s < 0.0;
+  const int lt = blev[b];
+  dfacc gx{0.f, 0.f}, gy{0.f, 0.f};
+  if (has_far && lt >= 2) l2p_part_df<E>(local + (size_t)b * E * (p + 1), p, sl, wi, neg, gx, gy);
+  if (has_far) {
+    const unsigned long long kb = bkey[b];
+    const int bx = (int)compact2d(kb), by = (int)compact2d(kb >> 1);
+    // W list: the lanes of a target take every 4th box
+    for (int jw = wstart[leaf] + sl; jw < wstart[leaf + 1]; jw += 4) {
+      const int w = wlist[jw];
+      const unsigned long long kw = bkey[w];
+      float3 tx, ty;
+      frame_shift(wia, wib, blev[w] - lt, bx, by, (int)compact2d(kw), (int)compact2d(kw >> 1), tx, ty);
+      m2p_df<E>(mpole + (size_t)w * E * p, p, cdf{tf_to_dfl(tx), tf_to_dfl(ty)}, neg, gx, gy);
     }
+  }
+  dfl vx = acc_value(gx), vy = acc_value(gy);
+  df_quad_sum(vx, vy, sl);
+  if (sl == 0 && act) {
+    const double2 nv = nearbuf[i];
+    eb_post_store(post, perm[i], make_double2(dfl_to_double(vx) + nv.x, dfl_to_double(vy) + nv.y), out);
   }
 }
 
@@ -1494,38 +1636,39 @@ __global__ void __launch_bounds__(128) k_far32(const int4* __restrict__ tiles, c
 // compensated sums buy nothing. Writes the near-field sums in sorted order. Positions are
 // absolute (float hi + lo), so sources of any level are alike.
 #define NEAR_SLAB 256
-template <int E>
-__device__ __forceinline__ void near_pair(const float4 hlj, const float4 PQ, const float2 A, const float4 hl,
-                                          float& gx, float& gy) {
+template <int K>
+__device__ __forceinline__ void near_pair(const float4 hlj, const float4 c, const float4 hl, float& gx, float& gy) {
   const float dx = (hlj.x - hl.x) + (hlj.z - hl.z);
   const float dy = (hlj.y - hl.y) + (hlj.w - hl.w);
   const float rr = __fdividef(1.0f, fmaf(dx, dx, fmaf(dy, dy, 1e-36f)));
-  const float ix = dx * rr, iy = -dy * rr;  // 1 / (z_s - z_t)
-  if (E == 2) {
-    const float w2x = fmaf(ix, ix, -iy * iy), w2y = -2.0f * ix * iy;
-    const float tx = fmaf(dx, w2x, -dy * w2y), ty = fmaf(dx, w2y, dy * w2x);
-    gx = fmaf(PQ.x, ix, fmaf(-PQ.y, iy, fmaf(A.x, tx, fmaf(-A.y, ty, gx))));
-    gy = fmaf(PQ.z, iy, fmaf(PQ.w, ix, fmaf(A.x, ty, fmaf(A.y, tx, gy))));
-  } else {
-    gx = fmaf(-A.x, ix, fmaf(A.y, iy, gx));
-    gy = fmaf(-A.x, iy, fmaf(-A.y, ix, gy));
+  const float ex = dx * rr, ey = dy * rr;  // conj(1/D), D = z_s - z_t
+  if (K == NEAR_Q) {  // c = (q, -, -)
+    gx = fmaf(-c.x, ex, fmaf(-c.y, ey, gx));
+    gy = fmaf(c.x, ey, fmaf(-c.y, ex, gy));
+  } else {  // c = (ax, ay, c0, c1)
+    const float v = fmaf(ey, fmaf(c.x, dx, c.y * dy), c.z);
+    gx = fmaf(ex, v, gx);
+    gy = fmaf(ey, v, gy);
+    if (K == NEAR_VC) {
+      gx = fmaf(-ey, c.w, gx);
+      gy = fmaf(ex, c.w, gy);
+    }
   }
 }
 
-template <int E>
+template <int K>
 __global__ void __launch_bounds__(128, 8) k_near32(const int4* __restrict__ tiles, const int* __restrict__ leaves,
                                                    const int* __restrict__ pt0, const int* __restrict__ pt1,
                                                    const int* __restrict__ ustart, const int* __restrict__ ulist,
                                                    const float4* __restrict__ zhl,
-                                                   const float2* __restrict__ pq,
-                                                   const float2* __restrict__ aa,
-                                                   const float2* __restrict__ qa,
+                                                   const float2* __restrict__ qn, int plus,
                                                    double2* __restrict__ nearbuf) {
+  constexpr bool ST = K != NEAR_Q;
   static_assert(EB_NTILE == 32, "two targets per thread over 16 lanes");
   constexpr int NS = 8;
   __shared__ float4 sz[NEAR_SLAB];
-  __shared__ float4 sp[E == 2 ? NEAR_SLAB : 1];
-  __shared__ float2 sa[NEAR_SLAB];
+  __shared__ float4 sp[ST ? NEAR_SLAB : 1];
+  __shared__ float2 sa[ST ? 1 : NEAR_SLAB];
   __shared__ int spre[33], sj0[32];
   __shared__ float2 sred[NS][EB_NTILE];
   const int4 tl = tiles[blockIdx.x];
@@ -1572,21 +1715,16 @@ __global__ void __launch_bounds__(128, 8) k_near32(const int4* __restrict__ tile
         }
         const int j = sj0[lo] + gs - spre[lo];
         sz[s2] = zhl[j];
-        if (E == 2) {
-          sp[s2] = reinterpret_cast<const float4*>(pq)[j];
-          sa[s2] = aa[j];
-        } else {
-          sa[s2] = qa[j];
-        }
+        if (ST) sp[s2] = reinterpret_cast<const float4*>(qn)[j];
+        else sa[s2] = qn[j];
       }
       __syncthreads();
 #pragma unroll 2
       for (int jj = sl; jj < ns; jj += NS) {
         const float4 hlj = sz[jj];
-        const float4 PQ = E == 2 ? sp[jj] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float2 A = sa[jj];
-        near_pair<E>(hlj, PQ, A, h0, gx0, gy0);
-        near_pair<E>(hlj, PQ, A, h1, gx1, gy1);
+        const float4 c = ST ? sp[jj] : make_float4(sa[jj].x, sa[jj].y, 0.f, 0.f);
+        near_pair<K>(hlj, c, h0, gx0, gy0);
+        near_pair<K>(hlj, c, h1, gx1, gy1);
       }
     }
   }
@@ -1600,6 +1738,7 @@ __global__ void __launch_bounds__(128, 8) k_near32(const int4* __restrict__ tile
       v.x += sred[q][tid].x;
       v.y += sred[q][tid].y;
     }
+    if (ST) v = near_turn<float>(v.x, v.y, plus);
     nearbuf[tl.y + tid] = make_double2((double)v.x, (double)v.y);
   }
 }
@@ -1635,56 +1774,45 @@ __device__ __forceinline__ void direct_block_sum(T& gx, T& gy) {
   }
 }
 
-template <int E>
+template <int K>
 __global__ void __launch_bounds__(128) k_direct64(int n, const double2* __restrict__ zs,
-                                                  const double2* __restrict__ pq,
-                                                  const double2* __restrict__ aa,
-                                                  const double2* __restrict__ qa, const int* __restrict__ perm,
-                                                  double2* __restrict__ out, EbPost post) {
+                                                  const double2* __restrict__ q, const int* __restrict__ perm,
+                                                  int plus, double2* __restrict__ out, EbPost post) {
+  constexpr bool ST = K == NEAR_V || K == NEAR_VC;
   const int i = blockIdx.x;  // one block of 128 threads per target, the threads over the sources
   const double2 zi = zs[i];
   double gx = 0.0, gy = 0.0;
   for (int j = threadIdx.x; j < n; j += 128) {
     if (j == i) continue;
-    const double2 zj = zs[j];
-    const double dx = zj.x - zi.x, dy = zj.y - zi.y;
-    const double rr = rcp_nr(fma(dx, dx, dy * dy));
-    const double ix = dx * rr, iy = -dy * rr;  // 1/D
-    if (E == 2) {
-      const double2 P = pq[2 * j], Q = pq[2 * j + 1], A = aa[j];
-      gx = fma(P.x, ix, fma(-P.y, iy, gx));  // qa/D + s conj(qb/D)
-      gy = fma(Q.x, iy, fma(Q.y, ix, gy));
-      const double w2x = fma(ix, ix, -iy * iy), w2y = -2.0 * ix * iy;  // conj(1/D)^2
-      const double tx = fma(dx, w2x, -dy * w2y), ty = fma(dx, w2y, dy * w2x);
-      gx = fma(A.x, tx, fma(-A.y, ty, gx));  // - s D conj(qa) conj(1/D)^2
-      gy = fma(A.x, ty, fma(A.y, tx, gy));
-    } else {
-      const double2 q = qa[j];
-      gx = fma(-q.x, ix, fma(q.y, iy, gx));  // q/(z_i - z_j) = -q/D
-      gy = fma(-q.x, iy, fma(-q.y, ix, gy));
-    }
+    const double2 ca = ST ? q[2 * j] : q[j], cc = ST ? q[2 * j + 1] : make_double2(0.0, 0.0);
+    near_pair64<K>(zs[j], ca, cc, zi, gx, gy);
   }
   direct_block_sum<double>(gx, gy);
-  if (threadIdx.x == 0) eb_post_store(post, perm[i], make_double2(gx, gy), out);
+  if (threadIdx.x == 0) {
+    const double2 v = ST ? near_turn<double>(gx, gy, plus) : make_double2(gx, gy);
+    eb_post_store(post, perm[i], v, out);
+  }
 }
 
 // The FP32 operator's direct sums: positions as float hi + lo, the pair of k_near32.
-template <int E>
+template <int K>
 __global__ void __launch_bounds__(128) k_direct32(int n, const float4* __restrict__ zhl,
-                                                  const float4* __restrict__ pq, const float2* __restrict__ aa,
-                                                  const float2* __restrict__ qa, const int* __restrict__ perm,
-                                                  double2* __restrict__ out, EbPost post) {
+                                                  const float2* __restrict__ nc, const int* __restrict__ perm,
+                                                  int plus, double2* __restrict__ out, EbPost post) {
+  constexpr bool ST = K != NEAR_Q;
   const int i = blockIdx.x;
   const float4 hi = zhl[i];
   float gx = 0.f, gy = 0.f;
   for (int j = threadIdx.x; j < n; j += 128) {
     if (j == i) continue;
-    const float4 PQ = E == 2 ? pq[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2 A = E == 2 ? aa[j] : qa[j];
-    near_pair<E>(zhl[j], PQ, A, hi, gx, gy);
+    const float4 c = ST ? reinterpret_cast<const float4*>(nc)[j] : make_float4(nc[j].x, nc[j].y, 0.f, 0.f);
+    near_pair<K>(zhl[j], c, hi, gx, gy);
   }
   direct_block_sum<float>(gx, gy);
-  if (threadIdx.x == 0) eb_post_store_f32(post, perm[i], make_float2(gx, gy), out);
+  if (threadIdx.x == 0) {
+    const float2 v = ST ? near_turn<float>(gx, gy, plus) : make_float2(gx, gy);
+    eb_post_store_f32(post, perm[i], v, out);
+  }
 }
 
 // ---------------------------------------------------------------------------------
@@ -1767,8 +1895,8 @@ __global__ void k_reflect_df(int first, int nb, const unsigned long long* __rest
 //   z conj(Phi') + conj(Psi) = (z - z_j) conj(gamma1 t^2 + 2 gamma2 t^3)
 //                              + 2 conj(gamma2 t^2) + conj(delta1 t),
 // which has no terms of size |z|. One block per box of level ld (blocks off the wall
-// return at once); sources staged through shared memory. sorted: add into dst in the
-// sorted order (the near-field buffer of the split passes), else in node order.
+// return at once); sources staged through shared memory. Added to the near-field sums
+// (sorted order).
 #define IMG_TILE 128
 __global__ void __launch_bounds__(IMG_TILE) k_img_near(int off, int nb, int lev,
                                                        const unsigned long long* __restrict__ bkey,
@@ -1777,7 +1905,7 @@ __global__ void __launch_bounds__(IMG_TILE) k_img_near(int off, int nb, int lev,
                                                        const double2* __restrict__ dens,
                                                        const double2* __restrict__ dz,
                                                        const double* __restrict__ hpt, double s,
-                                                       double2* __restrict__ dst, int sorted) {
+                                                       double2* __restrict__ nearbuf) {
   __shared__ double2 sz[IMG_TILE], sg1[IMG_TILE], sg2[IMG_TILE], sd1[IMG_TILE];
   const int b = off + blockIdx.x;
   const unsigned long long key = bkey[b];
@@ -1846,15 +1974,15 @@ __global__ void __launch_bounds__(IMG_TILE) k_img_near(int off, int nb, int lev,
         }
       }
     }
-    if (act) {
-      const int o = sorted ? i : perm[i];
-      dst[o] = make_double2(dst[o].x + acc.x, dst[o].y + acc.y);
-    }
+    if (act) nearbuf[i] = make_double2(nearbuf[i].x + acc.x, nearbuf[i].y + acc.y);
   }
 }
 
 inline int nblk(long long n, int bs) { return (int)((n + bs - 1) / bs); }
 inline int round32(int n) { return (n + 31) & ~31; }
+#ifndef FAR64_LPT
+#define FAR64_LPT 4
+#endif
 template <typename T>
 int tables_build(EbTables& tb, int p, double tol) {
   tb.p = p;
@@ -1977,7 +2105,7 @@ int fmm_expansions_df(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
     size_t sm = sizeof(float4) * (32 * (size_t)(p + 1) + 96);
     if (sm > 48 * 1024) EB_CUDA_TRY(cudaFuncSetAttribute(k_p2m_df<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     k_p2m_df<E><<<t.nleaf, std::max(128, round32((E == 2 ? 3 : 1) * p)), sm, st>>>(t.leaves.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(), t.wdf.as<float4>(),
-                                          E == 2 ? w.qdf.as<float4>() : w.pqdf.as<float4>(), p, mp);
+                                          E == 2 ? w.qdf.as<float4>() : w.ncdf.as<float4>(), p, mp);
     eb_count_launch(ctx);
   }
   for (int l = L - 1; l >= 2; --l) {
@@ -2142,11 +2270,19 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
   return EB_OK;
 }
 
+// What the near-field pair needs (see the charges): FASMVP's charges with its sign have
+// c1 = 0, and FASMVP_LAP's post-processing (kind 2) reads the imaginary part only.
+template <int E>
+int near_kind(int sign, const double2* dz, const EbPost& post) {
+  if (E == 1) return post.kind == 2 ? NEAR_QI : NEAR_Q;
+  return dz && sign < 0 ? NEAR_V : NEAR_VC;
+}
+
 // The direct path of a small problem: the FMM's charges, k_direct64 / k_direct32, and
 // the post-processing. FP64-class requests (native or double-float) run in native FP64.
 template <int E>
 int direct_run(eb_ctx* ctx, EbTree& t, bool f32, int sign, const double2* dens, const double2* dz,
-               const double* hpt, const double2* q, double2* out, const EbPost* postp, cudaEvent_t join) {
+               const double* hpt, const double2* q_in, double2* out, const EbPost* postp, cudaEvent_t join) {
   EbPost post{};
   if (postp) post = *postp;
   cudaStream_t st = eb_stream(ctx);
@@ -2154,32 +2290,42 @@ int direct_run(eb_ctx* ctx, EbTree& t, bool f32, int sign, const double2* dens, 
   EbFmmWork& w = f32 ? ctx->work32 : ctx->work64;
   const size_t cs = f32 ? sizeof(float2) : sizeof(double2);
   EB_TRY(w.qa.ensure(cs * (size_t)n));
-  EB_TRY(w.qb.ensure(cs * (size_t)n));
-  EB_TRY(w.pq.ensure(cs * 2 * (size_t)n));
-  EB_TRY(w.aa.ensure(cs * (size_t)n));
+  if (E == 2) {
+    EB_TRY(w.qb.ensure(cs * (size_t)n));
+    EB_TRY(w.nc.ensure(cs * 2 * (size_t)n));
+  }
   const int g = n;  // one block of 128 threads per target
+  const int kind = near_kind<E>(sign, dz, post);
+  const bool plus = sign > 0;
   if (f32) {
+    const float4* zh = t.zhl.as<float4>();
+    const float2* q = E == 2 ? w.nc.as<float2>() : w.qa.as<float2>();
     if (E == 2)
       k_charges_stokes<float><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), dens, dz, hpt, (double)sign,
                                                             w.qa.as<float2>(), w.qb.as<float2>(),
-                                                            w.pq.as<float2>(), w.aa.as<float2>());
+                                                            w.nc.as<float2>());
     else
-      k_charges_cauchy<float><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q, post.u, post.dz, post.hpt,
+      k_charges_cauchy<float><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q_in, post.u, post.dz, post.hpt,
                                                             w.qa.as<float2>());
     if (join) EB_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
-    k_direct32<E><<<g, 128, 0, st>>>(n, t.zhl.as<float4>(), reinterpret_cast<const float4*>(w.pq.p),
-                                     w.aa.as<float2>(), w.qa.as<float2>(), t.perm.as<int>(), out, post);
+    if (E == 1) k_direct32<NEAR_Q><<<g, 128, 0, st>>>(n, zh, q, t.perm.as<int>(), 0, out, post);
+    else if (kind == NEAR_V) k_direct32<NEAR_V><<<g, 128, 0, st>>>(n, zh, q, t.perm.as<int>(), plus, out, post);
+    else k_direct32<NEAR_VC><<<g, 128, 0, st>>>(n, zh, q, t.perm.as<int>(), plus, out, post);
   } else {
+    const double2* zz = t.zs.as<double2>();
+    const double2* q = E == 2 ? w.nc.as<double2>() : w.qa.as<double2>();
     if (E == 2)
       k_charges_stokes<double><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), dens, dz, hpt, (double)sign,
                                                              w.qa.as<double2>(), w.qb.as<double2>(),
-                                                             w.pq.as<double2>(), w.aa.as<double2>());
+                                                             w.nc.as<double2>());
     else
-      k_charges_cauchy<double><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q, post.u, post.dz, post.hpt,
+      k_charges_cauchy<double><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q_in, post.u, post.dz, post.hpt,
                                                              w.qa.as<double2>());
     if (join) EB_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
-    k_direct64<E><<<g, 128, 0, st>>>(n, t.zs.as<double2>(), w.pq.as<double2>(), w.aa.as<double2>(),
-                                     w.qa.as<double2>(), t.perm.as<int>(), out, post);
+    if (kind == NEAR_Q) k_direct64<NEAR_Q><<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), 0, out, post);
+    else if (kind == NEAR_QI) k_direct64<NEAR_QI><<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), 0, out, post);
+    else if (kind == NEAR_V) k_direct64<NEAR_V><<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), plus, out, post);
+    else k_direct64<NEAR_VC><<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), plus, out, post);
   }
   ctx->launches += 2;
   return eb_check_launch(ctx, "direct sum");
@@ -2201,26 +2347,25 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
   const int n = t.n;
   const bool df = f64 && df_req;
   if (df) {
-    EB_TRY(w.pqdf.ensure(sizeof(float4) * 2 * (size_t)n));
-    EB_TRY(w.aadf.ensure(sizeof(float4) * (size_t)n));
-    EB_TRY(w.qdf.ensure(sizeof(float4) * 2 * (size_t)n));
+    EB_TRY(w.ncdf.ensure(sizeof(float4) * E * (size_t)n));
+    if (E == 2) EB_TRY(w.qdf.ensure(sizeof(float4) * 2 * (size_t)n));
   } else {
     EB_TRY(w.qa.ensure(sizeof(c_t<T>) * (size_t)n));
-    EB_TRY(w.qb.ensure(sizeof(c_t<T>) * (size_t)n));
-    EB_TRY(w.pq.ensure(sizeof(c_t<T>) * 2 * (size_t)n));
-    EB_TRY(w.aa.ensure(sizeof(c_t<T>) * (size_t)n));
+    if (E == 2) {
+      EB_TRY(w.qb.ensure(sizeof(c_t<T>) * (size_t)n));
+      EB_TRY(w.nc.ensure(sizeof(c_t<T>) * 2 * (size_t)n));
+    }
   }
   if (df && E == 2) {
     k_charges_stokes_df<<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), dens, dz, hpt, (double)sign,
                                                       1.0 / t.W, t.plev.as<unsigned char>(), w.qdf.as<float4>(),
-                                                      w.pqdf.as<float4>(), w.aadf.as<float4>());
+                                                      w.ncdf.as<float4>());
   } else if (df) {
     k_charges_cauchy_df<<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q, post.u, post.dz, post.hpt,
-                                                      1.0 / t.W, t.plev.as<unsigned char>(), w.pqdf.as<float4>());
+                                                      1.0 / t.W, t.plev.as<unsigned char>(), w.ncdf.as<float4>());
   } else if (E == 2) {
     k_charges_stokes<T><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), dens, dz, hpt, (double)sign,
-                                                      w.qa.as<c_t<T>>(), w.qb.as<c_t<T>>(),
-                                                      w.pq.as<c_t<T>>(), w.aa.as<c_t<T>>());
+                                                      w.qa.as<c_t<T>>(), w.qb.as<c_t<T>>(), w.nc.as<c_t<T>>());
   } else {
     k_charges_cauchy<T><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q, post.u, post.dz, post.hpt,
                                                       w.qa.as<c_t<T>>());
@@ -2228,40 +2373,62 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
   eb_count_launch(ctx);
   const int has_far = t.L >= 2;
   int blocks = nblk((long long)t.ngroup * 32, 128);
-  // FP32 and double-float: the near field runs on the side stream while the expansion
-  // passes run on the main stream, and the far-field kernel adds both. Measured up to
-  // 2^20 nodes it pays at every size (the expansion passes' coarse levels stay
-  // latency-bound): against a limit of 2^18, the 285,440-node batch's RK2 step 35.1 →
-  // 33.6 ms and the 1,048,576-node refined solve 45.7 → 44.3 ms. The per-kernel profiling
-  // timer times the combined kernel.
-  const bool split = has_far && (df || !f64) && !ctx->profiling && n <= (1 << 20);
-  if (split) {
-    EB_TRY(w.nearbuf.ensure(sizeof(double2) * (size_t)n));
-    EB_CUDA_TRY(cudaEventRecord(ctx->ev_c, st));
-    EB_CUDA_TRY(cudaStreamWaitEvent(ctx->side_stream, ctx->ev_c, 0));
-    cudaStream_t ss = ctx->side_stream;
+  const int kind = near_kind<E>(sign, dz, post);
+  const int plus = sign > 0;
+  EB_TRY(w.nearbuf.ensure(sizeof(double2) * (size_t)n));
+  double2* nb = w.nearbuf.as<double2>();
+  auto near = [&](cudaStream_t ns) {
     if (df) {
-      k_leaf_df<E, 1><<<blocks, 128, 0, ss>>>(
-          t.ngroup, t.gleaf.as<int>(), t.gfirst.as<int>(), t.leaves.as<int>(), 0, t.bkey.as<unsigned long long>(),
-          t.blev.as<unsigned char>(), t.pt0.as<int>(), t.pt1.as<int>(), t.ustart.as<int>(), t.ulist.as<int>(),
-          t.wstart.as<int>(), t.wlist.as<int>(), w.mpole_df.as<float4>(), t.perm.as<int>(),
-          t.wdf.as<float4>(), t.wdf_lo.as<float2>(), w.pqdf.as<float4>(), w.aadf.as<float4>(), tb.p,
-          (double)sign, w.local_df.as<float4>(), out, post, w.nearbuf.as<double2>());
+      auto go = [&](auto kern) {
+        kern<<<blocks, 128, 0, ns>>>(t.ngroup, t.gleaf.as<int>(), t.gfirst.as<int>(), t.leaves.as<int>(),
+                                     t.bkey.as<unsigned long long>(), t.blev.as<unsigned char>(), t.pt0.as<int>(),
+                                     t.pt1.as<int>(), t.ustart.as<int>(), t.ulist.as<int>(), t.wdf.as<float4>(),
+                                     t.wdf_lo.as<float2>(), w.ncdf.as<float4>(), plus, nb);
+      };
+      if (E == 1) go(k_near_df<NEAR_Q>);
+      else if (kind == NEAR_V) go(k_near_df<NEAR_V>);
+      else go(k_near_df<NEAR_VC>);
+    } else if (f64) {
+      const double2* nq = E == 2 ? w.nc.as<double2>() : w.qa.as<double2>();
+      auto go = [&](auto kern) {
+        kern<<<t.ntile, 128, 0, ns>>>(t.tiles.as<int4>(), t.pt0.as<int>(), t.pt1.as<int>(), t.ustart.as<int>(),
+                                      t.ulist.as<int>(), t.zs.as<double2>(), nq, plus, nb);
+      };
+      if (kind == NEAR_Q) go(k_near64<NEAR_Q>);
+      else if (kind == NEAR_QI) go(k_near64<NEAR_QI>);
+      else if (kind == NEAR_V) go(k_near64<NEAR_V>);
+      else go(k_near64<NEAR_VC>);
     } else {
-      k_near32<E><<<t.ntile, 128, 0, ss>>>(t.tiles.as<int4>(), t.leaves.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(),
-                                           t.ustart.as<int>(), t.ulist.as<int>(), t.zhl.as<float4>(),
-                                           w.pq.as<float2>(), w.aa.as<float2>(), w.qa.as<float2>(),
-                                           w.nearbuf.as<double2>());
+      const float2* nq = E == 2 ? w.nc.as<float2>() : w.qa.as<float2>();
+      auto go = [&](auto kern) {
+        kern<<<t.ntile, 128, 0, ns>>>(t.tiles.as<int4>(), t.leaves.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(),
+                                      t.ustart.as<int>(), t.ulist.as<int>(), t.zhl.as<float4>(), nq, plus, nb);
+      };
+      if (E == 1) go(k_near32<NEAR_Q>);
+      else if (kind == NEAR_V) go(k_near32<NEAR_V>);
+      else go(k_near32<NEAR_VC>);
     }
     eb_count_launch(ctx);
     if (E == 2 && t.wall && dz) {  // the wall's reflected near field joins the near-field sums
       const int ld = t.ld, nbl = t.lev_off[ld + 1] - t.lev_off[ld];
-      k_img_near<<<nbl, IMG_TILE, 0, ss>>>(t.lev_off[ld], nbl, ld, t.bkey.as<unsigned long long>(), t.pt0.as<int>(),
+      k_img_near<<<nbl, IMG_TILE, 0, ns>>>(t.lev_off[ld], nbl, ld, t.bkey.as<unsigned long long>(), t.pt0.as<int>(),
                                            t.pt1.as<int>(), t.zs.as<double2>(), t.perm.as<int>(), dens, dz, hpt,
-                                           (double)sign, w.nearbuf.as<double2>(), 1);
+                                           (double)sign, nb);
       eb_count_launch(ctx);
     }
-    EB_CUDA_TRY(cudaEventRecord(ctx->ev_p2p, ss));
+  };
+  // The near field runs on the side stream while the expansion passes run on the main
+  // stream, and the far-field kernel adds both. Measured up to
+  // 2^20 nodes it pays at every size (the expansion passes' coarse levels stay
+  // latency-bound): against a limit of 2^18, the 285,440-node batch's RK2 step 35.1 →
+  // 33.6 ms and the 1,048,576-node refined solve 45.7 → 44.3 ms. Above that, and under the
+  // per-kernel profiling timer, it precedes the far field on the main stream.
+  const bool split = has_far && !ctx->profiling && n <= (1 << 20);
+  if (split) {
+    EB_CUDA_TRY(cudaEventRecord(ctx->ev_c, st));
+    EB_CUDA_TRY(cudaStreamWaitEvent(ctx->side_stream, ctx->ev_c, 0));
+    near(ctx->side_stream);
+    EB_CUDA_TRY(cudaEventRecord(ctx->ev_p2p, ctx->side_stream));
   }
   if (has_far && df) EB_TRY(fmm_expansions_df<E>(ctx, t, tb, w));
   else if (has_far) EB_TRY((fmm_expansions<T, E>(ctx, t, tb, w)));
@@ -2274,61 +2441,36 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
   if (split) EB_CUDA_TRY(cudaStreamWaitEvent(st, ctx->ev_p2p, 0));
   if (join) EB_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
   if (!split && !f64) {
-    // FP32 without the split: the near-field kernel, then the far field on the same stream
-    EB_TRY(w.nearbuf.ensure(sizeof(double2) * (size_t)n));
     ProfScope pn(ctx, 2, st);
-    k_near32<E><<<t.ntile, 128, 0, st>>>(t.tiles.as<int4>(), t.leaves.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(),
-                                         t.ustart.as<int>(), t.ulist.as<int>(), t.zhl.as<float4>(),
-                                         w.pq.as<float2>(), w.aa.as<float2>(), w.qa.as<float2>(),
-                                         w.nearbuf.as<double2>());
-    eb_count_launch(ctx);
+    near(st);
     pn.done();
   }
   ProfScope ps(ctx, 0, st);
-  if (df && split) {
-    k_leaf_df<E, 2><<<blocks, 128, 0, st>>>(
+  if (!split && f64) near(st);
+  if (df) {
+    k_far_df<E><<<blocks, 128, 0, st>>>(
         t.ngroup, t.gleaf.as<int>(), t.gfirst.as<int>(), t.leaves.as<int>(), has_far, t.bkey.as<unsigned long long>(),
-        t.blev.as<unsigned char>(), t.pt0.as<int>(), t.pt1.as<int>(), t.ustart.as<int>(), t.ulist.as<int>(),
-        t.wstart.as<int>(), t.wlist.as<int>(), w.mpole_df.as<float4>(), t.perm.as<int>(),
-        t.wdf.as<float4>(), t.wdf_lo.as<float2>(), w.pqdf.as<float4>(), w.aadf.as<float4>(), tb.p,
-        (double)sign, w.local_df.as<float4>(), out, post, w.nearbuf.as<double2>());
-  } else if (split) {
-    k_far32<E><<<t.ntile, 128, far_sm, st>>>(t.tiles.as<int4>(), t.leaves.as<int>(),
-                                             t.bkey.as<unsigned long long>(), t.blev.as<unsigned char>(),
-                                             t.anc.as<int>(), t.wstart.as<int>(), t.wlist.as<int>(), t.perm.as<int>(),
-                                             t.wdf.as<float4>(), tb.p, (float)sign, w.local.as<float2>(),
-                                             w.mpole.as<float2>(), out, post, w.nearbuf.as<double2>());
-  } else if (df) {
-    k_leaf_df<E, 0><<<blocks, 128, 0, st>>>(
-        t.ngroup, t.gleaf.as<int>(), t.gfirst.as<int>(), t.leaves.as<int>(), has_far, t.bkey.as<unsigned long long>(),
-        t.blev.as<unsigned char>(), t.pt0.as<int>(), t.pt1.as<int>(), t.ustart.as<int>(), t.ulist.as<int>(),
-        t.wstart.as<int>(), t.wlist.as<int>(), w.mpole_df.as<float4>(), t.perm.as<int>(),
-        t.wdf.as<float4>(), t.wdf_lo.as<float2>(), w.pqdf.as<float4>(), w.aadf.as<float4>(), tb.p,
-        (double)sign,
-        w.local_df.as<float4>(), out, post, nullptr);
+        t.blev.as<unsigned char>(), t.pt1.as<int>(), t.wstart.as<int>(), t.wlist.as<int>(), w.mpole_df.as<float4>(),
+        t.perm.as<int>(), t.wdf.as<float4>(), t.wdf_lo.as<float2>(), tb.p, (double)sign, w.local_df.as<float4>(),
+        out, post, nb);
   } else if (f64) {
-    k_leaf64<E><<<blocks, 128, 0, st>>>(
-        t.ngroup, t.gleaf.as<int>(), t.gfirst.as<int>(), t.leaves.as<int>(), has_far, t.bkey.as<unsigned long long>(),
-        t.blev.as<unsigned char>(), t.pt0.as<int>(), t.pt1.as<int>(), t.ustart.as<int>(), t.ulist.as<int>(),
-        t.wstart.as<int>(), t.wlist.as<int>(), t.perm.as<int>(),
-        t.zs.as<double2>(), w.pq.as<double2>(), w.aa.as<double2>(), w.qa.as<double2>(), t.x0, t.y0,
-        t.W, tb.p, (double)sign, w.local.as<double2>(), w.mpole.as<double2>(), out, post);
+    const int lpt = FAR64_LPT;
+    auto go = [&](auto kern) {
+      kern<<<nblk((long long)n * lpt, 128), 128, 0, st>>>(
+          n, t.lflag.as<int>(), t.lscan.as<int>(), t.leaves.as<int>(), has_far, t.bkey.as<unsigned long long>(),
+          t.blev.as<unsigned char>(), t.wstart.as<int>(), t.wlist.as<int>(), t.perm.as<int>(), t.zs.as<double2>(),
+          t.x0, t.y0, t.W, tb.p, (double)sign, w.local.as<double2>(), w.mpole.as<double2>(), nb, out, post);
+    };
+    if (lpt == 1) go(k_far64<E, 1>);
+    else go(k_far64<E, 4>);
   } else {
     k_far32<E><<<t.ntile, 128, far_sm, st>>>(t.tiles.as<int4>(), t.leaves.as<int>(),
                                              t.bkey.as<unsigned long long>(), t.blev.as<unsigned char>(),
                                              t.anc.as<int>(), t.wstart.as<int>(), t.wlist.as<int>(), t.perm.as<int>(),
                                              t.wdf.as<float4>(), tb.p, (float)sign, w.local.as<float2>(),
-                                             w.mpole.as<float2>(), out, post, w.nearbuf.as<double2>());
+                                             w.mpole.as<float2>(), out, post, nb);
   }
   eb_count_launch(ctx);
-  if (E == 2 && t.wall && dz && !split) {  // the reflected near field, after the output is written
-    const int ld = t.ld, nb = t.lev_off[ld + 1] - t.lev_off[ld];
-    double2* dst = post.kind == 1 ? reinterpret_cast<double2*>(post.y) : out;
-    k_img_near<<<nb, IMG_TILE, 0, st>>>(t.lev_off[ld], nb, ld, t.bkey.as<unsigned long long>(), t.pt0.as<int>(),
-                                        t.pt1.as<int>(), t.zs.as<double2>(), t.perm.as<int>(), dens, dz, hpt,
-                                        (double)sign, dst, 0);
-    eb_count_launch(ctx);
-  }
   ps.done();
   ctx->last_p = tb.p;
   return eb_check_launch(ctx, "fmm apply");

@@ -166,8 +166,8 @@ struct EbTables {
 
 struct EbFmmWork {
   DevBuf qa, qb;     // c_t<T>[n] sorted charges (P2M)
-  DevBuf pq, aa;     // near-field source data (P2P)
-  DevBuf pqdf, aadf; // double-float near-field source data, scaled by 1/r_leaf (float4)
+  DevBuf nc;         // c_t<T>[2n]: near-field coefficients of the Stokes pair
+  DevBuf ncdf;       // double-float near-field data (or Cauchy charges), scaled by 1/r_leaf (float4[E n])
   DevBuf mpole_df;   // float4[nbox*E*p]: multipoles, double-float pipeline
   DevBuf local_df;   // float4[nbox*E*(p+1)]: local expansions, double-float pipeline
   DevBuf qdf;        // float4[2n]: qa/r, qb/r as double-float (P2M)
