@@ -2088,6 +2088,15 @@ struct ProfScope {
   }
 };
 
+constexpr int FX_DF = 16384;
+
+// Boxes of the levels 2, 3, .. of at most 384 boxes: their V lists are the long ones.
+int coarse_boxes(const EbTree& t) {
+  int l = 2;
+  while (l <= t.L && t.lev_off[l + 1] - t.lev_off[l] <= 384) ++l;
+  return t.lev_off[l] - t.lev_off[2];
+}
+
 // Upward pass, M2L and downward pass, shared by both kernels. Leaves the local
 // expansions of every box in w.local.
 // Expansions of the double-float pipeline (FP64-class accuracy on the FP32 pipes):
@@ -2122,7 +2131,13 @@ int fmm_expansions_df(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
     if (sm > 48 * 1024)
       EB_CUDA_TRY(cudaFuncSetAttribute(k_m2l_df<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     ProfScope ps(ctx, 1, st);
-    if (nt > 0) {
+    // the fixed-point M2L from FX_DF boxes on (measured in eb_m2l_fx.cu)
+    const bool fixed = p <= EB_FX_MAXP && nt >= FX_DF;
+    const int ncoarse = coarse_boxes(t);
+    if (nt > 0 && fixed) {
+      EB_TRY(eb_m2l_fx(ctx, E, true, first, nt, nt, ncoarse, t.vlist.as<int>(), t.vcode.as<unsigned char>(), t.vcount.as<int>(),
+                       tb, w, mp, lo, 0, st));
+    } else if (nt > 0) {
       k_m2l_df<E><<<nt, 128, sm, st>>>(first, t.vlist.as<int>(), t.vcode.as<unsigned char>(), t.vcount.as<int>(),
                                        p, tb.binom_df.as<float2>(), ldb, tb.dinv_df.as<float4>(), tb.pd.as<int>(),
                                        mp, lo, 0);
@@ -2133,10 +2148,16 @@ int fmm_expansions_df(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
       EB_TRY(w.mimg.ensure(sizeof(float4) * (size_t)nimg * E * p));
       k_reflect_df<<<nblk((long long)nbi * p, 128), 128, 0, st>>>(first, nbi, t.bkey.as<unsigned long long>(), p,
                                                                  mp, w.mimg.as<float4>());
-      k_m2l_df<E><<<nbi, 128, sm, st>>>(first, t.ilist.as<int>(), t.icode.as<unsigned char>(), t.icount.as<int>(),
-                                        p, tb.binom_df.as<float2>(), ldb, tb.dinv_df.as<float4>(), tb.pd.as<int>(),
-                                        w.mimg.as<float4>(), lo, 1);
-      ctx->launches += 2;
+      eb_count_launch(ctx);
+      if (fixed) {
+        EB_TRY(eb_m2l_fx(ctx, E, true, first, nbi, nbi, ncoarse, t.ilist.as<int>(), t.icode.as<unsigned char>(),
+                         t.icount.as<int>(), tb, w, w.mimg.p, lo, 1, st));
+      } else {
+        k_m2l_df<E><<<nbi, 128, sm, st>>>(first, t.ilist.as<int>(), t.icode.as<unsigned char>(), t.icount.as<int>(),
+                                          p, tb.binom_df.as<float2>(), ldb, tb.dinv_df.as<float4>(), tb.pd.as<int>(),
+                                          w.mimg.as<float4>(), lo, 1);
+        eb_count_launch(ctx);
+      }
     }
     ps.done();
   }
@@ -2213,6 +2234,8 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
     if (sm > 48 * 1024)
       EB_CUDA_TRY(cudaFuncSetAttribute(k_m2l<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     ProfScope ps(ctx, 1, st);
+    const bool fixed = sizeof(T) == 8 && p <= EB_FX_MAXP;
+    const int ncoarse = coarse_boxes(t);
     if (nt > 0 && sizeof(T) == 4 && p == 20 && ctx->opts.m2l_tc > 0) {
       EB_TRY(eb_m2l_tc(ctx, E, first, nt, t.vlist.as<int>(), t.vcode.as<unsigned char>(), t.vcount.as<int>(),
                        reinterpret_cast<const float*>(tb.binom.p), ldb, reinterpret_cast<const float2*>(tb.dinv.p),
@@ -2225,6 +2248,9 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
                                             reinterpret_cast<const float2*>(w.mpole.p),
                                             reinterpret_cast<float2*>(w.local.p), 0);
       eb_count_launch(ctx);
+    } else if (nt > 0 && fixed) {
+      EB_TRY(eb_m2l_fx(ctx, E, false, first, nt, nt, ncoarse, t.vlist.as<int>(), t.vcode.as<unsigned char>(),
+                       t.vcount.as<int>(), tb, w, w.mpole.p, w.local.p, 0, st));
     } else if (nt > 0) {
       k_m2l<T, E><<<nt, 128, sm, st>>>(first, t.vlist.as<int>(), t.vcode.as<unsigned char>(),
                                        t.vcount.as<int>(), p, tb.binom.as<T>(), ldb,
@@ -2243,11 +2269,14 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
                                                reinterpret_cast<const float2*>(tb.dinv.p), tb.pd.as<int>(),
                                                reinterpret_cast<const float2*>(w.mimg.p),
                                                reinterpret_cast<float2*>(w.local.p), 1);
+      else if (fixed)
+        EB_TRY(eb_m2l_fx(ctx, E, false, first, nbi, nbi, ncoarse, t.ilist.as<int>(), t.icode.as<unsigned char>(),
+                         t.icount.as<int>(), tb, w, w.mimg.p, w.local.p, 1, st));
       else
         k_m2l<T, E><<<nbi, 128, sm, st>>>(first, t.ilist.as<int>(), t.icode.as<unsigned char>(), t.icount.as<int>(),
                                           p, tb.binom.as<T>(), ldb, tb.dinv.as<c_t<T>>(), tb.pd.as<int>(),
                                           w.mimg.as<c_t<T>>(), w.local.as<c_t<T>>(), 1);
-      ctx->launches += 2;
+      ctx->launches += fixed ? 1 : 2;
     }
     ps.done();
   }
@@ -2485,6 +2514,7 @@ int eb_tables_init(eb_ctx* ctx) {
     return EB_ERR_TOL;
   }
   EB_TRY(tables_build<double>(ctx->tab64, p64, ctx->opts.tol64));
+  EB_TRY(eb_m2l_fx_tables(ctx->tab64));
   EB_TRY(tables_build<float>(ctx->tab32, p32, ctx->opts.tol32));
   return EB_OK;
 }

@@ -162,7 +162,12 @@ struct EbTables {
   DevBuf dinv_df;   // float4[EB_NCODE*(p+2)]
   DevBuf epow_df;   // float4[4*(p+2)]
   DevBuf einv_df;   // float4[4*(p+2)]
+  // fixed-point M2L (FP64 tables of order <= EB_FX_MAXP): the binomial matrix's digits, the
+  // powers (2/d)^j as limbs of 2^62 fractions, and the matrix's row scalings
+  DevBuf fxb, fxt, fxr;
 };
+#define EB_FX_K 48      // orders of the fixed-point M2L's operand tiles
+#define EB_FX_MAXP 47   // its largest expansion order (p + 1 local orders)
 
 struct EbFmmWork {
   DevBuf qa, qb;     // c_t<T>[n] sorted charges (P2M)
@@ -175,6 +180,8 @@ struct EbFmmWork {
   DevBuf mpole;      // c_t<T>[nbox*E*p]
   DevBuf mpart;      // c_t<T>[nchunk*E*p]: per-chunk partial multipoles (FP32 direct P2M)
   DevBuf local;      // c_t<T>[nbox*E*(p+1)]
+  DevBuf next;       // int: the FP64 near field's tile counter
+  DevBuf mfix;       // fixed-point multipoles of the M2L: longlong2[nbox*E*p], int4[nbox] exponents
   DevBuf mimg;       // multipoles mirrored across the wall, in the pipeline's format
 };
 
@@ -407,6 +414,12 @@ int eb_laplace_matvec_adj_dev(eb_ctx* ctx, const double* x, double* y, int prec)
 int eb_m2l_tc(eb_ctx* ctx, int E, int first, int ntarget, const int* vlist, const unsigned char* vcode,
               const int* vcount, const float* binom, int ldb, const float2* dinv, const int* pd,
               const float2* mpole, float2* local, cudaStream_t st);
+
+// m2l_fx.cu: the FP64-class M2L in fixed point on the tensor cores (orders <= EB_FX_MAXP)
+int eb_m2l_fx(eb_ctx* ctx, int E, bool df, int first, int ntarget, int nsrc, int ncoarse, const int* vlist,
+              const unsigned char* vcode, const int* vcount, EbTables& tb, EbFmmWork& w, const void* mpole,
+              void* local, int accumulate, cudaStream_t st);
+int eb_m2l_fx_tables(EbTables& tb);
 
 // api.cu: (re)build the installed geometry's tree with the current eb_opts
 int eb_geom_tree(eb_ctx* ctx);
