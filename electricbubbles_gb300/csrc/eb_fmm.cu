@@ -22,6 +22,7 @@
 //    separation ratio needs for the requested tolerance.
 #include <algorithm>
 #include <cmath>
+#include <functional>
 #include <vector>
 
 #include "eb_df.cuh"
@@ -53,6 +54,8 @@ __device__ __forceinline__ double2 box_center(unsigned long long key, double x0,
   unsigned int ix = compact2d(key), iy = compact2d(key >> 1);
   return make_double2(x0 + ((double)ix + 0.5) * r, y0 + ((double)iy + 0.5) * r);
 }
+
+__device__ __forceinline__ double pow2d(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 
 __device__ __forceinline__ int quadrant(unsigned long long key) {
   return (int)(key & 3ull);  // bit 0: ix & 1, bit 1: iy & 1
@@ -88,14 +91,16 @@ __device__ __forceinline__ void near_charge(c_t<T> a, c_t<T> b, T s, T f, c_t<T>
 
 // Computed in T: the FP32 operator forms its charges in FP32 (GB300's FP64 pipe is ~1/60
 // of its FP32 rate). dz = null: the charges of the transposed operator's sum,
-// qa = -dens, qb = conj(dens). nc: the near field's (ax, ay), (c0, c1).
+// qa = -dens, qb = conj(dens). nc: the near field's (ax, ay), (c0, c1). next: the FP64 near
+// field's tile counter, set to zero.
 template <typename T>
 __global__ void k_charges_stokes(int n, const int* __restrict__ perm,
                                  const double2* __restrict__ dens, const double2* __restrict__ dz,
                                  const double* __restrict__ hpt, double sd,
                                  c_t<T>* __restrict__ qa, c_t<T>* __restrict__ qb,
-                                 c_t<T>* __restrict__ nc) {
+                                 c_t<T>* __restrict__ nc, int* __restrict__ next) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0 && next) *next = 0;
   if (i >= n) return;
   int o = perm[i];
   const double2 ud = dens[o];
@@ -178,8 +183,9 @@ template <typename T>
 __global__ void k_charges_cauchy(int n, const int* __restrict__ perm,
                                  const double2* __restrict__ q, const double* __restrict__ lu,
                                  const double2* __restrict__ dz, const double* __restrict__ hpt,
-                                 c_t<T>* __restrict__ qa) {
+                                 c_t<T>* __restrict__ qa, int* __restrict__ next) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0 && next) *next = 0;
   if (i >= n) return;
   const int o = perm[i];
   if (q) {
@@ -255,126 +261,274 @@ __device__ __forceinline__ c_t<T> cpow_int(c_t<T> u, int n) {
 // write their powers w^j to shared memory, then thread j forms the power sums
 //   A_j = sum a w^j,  B_j = sum b w^j,  C_j = sum conj(w) a w^j   (a = qa/r, b = qb/r)
 // and M_phi[k] = -A_{k-1}, M_psi[k] = -(B_{k-1} + (k-1) C_{k-2}).
+//
+// FP64-bound: about 15 FP64 instructions per point and order. The powers come by doubling
+// (w^j = w^(j-len) w^len, all points and orders of a step at once), and four groups of
+// threads take a quarter of the points each, every thread all three sums of its order, so
+// that 176 of 192 lanes are busy at p = 44. BREAL: real charges b (FASMVP's own, see the
+// charges). Measured alone: 96 -> 72 us at 64 x 512, 2.25 -> 1.50 ms at 1,024 x 1,024.
 // ---------------------------------------------------------------------------------
-template <typename T, int E>
-__global__ void __launch_bounds__(64) k_p2m(const int* __restrict__ leaves,
-                                            const unsigned long long* __restrict__ bkey,
-                                            const unsigned char* __restrict__ blev,
-                                            const int* __restrict__ pt0, const int* __restrict__ pt1,
-                                            const double2* __restrict__ zs,
-                                            const c_t<T>* __restrict__ qa,
-                                            const c_t<T>* __restrict__ qb, double x0, double y0,
-                                            double W, int p, c_t<T>* __restrict__ mpole) {
-  extern __shared__ unsigned char smem_raw[];
+constexpr int P2M_NG = 4;  // groups of points
+template <int E, bool BREAL>
+__global__ void __launch_bounds__(256) k_p2m64(const int* __restrict__ leaves,
+                                               const unsigned long long* __restrict__ bkey,
+                                               const unsigned char* __restrict__ blev,
+                                               const int* __restrict__ pt0, const int* __restrict__ pt1,
+                                               const double2* __restrict__ zs,
+                                               const double2* __restrict__ qa,
+                                               const double2* __restrict__ qb, double x0, double y0,
+                                               double W, double winv, int p, double2* __restrict__ mpole) {
+  extern __shared__ double2 sm2d[];
   const int ps = p + 1;  // odd row stride: conflict-free rows
-  c_t<T>* pw = reinterpret_cast<c_t<T>*>(smem_raw);
-  c_t<T>* sc = pw + 32 * ps;
+  double2* pw = sm2d;                // [32][p + 1]: w^j per point
+  double2* sc = pw + 32 * ps;        // a, b, conj(w) a per point
   const int b = leaves[blockIdx.x];
-  int tid = threadIdx.x;
-  const double r = ldexp(W, -(int)blev[b]);
-  double2 c = box_center(bkey[b], x0, y0, r);
-  const T rinv = (T)(1.0 / r);
-  c_t<T> A = cmk<T>(0, 0), B = cmk<T>(0, 0), C = cmk<T>(0, 0);
-  int i0 = pt0[b], i1 = pt1[b];
-  for (int base = i0; base < i1; base += 32) {
-    int cnt = min(32, i1 - base);
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int lev = blev[b];
+  const double rinv = winv * pow2d(lev);
+  const int grp = tid / p, k = tid - grp * p;
+  double2 A = make_double2(0.0, 0.0), B = A, C = A;
+  const int i0 = pt0[b], i1 = pt1[b];
+  const int nbat = (i1 - i0 + 31) / 32;  // batches of equal size
+  for (int bt = 0; bt < nbat; ++bt) {
+    const int base = i0 + bt * (i1 - i0) / nbat, cnt = i0 + (bt + 1) * (i1 - i0) / nbat - base;
     __syncthreads();
     if (tid < cnt) {
-      int i = base + tid;
-      double2 zi = zs[i];
-      c_t<T> w = cmk<T>((T)((zi.x - c.x) / r), (T)((zi.y - c.y) / r));
-      c_t<T> ah = cscale<T>(qa[i], rinv);
+      const int i = base + tid;
+      const double2 zi = zs[i];
+      const double2 c = box_center(bkey[b], x0, y0, W * pow2d(-lev));
+      const double2 w = make_double2((zi.x - c.x) * rinv, (zi.y - c.y) * rinv);
+      const double2 ah = cscale<double>(qa[i], rinv);
       sc[tid] = ah;
       if (E == 2) {
-        sc[32 + tid] = cscale<T>(qb[i], rinv);
-        sc[64 + tid] = cmul<T>(cconj<T>(w), ah);
+        sc[32 + tid] = cscale<double>(qb[i], rinv);
+        sc[64 + tid] = cmul<double>(cconj<double>(w), ah);
       }
-      c_t<T> pwr = cmk<T>(1, 0);
-      c_t<T>* row = pw + tid * ps;
-      for (int j = 0; j < p; ++j) {
-        row[j] = pwr;
-        pwr = cmul<T>(pwr, w);
-      }
+      pw[tid * ps] = make_double2(1.0, 0.0);
+      pw[tid * ps + 1] = w;
     }
     __syncthreads();
-    if (tid < p) {
-      for (int s = 0; s < cnt; ++s) {
-        c_t<T> v = pw[s * ps + tid];
-        cfma<T>(A, sc[s], v);
+    for (int len = 1; len + 1 < p; len <<= 1) {
+      const int span = min(len, p - 1 - len);
+      for (int pr = tid; pr < cnt * span; pr += nt) {
+        const int j = pr / cnt, sp = pr - j * cnt;  // lanes over the points first
+        double2* row = pw + sp * ps + len + 1 + j;
+        *row = cmul<double>(*(row - len), pw[sp * ps + len]);
+      }
+      __syncthreads();
+    }
+    if (grp < P2M_NG) {
+      for (int s = grp; s < cnt; s += P2M_NG) {
+        const double2 v = pw[s * ps + k];
+        cfma<double>(A, sc[s], v);
         if (E == 2) {
-          cfma<T>(B, sc[32 + s], v);
-          cfma<T>(C, sc[64 + s], v);
+          if (BREAL) crfma<double>(B, sc[32 + s].x, v);
+          else cfma<double>(B, sc[32 + s], v);
+          cfma<double>(C, sc[64 + s], v);
         }
       }
     }
   }
   __syncthreads();
-  if (tid < p) pw[tid] = C;
-  __syncthreads();
-  if (tid < p) {
-    c_t<T>* mp = mpole + (size_t)b * E * p;
-    mp[tid] = cmk<T>(-A.x, -A.y);
+  double2* red = sm2d;  // [E == 2 ? 3 : 1][P2M_NG][p]
+  if (grp < P2M_NG) {
+    red[grp * p + k] = A;
     if (E == 2) {
-      c_t<T> v = B;
-      if (tid >= 1) crfma<T>(v, (T)tid, pw[tid - 1]);
-      mp[p + tid] = cmk<T>(-v.x, -v.y);
+      red[(P2M_NG + grp) * p + k] = B;
+      red[(2 * P2M_NG + grp) * p + k] = C;
     }
+  }
+  __syncthreads();
+  auto total = [&](int which, int kk) {
+    const double2* q = red + which * P2M_NG * p + kk;
+    return cadd<double>(cadd<double>(q[0], q[p]), cadd<double>(q[2 * p], q[3 * p]));
+  };
+  for (int o = tid; o < E * p; o += nt) {
+    double2 v;
+    if (o < p) {
+      v = total(0, o);
+    } else {
+      const int kk = o - p;
+      v = total(1, kk);
+      if (kk >= 1) crfma<double>(v, (double)kk, total(2, kk - 1));
+    }
+    mpole[(size_t)b * E * p + o] = make_double2(-v.x, -v.y);
   }
 }
 
+// the sum of the 4 lanes of an output (lanes 4o .. 4o+3) in a fixed order, in every lane
+__device__ __forceinline__ double2 quad_sum(double2 v) {
+#pragma unroll
+  for (int o = 1; o <= 2; o <<= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  return v;
+}
+
 // ---------------------------------------------------------------------------------
-// M2M: one block per parent, one thread per output coefficient (e, n). With e the child
+// M2M into the boxes of one level. With e the child
 // centre offset in child units and a_k = e^-k M_k:  M'_n = (e/2)^n sum_{k<=n} C(n-1,k-1) a_k.
 // psi is first moved to the parent centre: psi_k += conj(e) (k-1) phi_{k-1}.
+//
+// The four children's offsets are e_0 = (1 + i)/2 times 1, i, -1, -i (rot), so that with
+// b_k = e_0^-k M_k of each child and c_k^r = sum over the children of i^(rot r) b_k,
+//   M'_n = (e_0/2)^n sum_k C(n-1,k-1) c_k^((n-k) mod 4):
+// one binomial sum for all children, the kernel's bulk, where a sum per child took up to
+// four times the FP64 work. Four lanes per output take every 4th term each (one r per lane).
+// An SM takes 16 cycles per FP64 warp instruction, so that one parent's outputs alone keep
+// it busy for microseconds; on a level of few boxes they are dealt to nsplit blocks (each
+// forms c anew).
+// Measured (E = 2): 25.2 -> 11.9 us a level of 64 x 512 (beside the near field), 21.6 -> 8.4
+// us at 4,096 nodes.
 // ---------------------------------------------------------------------------------
-template <typename T, int E>
-__global__ void k_m2m(int offp, const unsigned long long* __restrict__ bkey,
-                      const int* __restrict__ child0, const int* __restrict__ nchild, int p,
-                      const T* __restrict__ binom, int ldb, const c_t<T>* __restrict__ epow2,
-                      const c_t<T>* __restrict__ einv, c_t<T>* __restrict__ mpole) {
-  extern __shared__ unsigned char smem_raw[];
-  c_t<T>* a = reinterpret_cast<c_t<T>*>(smem_raw);
-  const int P = offp + blockIdx.x, tid = threadIdx.x, ld = p + 2, nout = E * p;
-  const int e = tid / p, nn = tid - e * p;
-  const bool active = tid < nout;
-  c_t<T> acc = cmk<T>(0, 0);
-  int c0 = child0[P], nc = nchild[P];
+__device__ __forceinline__ int quad_rot(int q) { return q == 3 ? 0 : q == 2 ? 1 : q == 0 ? 2 : 3; }
+
+template <int E>
+__global__ void k_m2m64(int offp, int nsplit, const unsigned long long* __restrict__ bkey,
+                        const int* __restrict__ child0, const int* __restrict__ nchild, int p,
+                        const double* __restrict__ binom, int ldb, const double2* __restrict__ epow2,
+                        const double2* __restrict__ einv, double2* __restrict__ mpole) {
+  extern __shared__ double2 sm2d[];
+  double2* cr = sm2d;  // [r][E*p]
+  const int P = offp + blockIdx.x / nsplit, sp = blockIdx.x % nsplit;
+  const int tid = threadIdx.x, ld = p + 2, nout = E * p;
+  const int c0 = child0[P], nc = nchild[P];
   if (nc == 0) return;  // a leaf: its multipole comes from its points
-  for (int ci = 0; ci < nc; ++ci) {
-    int c = c0 + ci;
-    int q = quadrant(bkey[c]);
-    c_t<T> ec = cscale<T>(epow2[q * ld + 1], (T)2);
-    const c_t<T>* mc = mpole + (size_t)c * E * p;
-    __syncthreads();
-    for (int idx = tid; idx < nout; idx += blockDim.x) {
-      int e2 = idx / p, kk = idx - e2 * p, k = kk + 1;
-      c_t<T> v = mc[idx];
-      if (e2 == 1 && k >= 2) cfma<T>(v, cscale<T>(cconj<T>(ec), (T)(k - 1)), mc[kk - 1]);
-      a[idx] = cmul<T>(v, einv[q * ld + k]);
-    }
-    __syncthreads();
-    if (active) {
-      int n = nn + 1;
-      const T* brow = binom + (size_t)(n - 1) * ldb;
-      const c_t<T>* ae = a + e * p;
-      c_t<T> s0 = cmk<T>(0, 0), s1 = cmk<T>(0, 0);
-      int k = 0;
-      for (; k + 1 < n; k += 2) {
-        crfma<T>(s0, brow[k], ae[k]);
-        crfma<T>(s1, brow[k + 1], ae[k + 1]);
+  const double2* e0inv = einv + 3 * ld;
+  const double2* e0pow = epow2 + 3 * ld;
+  for (int o = tid; o < nout; o += blockDim.x) {
+    const int e2 = o / p, kk = o - e2 * p, k = kk + 1;
+    double2 c[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) c[r] = make_double2(0.0, 0.0);
+    const double2 sc = e0inv[k];
+    for (int ci = 0; ci < nc; ++ci) {
+      const double2* mc = mpole + (size_t)(c0 + ci) * nout;
+      const int q = quadrant(bkey[c0 + ci]), rot = quad_rot(q);
+      double2 v = mc[o];
+      if (e2 == 1 && k >= 2) {
+        const double2 ec = epow2[q * ld + 1];  // e / 2
+        cfma<double>(v, cscale<double>(cconj<double>(ec), 2.0 * (k - 1)), mc[kk - 1]);
       }
-      if (k < n) crfma<T>(s0, brow[k], ae[k]);
-      cfma<T>(acc, epow2[q * ld + n], cadd<T>(s0, s1));
+      const double2 b = cmul<double>(v, sc);
+      c[0] = cadd<double>(c[0], b);
+      if (rot == 0) {
+#pragma unroll
+        for (int r = 1; r < 4; ++r) c[r] = cadd<double>(c[r], b);
+      } else if (rot == 2) {
+        c[1] = csub<double>(c[1], b);
+        c[2] = cadd<double>(c[2], b);
+        c[3] = csub<double>(c[3], b);
+      } else {
+        const double2 ib = rot == 1 ? make_double2(-b.y, b.x) : make_double2(b.y, -b.x);
+        c[1] = cadd<double>(c[1], ib);
+        c[2] = csub<double>(c[2], b);
+        c[3] = csub<double>(c[3], ib);
+      }
     }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) cr[r * nout + o] = c[r];
   }
-  if (active) mpole[(size_t)P * E * p + tid] = acc;
+  __syncthreads();
+  // a warp's 8 outputs: every nsplit-th group of 8
+  const int o = ((tid >> 5) * nsplit + sp) * 8 + ((tid >> 2) & 7), part = tid & 3;
+  const bool act = o < nout;
+  const int oo = act ? o : 0;
+  const int e = oo / p, n = oo - e * p + 1;
+  double2 v = make_double2(0.0, 0.0);
+  if (act) {
+    const double* brow = binom + (size_t)(n - 1) * ldb;
+    const double2* src = cr + ((n - 1 - part) & 3) * nout + e * p;
+#pragma unroll 4
+    for (int k = part; k < n; k += 4) crfma<double>(v, brow[k], src[k]);
+  }
+  v = quad_sum(v);
+  if (act && part == 0) mpole[(size_t)P * nout + o] = cmul<double>(e0pow[n], v);
 }
 
 // ---------------------------------------------------------------------------------
-// L2L: one block per child box, one thread per output (e, j). With e the child offset
-// in child units and a_m = (e/2)^m L_m:  L'_j += e^-j sum_{m>=j} C(m, j) a_m.
-// psi is first moved to the child centre: psi_m += conj(e/2) (m+1) phi_{m+1}.
+// L2L from the boxes of one level to their children. With e the child offset
+// in child units and a_m = (e/2)^m L_m:  L'_j += e^-j sum_{m>=j} C(m, j) a_m,
+// and psi is moved to the child centre: psi'_j += conj(e) (j+1) phi'_{j+1} (of the shifted
+// coefficients; shifting and moving polynomials commute).
+//
+// For the children e_0 i^rot (see the M2M), with a_m = (e_0/2)^m L_m and
+// S_r = sum_{m = j+r mod 4} C(m, j) a_m:  L'_j = e_0^-j sum_r i^(rot r) S_r, so that the
+// four lanes of an output form the S_r of all children at once and then one child each.
+// On levels of few boxes the orders are dealt to nsplit blocks in ranges of about equal
+// work.
 // ---------------------------------------------------------------------------------
+template <int E>
+__global__ void k_l2l64(int offp, int nsplit, const unsigned long long* __restrict__ bkey,
+                        const int* __restrict__ child0, const int* __restrict__ nchild, int p,
+                        const double* __restrict__ binom, int ldb, const double2* __restrict__ epow2,
+                        const double2* __restrict__ einv, double2* __restrict__ local) {
+  extern __shared__ double2 sm2d[];
+  double2* a = sm2d;                    // [E][p + 1]
+  double2* sph = a + E * (p + 1);       // [rot][p + 1]: the children's phi', for psi
+  __shared__ int s_child[4];
+  const int ldl = p + 1, ld = p + 2, nout = E * ldl, tid = threadIdx.x;
+  const int P = offp + blockIdx.x / nsplit, sp = blockIdx.x % nsplit;
+  const int c0 = child0[P], nc = nchild[P];
+  if (nc == 0) return;
+  // orders [ja, jb): the work of order j is p + 1 - j terms
+  auto cut = [&](int i) { return i >= nsplit ? ldl : (int)(ldl * (1.f - sqrtf(1.f - (float)i / nsplit))); };
+  const int ja = cut(sp), jb = cut(sp + 1), nj = jb - ja;
+  if (tid < 4) s_child[tid] = -1;
+  __syncthreads();
+  if (tid < nc) s_child[quad_rot(quadrant(bkey[c0 + tid]))] = c0 + tid;
+  const double2* e0inv = einv + 3 * ld;
+  const double2* e0pow = epow2 + 3 * ld;
+  const double2* lp = local + (size_t)P * nout;
+  for (int idx = tid; idx < nout; idx += blockDim.x) {
+    const int m = idx % ldl;
+    if (m >= ja) a[idx] = cmul<double>(lp[idx], e0pow[m]);
+  }
+  __syncthreads();
+  // outputs: phi of the orders [ja, min(jb + 1, p + 1)) (psi of the last one needs the next
+  // phi), then psi of [ja, jb)
+  const int nphi = E == 2 ? min(nj + 1, ldl - ja) : nj;
+  const int o = tid >> 2, part = tid & 3;
+  const bool psi = o >= nphi, act = o < nphi + (E == 2 ? nj : 0);
+  const int j = !act ? p : ja + (psi ? o - nphi : o);
+  const double2* ae = a + (psi && act ? ldl : 0);
+  double2 s = make_double2(0.0, 0.0);
+  if (act) {
+#pragma unroll 4
+    for (int m = j + part; m <= p; m += 4) crfma<double>(s, binom[(size_t)m * ldb + j], ae[m]);
+  }
+  // child `part` (rot): sum_r i^(rot r) S_r, S_r in the quad's lane r
+  const int q0 = (threadIdx.x & 31) & ~3;
+  double2 v = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const double x = __shfl_sync(0xffffffffu, s.x, q0 + r), y = __shfl_sync(0xffffffffu, s.y, q0 + r);
+    const int k = (part * r) & 3;  // times i^k
+    const double tx = k & 1 ? y : x, ty = k & 1 ? x : y;
+    v.x += k == 1 || k == 2 ? -tx : tx;
+    v.y += k >= 2 ? -ty : ty;
+  }
+  v = cmul<double>(e0inv[j], v);
+  if (E == 2) {
+    if (act && !psi) sph[part * ldl + j] = v;
+    __syncthreads();
+    if (act && psi && j < p) {
+      // conj(e_0 i^rot) (j + 1) phi'
+      const double f = 0.5 * (j + 1);
+      const double2 ec = make_double2(part == 0 || part == 3 ? f : -f, part <= 1 ? -f : f);
+      cfma<double>(v, ec, sph[part * ldl + j + 1]);
+    }
+  }
+  const int c = s_child[part];
+  if (act && c >= 0 && (psi || j < jb)) {
+    double2* lc = local + (size_t)c * nout + (psi ? ldl : 0) + j;
+    *lc = cadd<double>(*lc, v);
+  }
+}
+
+// FP32 L2L: one block per child box, one thread per output (e, j), psi moved before the
+// shift: psi_m += conj(e/2) (m+1) phi_{m+1}.
 template <typename T, int E>
 __global__ void k_l2l(int offc, const unsigned long long* __restrict__ bkey,
                       const int* __restrict__ parent, int p, const T* __restrict__ binom,
@@ -703,8 +857,7 @@ __global__ void __launch_bounds__(128) k_m2l_df(int first, const int* __restrict
 }
 
 // ---------------------------------------------------------------------------------
-// Upward and downward passes of the double-float pipeline: the P2M, M2M and L2L of the
-// FP64 kernels above with double-float operands and compensated sums.
+// The P2M of the double-float pipeline (its M2M and L2L are the FP64 kernels above).
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ cdf cdf_conj(cdf a) { return cdf{a.x, dfl_neg(a.y)}; }
 __device__ __forceinline__ cdf cdf_scale(cdf a, float f) { return cdf{dfl_mul_f(a.x, f), dfl_mul_f(a.y, f)}; }
@@ -1061,6 +1214,13 @@ __global__ void k_m2m_f32(int offp, const unsigned long long* __restrict__ bkey,
 // sources (and the terms of the local expansion), and their partial sums are added
 // with two shuffles in a fixed order.
 // ---------------------------------------------------------------------------------
+// a u + c
+template <typename T>
+__device__ __forceinline__ c_t<T> chorner(c_t<T> a, c_t<T> u, c_t<T> c) {
+  cfma<T>(c, a, u);
+  return c;
+}
+
 // Terms m0 <= m < m1 of the local expansions at u.
 template <typename T, int E>
 __device__ __forceinline__ void l2p_range(const c_t<T>* lb, int p, int m0, int m1, c_t<T> u, T s, T& gx,
@@ -1068,19 +1228,16 @@ __device__ __forceinline__ void l2p_range(const c_t<T>* lb, int p, int m0, int m
   const int ldl = p + 1;
   if (m0 >= m1) return;
   c_t<T> ph = lb[m1 - 1], dph = cmk<T>(0, 0);
+  c_t<T> ps = E == 2 ? lb[ldl + m1 - 1] : cmk<T>(0, 0);
   for (int m = m1 - 2; m >= m0; --m) {
-    dph = cadd<T>(cmul<T>(dph, u), ph);
-    ph = cadd<T>(cmul<T>(ph, u), lb[m]);
-  }
-  c_t<T> ps = cmk<T>(0, 0);
-  if (E == 2) {
-    ps = lb[ldl + m1 - 1];
-    for (int m = m1 - 2; m >= m0; --m) ps = cadd<T>(cmul<T>(ps, u), lb[ldl + m]);
+    if (E == 2) dph = chorner<T>(dph, u, ph);
+    ph = chorner<T>(ph, u, lb[m]);
+    if (E == 2) ps = chorner<T>(ps, u, lb[ldl + m]);
   }
   if (m0 > 0) {
     c_t<T> um1 = cpow_int<T>(u, m0 - 1);  // u^(m0-1)
     // d/du (u^m0 H) = u^(m0-1) (u H' + m0 H)
-    dph = cmul<T>(um1, cadd<T>(cmul<T>(u, dph), cscale<T>(ph, (T)m0)));
+    if (E == 2) dph = cmul<T>(um1, cadd<T>(cmul<T>(u, dph), cscale<T>(ph, (T)m0)));
     c_t<T> um = cmul<T>(um1, u);
     ph = cmul<T>(um, ph);
     if (E == 2) ps = cmul<T>(um, ps);
@@ -1115,14 +1272,14 @@ __device__ __forceinline__ void m2p_eval(const c_t<T>* M, int p, c_t<T> u, T s, 
   c_t<T> a = M[p - 1];
   c_t<T> da = cscale<T>(M[p - 1], (T)p);
   for (int k = p - 1; k >= 1; --k) {
-    a = cadd<T>(cmul<T>(a, v), M[k - 1]);
-    if (E == 2) da = cadd<T>(cmul<T>(da, v), cscale<T>(M[k - 1], (T)k));
+    a = chorner<T>(a, v, M[k - 1]);
+    if (E == 2) da = chorner<T>(da, v, cscale<T>(M[k - 1], (T)k));
   }
   const c_t<T> ph = cmul<T>(a, v);  // sum M_k v^k
   if (E == 2) {
     const c_t<T> dph = cmul<T>(da, cmul<T>(v, v));  // sum k M_k v^(k+1) = -phi_u
     c_t<T> b = M[2 * p - 1];
-    for (int k = p - 1; k >= 1; --k) b = cadd<T>(cmul<T>(b, v), M[p + k - 1]);
+    for (int k = p - 1; k >= 1; --k) b = chorner<T>(b, v, M[p + k - 1]);
     const c_t<T> ps = cmul<T>(b, v);
     const c_t<T> t = cmulc<T>(u, dph);  // -u conj(phi_u)
     gx += ph.x + s * (ps.x - t.x);
@@ -1140,88 +1297,107 @@ __device__ __forceinline__ void m2p_eval(const c_t<T>* M, int p, c_t<T> u, T s, 
 // targets (87 % of the lanes busy at T = 28, where 32-target tiles with fixed slices have
 // 77 % on average). Sources are staged through shared memory in slabs; a warp reads two or
 // three of them at once (broadcasts). The slices are added in a fixed order; the sums go
-// to nearbuf (sorted order), so that the near field runs beside the expansion passes.
+// to nearbuf (sorted order), so that the near field runs beside the expansion passes. It
+// does so with NEAR64_CTAS blocks per SM that draw tiles from a counter (zeroed by the
+// charges' kernel): eight warps keep the FP64 pipe busy, while as many blocks as fit left
+// the expansion passes, which share the pipe warp by warp, a seventh of it and the
+// fixed-point M2L no shared memory.
 // Measured: 3.25 ms for the 110.6 M pairs of 1,048,576 nodes (82 % of the FP64 issue rate
 // at 14 instructions a pair), 149 us for the 4.0 M of 64 x 512; with a warp per 8 targets
 // reading every source from global memory and the longer pair, near and far field
 // together took 9.76 ms and 392 us (now, with the far field below, 5.7 ms and 233 us).
 #define NEAR64_SLAB 128
+#define NEAR64_CTAS 4
 template <int K>
-__global__ void __launch_bounds__(128) k_near64(const int4* __restrict__ tiles, const int* __restrict__ pt0,
+__global__ void __launch_bounds__(128) k_near64(int ntile, int* __restrict__ next,
+                                                const int4* __restrict__ tiles, const int* __restrict__ pt0,
                                                 const int* __restrict__ pt1, const int* __restrict__ ustart,
                                                 const int* __restrict__ ulist, const double2* __restrict__ zs,
                                                 const double2* __restrict__ q, int plus,
                                                 double2* __restrict__ nearbuf) {
   constexpr bool ST = K == NEAR_V || K == NEAR_VC;
   __shared__ double2 sz[NEAR64_SLAB], sa[NEAR64_SLAB], sc[ST ? NEAR64_SLAB : 1], sred[128];
-  __shared__ int sidx[NEAR64_SLAB], spre[33], sj0[32];
-  const int4 tl = tiles[blockIdx.x];
-  const int tid = threadIdx.x, T = tl.z - tl.y, nsl = 128 / T;
-  const int sl = tid / T, i = tl.y + tid - sl * T;
-  const double2 zi = zs[i];
-  double gx = 0.0, gy = 0.0;
-  const int ub = ustart[tl.x], ue = ustart[tl.x + 1];
-  for (int cb = ub; cb < ue; cb += 32) {
-    const int nc = min(32, ue - cb);
-    if (cb > ub) __syncthreads();  // the previous boxes' slabs are consumed
-    if (tid < 32) {
-      int c = 0, j0 = 0;
-      if (tid < nc) {
-        const int sbx = ulist[cb + tid];
-        j0 = pt0[sbx];
-        c = pt1[sbx] - j0;
-      }
-      int x = c;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (tid >= o) x += y;
-      }
-      sj0[tid] = j0;
-      spre[tid + 1] = x;
-      if (tid == 0) spre[0] = 0;
-    }
+  __shared__ int sidx[NEAR64_SLAB], spre[33], sj0[32], s_tile;
+  const int tid = threadIdx.x;
+  for (;;) {
+    if (tid == 0) s_tile = atomicAdd(next, 1);
     __syncthreads();
-    const int total = spre[nc];
-    for (int base = 0; base < total; base += NEAR64_SLAB) {
-      const int ns = min(NEAR64_SLAB, total - base);
-      if (base > 0) __syncthreads();
-      if (tid < ns) {
-        const int gs = base + tid;
-        int lo = 0, hi = nc;  // the box k with spre[k] <= gs < spre[k + 1]
-        while (hi - lo > 1) {
-          const int mid = (lo + hi) >> 1;
-          if (spre[mid] <= gs) lo = mid;
-          else hi = mid;
+    const int tile = s_tile;
+    if (tile >= ntile) return;
+    const int4 tl = tiles[tile];
+    const int T = tl.z - tl.y, nsl = 128 / T;
+    const int sl = tid / T, i = tl.y + tid - sl * T;
+    const double2 zi = zs[i];
+    double gx = 0.0, gy = 0.0;
+    const int ub = ustart[tl.x], ue = ustart[tl.x + 1];
+    for (int cb = ub; cb < ue; cb += 32) {
+      const int nc = min(32, ue - cb);
+      if (cb > ub) __syncthreads();  // the previous boxes' slabs are consumed
+      if (tid < 32) {
+        int c = 0, j0 = 0;
+        if (tid < nc) {
+          const int sbx = ulist[cb + tid];
+          j0 = pt0[sbx];
+          c = pt1[sbx] - j0;
         }
-        const int j = sj0[lo] + gs - spre[lo];
-        sidx[tid] = j;
-        sz[tid] = zs[j];
-        if (ST) {
-          sa[tid] = q[2 * (size_t)j];
-          sc[tid] = q[2 * (size_t)j + 1];
-        } else {
-          sa[tid] = q[j];
+        int x = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, x, o);
+          if (tid >= o) x += y;
         }
+        sj0[tid] = j0;
+        spre[tid + 1] = x;
+        if (tid == 0) spre[0] = 0;
       }
       __syncthreads();
-      if (sl < nsl) {
+      const int total = spre[nc];
+      for (int base = 0; base < total; base += NEAR64_SLAB) {
+        const int ns = min(NEAR64_SLAB, total - base);
+        if (base > 0) __syncthreads();
+        if (tid < ns) {
+          const int gs = base + tid;
+          int lo = 0, hi = nc;  // the box k with spre[k] <= gs < spre[k + 1]
+          while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (spre[mid] <= gs) lo = mid;
+            else hi = mid;
+          }
+          const int j = sj0[lo] + gs - spre[lo];
+          sidx[tid] = j;
+          sz[tid] = zs[j];
+          if (ST) {
+            sa[tid] = q[2 * (size_t)j];
+            sc[tid] = q[2 * (size_t)j + 1];
+          } else {
+            sa[tid] = q[j];
+          }
+        }
+        __syncthreads();
+        if (sl < nsl) {
 #pragma unroll 2
-        for (int jj = sl; jj < ns; jj += nsl) {
-          if (sidx[jj] == i) continue;
-          near_pair64<K>(sz[jj], sa[jj], ST ? sc[jj] : make_double2(0.0, 0.0), zi, gx, gy);
+          for (int jj = sl; jj < ns; jj += nsl) {
+            if (sidx[jj] == i) continue;
+            near_pair64<K>(sz[jj], sa[jj], ST ? sc[jj] : make_double2(0.0, 0.0), zi, gx, gy);
+          }
         }
       }
     }
-  }
-  sred[tid] = make_double2(gx, gy);
-  __syncthreads();
-  if (tid < T) {
-    double2 v = sred[tid];
-    for (int k = 1; k < nsl; ++k) v = cadd<double>(v, sred[k * T + tid]);
-    nearbuf[i] = ST ? near_turn<double>(v.x, v.y, plus) : v;
+    sred[tid] = make_double2(gx, gy);
+    __syncthreads();
+    if (tid < T) {
+      double2 v = sred[tid];
+      for (int k = 1; k < nsl; ++k) v = cadd<double>(v, sred[k * T + tid]);
+      nearbuf[i] = ST ? near_turn<double>(v.x, v.y, plus) : v;
+    }
   }
 }
+
+// Points from which the FP64 far field takes one lane per target: with fewer, a lane's whole
+// Horner chain is longer than the FP64 pipe is busy. Measured, Horner steps
+// as four FMAs and no divisions included: 83.5 -> 38.8 us at 64 x 512 and 2.48 -> 0.97 ms at
+// 1,024 x 1,024 with one lane, 15.3 -> 12.3 us at 4,096 nodes with four.
+constexpr int FAR64_ONE = 12288;
 
 // FP64 far field: L2P of the leaf's local expansions and the W list, LPT lanes per target
 // (LPT = 4: a warp per group of 8 targets, each lane a quarter of the terms; LPT = 1: a
@@ -1234,7 +1410,7 @@ __global__ void __launch_bounds__(128) k_far64(int n, const int* __restrict__ lf
                                                const unsigned char* __restrict__ blev,
                                                const int* __restrict__ wstart, const int* __restrict__ wlist,
                                                const int* __restrict__ perm, const double2* __restrict__ zs,
-                                               double x0, double y0, double W, int p, double s,
+                                               double x0, double y0, double W, double winv, int p, double s,
                                                const double2* __restrict__ local,
                                                const double2* __restrict__ mpole,
                                                const double2* __restrict__ nearbuf, double2* __restrict__ out,
@@ -1247,18 +1423,20 @@ __global__ void __launch_bounds__(128) k_far64(int n, const int* __restrict__ lf
     const int leaf = lscan[i] + lflag[i] - 1, b = leaves[leaf];  // leaf heads up to point i
     const double2 zi = zs[i];
     if (blev[b] >= 2) {
-      const double r = ldexp(W, -(int)blev[b]);
-      const double2 c = box_center(bkey[b], x0, y0, r);
-      const double2 u = make_double2((zi.x - c.x) / r, (zi.y - c.y) / r);
+      const int lev = blev[b];
+      const double2 c = box_center(bkey[b], x0, y0, W * pow2d(-lev));
+      const double rinv = winv * pow2d(lev);
+      const double2 u = make_double2((zi.x - c.x) * rinv, (zi.y - c.y) * rinv);
       const double2* lb = local + (size_t)b * E * (p + 1);
       if (LPT == 1) l2p_range<double, E>(lb, p, 0, p + 1, u, s, gx, gy);
       else l2p_part<double, E>(lb, p, sl, u, s, gx, gy);
     }
     for (int jw = wstart[leaf] + sl; jw < wstart[leaf + 1]; jw += LPT) {
       const int w = wlist[jw];
-      const double rw = ldexp(W, -(int)blev[w]);
-      const double2 cw = box_center(bkey[w], x0, y0, rw);
-      m2p_eval<double, E>(mpole + (size_t)w * E * p, p, make_double2((zi.x - cw.x) / rw, (zi.y - cw.y) / rw),
+      const int lev = blev[w];
+      const double2 cw = box_center(bkey[w], x0, y0, W * pow2d(-lev));
+      const double rinv = winv * pow2d(lev);
+      m2p_eval<double, E>(mpole + (size_t)w * E * p, p, make_double2((zi.x - cw.x) * rinv, (zi.y - cw.y) * rinv),
                           s, gx, gy);
     }
   }
@@ -1980,9 +2158,6 @@ __global__ void __launch_bounds__(IMG_TILE) k_img_near(int off, int nb, int lev,
 
 inline int nblk(long long n, int bs) { return (int)((n + bs - 1) / bs); }
 inline int round32(int n) { return (n + 31) & ~31; }
-#ifndef FAR64_LPT
-#define FAR64_LPT 4
-#endif
 template <typename T>
 int tables_build(EbTables& tb, int p, double tol) {
   tb.p = p;
@@ -2088,6 +2263,28 @@ struct ProfScope {
   }
 };
 
+// Blocks per box of the FP64 M2M / L2L of a level of nb boxes.
+int level_split(const eb_ctx* ctx, int nb) { return nb <= ctx->nsm ? 4 : nb <= 3 * ctx->nsm ? 2 : 1; }
+
+// M2M into the boxes of level l, L2L out of them.
+template <int E>
+void launch_m2m64(eb_ctx* ctx, EbTree& t, EbTables& tb, int l, double2* mpole, cudaStream_t st) {
+  const int p = tb.p, nb = t.lev_off[l + 1] - t.lev_off[l], ns = level_split(ctx, nb);
+  const int groups = ((E * p + 7) / 8 + ns - 1) / ns;
+  k_m2m64<E><<<nb * ns, 32 * groups, sizeof(double2) * 4 * E * p, st>>>(
+      t.lev_off[l], ns, t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
+      tb.binom.as<double>(), 2 * p + 2, tb.epow.as<double2>(), tb.einv.as<double2>(), mpole);
+}
+template <int E>
+void launch_l2l64(eb_ctx* ctx, EbTree& t, EbTables& tb, int l, double2* local, cudaStream_t st) {
+  const int p = tb.p, nb = t.lev_off[l + 1] - t.lev_off[l], ns = level_split(ctx, nb);
+  // the widest range of orders is the last one
+  const int ldl = p + 1, nj = ldl - (ns == 1 ? 0 : (int)(ldl * (1.f - std::sqrt(1.f / ns)))) + 1;
+  k_l2l64<E><<<nb * ns, round32(4 * (E * nj + E - 1)), sizeof(double2) * (E + 4) * (p + 1), st>>>(
+      t.lev_off[l], ns, t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
+      tb.binom.as<double>(), 2 * p + 2, tb.epow.as<double2>(), tb.einv.as<double2>(), local);
+}
+
 constexpr int FX_DF = 16384;
 
 // Boxes of the levels 2, 3, .. of at most 384 boxes: their V lists are the long ones.
@@ -2119,10 +2316,9 @@ int fmm_expansions_df(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
   }
   for (int l = L - 1; l >= 2; --l) {
     int nb = t.lev_off[l + 1] - t.lev_off[l];
-    size_t sm = sizeof(float4) * 4 * E * p;
-    k_m2m_df<E><<<nb, round32(4 * E * p), sm, st>>>(t.lev_off[l], t.bkey.as<unsigned long long>(), t.child0.as<int>(),
-                                                t.nchild.as<int>(), p, tb.binom_df.as<float2>(), ldb,
-                                                tb.epow_df.as<float4>(), tb.einv_df.as<float4>(), mp);
+    k_m2m_df<E><<<nb, round32(4 * E * p), sizeof(float4) * 4 * E * p, st>>>(
+        t.lev_off[l], t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
+        tb.binom_df.as<float2>(), ldb, tb.epow_df.as<float4>(), tb.einv_df.as<float4>(), mp);
     eb_count_launch(ctx);
   }
   {
@@ -2163,17 +2359,18 @@ int fmm_expansions_df(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
   }
   for (int l = 3; l <= L; ++l) {
     int nb = t.lev_off[l + 1] - t.lev_off[l];
-    size_t sm = sizeof(float4) * E * (p + 1);
-    k_l2l_df<E><<<nb, round32(4 * E * (p + 1)), sm, st>>>(t.lev_off[l], t.bkey.as<unsigned long long>(),
-                                                     t.parent.as<int>(), p, tb.binom_df.as<float2>(), ldb,
-                                                     tb.epow_df.as<float4>(), tb.einv_df.as<float4>(), lo);
+    k_l2l_df<E><<<nb, round32(4 * E * (p + 1)), sizeof(float4) * E * (p + 1), st>>>(
+          t.lev_off[l], t.bkey.as<unsigned long long>(), t.parent.as<int>(), p, tb.binom_df.as<float2>(), ldb,
+          tb.epow_df.as<float4>(), tb.einv_df.as<float4>(), lo);
     eb_count_launch(ctx);
   }
   return EB_OK;
 }
 
+// breal: the charges b are real (see the charges).
 template <typename T, int E>
-int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
+int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w, bool breal,
+                   const std::function<int()>& after_p2m) {
   cudaStream_t st = eb_stream(ctx);
   const int p = tb.p, L = t.L;
   const int ldb = 2 * p + 2;
@@ -2210,20 +2407,22 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
       eb_count_launch(ctx);
     }
   } else {
-    size_t sm = sizeof(c_t<T>) * (32 * (size_t)(p + 1) + 96);
-    k_p2m<T, E><<<t.nleaf, 64, sm, st>>>(t.leaves.as<int>(), t.bkey.as<unsigned long long>(),
-                                          t.blev.as<unsigned char>(), t.pt0.as<int>(),
-                                          t.pt1.as<int>(), t.zs.as<double2>(), w.qa.as<c_t<T>>(),
-                                          w.qb.as<c_t<T>>(), t.x0, t.y0, t.W, p,
-                                          w.mpole.as<c_t<T>>());
+    const size_t sm = sizeof(double2) * std::max(32 * (size_t)(p + 1) + 96, (size_t)(E == 2 ? 3 : 1) * P2M_NG * p);
+    auto go = [&](auto kern) -> int {
+      if (sm > 48 * 1024)
+        EB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+      kern<<<t.nleaf, round32(P2M_NG * p), sm, st>>>(t.leaves.as<int>(), t.bkey.as<unsigned long long>(),
+                                                     t.blev.as<unsigned char>(), t.pt0.as<int>(), t.pt1.as<int>(),
+                                                     t.zs.as<double2>(), w.qa.as<double2>(), w.qb.as<double2>(), t.x0,
+                                                     t.y0, t.W, 1.0 / t.W, p, w.mpole.as<double2>());
+      return EB_OK;
+    };
+    if (E == 2 && breal) EB_TRY(go(k_p2m64<E, true>));
+    else EB_TRY(go(k_p2m64<E, false>));
     eb_count_launch(ctx);
+    if (after_p2m) EB_TRY(after_p2m());
     for (int l = L - 1; l >= 2; --l) {
-      int nb = t.lev_off[l + 1] - t.lev_off[l];
-      size_t sm2 = sizeof(c_t<T>) * E * p;
-      k_m2m<T, E><<<nb, round32(E * p), sm2, st>>>(t.lev_off[l], t.bkey.as<unsigned long long>(),
-                                                   t.child0.as<int>(), t.nchild.as<int>(), p,
-                                                   tb.binom.as<T>(), ldb, tb.epow.as<c_t<T>>(),
-                                                   tb.einv.as<c_t<T>>(), w.mpole.as<c_t<T>>());
+      launch_m2m64<E>(ctx, t, tb, l, w.mpole.as<double2>(), st);
       eb_count_launch(ctx);
     }
   }
@@ -2288,11 +2487,12 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
     const int lend = sizeof(T) == 8 ? L : t.lend;
     for (int l = 3; l <= lend; ++l) {
       int nb = t.lev_off[l + 1] - t.lev_off[l];
-      size_t sm = sizeof(c_t<T>) * E * (p + 1);
-      k_l2l<T, E><<<nb, round32(E * (p + 1)), sm, st>>>(t.lev_off[l], t.bkey.as<unsigned long long>(),
-                                                       t.parent.as<int>(), p, tb.binom.as<T>(), ldb,
-                                                       tb.epow.as<c_t<T>>(), tb.einv.as<c_t<T>>(),
-                                                       w.local.as<c_t<T>>());
+      if (sizeof(T) == 8)
+        launch_l2l64<E>(ctx, t, tb, l - 1, w.local.as<double2>(), st);
+      else
+        k_l2l<float, E><<<nb, round32(E * (p + 1)), sizeof(float2) * E * (p + 1), st>>>(
+            t.lev_off[l], t.bkey.as<unsigned long long>(), t.parent.as<int>(), p, tb.binom.as<float>(), ldb,
+            tb.epow.as<float2>(), tb.einv.as<float2>(), w.local.as<float2>());
       eb_count_launch(ctx);
     }
   }
@@ -2332,10 +2532,10 @@ int direct_run(eb_ctx* ctx, EbTree& t, bool f32, int sign, const double2* dens, 
     if (E == 2)
       k_charges_stokes<float><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), dens, dz, hpt, (double)sign,
                                                             w.qa.as<float2>(), w.qb.as<float2>(),
-                                                            w.nc.as<float2>());
+                                                            w.nc.as<float2>(), nullptr);
     else
       k_charges_cauchy<float><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q_in, post.u, post.dz, post.hpt,
-                                                            w.qa.as<float2>());
+                                                            w.qa.as<float2>(), nullptr);
     if (join) EB_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
     if (E == 1) k_direct32<NEAR_Q><<<g, 128, 0, st>>>(n, zh, q, t.perm.as<int>(), 0, out, post);
     else if (kind == NEAR_V) k_direct32<NEAR_V><<<g, 128, 0, st>>>(n, zh, q, t.perm.as<int>(), plus, out, post);
@@ -2346,10 +2546,10 @@ int direct_run(eb_ctx* ctx, EbTree& t, bool f32, int sign, const double2* dens, 
     if (E == 2)
       k_charges_stokes<double><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), dens, dz, hpt, (double)sign,
                                                              w.qa.as<double2>(), w.qb.as<double2>(),
-                                                             w.nc.as<double2>());
+                                                             w.nc.as<double2>(), nullptr);
     else
       k_charges_cauchy<double><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q_in, post.u, post.dz, post.hpt,
-                                                             w.qa.as<double2>());
+                                                             w.qa.as<double2>(), nullptr);
     if (join) EB_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
     if (kind == NEAR_Q) k_direct64<NEAR_Q><<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), 0, out, post);
     else if (kind == NEAR_QI) k_direct64<NEAR_QI><<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), 0, out, post);
@@ -2385,6 +2585,11 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
       EB_TRY(w.nc.ensure(sizeof(c_t<T>) * 2 * (size_t)n));
     }
   }
+  int* next = nullptr;
+  if (f64 && !df) {
+    EB_TRY(w.next.ensure(sizeof(int)));
+    next = w.next.as<int>();
+  }
   if (df && E == 2) {
     k_charges_stokes_df<<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), dens, dz, hpt, (double)sign,
                                                       1.0 / t.W, t.plev.as<unsigned char>(), w.qdf.as<float4>(),
@@ -2394,10 +2599,11 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
                                                       1.0 / t.W, t.plev.as<unsigned char>(), w.ncdf.as<float4>());
   } else if (E == 2) {
     k_charges_stokes<T><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), dens, dz, hpt, (double)sign,
-                                                      w.qa.as<c_t<T>>(), w.qb.as<c_t<T>>(), w.nc.as<c_t<T>>());
+                                                      w.qa.as<c_t<T>>(), w.qb.as<c_t<T>>(), w.nc.as<c_t<T>>(),
+                                                      next);
   } else {
     k_charges_cauchy<T><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q, post.u, post.dz, post.hpt,
-                                                      w.qa.as<c_t<T>>());
+                                                      w.qa.as<c_t<T>>(), next);
   }
   eb_count_launch(ctx);
   const int has_far = t.L >= 2;
@@ -2420,8 +2626,9 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
     } else if (f64) {
       const double2* nq = E == 2 ? w.nc.as<double2>() : w.qa.as<double2>();
       auto go = [&](auto kern) {
-        kern<<<t.ntile, 128, 0, ns>>>(t.tiles.as<int4>(), t.pt0.as<int>(), t.pt1.as<int>(), t.ustart.as<int>(),
-                                      t.ulist.as<int>(), t.zs.as<double2>(), nq, plus, nb);
+        kern<<<std::min(t.ntile, NEAR64_CTAS * ctx->nsm), 128, 0, ns>>>(
+            t.ntile, next, t.tiles.as<int4>(), t.pt0.as<int>(), t.pt1.as<int>(), t.ustart.as<int>(),
+            t.ulist.as<int>(), t.zs.as<double2>(), nq, plus, nb);
       };
       if (kind == NEAR_Q) go(k_near64<NEAR_Q>);
       else if (kind == NEAR_QI) go(k_near64<NEAR_QI>);
@@ -2453,14 +2660,21 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
   // 33.6 ms and the 1,048,576-node refined solve 45.7 → 44.3 ms. Above that, and under the
   // per-kernel profiling timer, it precedes the far field on the main stream.
   const bool split = has_far && !ctx->profiling && n <= (1 << 20);
-  if (split) {
+  auto fork_near = [&]() -> int {
     EB_CUDA_TRY(cudaEventRecord(ctx->ev_c, st));
     EB_CUDA_TRY(cudaStreamWaitEvent(ctx->side_stream, ctx->ev_c, 0));
     near(ctx->side_stream);
     EB_CUDA_TRY(cudaEventRecord(ctx->ev_p2p, ctx->side_stream));
-  }
+    return EB_OK;
+  };
+  // FP64 on few tiles (the near field is the shorter side then): forked once the P2M, which
+  // the FP64 pipe bounds as well, has run. 4,096 nodes over a wall 3.68 -> 3.56 ms a solve,
+  // 14,401 nodes 233 -> 227 us an apply; 64 x 512 the other way, 6.72 -> 7.82 ms a solve.
+  const bool late = f64 && !df && t.ntile <= 8 * ctx->nsm;
+  if (split && !late) EB_TRY(fork_near());
   if (has_far && df) EB_TRY(fmm_expansions_df<E>(ctx, t, tb, w));
-  else if (has_far) EB_TRY((fmm_expansions<T, E>(ctx, t, tb, w)));
+  else if (has_far) EB_TRY((fmm_expansions<T, E>(ctx, t, tb, w, dz != nullptr,
+                                                 split && late ? std::function<int()>(fork_near) : nullptr)));
   if (!has_far) {
     EB_TRY(w.local.ensure(sizeof(c_t<T>) * (size_t)(E * (tb.p + 1))));
     EB_TRY(w.local_df.ensure(sizeof(float4) * (size_t)(E * (tb.p + 1))));
@@ -2483,12 +2697,12 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
         t.perm.as<int>(), t.wdf.as<float4>(), t.wdf_lo.as<float2>(), tb.p, (double)sign, w.local_df.as<float4>(),
         out, post, nb);
   } else if (f64) {
-    const int lpt = FAR64_LPT;
+    const int lpt = n >= FAR64_ONE ? 1 : 4;
     auto go = [&](auto kern) {
       kern<<<nblk((long long)n * lpt, 128), 128, 0, st>>>(
           n, t.lflag.as<int>(), t.lscan.as<int>(), t.leaves.as<int>(), has_far, t.bkey.as<unsigned long long>(),
           t.blev.as<unsigned char>(), t.wstart.as<int>(), t.wlist.as<int>(), t.perm.as<int>(), t.zs.as<double2>(),
-          t.x0, t.y0, t.W, tb.p, (double)sign, w.local.as<double2>(), w.mpole.as<double2>(), nb, out, post);
+          t.x0, t.y0, t.W, 1.0 / t.W, tb.p, (double)sign, w.local.as<double2>(), w.mpole.as<double2>(), nb, out, post);
     };
     if (lpt == 1) go(k_far64<E, 1>);
     else go(k_far64<E, 4>);

@@ -50,3 +50,23 @@ def test_cauchy_scales(gpu_ctx_factory, oracle, n, prec, df64, bar):
     q = rng.standard_normal(n) + 1j * rng.standard_normal(n)
     ctx = gpu_ctx_factory(leaf64=8, leaf_cap=8, df64=df64)
     assert relmax(ctx.dapif2(z, q, prec), oracle.cauchy_direct(z, z, q, True)) < bar
+
+
+@pytest.mark.parametrize("n", [300, 3000, 30000])
+@pytest.mark.parametrize("p64", [5, 44])
+def test_level_passes(gpu_ctx_factory, oracle, n, p64):
+    """M2M and L2L on levels of a few, some hundred and thousands of boxes (their outputs are
+    dealt to four, two or one blocks per box), and the far field's two lane layouts: at 1e-12
+    against direct sums, at a low order against the double-float kernels (1e-11)."""
+    rng = np.random.default_rng(n)
+    z = rng.uniform(-1, 1, n) + 1j * rng.uniform(-1, 1, n)
+    q = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    got = gpu_ctx_factory(p64=p64, leaf64=8, leaf_cap=8).dapif2(z, q)
+    if p64 == 44:
+        i = rng.integers(0, n, 200)
+        d = z[i][:, None] - z[None, :]
+        d[np.arange(200), i] = np.inf
+        assert relmax(got[i], (q[None, :] / d).sum(1)) < 1e-12
+    else:
+        ref = gpu_ctx_factory(p64=p64, leaf64=8, leaf_cap=8, df64=1).dapif2(z, q)
+        assert relmax(got, ref) < 1e-11
