@@ -26,6 +26,8 @@
 // right-preconditioned operator A M^-1 in the variable t = M x (k_deflate below), from
 // t0 = M rhs; x = M^-1 t at the end. Its residual b - A M^-1 t is b - A x, so the
 // stopping test and the reported error are those of the unpreconditioned solve.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -358,6 +360,15 @@ int laplace_matvec_deflated(eb_ctx* ctx, const double* x, double* y, int prec) {
   return eb_laplace_matvec_dev(ctx, t, y, prec);
 }
 
+// The Arnoldi step of a small system in one launch (below; GM_CL_ROWS rows at most).
+struct GmCtl;
+constexpr int GM_CL = 16;          // blocks of the cluster
+constexpr int GM_CL_THREADS = 512;
+constexpr int GM_CL_ROWS = GM_CL * GM_CL_THREADS;
+template <int PASSES>
+int gm_step(cudaStream_t s, int n, int ncol, double* V, size_t ldv, double* w, double* h1, double* h2, double* nw,
+            GmCtl* c = nullptr, double* hdev = nullptr, double* xin = nullptr, cudaGraphConditionalHandle h = 0);
+
 // One GMRES cycle (DGMRES with NRMAX = 0). x holds x0 on entry unless x0_zero.
 // Returns the DGMRES IERR convention in *ierr.
 int gmres_cycle(Gm& g, op_fn op, int prec, const double* b, double* x, bool x0_zero,
@@ -371,6 +382,7 @@ int gmres_cycle(Gm& g, op_fn op, int prec, const double* b, double* x, bool x0_z
   // classical Gram-Schmidt twice for the FP64 solve; once for the inner FP32 cycle of
   // the refined solve, whose tolerance (1e-5) is far above the loss of orthogonality
   const bool cgs2 = prec == EB_FP64;
+  const bool small = n <= GM_CL_ROWS;
   EB_TRY(ctx->gV.ensure(sizeof(double) * ldv * (maxl + 1)));
   double* V = ctx->gV.as<double>();
   double* part = ctx->gPart.as<double>();
@@ -432,11 +444,16 @@ int gmres_cycle(Gm& g, op_fn op, int prec, const double* b, double* x, bool x0_z
     double snormw;
     if (cgs2) {
       // pass 1: h1 = V^T w; w -= V h1; pass 2: h2 = V^T w; w -= V h2 with ||w||^2
-      k_vtw<<<g.nb, RBS, 0, g.s>>>(n, ll, nullptr, V, ldv, w, part, hdev, g.ticket);
-      k_update_vtw<<<g.nb, RBS, 0, g.s>>>(n, ll, nullptr, V, ldv, hdev, w, part, hdev + (maxl + 2), g.ticket);
-      k_gemv_sub<<<g.nb, RBS, 0, g.s>>>(n, ll, nullptr, V, ldv, hdev + (maxl + 2), w, part,
-                                        hdev + 2 * (maxl + 2), g.ticket);
-      ctx->launches += 3;
+      if (small) {
+        EB_TRY(gm_step<2>(g.s, n, ll, V, ldv, w, hdev, hdev + (maxl + 2), hdev + 2 * (maxl + 2)));
+        eb_count_launch(ctx);
+      } else {
+        k_vtw<<<g.nb, RBS, 0, g.s>>>(n, ll, nullptr, V, ldv, w, part, hdev, g.ticket);
+        k_update_vtw<<<g.nb, RBS, 0, g.s>>>(n, ll, nullptr, V, ldv, hdev, w, part, hdev + (maxl + 2), g.ticket);
+        k_gemv_sub<<<g.nb, RBS, 0, g.s>>>(n, ll, nullptr, V, ldv, hdev + (maxl + 2), w, part,
+                                          hdev + 2 * (maxl + 2), g.ticket);
+        ctx->launches += 3;
+      }
       EB_CUDA_TRY(cudaMemcpyAsync(hbuf.data(), hdev, sizeof(double) * 3 * (maxl + 2),
                                   cudaMemcpyDeviceToHost, g.s));
       EB_CUDA_TRY(cudaStreamSynchronize(g.s));
@@ -444,7 +461,9 @@ int gmres_cycle(Gm& g, op_fn op, int prec, const double* b, double* x, bool x0_z
       snormw = std::sqrt(std::max(hbuf[2 * (maxl + 2)], 0.0));
     } else {
       // one pass: h = V^T w and w . w; the update waits for the decision below
-      k_vtw<<<g.nb, RBS, 0, g.s>>>(n, ll, nullptr, V, ldv, w, part, hdev, g.ticket, 1);
+      // (a small system's kernel has made it already)
+      if (small) EB_TRY(gm_step<1>(g.s, n, ll, V, ldv, w, hdev, nullptr, hdev + 2 * (maxl + 2)));
+      else k_vtw<<<g.nb, RBS, 0, g.s>>>(n, ll, nullptr, V, ldv, w, part, hdev, g.ticket, 1);
       eb_count_launch(ctx);
       EB_CUDA_TRY(cudaMemcpyAsync(hbuf.data(), hdev, sizeof(double) * (ll + 1), cudaMemcpyDeviceToHost, g.s));
       EB_CUDA_TRY(cudaStreamSynchronize(g.s));
@@ -464,7 +483,7 @@ int gmres_cycle(Gm& g, op_fn op, int prec, const double* b, double* x, bool x0_z
     if (*err <= tol) { iflag = 0; break; }
     if (ll == maxl) break;
     if (snormw == 0.0) { iflag = 2; break; }
-    if (cgs2) {
+    if (cgs2 || small) {
       k_scale<<<g.nb, RBS, 0, g.s>>>(n, 1.0 / snormw, w);
     } else {
       k_sub_scale<<<g.nb, RBS, 0, g.s>>>(n, ll, V, ldv, hdev, w, 1.0 / snormw);
@@ -607,6 +626,135 @@ __device__ void gm_arnoldi_warp(GmCtl* c, const double* __restrict__ hdev, cudaG
   }
   c->cont = cont;
   cudaGraphSetConditional(h, cont ? 1u : 0u);
+}
+
+// A whole Arnoldi step of a small system after its operator apply, in one launch: both
+// Gram-Schmidt passes of classical Gram-Schmidt twice (PASSES = 2) or the one pass with the
+// norm by Pythagoras (PASSES = 1), and the new column. One cluster of GM_CL blocks, a row
+// per thread; the sums over the blocks go through distributed shared memory in rank order.
+// With `c` (graph mode) the first block then ends the step (gm_arnoldi_warp) and the column is
+// stored scaled, into V and xin; without it (host-driven loop) the coefficients go to h1, h2
+// and the norm to nw (PASSES = 1: w . w to h1[ncol]) and w is overwritten unscaled. A NaN
+// norm fails the comparison and is summed, so it reaches the NaN test as before.
+//
+// Up to GM_CL_ROWS rows the four kernels it replaces are bound by their launches and the
+// three grid-wide reductions (5 to 9 us each); this one by the FP64 latency and rate of 16
+// SMs, 4 ncol n FMAs. Measured, FP64 mode: 16.5 -> 8.5 us a step at 512 rows, 19 -> 14 us at
+// 8,192 (ncol about 10); above that the grid-wide kernels have the SMs for it.
+template <int PASSES>
+__global__ void __cluster_dims__(GM_CL, 1, 1) __launch_bounds__(GM_CL_THREADS)
+    k_gm_step(int n, int ncol, double* V, size_t ldv, double* w, double* h1, double* h2, double* nw, GmCtl* c,
+              double* hdev, double* __restrict__ xin, cudaGraphConditionalHandle h) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ double ws[GM_CL_THREADS];
+  __shared__ double part[2][EB_GM_MAXL + 2], hs[2][EB_GM_MAXL + 2], sq[1], red[32], s_nw;
+  const int tid = threadIdx.x, wi = tid >> 5, lane = tid & 31;
+  const int rank = (int)cl.block_rank();
+  if (c) ncol = c->ll;
+  const int rows = (n + GM_CL - 1) / GM_CL, r0 = rank * rows, nr = max(0, min(n, r0 + rows) - r0);
+  const bool act = tid < nr;
+  const double* Vr = V + r0;
+  double wv = act ? w[r0 + tid] : 0.0;
+  ws[tid] = wv;
+  __syncthreads();
+#pragma unroll
+  for (int ps = 0; ps < PASSES; ++ps) {
+    // V^T w, in the last pass with w . w: a warp per column
+    const int nc = ncol + (ps == PASSES - 1);
+    for (int j = wi; j < nc; j += GM_CL_THREADS / 32) {
+      const double* v = j < ncol ? Vr + (size_t)j * ldv : ws;
+      double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+      for (int i = lane; i < nr; i += 128) {
+        s0 = fma(v[i], ws[i], s0);
+        if (i + 32 < nr) s1 = fma(v[i + 32], ws[i + 32], s1);
+        if (i + 64 < nr) s2 = fma(v[i + 64], ws[i + 64], s2);
+        if (i + 96 < nr) s3 = fma(v[i + 96], ws[i + 96], s3);
+      }
+      const double s = warp_sum<double>((s0 + s1) + (s2 + s3));
+      if (lane == 0) part[ps][j] = s;
+    }
+    cl.sync();
+    for (int j = tid; j < nc; j += GM_CL_THREADS) {
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int b = 0; b < GM_CL; ++b) s[b & 3] += cl.map_shared_rank(part[ps], b)[j];
+      hs[ps][j] = (s[0] + s[1]) + (s[2] + s[3]);
+    }
+    __syncthreads();
+    // w -= V h
+    if (act) {
+      double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+      int j = 0;
+      for (; j + 4 <= ncol; j += 4) {
+        const double* v = Vr + (size_t)j * ldv + tid;
+        a0 = fma(v[0], hs[ps][j], a0);
+        a1 = fma(v[ldv], hs[ps][j + 1], a1);
+        a2 = fma(v[2 * ldv], hs[ps][j + 2], a2);
+        a3 = fma(v[3 * ldv], hs[ps][j + 3], a3);
+      }
+      for (; j < ncol; ++j) a0 = fma(Vr[(size_t)j * ldv + tid], hs[ps][j], a0);
+      wv -= (a0 + a1) + (a2 + a3);
+      ws[tid] = wv;
+    }
+    __syncthreads();
+  }
+  // the new vector's norm
+  if (PASSES == 2) {
+    // by Pythagoras from the second pass, whose coefficients are rounding residues:
+    // ||w - V h||^2 = w . w - h . h to rounding, unless they are not small (a new direction
+    // lost in rounding), where the norm is summed
+    if (wi == 0) {
+      double t = 0.0;
+      for (int j = lane; j < ncol; j += 32) t = fma(hs[1][j], hs[1][j], t);
+      t = warp_sum<double>(t);
+      if (lane == 0) s_nw = t <= 1e-3 * hs[1][ncol] ? hs[1][ncol] - t : -1.0;
+    }
+    __syncthreads();
+    if (s_nw < 0.0) {  // the same values, so the same branch, in every block
+      const double s = block_sum(wv * wv, red);
+      if (tid == 0) sq[0] = s;
+      cl.sync();
+      if (tid == 0) {
+        double t = 0.0;
+        for (int b = 0; b < GM_CL; ++b) t += *cl.map_shared_rank(sq, b);
+        s_nw = t;
+      }
+    }
+  } else if (tid == 0) {
+    s_nw = pyth_norm2(hs[0], ncol, hs[0][ncol]);
+  }
+  __syncthreads();
+  const double nn = s_nw;
+  if (rank == 0) {
+    for (int j = tid; j < ncol + (PASSES == 1); j += GM_CL_THREADS) {
+      h1[j] = hs[0][j];
+      if (PASSES == 2) h2[j] = hs[1][j];
+    }
+    if (tid == 0) *nw = nn;
+    __syncthreads();
+    if (c && tid < 32) gm_arnoldi_warp(c, hdev, h);
+  }
+  if (act) {
+    if (c) {
+      // (an invariant space, norm 0, ends the iteration: its column is not read)
+      const double v = wv * (1.0 / sqrt(fmax(nn, 0.0)));
+      V[(size_t)ncol * ldv + r0 + tid] = v;
+      xin[r0 + tid] = v;
+    } else {
+      w[r0 + tid] = wv;
+    }
+  }
+  cl.sync();  // no block leaves while others read its sums
+}
+
+// Launches k_gm_step (n <= GM_CL_ROWS).
+template <int PASSES>
+int gm_step(cudaStream_t s, int n, int ncol, double* V, size_t ldv, double* w, double* h1, double* h2, double* nw,
+            GmCtl* c, double* hdev, double* xin, cudaGraphConditionalHandle h) {
+  EB_CUDA_TRY(cudaFuncSetAttribute(k_gm_step<PASSES>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  k_gm_step<PASSES><<<GM_CL, GM_CL_THREADS, 0, s>>>(n, ncol, V, ldv, w, h1, h2, nw, c, hdev, xin, h);
+  return EB_OK;
 }
 
 // The last Gram-Schmidt update (w -= V h with ||w||^2 into hdev[GM_NW]); the block that
@@ -791,6 +939,14 @@ int build_graph(eb_ctx* ctx, GmGraph& G, int kind, op_fn op, int n, int maxl) {
   cst = eb_capture_into(ctx, body, nullptr, 0, nullptr, &G.n_body, &body_lost, [&]() -> int {
     cudaStream_t s = ctx->stream;
     EB_TRY(op(ctx, xin, wbuf, prec));
+    if (n <= GM_CL_ROWS) {
+      if (refine)
+        EB_TRY(gm_step<1>(s, n, 0, V, ldv, wbuf, hdev + GM_H1, nullptr, hdev + GM_NW, ctl, hdev, xin, h));
+      else
+        EB_TRY(gm_step<2>(s, n, 0, V, ldv, wbuf, hdev + GM_H1, hdev + GM_H2, hdev + GM_NW, ctl, hdev, xin, h));
+      eb_count_launch(ctx);
+      return eb_check_launch(ctx, "gmres graph (body)");
+    }
     if (refine) {
       // one Gram-Schmidt pass for the inner FP32 cycle (the H2 slots stay zero), its
       // norm by Pythagoras from the same reduction, the update fused with the store
