@@ -466,19 +466,24 @@ int eb_stokes_matvec_dev(eb_ctx* ctx, const double* x, double* y, int prec) {
   EB_TRY(ctx->za.ensure(sizeof(double2) * k));
   EB_TRY(ctx->pk.ensure(sizeof(double) * k));
   // the per-drop sums run on the side stream, overlapping the FMM; the leaf kernel, whose
-  // fused post-processing reads them, waits for them
-  EB_CUDA_TRY(cudaEventRecord(ctx->ev_fork, s));
-  EB_CUDA_TRY(cudaStreamWaitEvent(ctx->side_stream, ctx->ev_fork, 0));
-  k_drop_reduce_stokes<<<k, 256, 0, ctx->side_stream>>>(ctx->start.as<int>(), dens, ctx->pkw.as<double2>(),
-                                                       ctx->za.as<double2>(), ctx->pk.as<double>());
-  eb_count_launch(ctx);
-  EB_CUDA_TRY(cudaEventRecord(ctx->ev_join, ctx->side_stream));
+  // fused post-processing reads them, waits for them. The direct sums' charge kernel forms
+  // them itself (EbPost::start).
+  const bool direct = ctx->tree.direct;
+  if (!direct) {
+    EB_CUDA_TRY(cudaEventRecord(ctx->ev_fork, s));
+    EB_CUDA_TRY(cudaStreamWaitEvent(ctx->side_stream, ctx->ev_fork, 0));
+    k_drop_reduce_stokes<<<k, 256, 0, ctx->side_stream>>>(ctx->start.as<int>(), dens, ctx->pkw.as<double2>(),
+                                                         ctx->za.as<double2>(), ctx->pk.as<double>());
+    eb_count_launch(ctx);
+    EB_CUDA_TRY(cudaEventRecord(ctx->ev_join, ctx->side_stream));
+  }
   EbPost post{1, dens, nullptr, ctx->z.as<double2>(), ctx->dz.as<double2>(), ctx->hpt.as<double>(),
                ctx->pc1.as<double>(), ctx->pc2.as<double2>(), ctx->drop_of.as<int>(),
                ctx->za.as<double2>(), ctx->pk.as<double>(), y, ctx->pc1f.as<float>(),
-               ctx->pc2f.as<float2>(), ctx->nsim > 0 ? ctx->b_pinf.as<int>() : nullptr};
+               ctx->pc2f.as<float2>(), ctx->nsim > 0 ? ctx->b_pinf.as<int>() : nullptr,
+               direct ? ctx->start.as<int>() : nullptr, ctx->pkw.as<double2>(), k};
   EB_TRY(eb_fmm_apply(ctx, ctx->tree, 0, -1, prec, dens, ctx->dz.as<double2>(), ctx->hpt.as<double>(),
-                      nullptr, &post, ctx->ev_join));
+                      nullptr, &post, direct ? nullptr : ctx->ev_join));
   return eb_check_launch(ctx, "stokes matvec");
 }
 

@@ -21,6 +21,11 @@ struct EbPost {
   const float2* c2f;
   const int* pinf_drop;   // kind 1: per drop, the drop whose pressure is pinf (the first
                           // drop of its simulation); null: drop 0
+  // kind 1, for the direct sums' charge kernel, which forms za and pk too (null: formed
+  // already): the drops' starts, the weights of the singular-term sums and the drops' count
+  const int* start;
+  const double2* pkw;
+  int k;
 };
 
 // Per-node coefficients of the post-processing, formed once per geometry (they hold the
