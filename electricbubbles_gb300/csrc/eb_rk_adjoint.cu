@@ -960,7 +960,8 @@ __global__ void k_sum3(int n, const double* __restrict__ x, const double* __rest
 }
 
 int set_smem(const void* fn, size_t bytes) {
-  if (bytes > 48 * 1024)
+  // (48 KiB without it, the kernel's static shared memory included)
+  if (bytes > 40 * 1024)
     EB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   return EB_OK;
 }

@@ -340,7 +340,9 @@ int check_pow2(eb_ctx* ctx, int& nmax) {
 }
 
 int set_smem(const void* fn, size_t bytes) {
-  if (bytes > 48 * 1024)
+  // (48 KiB without it, the kernel's static shared memory included: k_setvelf's largest drop
+  // of 2,048 nodes takes exactly 48 KiB of dynamic memory)
+  if (bytes > 40 * 1024)
     EB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   return EB_OK;
 }
