@@ -177,7 +177,7 @@ __global__ void k_charges_stokes_df(int n, const int* __restrict__ perm, const d
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int o = perm[i];
-  const double rinv = ldexp(winv, (int)plev[i]);
+  const double rinv = winv * pow2d((int)plev[i]);
   double2 u = dens[o], a, b;
   if (dz) {
     double2 d = dz[o];
@@ -213,7 +213,7 @@ __global__ void k_charges_cauchy_df(int n, const int* __restrict__ perm, const d
                                     const unsigned char* __restrict__ plev, float4* __restrict__ qdf) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double rinv = ldexp(winv, (int)plev[i]);
+  const double rinv = winv * pow2d((int)plev[i]);
   double2 v = cauchy_charge(perm[i], q, lu, dz, hpt);
   qdf[i] = df4(make_double2(v.x * rinv, v.y * rinv));
 }
@@ -999,48 +999,62 @@ __device__ __forceinline__ cdf quad_merge(dfacc rx, dfacc ry) {
   return v;
 }
 
-// M2M: 4 lanes per output coefficient, each summing every 4th term, so the dependent
-// chain of compensated products is a quarter as long.
+// M2M: k_m2m64's scheme (one binomial sum for all children's rotations) in double-float: 4
+// lanes per output coefficient, each summing every 4th term, so that the dependent chain of
+// compensated products is a sixteenth of a sum per child's. Measured (E = 2): 14.9 -> 9.4 us a level
+// of 64 x 512, 79 -> 56 us at 1,024 x 1,024 (its far field beside it, with the Horner steps
+// below: 22.6 -> 19.2 and 569 -> 482 us)
 template <int E>
 __global__ void k_m2m_df(int offp, const unsigned long long* __restrict__ bkey,
                          const int* __restrict__ child0, const int* __restrict__ nchild, int p,
                          const float2* __restrict__ binom, int ldb, const float4* __restrict__ epow2,
                          const float4* __restrict__ einv, float4* __restrict__ mpole) {
   extern __shared__ float4 sm4[];
-  float4* a = sm4;  // [child][E*p]
+  float4* cr = sm4;  // [r][E*p]
   const int P = offp + blockIdx.x, tid = threadIdx.x, ld = p + 2, nout = E * p;
   const int c0 = child0[P], nc = nchild[P];
   if (nc == 0) return;  // a leaf: its multipole comes from its points
-  for (int idx = tid; idx < nc * nout; idx += blockDim.x) {
-    const int ci = idx / nout, o = idx - ci * nout;
-    const int c = c0 + ci, q = quadrant(bkey[c]);
-    const int e2 = o / p, kk = o - e2 * p, k = kk + 1;
-    const float4* mc = mpole + (size_t)c * nout;
-    cdf v = cdf_from_float4(mc[o]);
-    if (e2 == 1 && k >= 2) {
-      const cdf ec = cdf_scale(cdf_from_float4(epow2[q * ld + 1]), 2.f);
-      v = cdf_add(v, cdf_mul(cdf_scale(cdf_conj(ec), (float)(k - 1)), cdf_from_float4(mc[kk - 1])));
-    }
-    a[idx] = cdf_f4(cdf_mul(v, cdf_from_float4(einv[q * ld + k])));
-  }
-  __syncthreads();
+  // four lanes per coefficient: lane r forms c^r from the children's b (lane ci forms child ci's)
   const int o = tid >> 2, part = tid & 3;
   const bool act = o < nout;
   const int oo = act ? o : 0;
   const int e = oo / p, n = oo - e * p + 1;
-  const float2* brow = binom + (size_t)(n - 1) * ldb;
+  {
+    const int q = part < nc ? quadrant(bkey[c0 + part]) : 0;
+    cdf b{{0.f, 0.f}, {0.f, 0.f}};
+    if (part < nc) {
+      const float4* mc = mpole + (size_t)(c0 + part) * nout;
+      cdf v = cdf_from_float4(mc[oo]);
+      if (e == 1 && n >= 2) {
+        const cdf ec = cdf_scale(cdf_from_float4(epow2[q * ld + 1]), 2.f);
+        v = cdf_add(v, cdf_mul(cdf_scale(cdf_conj(ec), (float)(n - 1)), cdf_from_float4(mc[n - 2])));
+      }
+      b = cdf_mul(v, cdf_from_float4(einv[3 * ld + n]));
+    }
+    const int rot = quad_rot(q), q0 = (tid & 31) & ~3;
+    cdf c{{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+    for (int ci = 0; ci < 4; ++ci) {
+      const float4 f = make_float4(__shfl_sync(0xffffffffu, b.x.hi, q0 + ci), __shfl_sync(0xffffffffu, b.x.lo, q0 + ci),
+                                   __shfl_sync(0xffffffffu, b.y.hi, q0 + ci), __shfl_sync(0xffffffffu, b.y.lo, q0 + ci));
+      const int k = (part * __shfl_sync(0xffffffffu, rot, q0 + ci)) & 3;  // times i^k
+      const cdf v = cdf_from_float4(f);
+      const dfl tx = k & 1 ? v.y : v.x, ty = k & 1 ? v.x : v.y;
+      c.x = dfl_add(c.x, k == 1 || k == 2 ? dfl_neg(tx) : tx);
+      c.y = dfl_add(c.y, k >= 2 ? dfl_neg(ty) : ty);
+    }
+    if (act) cr[part * nout + o] = cdf_f4(c);
+  }
+  __syncthreads();
   dfacc rx{0.f, 0.f}, ry{0.f, 0.f};
   if (act) {
-    for (int ci = 0; ci < nc; ++ci) {
-      const int q = quadrant(bkey[c0 + ci]);
-      const float4* ae = a + ci * nout + e * p;
-      dfacc sx{0.f, 0.f}, sy{0.f, 0.f};
-      for (int k = part; k < n; k += 4) cacc_rmul(sx, sy, dfl{brow[k].x, brow[k].y}, cdf_from_float4(ae[k]));
-      cacc_mul(rx, ry, cdf_from_float4(epow2[q * ld + n]), cacc_value(sx, sy));
-    }
+    const float2* brow = binom + (size_t)(n - 1) * ldb;
+    const float4* src = cr + ((n - 1 - part) & 3) * nout + e * p;
+#pragma unroll 4
+    for (int k = part; k < n; k += 4) cacc_rmul(rx, ry, dfl{brow[k].x, brow[k].y}, cdf_from_float4(src[k]));
   }
   const cdf v = quad_merge(rx, ry);
-  if (act && part == 0) mpole[(size_t)P * nout + o] = cdf_f4(v);
+  if (act && part == 0) mpole[(size_t)P * nout + o] = cdf_f4(cdf_mul(cdf_from_float4(epow2[3 * ld + n]), v));
 }
 
 template <int E>
@@ -1525,6 +1539,21 @@ __device__ __forceinline__ dfl tf_diff(float ah, float am, float al, float3 b) {
   return fast_two_sum(h.hi, __fadd_rn(h.lo, u));
 }
 
+// a u + c: the two products and the addend of each part summed at once
+__device__ __forceinline__ dfl dfl_dot2_add(dfl a, dfl b, dfl c, dfl d, dfl s) {  // a b + c d + s
+  const float p = __fmul_rn(a.hi, b.hi), q = __fmul_rn(c.hi, d.hi);
+  float e = __fmaf_rn(a.hi, b.hi, -p), f = __fmaf_rn(c.hi, d.hi, -q);
+  e = __fmaf_rn(a.hi, b.lo, e);
+  f = __fmaf_rn(c.hi, d.lo, f);
+  e = __fmaf_rn(a.lo, b.hi, e);
+  f = __fmaf_rn(c.lo, d.hi, f);
+  const dfl t = two_sum(p, q), u = two_sum(t.hi, s.hi);
+  return fast_two_sum(u.hi, __fadd_rn(__fadd_rn(u.lo, t.lo), __fadd_rn(__fadd_rn(e, f), s.lo)));
+}
+__device__ __forceinline__ cdf cdf_horner(cdf a, cdf u, cdf c) {
+  return cdf{dfl_dot2_add(a.x, u.x, dfl_neg(a.y), u.y, c.x), dfl_dot2_add(a.x, u.y, a.y, u.x, c.y)};
+}
+
 template <int E>
 __device__ __forceinline__ void l2p_part_df(const float4* L, int p, int sl, cdf u, bool neg, dfacc& gx,
                                             dfacc& gy) {
@@ -1533,18 +1562,18 @@ __device__ __forceinline__ void l2p_part_df(const float4* L, int p, int sl, cdf 
   if (m0 >= m1) return;
   cdf ph = cdf_from_float4(L[m1 - 1]), dph = cdf{{0.f, 0.f}, {0.f, 0.f}};
   for (int m = m1 - 2; m >= m0; --m) {
-    dph = cdf_add(cdf_mul(dph, u), ph);
-    ph = cdf_add(cdf_mul(ph, u), cdf_from_float4(L[m]));
+    if (E == 2) dph = cdf_horner(dph, u, ph);
+    ph = cdf_horner(ph, u, cdf_from_float4(L[m]));
   }
   cdf ps = cdf{{0.f, 0.f}, {0.f, 0.f}};
   if (E == 2) {
     ps = cdf_from_float4(L[ldl + m1 - 1]);
-    for (int m = m1 - 2; m >= m0; --m) ps = cdf_add(cdf_mul(ps, u), cdf_from_float4(L[ldl + m]));
+    for (int m = m1 - 2; m >= m0; --m) ps = cdf_horner(ps, u, cdf_from_float4(L[ldl + m]));
   }
   if (m0 > 0) {
     cdf um1 = cdf_pow(u, m0 - 1);
-    cdf t = cdf_add(cdf_mul(u, dph), cdf{dfl_mul_f(ph.x, (float)m0), dfl_mul_f(ph.y, (float)m0)});
-    dph = cdf_mul(um1, t);
+    if (E == 2)
+      dph = cdf_mul(um1, cdf_horner(u, dph, cdf{dfl_mul_f(ph.x, (float)m0), dfl_mul_f(ph.y, (float)m0)}));
     cdf um = cdf_mul(um1, u);
     ph = cdf_mul(um, ph);
     if (E == 2) ps = cdf_mul(um, ps);
@@ -1610,14 +1639,14 @@ __device__ __forceinline__ void m2p_df(const float4* M, int p, cdf u, bool neg, 
   cdf da = cdf_scale(a, (float)p);
   for (int k = p - 1; k >= 1; --k) {
     const cdf mk = cdf_from_float4(M[k - 1]);
-    a = cdf_add(cdf_mul(a, v), mk);
-    if (E == 2) da = cdf_add(cdf_mul(da, v), cdf_scale(mk, (float)k));
+    a = cdf_horner(a, v, mk);
+    if (E == 2) da = cdf_horner(da, v, cdf_scale(mk, (float)k));
   }
   const cdf ph = cdf_mul(a, v);
   if (E == 2) {
     const cdf dph = cdf_mul(da, cdf_mul(v, v));  // -phi_u
     cdf b = cdf_from_float4(M[2 * p - 1]);
-    for (int k = p - 1; k >= 1; --k) b = cdf_add(cdf_mul(b, v), cdf_from_float4(M[p + k - 1]));
+    for (int k = p - 1; k >= 1; --k) b = cdf_horner(b, v, cdf_from_float4(M[p + k - 1]));
     const cdf ps = cdf_mul(b, v);
     const dfl tx = dfl_add(dfl_mul(u.x, dph.x), dfl_mul(u.y, dph.y));  // -u conj(phi_u)
     const dfl ty = dfl_sub(dfl_mul(u.y, dph.x), dfl_mul(u.x, dph.y));

@@ -162,9 +162,10 @@ struct EbTables {
   DevBuf dinv_df;   // float4[EB_NCODE*(p+2)]
   DevBuf epow_df;   // float4[4*(p+2)]
   DevBuf einv_df;   // float4[4*(p+2)]
-  // fixed-point M2L (FP64 tables of order <= EB_FX_MAXP): the binomial matrix's digits, the
-  // powers (2/d)^j as limbs of 2^62 fractions, and the matrix's row scalings
-  DevBuf fxb, fxt, fxr;
+  // fixed-point M2L (FP64 tables of order <= EB_FX_MAXP): the powers (2/d)^j as limbs of
+  // 2^62 fractions, then (fxb) the binomial matrix's digits and (fxr) its row scalings
+  DevBuf fxt;
+  const void *fxb = nullptr, *fxr = nullptr;
 };
 #define EB_FX_K 48      // orders of the fixed-point M2L's operand tiles
 #define EB_FX_MAXP 47   // its largest expansion order (p + 1 local orders)

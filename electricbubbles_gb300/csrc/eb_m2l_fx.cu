@@ -25,7 +25,7 @@
 // Errors of the sums against direct sums are those of the FP64 kernel (k_m2l) or smaller.
 //
 // What bounds it is the issue of the integer work before and after the products. One block
-// per SM (its accumulators fill the tensor memory) of two teams of eight warps, each with
+// per SM (its accumulators fill the tensor memory) of two teams of 16 warps, each with
 // its own digits, runs a round of one team's integer work under the other's: the team that
 // holds the tensor memory issues its products, reads the sums and passes it on.
 // Measured (E = 2, p = 44; k_m2l is the FP64 CUDA-core kernel): 13,290 entries of 64 x 512
@@ -37,6 +37,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -52,7 +53,7 @@ constexpr int FX_B = EB_FX_K * EB_FX_K * 2; // bytes of a digit of the matrix
 constexpr int FX_ND = 6;                    // digits of a number
 constexpr int FX_NACC = 7;                  // accumulators (digit pairs i + j = 0 .. 6)
 constexpr int FX_COLS = 512;                // tensor-memory columns (7 x 48, a power of two)
-constexpr int FX_TEAM = 256;                // threads of a team
+constexpr int FX_TEAM = 512;                // threads of a team
 constexpr int FX_THREADS = 2 * FX_TEAM;
 constexpr int FX_PITCH = FX_ROWS + 4;       // row pitch of the contributions (int64)
 constexpr int FX_GROUP = 8;                 // target boxes of a work item, at most
@@ -88,16 +89,22 @@ struct Limb {
   int hi, lo;
 };
 __device__ __forceinline__ Limb limbs(long long x) {
-  return Limb{(int)((x + 0x80000000ll) >> 32), (int)x};
+  return Limb{(int)(x >> 32) + (int)((uint32_t)x >> 31), (int)x};
+}
+
+// a b + c of 32-bit a and b and 64-bit c in one instruction (a product of sign-extended
+// truncations written in C becomes a 64-bit multiplication: three multiply-adds and shifts)
+__device__ __forceinline__ long long madw(int a, int b, long long c) {
+  long long d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
 }
 
 // (x yr + y yi) / 2^64, the lowest parts left out (an error of at most two units), for
 // |x|, |y| < 2^61.5 and table entries of at most 2^62: every partial sum is below 2^63
 __device__ __forceinline__ long long mul_add_hi(Limb x, int yrh, int yrl, Limb y, int yih, int yil) {
-  const long long hh = (long long)x.hi * yrh + (long long)y.hi * yih;
-  const long long mid = (long long)x.hi * yrl + (long long)x.lo * yrh + (long long)y.hi * yil +
-                        (long long)y.lo * yih + 0x80000000ll;
-  return hh + (mid >> 32);
+  const long long mid = madw(x.hi, yrl, madw(x.lo, yrh, madw(y.hi, yil, madw(y.lo, yih, 0x80000000ll))));
+  return madw(x.hi, yrh, madw(y.hi, yih, (long long)(int)(mid >> 32)));
 }
 
 // 2^e of any e: two factors, the first clamped so that a result in range stays exact
@@ -122,29 +129,45 @@ __device__ __forceinline__ int exp_above(uint32_t hiabs) {  // e with |v| < 2^e,
 // Multipoles of the boxes [first, first + nb) as 64-bit integers, one warp per box:
 // fx = v 2^(61 - S), 2^S above the box's largest part of phi (fs.x) and of psi (fs.y); fs.z is
 // the exponent above the largest part of k phi_k, which moving psi to another centre adds.
+// Double-float multipoles without FP64: the exponents are those of the high floats, and both
+// floats of a part are shifted into place as integers.
+__device__ __forceinline__ long long float_fix(float f, int S) {  // f 2^(61 - S), |f| < 2^S
+  const uint32_t b = __float_as_uint(f);
+  const int e = (int)((b >> 23) & 255u), m = (int)((b & 0x7fffffu) | (e ? 0x800000u : 0u));
+  const int sh = max(e, 1) - 89 - S;
+  const long long v = sh >= 0 ? (long long)m << min(sh, 40) : sh > -32 ? (long long)((m + (1 << (-sh - 1))) >> -sh) : 0;
+  return (int)b < 0 ? -v : v;
+}
+
 template <int E, bool DF>
 __global__ void __launch_bounds__(128) k_m2l_fix(int first, int nb, int p, const void* __restrict__ mpole,
                                                  longlong2* __restrict__ fx, int4* __restrict__ fs) {
   const int wb = (blockIdx.x * 128 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (wb >= nb) return;
   const size_t b = (size_t)(first + wb), n = (size_t)E * p;
-  auto ld = [&](int o) {
-    if (DF) {
-      const float4 v = reinterpret_cast<const float4*>(mpole)[b * n + o];
-      return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
-    }
-    return reinterpret_cast<const double2*>(mpole)[b * n + o];
-  };
+  const double2* md = reinterpret_cast<const double2*>(mpole) + b * n;
+  const float4* mf = reinterpret_cast<const float4*>(mpole) + b * n;
+  // the largest parts' magnitude bits (double: the high words; double-float: the high floats),
+  // and those of k phi_k rounded up
   uint32_t h[2] = {0u, 0u}, hk = 0u;
   for (int o = lane; o < E * p; o += 32) {
-    const double2 v = ld(o);
-    const uint32_t m = max((uint32_t)__double2hiint(v.x) & 0x7fffffffu, (uint32_t)__double2hiint(v.y) & 0x7fffffffu);
+    uint32_t m;
+    if (DF) {
+      const float4 v = mf[o];
+      m = max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.z) & 0x7fffffffu);
+    } else {
+      const double2 v = md[o];
+      m = max((uint32_t)__double2hiint(v.x) & 0x7fffffffu, (uint32_t)__double2hiint(v.y) & 0x7fffffffu);
+    }
     if (E == 1 || o < p) {
       h[0] = max(h[0], m);
       if (E == 2) {
-        // (m's top 20 mantissa bits plus one, times k) bounds k |v|
-        const double f = __hiloint2double((int)min(m + 1u, 0x7fefffffu), 0) * (double)(o + 1);
-        hk = max(hk, (uint32_t)__double2hiint(f));
+        const float k = (float)(o + 1);
+        if (DF) hk = max(hk, __float_as_uint(__fmul_ru(__uint_as_float(m), k)));
+        else {  // the exponent field plus that of (top mantissa bits + 1) x k
+          const float t = __fmul_ru(__uint_as_float(0x3f800000u + (((m & 0xfffffu) + 1u) << 3)), k);
+          hk = max(hk, (m & 0x7ff00000u) + ((__float_as_uint(t) >> 23) - 127u) * (1u << 20));
+        }
       }
     } else {
       h[1] = max(h[1], m);
@@ -155,24 +178,27 @@ __global__ void __launch_bounds__(128) k_m2l_fix(int first, int nb, int p, const
     h[1] = __reduce_max_sync(0xffffffffu, h[1]);
     hk = __reduce_max_sync(0xffffffffu, hk);
   }
-  const bool bad = max(h[0], h[1]) >= 0x7ff00000u;
+  auto above = [](uint32_t m) { return DF ? (int)(m >> 23) - 126 : exp_above(m); };
+  const bool bad = max(h[0], h[1]) >= (DF ? 0x7f800000u : 0x7ff00000u);
   int S[2];
-  double f1[2], f2[2];
 #pragma unroll
-  for (int e = 0; e < E; ++e) {
-    S[e] = max(exp_above(h[e]), FX_EMIN);
-    // 2^(61 - S) as two factors (S from -900 to 1024)
-    const int e1 = (61 - S[e]) >> 1, e2 = 61 - S[e] - e1;
-    f1[e] = __hiloint2double((1023 + e1) << 20, 0);
-    f2[e] = __hiloint2double((1023 + e2) << 20, 0);
-  }
-  if (lane == 0) fs[b] = make_int4(bad ? FX_BAD : S[0], S[E - 1], max(exp_above(hk), S[0]), 0);
+  for (int e = 0; e < E; ++e) S[e] = max(above(h[e]), FX_EMIN);
+  if (lane == 0) fs[b] = make_int4(bad ? FX_BAD : S[0], S[E - 1], max(above(hk), S[0]), 0);
   for (int o = lane; o < E * p; o += 32) {
-    const double2 v = ld(o);
-    const int e = E == 1 || o < p ? 0 : 1;
-    longlong2 r;
-    r.x = bad ? 0 : __double2ll_rn(v.x * f1[e] * f2[e]);
-    r.y = bad ? 0 : __double2ll_rn(v.y * f1[e] * f2[e]);
+    const int Se = E == 1 || o < p ? S[0] : S[E - 1];
+    longlong2 r = make_longlong2(0, 0);
+    if (!bad && DF) {
+      const float4 v = mf[o];
+      r.x = float_fix(v.x, Se) + float_fix(v.y, Se);
+      r.y = float_fix(v.z, Se) + float_fix(v.w, Se);
+    } else if (!bad) {
+      const double2 v = md[o];
+      // 2^(61 - S) as two factors (S from -900 to 1024)
+      const int e1 = (61 - Se) >> 1, e2 = 61 - Se - e1;
+      const double f1 = __hiloint2double((1023 + e1) << 20, 0), f2 = __hiloint2double((1023 + e2) << 20, 0);
+      r.x = __double2ll_rn(v.x * f1 * f2);
+      r.y = __double2ll_rn(v.y * f1 * f2);
+    }
     fx[b * n + o] = r;
   }
 }
@@ -180,9 +206,9 @@ __global__ void __launch_bounds__(128) k_m2l_fix(int first, int nb, int p, const
 // (x c + y d) 2^-q for |x|, |y| < 2^61 and small integers (|c| + |d| < 2^10), q >= 1 such
 // that the result stays below 2^62: the operands in 31-bit parts
 __device__ __forceinline__ long long small_mul(long long x, int c, long long y, int d, int q) {
-  const long long mask = (1ll << 31) - 1;
-  const long long h = (long long)(int)(x >> 31) * c + (long long)(int)(y >> 31) * d;
-  const long long l = (long long)(int)(x & mask) * c + (long long)(int)(y & mask) * d;
+  const int mask = 0x7fffffff;
+  const long long h = madw((int)(x >> 31), c, madw((int)(y >> 31), d, 0));
+  const long long l = madw((int)x & mask, c, madw((int)y & mask, d, 0));
   return q <= 31 ? shl31(h, 31 - q) + sra31(l, q) : (h + (l >> 31)) >> min(q - 31, 63);
 }
 
@@ -234,17 +260,18 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
   __shared__ __align__(8) unsigned long long mbar[2];
   __shared__ uint32_t s_taddr;
   __shared__ int sv_src[2][NE], sv_code[2][NE], sv_pd[2][NE], sv_box[2][NE], sv_exp[2][E][NE];
-  __shared__ int sv_e0[2][FX_GROUP + 1], sv_E[2][E][FX_GROUP];
+  __shared__ int sv_e0[2][FX_GROUP + 1], sv_E[2][E][FX_GROUP], sv_cnt[2][FX_GROUP], s_pdv[EB_NCODE];
   __shared__ int s_fail, s_lock;
   const int team = threadIdx.x / FX_TEAM, tid = threadIdx.x - team * FX_TEAM, warp = tid >> 5, lane = tid & 31;
   int *s_src = sv_src[team], *s_code = sv_code[team], *s_pd = sv_pd[team], *s_box = sv_box[team];
-  int *s_e0 = sv_e0[team], (*s_exp)[NE] = sv_exp[team], (*s_E)[FX_GROUP] = sv_E[team];
+  int *s_cnt = sv_cnt[team], *s_e0 = sv_e0[team], (*s_exp)[NE] = sv_exp[team], (*s_E)[FX_GROUP] = sv_E[team];
   unsigned char* sB = sm;                                                   // [digit][48 x 48]
   unsigned char* sA = sm + FX_ND * FX_B + (size_t)team * FX_ND * FX_A;      // [digit][128 x 48], then
   long long* sC = reinterpret_cast<long long*>(sA);                         // the contributions
   const int ldl = p + 1, ldt = p + 2;
   const int4* tabp = tab + (size_t)EB_NCODE * ldt;  // (-1)^m (2/d)^m
   for (int i = threadIdx.x; i < FX_ND * FX_B / 16; i += FX_THREADS) reinterpret_cast<uint4*>(sB)[i] = bdig[i];
+  for (int i = threadIdx.x; i < EB_NCODE; i += FX_THREADS) s_pdv[i] = pdv[i];
   if (threadIdx.x == 0) {
     s_fail = 0;
     s_lock = 0;
@@ -268,87 +295,89 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
   const int nitem = nsingle + (ntarget - nsingle + group - 1) / group, step = 2 * gridDim.x;
   auto item_box = [&](int g) { return g < nsingle ? g : min(ntarget, nsingle + (g - nsingle) * group); };
   for (int g = team * gridDim.x + blockIdx.x; g < nitem; g += step) {
-    const int gb1 = item_box(g + 1);
-    int b0 = item_box(g);
+    const int gb0 = item_box(g), gb1 = item_box(g + 1);
+    if (tid < gb1 - gb0) s_cnt[tid] = vcount[first + gb0 + tid];
+    team_sync(team);
+    int b0 = gb0;
     while (b0 < gb1) {
-      // a round: the next boxes of the group whose entries fit (a box has at most 27)
-      int b1 = b0, ne = 0;
+      // a round: the next boxes of the item whose entries fit (a box has at most 27)
+      int b1 = b0, ne = 0, mine = -1, mine0 = 0;
       while (b1 < gb1) {
-        const int c = vcount[first + b1];
+        const int c = s_cnt[b1 - gb0];
         if (ne + c > NE) break;
         if (tid == 0) s_e0[b1 - b0] = ne;
-        if (tid < c) {
-          const size_t at = (size_t)(first + b1) * EB_VMAX + tid;
-          const int code = vcode[at];
-          s_src[ne + tid] = vlist[at];
-          s_code[ne + tid] = code;
-          s_pd[ne + tid] = pdv[code];
-          s_box[ne + tid] = b1 - b0;
+        if (tid >= ne && tid < ne + c) {
+          mine = b1;
+          mine0 = ne;
         }
         ne += c;
         ++b1;
       }
       const int nbx = b1 - b0;
       if (tid == 0) s_e0[nbx] = ne;
+      if (mine >= 0) {
+        const size_t at = (size_t)(first + mine) * EB_VMAX + tid - mine0;
+        const int code = vcode[at];
+        s_src[tid] = vlist[at];
+        s_code[tid] = code;
+        s_pd[tid] = s_pdv[code];
+        s_box[tid] = mine - b0;
+      }
       team_sync(team);
       if (ne > 0) {
-        // the digits of a: a warp per entry, two columns per lane (the rows of entries beyond
-        // ne hold anything: a row's products stay in its row)
-        for (int en = warp; en < ne; en += NW) {
+        // the digits of a: a warp per entry and expansion, two columns per lane (the rows of
+        // entries beyond ne hold anything: a row's products stay in its row)
+        for (int it = warp; it < E * ne; it += NW) {
+          const int en = E == 2 ? it >> 1 : it, e = E == 2 ? it & 1 : 0;
           const int kk = 2 * lane;  // columns kk, kk + 1: orders k = kk + 1, kk + 2
-          const int code = s_code[en], pd = s_pd[en];
-          const longlong2* ms = fx + (size_t)s_src[en] * E * p;
-          const int4 S = fs[s_src[en]];
-          const int4* tb = tab + (size_t)code * ldt;
-          const int dx = code % 7 - 3, dy = code / 7 - 3;
-          longlong2 ph[2], ps[2];
+          const int code = s_code[en], pd = s_pd[en], src = s_src[en];
+          const longlong2* ms = fx + (size_t)src * E * p + kk;
+          const int4 S = fs[src];
+          const int4* tb = tab + (size_t)code * ldt + kk + 1;
+          longlong2 y[2];
           int4 t[2];
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
             const bool in = kk + q < pd;
-            ph[q] = in ? ms[kk + q] : make_longlong2(0, 0);
-            if (E == 2) ps[q] = in ? ms[p + kk + q] : make_longlong2(0, 0);
-            t[q] = in ? tb[kk + q + 1] : make_int4(0, 0, 0, 0);
+            y[q] = in ? ms[q + e * p] : make_longlong2(0, 0);
+            t[q] = in ? tb[q] : make_int4(0, 0, 0, 0);
           }
-          long long a[2 * E][2];
-          longlong2 before;  // phi of the column before kk
-          before.x = __shfl_up_sync(0xffffffffu, ph[1].x, 1);
-          before.y = __shfl_up_sync(0xffffffffu, ph[1].y, 1);
-          // psi moved to the target centre, 61 bits below 2^Sp: |psi'| <= |psi| + |d|_1 k |phi_k|
-          const int lg = 32 - __clz(abs(dx) + abs(dy));
-          const int Sp = E == 2 ? max(S.y, S.z + lg) + 1 : 0, q_phi = Sp - S.x, q_psi = min(Sp - S.y, 63);
+          int ex = S.x;
+          if (e) {
+            // psi moved to the target centre: psi -= conj(d) (k - 1) phi of the order before
+            // (none before the first), 61 bits below 2^ex: |psi'| <= |psi| + |d|_1 k |phi_k|
+            const int dx = code % 7 - 3, dy = code / 7 - 3;
+            ex = max(S.y, S.z + 32 - __clz(abs(dx) + abs(dy))) + 1;
+            const int q_phi = ex - S.x, q_psi = min(ex - S.y, 63);
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const Limb xr = limbs(ph[q].x), xi = limbs(ph[q].y);
-            a[0][q] = mul_add_hi(xr, t[q].x, t[q].y, xi, -t[q].z, -t[q].w);
-            a[1][q] = mul_add_hi(xr, t[q].z, t[q].w, xi, t[q].x, t[q].y);
-            if (E == 2) {
-              // psi -= conj(d) (k - 1) phi of the order before (none before the first)
-              const longlong2 pb = q == 0 ? before : ph[0];
+            for (int q = 0; q < 2; ++q) {
+              const longlong2 pb = kk + q >= 1 && kk + q < pd ? ms[q - 1] : make_longlong2(0, 0);
               const int dxf = dx * (kk + q), dyf = dy * (kk + q);
-              const Limb yr = limbs((ps[q].x >> q_psi) - small_mul(pb.x, dxf, pb.y, dyf, q_phi));
-              const Limb yi = limbs((ps[q].y >> q_psi) - small_mul(pb.y, dxf, pb.x, -dyf, q_phi));
-              a[2 * E - 2][q] = mul_add_hi(yr, t[q].x, t[q].y, yi, -t[q].z, -t[q].w);
-              a[2 * E - 1][q] = mul_add_hi(yr, t[q].z, t[q].w, yi, t[q].x, t[q].y);
+              y[q].x = (y[q].x >> q_psi) - small_mul(pb.x, dxf, pb.y, dyf, q_phi);
+              y[q].y = (y[q].y >> q_psi) - small_mul(pb.y, dxf, pb.x, -dyf, q_phi);
             }
           }
+          long long a[2][2];
+          uint32_t mx = 0;
 #pragma unroll
-          for (int e = 0; e < E; ++e) {
-            const uint32_t m = max(max(hi_abs(a[2 * e][0]), hi_abs(a[2 * e][1])),
-                                   max(hi_abs(a[2 * e + 1][0]), hi_abs(a[2 * e + 1][1])));
-            // |a| < 2^(64 - clz): brought below 2^53, or halved where it is far below the
-            // box's scale (its last bits are those of the product then)
-            const int r = max(11 - __clz(__reduce_max_sync(0xffffffffu, m)), 1);
-            // a is this integer times 2^(S - 59) (the product kept 2^-2 of it), times 2^r
-            if (lane == 0) s_exp[e][en] = S.x == FX_BAD ? FX_BAD : (e ? Sp : S.x) - 59 + r;
-            if (kk < EB_FX_K) {
-              const long long bias = (BIAS << r) + (1ll << (r - 1));
+          for (int q = 0; q < 2; ++q) {
+            const Limb yr = limbs(y[q].x), yi = limbs(y[q].y);
+            a[0][q] = mul_add_hi(yr, t[q].x, t[q].y, yi, -t[q].z, -t[q].w);
+            a[1][q] = mul_add_hi(yr, t[q].z, t[q].w, yi, t[q].x, t[q].y);
+            mx = max(mx, max(hi_abs(a[0][q]), hi_abs(a[1][q])));
+          }
+          // |a| < 2^(64 - clz): brought below 2^53, or halved where it is far below the
+          // box's scale (its last bits are those of the product then)
+          const int r = max(11 - __clz(__reduce_max_sync(0xffffffffu, mx)), 1);
+          // a is this integer times 2^(ex - 59) (the product kept 2^-2 of it), times 2^r
+          if (lane == 0) s_exp[e][en] = S.x == FX_BAD ? FX_BAD : ex - 59 + r;
+          if (kk < EB_FX_K) {
+            const long long bias = (BIAS << r) + (1ll << (r - 1));
 #pragma unroll
-              for (int c = 2 * e; c < 2 * e + 2; ++c) {
-                const int row = 2 * E * en + c;
-                store_digits(sA + ((row >> 3) * FX_KCH + (kk >> 3)) * 128 + (row & 7) * 16 + (kk & 7) * 2, a[c][0],
-                             a[c][1], r, bias);
-              }
+            for (int c = 0; c < 2; ++c) {
+              const int row = 2 * E * en + 2 * e + c;
+              store_digits(sA + ((row >> 3) * FX_KCH + (kk >> 3)) * 128 + (row & 7) * 16 + (kk & 7) * 2, a[c][0],
+                           a[c][1], r, bias);
             }
           }
         }
@@ -399,8 +428,8 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
         const bool fail = *(volatile int*)&s_fail;
         asm volatile("tcgen05.fence::after_thread_sync;");
         // b_m out of the tensor memory, as integers: a warp reads the 32 rows of its quarter,
-        // half of the orders. The team then gives the tensor memory back.
-        constexpr int MH = EB_FX_K / 2;
+        // a part of the orders. The team then gives the tensor memory back.
+        constexpr int MH = EB_FX_K / (NW / 4);
         const int row = (warp & 3) * 32 + lane, mlo = (warp >> 2) * MH;
         if (!fail) {
           for (int m0 = mlo; m0 < mlo + MH; m0 += 4) {
@@ -417,8 +446,8 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
 #pragma unroll
               for (int d = 0; d < FX_NACC; ++d) w[d] = __float2int_rn(__uint_as_float(v[d][q]));
               // sum of w_d 2^(42 - 9 d), below 2^62 (no row of the matrix sums to 8)
-              const long long top = (long long)w[0] * (1 << 18) + ((long long)w[1] * (1 << 9) + w[2]);
-              const long long low = (long long)w[3] * (1 << 15) + ((long long)w[4] * 64 + ((w[5] >> 3) + (w[6] >> 12)));
+              const long long top = madw(w[0], 1 << 18, madw(w[1], 1 << 9, w[2]));
+              const long long low = madw(w[3], 1 << 15, madw(w[4], 64, (w[5] >> 3) + (w[6] >> 12)));
               sC[(m0 + q) * FX_PITCH + row] = shl31(top, 24) + low;
             }
           }
@@ -428,7 +457,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
         if (tid == 0) atomicExch(&s_lock, 0);
         if (fail) break;
         // contributions (-1)^m (2/d)^m b_m of the entries to their boxes, in place: a thread
-        // per row and half of the orders reads both parts before either is replaced
+        // per row and part of the orders reads both parts before either is replaced
         {
           const int en = row / (2 * E), e = E == 2 ? (row >> 1) & 1 : 0;
           const bool im = row & 1, act = en < ne;
@@ -507,8 +536,8 @@ int fx_launch(eb_ctx* ctx, int first, int ntarget, int nsrc, int ncoarse, const 
   const int nsingle = std::min(ncoarse, ntarget);
   const int nitem = nsingle + (ntarget - nsingle + group - 1) / group;
   const int grid = std::min((nitem + 1) / 2, ctx->nsm);
-  k_m2l_fx<E, DF><<<grid, FX_THREADS, sm, st>>>(first, ntarget, vlist, vcode, vcount, p, tb.fxb.as<uint4>(),
-                                               tb.fxt.as<int4>(), tb.fxr.as<int>(), tb.pd.as<int>(), fx, fs, local,
+  k_m2l_fx<E, DF><<<grid, FX_THREADS, sm, st>>>(first, ntarget, vlist, vcode, vcount, p, reinterpret_cast<const uint4*>(tb.fxb),
+                                               tb.fxt.as<int4>(), reinterpret_cast<const int*>(tb.fxr), tb.pd.as<int>(), fx, fs, local,
                                                accumulate, nsingle, group);
   ctx->launches += 2;
   return EB_OK;
@@ -615,11 +644,15 @@ int eb_m2l_fx_tables(EbTables& tb) {
   const std::vector<unsigned short>& dig = T.dig;
   const std::vector<int>& rsc = T.rsc;
   const std::vector<int4>& t = T.t;
-  EB_TRY(tb.fxb.ensure(dig.size() * 2));
-  EB_TRY(tb.fxr.ensure(rsc.size() * sizeof(int)));
-  EB_TRY(tb.fxt.ensure(t.size() * sizeof(int4)));
-  EB_CUDA_TRY(cudaMemcpy(tb.fxb.p, dig.data(), dig.size() * 2, cudaMemcpyHostToDevice));
-  EB_CUDA_TRY(cudaMemcpy(tb.fxr.p, rsc.data(), rsc.size() * sizeof(int), cudaMemcpyHostToDevice));
-  EB_CUDA_TRY(cudaMemcpy(tb.fxt.p, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  // one buffer and one copy: the powers, the digits, the row scalings (16-byte aligned)
+  const size_t nt = t.size() * sizeof(int4), nd = dig.size() * 2, nr = rsc.size() * sizeof(int);
+  std::vector<char> all(nt + nd + nr);
+  memcpy(all.data(), t.data(), nt);
+  memcpy(all.data() + nt, dig.data(), nd);
+  memcpy(all.data() + nt + nd, rsc.data(), nr);
+  EB_TRY(tb.fxt.ensure(all.size()));
+  tb.fxb = tb.fxt.as<char>() + nt;
+  tb.fxr = tb.fxt.as<char>() + nt + nd;
+  EB_CUDA_TRY(cudaMemcpy(tb.fxt.p, all.data(), all.size(), cudaMemcpyHostToDevice));
   return EB_OK;
 }

@@ -705,7 +705,7 @@ void DevBuf::release() {
 // leaf units, with both subtractions carried exactly (two-sum, two-product), so that
 // for two nodes the offsets differ by exactly (z_j - z_i)/r minus the integer index
 // offset of their leaves, up to the final rounding (about 2^-53 of a leaf side).
-__device__ __forceinline__ double leaf_offset(double z, double x0, unsigned int i, double r) {
+__device__ __forceinline__ double leaf_offset(double z, double x0, unsigned int i, double r, double rinv) {
   double s = __dsub_rn(z, x0);
   double bb = __dsub_rn(s, z);
   double e1 = __dadd_rn(__dsub_rn(z, __dsub_rn(s, bb)), __dsub_rn(-x0, bb));
@@ -715,7 +715,7 @@ __device__ __forceinline__ double leaf_offset(double z, double x0, unsigned int 
   double u = __dsub_rn(s, c);
   double bb2 = __dsub_rn(u, s);
   double e3 = __dadd_rn(__dsub_rn(s, __dsub_rn(u, bb2)), __dsub_rn(-c, bb2));
-  return __ddiv_rn(__dadd_rn(u, __dadd_rn(__dsub_rn(e1, e2), e3)), r);
+  return __dmul_rn(__dadd_rn(u, __dadd_rn(__dsub_rn(e1, e2), e3)), rinv);
 }
 
 // Leaf-relative node coordinates as three floats hi + mid + lo (all 53 bits of the
@@ -731,16 +731,20 @@ __device__ __forceinline__ void split3(double w, float& hi, float& mid, float& l
 __global__ void k_leaf_coords(const int* __restrict__ leaves, const unsigned long long* __restrict__ bkey,
                               const unsigned char* __restrict__ blev, const int* __restrict__ pt0,
                               const int* __restrict__ pt1, const double2* __restrict__ zs, double x0, double y0,
-                              double W, float4* __restrict__ wa, float2* __restrict__ wb) {
+                              double W, double winv, float4* __restrict__ wa, float2* __restrict__ wb) {
   const int b = leaves[blockIdx.x];
   const unsigned long long k = bkey[b];
   const unsigned int ix = compact2(k), iy = compact2(k >> 1);
-  const double r = ldexp(W, -(int)blev[b]);  // W / 2^level, exact
+  // W / 2^level, exact, and its reciprocal: every offset of the tree carries the same relative
+  // rounding of 1 / W (a change of unit), and an FP64 division is some twenty instructions on
+  // a pipe of two lanes a cycle
+  const double r = W * __hiloint2double((1023 - (int)blev[b]) << 20, 0);
+  const double rinv = winv * __hiloint2double((1023 + (int)blev[b]) << 20, 0);
   for (int i = pt0[b] + threadIdx.x; i < pt1[b]; i += blockDim.x) {
     double2 z = zs[i];
     float xh, xm, xl, yh, ym, yl;
-    split3(leaf_offset(z.x, x0, ix, r), xh, xm, xl);
-    split3(leaf_offset(z.y, y0, iy, r), yh, ym, yl);
+    split3(leaf_offset(z.x, x0, ix, r, rinv), xh, xm, xl);
+    split3(leaf_offset(z.y, y0, iy, r, rinv), yh, ym, yl);
     wa[i] = make_float4(xh, yh, xm, ym);
     wb[i] = make_float2(xl, yl);
   }
@@ -1079,7 +1083,7 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
   EB_TRY(t.wdf_lo.ensure(sizeof(float2) * (size_t)n));
   k_leaf_coords<<<nl, 64, 0, st>>>(t.leaves.as<int>(), t.bkey.as<unsigned long long>(), t.blev.as<unsigned char>(),
                                    t.pt0.as<int>(), t.pt1.as<int>(), t.zs.as<double2>(), t.x0, t.y0, t.W,
-                                   t.wdf.as<float4>(), t.wdf_lo.as<float2>());
+                                   1.0 / t.W, t.wdf.as<float4>(), t.wdf_lo.as<float2>());
   eb_count_launch(ctx);
   EB_TRY(eb_check_launch(ctx, "tree build"));
   t.valid = true;
