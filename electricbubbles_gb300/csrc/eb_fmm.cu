@@ -23,7 +23,11 @@
 #include <algorithm>
 #include <cmath>
 #include <functional>
+#include <type_traits>
+#include <utility>
 #include <vector>
+
+#include <cuda_pipeline.h>
 
 #include "eb_df.cuh"
 #include "eb_internal.h"
@@ -708,79 +712,333 @@ __global__ void __launch_bounds__(128) k_m2l(int first, const int* __restrict__ 
   }
 }
 
-// The FP32 M2L for the default order P (20): lane m <= P owns output order m of both
-// expansions. Its binomial column C(m+k-1, m) stays in registers, the warp's entries are
-// accumulated in registers, the loops over k run to P with a_k = 0 beyond the entry's
-// truncation order pd, and outputs m > pd are skipped, so each entry gives exactly the
-// sums of k_m2l (same terms, same order).
+// Two floats in a register pair: one issue slot for two multiply-adds (the rate of the
+// multiply-adds themselves is the same, 64 pairs or 128 lanes a cycle and SM)
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk2(float x, float y) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 upk2(f32x2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// The FP32 M2L for the default order P (20) on few boxes: a block per box, its four warps
+// with a quarter of the list each. An entry's multipoles and powers d^-j come by
+// asynchronous copies (all in flight at once), a_k takes the multipoles' place with a lane
+// per coefficient, and then lane m <= P owns output order m of both expansions: its binomial
+// column C(m+k-1, m) stays in registers (as pairs: a complex term is one packed
+// multiply-add), two entries at a time, and the loop over k stops at the first multiple of 4
+// past their truncation orders pd (a_k = 0 beyond an entry's own).
+// The longest list decides: a warp alone issues an instruction every four cycles, and the
+// 27 entries of a coarse level's box took one warp 11.5 us. At 64 x 512 (13,290 entries): 10.0 -> 8.9 us.
+constexpr int M2L32_CTAS = 5;  // blocks per SM
+
 template <int E, int P>
-__global__ void __launch_bounds__(128) k_m2l_f32p(int first, const int* __restrict__ vlist,
+__global__ void __launch_bounds__(128, M2L32_CTAS) k_m2l_f32w(int first, int nt, const int* __restrict__ vlist,
                                                   const unsigned char* __restrict__ vcode,
                                                   const int* __restrict__ vcount,
-                                                  const float* __restrict__ binom, int ldb,
+                                                  const float* __restrict__ bt,
                                                   const float2* __restrict__ dinv,
                                                   const int* __restrict__ pdv,
                                                   const float2* __restrict__ mpole,
                                                   float2* __restrict__ local, int accumulate) {
   constexpr int ldl = P + 1, ldd = P + 2;
-  __shared__ float2 sa[4][E][P];
-  __shared__ float2 sred[4][E][ldl];
+  constexpr int CM = E * P / 2, CD = ldd / 2, CPE = CM + CD;  // 16-byte pieces of an entry
+  static_assert(P % 4 == 0 && P <= 31 && EB_VMAX <= 32, "whole chunks, a lane per order and entry");
+  constexpr int WPB = 4, NE = (EB_VMAX + WPB - 1) / WPB;
+  __shared__ float4 sa[WPB][NE * CPE];  // per entry [e][k] M_k, then a_k; d^-j
+  __shared__ float2 sred[WPB][E][ldl];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gid = first + blockIdx.x;
-  const int nv = vcount[gid];
-  const int m = lane <= P ? lane : P;
-  float c2[P];
+  const int m = min(lane, P);
+  f32x2 c2[P];
 #pragma unroll
-  for (int k = 1; k <= P; ++k) c2[k - 1] = binom[(size_t)(m + k - 1) * ldb + m];
-  float2 acc[E];
+  for (int k = 0; k < P; ++k) {
+    const float c = bt[k * ldl + m];
+    c2[k] = pk2(c, c);
+  }
+  const float sgn = (m & 1) ? -1.f : 1.f;
+  float4* buf = sa[w];
+  float2* buf2 = reinterpret_cast<float2*>(buf);
+  for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+    const int gid = first + t;
+    const int nv = vcount[gid];
+    // this warp's entries
+    const int per = (nv + WPB - 1) / WPB, e0 = min(nv, w * per), ne = min(nv, e0 + per) - e0;
+    int lsrc = 0, lcode = 0, lpd = 0;
+    if (lane < ne) {
+      lsrc = vlist[(size_t)gid * EB_VMAX + e0 + lane];
+      lcode = vcode[(size_t)gid * EB_VMAX + e0 + lane];
+      lpd = pdv[lcode];
+    }
+    float2 acc[E];
 #pragma unroll
-  for (int e = 0; e < E; ++e) acc[e] = make_float2(0.f, 0.f);
-  for (int j = w; j < nv; j += 4) {
-    const int src = vlist[(size_t)gid * EB_VMAX + j];
-    const int code = vcode[(size_t)gid * EB_VMAX + j];
-    const int pd = pdv[code];
-    const float2* dv = dinv + (size_t)code * ldd;
-    const float2* ms = mpole + (size_t)src * E * P;
-    if (lane < P) {
-      const int kk = lane, k = kk + 1;
-      float2 v0 = make_float2(0.f, 0.f), v1 = v0;
-      if (kk < pd) {
-        const float2 sc = dv[k];
-        v0 = cmul<float>(ms[kk], sc);
-        if (E == 2) {
-          float2 mpsi = ms[P + kk];
-          const float dxr = (float)(code % 7 - 3), dyr = (float)(code / 7 - 3);
-          if (k >= 2) cfma<float>(mpsi, make_float2(-dxr * (float)(k - 1), dyr * (float)(k - 1)), ms[kk - 1]);
-          v1 = cmul<float>(mpsi, sc);
+    for (int e = 0; e < E; ++e) acc[e] = make_float2(0.f, 0.f);
+    if (ne > 0) {
+      for (int c0 = 0; c0 < ne * CPE; c0 += 32) {
+        const int c = c0 + lane, j = min(c / CPE, ne - 1), x = c - j * CPE;
+        const int src = __shfl_sync(0xffffffffu, lsrc, j), code = __shfl_sync(0xffffffffu, lcode, j);
+        const float4* g = x < CM ? reinterpret_cast<const float4*>(mpole) + (size_t)src * CM + x
+                                 : reinterpret_cast<const float4*>(dinv) + code * CD + (x - CM);
+        if (c < ne * CPE) __pipeline_memcpy_async(buf + c, g, 16);
+      }
+      __pipeline_commit();
+      __pipeline_wait_prior(0);
+      __syncwarp();
+      // a_k in place, from the last coefficient to the first: psi's shift reads phi_(k-1)
+      for (int c0 = (ne * P - 1) & ~31; c0 >= 0; c0 -= 32) {
+        const int c = c0 + lane, j = min(c / P, ne - 1), kk = c - j * P;
+        const int code = __shfl_sync(0xffffffffu, lcode, j), pd = __shfl_sync(0xffffffffu, lpd, j);
+        const bool act = c < ne * P;
+        float2* mj = buf2 + j * 2 * CPE + kk;
+        float2 v0 = make_float2(0.f, 0.f), v1 = v0;
+        if (act && kk < pd) {
+          const float2 sc = mj[E * P + 1];
+          v0 = cmul<float>(mj[0], sc);
+          if (E == 2) {  // psi moved to the target's centre
+            float2 ps = mj[P];
+            const float f = (float)kk;
+            const float dxr = (float)(code % 7 - 3) * f, dyr = (float)(code / 7 - 3) * f;
+            if (kk > 0) cfma<float>(ps, make_float2(-dxr, dyr), mj[-1]);
+            v1 = cmul<float>(ps, sc);
+          }
+        }
+        __syncwarp();
+        if (act) {
+          mj[0] = v0;
+          if (E == 2) mj[P] = v1;
+        }
+        __syncwarp();
+      }
+      for (int j = 0; j < ne; j += 2) {
+        const int j1 = min(j + 1, ne - 1);
+        const int pd0 = __shfl_sync(0xffffffffu, lpd, j), pd1 = __shfl_sync(0xffffffffu, lpd, j1);
+        const int pdm = __reduce_max_sync(0xffffffffu, max(pd0, pd1));  // (in a uniform register)
+        const float4 *b0 = buf + j * CPE, *b1 = buf + j1 * CPE;
+        const float2 po0 = cscale<float>(reinterpret_cast<const float2*>(b0 + CM)[m], lane <= pd0 ? sgn : 0.f);
+        const float2 po1 = cscale<float>(reinterpret_cast<const float2*>(b1 + CM)[m], lane <= pd1 && j1 > j ? sgn : 0.f);
+        const ulonglong2 *av = reinterpret_cast<const ulonglong2*>(b0), *bv = reinterpret_cast<const ulonglong2*>(b1);
+        f32x2 b[E][2];
+#pragma unroll
+        for (int e = 0; e < E; ++e) b[e][0] = b[e][1] = 0;
+#pragma unroll
+        for (int k0 = 0; k0 < P; k0 += 4) {
+          if (k0 < pdm) {
+#pragma unroll
+            for (int k = k0; k < k0 + 4; k += 2) {
+#pragma unroll
+              for (int e = 0; e < E; ++e) {
+                const ulonglong2 a0 = av[(e * P + k) / 2], a1 = bv[(e * P + k) / 2];
+                b[e][0] = fma2(c2[k], a0.x, b[e][0]);
+                b[e][1] = fma2(c2[k], a1.x, b[e][1]);
+                b[e][0] = fma2(c2[k + 1], a0.y, b[e][0]);
+                b[e][1] = fma2(c2[k + 1], a1.y, b[e][1]);
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          cfma<float>(acc[e], po0, upk2(b[e][0]));
+          cfma<float>(acc[e], po1, upk2(b[e][1]));
         }
       }
-      sa[w][0][kk] = v0;
-      if (E == 2) sa[w][1][kk] = v1;
     }
+    if (lane <= P) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) sred[w][e][lane] = acc[e];
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < E * ldl; idx += 128) {
+      const int e = idx / ldl, mm = idx - e * ldl;
+      float2 v = sred[0][e][mm];
+#pragma unroll
+      for (int q = 1; q < WPB; ++q) v = cadd<float>(v, sred[q][e][mm]);
+      float2* lc = local + (size_t)gid * E * ldl + idx;
+      if (accumulate) v = cadd<float>(*lc, v);
+      *lc = v;
+    }
+    __syncthreads();
+  }
+}
+
+// The FP32 M2L for the default order P (20) on many boxes: a lane per list entry. A warp takes as many
+// whole boxes as have 32 entries between them; the entries' multipoles come through shared
+// memory (asynchronous copies, all in flight at once), each lane scales its own to a_k in
+// registers and forms its 21 outputs of both expansions with the binomials C(m+k-1, m) as
+// immediate operands, and the entries of a box are added through shared memory in their
+// order. a_k = 0 beyond the entry's truncation order pd, outputs m > pd are left out.
+// With a lane per output order every a_k is a shared-memory broadcast, and a 16-byte one
+// costs four cycles of an SM however few addresses there are: two thirds of the lanes busy
+// and 68 to 80 of those cycles an entry, where this way an entry takes 98 warp instructions,
+// 60 of them multiply-adds. Measured (E = 2): 1,024 x 1,024 (497,412
+// entries) 287 -> 113 us.
+// Coarse levels' boxes, with up to 27 entries each, go one to a warp, the others nb to a
+// warp. From M2L32_WIDE boxes on: an apply of 256 x 512
+// (12,000 boxes) takes 125 against 134 us with a block per box, one of 64 x 1,024 (4,500)
+// 66.5 against 67.3 us and one of 64 x 512 (2,244) 45.6 against 40.2 us.
+constexpr int M2L32_WIDE = 8192;
+template <int P>
+struct M2lBinom {  // C(m+k, m) for k < P, m <= P: exact in double
+  __host__ __device__ static constexpr float at(int k, int m) {
+    double c = 1.0;
+    for (int i = 1; i <= m; ++i) c = c * (k + i) / i;
+    return (float)c;
+  }
+};
+template <typename F, int... I>
+__device__ __forceinline__ void static_for_impl(F&& f, std::integer_sequence<int, I...>) {
+  (f(std::integral_constant<int, I>()), ...);
+}
+template <int N, typename F>
+__device__ __forceinline__ void static_for(F&& f) {
+  static_for_impl(f, std::make_integer_sequence<int, N>());
+}
+
+constexpr int M2L32_WARPS = 4;
+template <int E, int P>
+struct M2l32Smem {
+  static constexpr int CM = E * P / 2;       // 16-byte pieces of a box's multipoles
+  static constexpr int PITCH = CM | 1;       // rows of an odd number of pieces: no bank conflicts
+  static constexpr int NOUT = E * (P + 1), CP = 33;
+  static constexpr int WARP = PITCH * 32 * 2 > NOUT * CP ? PITCH * 32 * 2 : (NOUT * CP + 1) & ~1;  // float2
+  float2 buf[M2L32_WARPS][WARP];             // the multipoles, then the outputs [NOUT][CP]
+  float2 d[(P + 2) * EB_NCODE];              // d^-j at [j][code]
+};
+
+template <int E, int P>
+__global__ void __launch_bounds__(32 * M2L32_WARPS, 4)
+    k_m2l_f32p(int first, int nt, int ncoarse, int nb, const int* __restrict__ vlist,
+               const unsigned char* __restrict__ vcode, const int* __restrict__ vcount,
+               const float2* __restrict__ dinv, const int* __restrict__ pdv, const float2* __restrict__ mpole,
+               float2* __restrict__ local, int accumulate) {
+  typedef M2l32Smem<E, P> Smem;
+  constexpr int ldd = P + 2, CM = Smem::CM, PITCH = Smem::PITCH, NOUT = Smem::NOUT, CP = Smem::CP;
+  static_assert(EB_VMAX <= 32 && (E * P) % 2 == 0, "a box's entries fit a warp");
+  extern __shared__ float4 sm4[];
+  Smem& S = *reinterpret_cast<Smem*>(sm4);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < EB_NCODE * ldd; i += 32 * M2L32_WARPS)
+    S.d[(i % ldd) * EB_NCODE + i / ldd] = dinv[i];
+  __syncthreads();
+  float2* buf = S.buf[w];
+  const int wid = blockIdx.x * M2L32_WARPS + w;
+  const int t0 = wid < ncoarse ? wid : ncoarse + (wid - ncoarse) * nb;
+  const int n = wid < ncoarse ? 1 : min(nb, nt - t0);  // this warp's boxes, at most 32
+  if (n <= 0) return;
+  const int cnt = lane < n ? vcount[first + t0 + lane] : 0;
+  int end = cnt;  // of the lane's box in the warp's entries
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= o) end += y;
+  }
+  for (int s = 0; s < n;) {
+    const int base = __shfl_sync(0xffffffffu, end - cnt, s);
+    const int e = s + __popc(__ballot_sync(0xffffffffu, lane >= s && lane < n && end - base <= 32));
+    const int ne = __shfl_sync(0xffffffffu, end, e - 1) - base;
+    // the lane's entry
+    int bx = s, o0 = 0;
+    for (int b = s; b < e; ++b) {
+      const int o = __shfl_sync(0xffffffffu, end - cnt, b) - base;
+      if (lane >= o) {
+        bx = b;
+        o0 = o;
+      }
+    }
+    int src = 0, code = 0, pd = -1;
+    if (lane < ne) {
+      const size_t x = (size_t)(first + t0 + bx) * EB_VMAX + (lane - o0);
+      src = vlist[x];
+      code = vcode[x];
+      pd = pdv[code];
+    }
+    for (int c0 = 0; c0 < ne * CM; c0 += 32) {
+      const int c = c0 + lane, j = min(c / CM, ne - 1), x = c - j * CM;
+      const int sj = __shfl_sync(0xffffffffu, src, j);
+      if (c < ne * CM)
+        __pipeline_memcpy_async(reinterpret_cast<float4*>(buf) + j * PITCH + x,
+                                reinterpret_cast<const float4*>(mpole) + (size_t)sj * CM + x, 16);
+    }
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
     __syncwarp();
-    if (lane <= pd) {
-      float2 post = dv[m];
-      if (m & 1) post = make_float2(-post.x, -post.y);
+    float2 a[E][P];
+    {
+      const float4* row = reinterpret_cast<const float4*>(buf) + (lane < ne ? lane : 0) * PITCH;
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        float2 b = make_float2(0.f, 0.f);
+      for (int x = 0; x < CM; ++x) {
+        const float4 v = row[x];
+        const int q = 2 * x;
+        a[q / P][q % P] = make_float2(v.x, v.y);
+        a[(q + 1) / P][(q + 1) % P] = make_float2(v.z, v.w);
+      }
+    }
+    const float dx = (float)(code % 7 - 3), dy = (float)(code / 7 - 3);
+    float2 below = make_float2(0.f, 0.f);  // phi's coefficient k - 1
 #pragma unroll
-        for (int k = 0; k < P; ++k) crfma<float>(b, c2[k], sa[w][e][k]);
-        cfma<float>(acc[e], post, b);
+    for (int k = 0; k < P; ++k) {
+      float2 sc = S.d[(k + 1) * EB_NCODE + code];
+      if (k >= pd) sc = make_float2(0.f, 0.f);
+      const float2 ph = a[0][k];
+      a[0][k] = cmul<float>(ph, sc);
+      if (E == 2) {  // psi moved to the target's centre
+        float2 ps = a[E - 1][k];
+        if (k > 0) cfma<float>(ps, make_float2(-dx * (float)k, dy * (float)k), below);
+        a[E - 1][k] = cmul<float>(ps, sc);
+        below = ph;
+      }
+    }
+    __syncwarp();  // the multipoles are consumed
+    static_for<P + 1>([&](auto mc) {
+      constexpr int m = decltype(mc)::value;
+      float2 b[E];
+#pragma unroll
+      for (int x = 0; x < E; ++x) b[x] = make_float2(0.f, 0.f);
+      static_for<P>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        constexpr float c = M2lBinom<P>::at(k, m);
+#pragma unroll
+        for (int x = 0; x < E; ++x) crfma<float>(b[x], c, a[x][k]);
+      });
+      float2 po = S.d[m * EB_NCODE + code];
+      if (m > pd) po = make_float2(0.f, 0.f);
+      if (m & 1) po = make_float2(-po.x, -po.y);
+#pragma unroll
+      for (int x = 0; x < E; ++x) buf[(x * (P + 1) + m) * CP + lane] = cmul<float>(po, b[x]);
+    });
+    __syncwarp();
+    for (int i0 = 0; i0 < (e - s) * NOUT; i0 += 32) {
+      const int i = i0 + lane, bi = min(i / NOUT, e - s - 1), o = i - bi * NOUT;
+      const int j1 = __shfl_sync(0xffffffffu, end, s + bi) - base, j0 = j1 - __shfl_sync(0xffffffffu, cnt, s + bi);
+      if (i < (e - s) * NOUT) {
+        float2 v = make_float2(0.f, 0.f);
+        for (int j = j0; j < j1; ++j) v = cadd<float>(v, buf[o * CP + j]);
+        float2* lc = local + (size_t)(first + t0 + s + bi) * NOUT + o;
+        if (accumulate) v = cadd<float>(*lc, v);
+        *lc = v;
       }
     }
     __syncwarp();
-  }
-  if (lane <= P) {
-#pragma unroll
-    for (int e = 0; e < E; ++e) sred[w][e][lane] = acc[e];
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < E * ldl; idx += blockDim.x) {
-    const int e = idx / ldl, mm = idx - e * ldl;
-    float2 v = cadd<float>(cadd<float>(sred[0][e][mm], sred[1][e][mm]), cadd<float>(sred[2][e][mm], sred[3][e][mm]));
-    if (accumulate) v = cadd<float>(local[(size_t)gid * E * ldl + idx], v);
-    local[(size_t)gid * E * ldl + idx] = v;
+    s = e;
   }
 }
 
@@ -1105,7 +1363,7 @@ __global__ void k_l2l_df(int offc, const unsigned long long* __restrict__ bkey,
 
 // ---------------------------------------------------------------------------------
 // FP32 multipoles of every box of the finest levels directly from its points, in
-// parallel over those levels (no dependent M2M chain): one block per chunk of at most
+// parallel over those levels (no dependent M2M chain): one warp per chunk of at most
 // EB_CHUNK points forms that chunk's contribution (the P2M sums of SLMKXP,
 // cadap2.f:412-468, scaled by the box side and relative to the box centre), and the
 // last chunk of a box to finish adds the chunks of the box in order. The offset of a point from an ancestor's centre in the
@@ -1118,100 +1376,222 @@ struct LevOff {
   float rinv[EB_KEY_LEVELS + 2];  // 1 / (box side) per level, rounded to float on the host
 };
 
+//
+// One warp per chunk, four to a block and without block-wide waits: a lane per point forms
+// the powers w^k of 32 points in shared memory (rows of an odd pitch: no bank conflicts),
+// then a lane per order sums the points, all three sums A, B, C from one read of a power.
+// With a block per chunk, a thread per sum and order, and half of the points each, a point
+// took 13 warp instructions and level, most of them addressing (E = 2, p = 20: 98 -> 72 us
+// for 524,288 nodes).
+constexpr int P2M_CW = 4;  // chunks of a block
+__host__ __device__ constexpr int p2m_pitch(int p) { return (p < 32 ? p : 32) | 1; }
+inline size_t p2m_smem(int p) { return P2M_CW * 32 * (sizeof(float2) * (p2m_pitch(p) + 1) + sizeof(float4)); }
+
+// A part of a box's sum is written: the warp that counts the last of nc adds them in order.
+__device__ __forceinline__ void p2m_finish(int lane, int nc, int nout, const float2* part, int* cdone, float2* mpole) {
+  __threadfence();
+  __syncwarp();
+  int done = 0;
+  if (lane == 0) done = atomicAdd(cdone, 1) == nc - 1;
+  if (!__shfl_sync(0xffffffffu, done, 0)) return;
+  __threadfence();
+  for (int o = lane; o < nout; o += 32) {
+    float2 acc = __ldcg(part + o);
+#pragma unroll 8
+    for (int q = 1; q < nc; ++q) acc = cadd<float>(acc, __ldcg(part + (size_t)q * nout + o));
+    mpole[o] = acc;
+  }
+  if (lane == 0) *cdone = 0;
+}
+
 template <int E>
-__global__ void __launch_bounds__(128) k_p2m_chunks(LevOff lo, int first2, const unsigned char* __restrict__ blev,
+__global__ void __launch_bounds__(32 * P2M_CW) k_p2m_chunks(LevOff lo, int nchunk, int first2,
+                                                    const unsigned char* __restrict__ blev,
                                                     const unsigned char* __restrict__ plev,
                                                     const int* __restrict__ chunk_box,
                                                     const int* __restrict__ cstart,
                                                     const unsigned long long* __restrict__ keys,
                                                     const int* __restrict__ pt0, const int* __restrict__ pt1,
                                                     const float4* __restrict__ wa, const float2* __restrict__ qa,
-                                                    const float2* __restrict__ qb, double W, int p,
+                                                    const float2* __restrict__ qb, int p,
                                                     float2* __restrict__ mpart, int* __restrict__ cdone,
                                                     float2* __restrict__ mpole) {
   // Sums per chunk: A_k = sum a w^k, B_k = sum b w^k, C_k = sum conj(w) a w^k (a, b the
   // scaled charges), multipole -A_k and -(B_k + k C_(k-1)).
-  constexpr int NA = E == 2 ? 3 : 1;
-  extern __shared__ float2 sm2[];
-  const int ps = p + 1, nacc = NA * p, nout = E * p;
-  float2* pw = sm2;                  // [EB_CHUNK][p + 1]: w^k per point
-  float2* sc = pw + EB_CHUNK * ps;   // [NA][EB_CHUNK]: a, b, conj(w) a per point
-  float2* red = sc + NA * EB_CHUNK;  // [2][nacc]: the sums over each half of the points
-  __shared__ int s_last;
-  const int c = blockIdx.x, tid = threadIdx.x;
+  extern __shared__ float4 sm4[];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c = blockIdx.x * P2M_CW + wid;
+  if (c >= nchunk) return;
+  const int pitch = p2m_pitch(p), nout = E * p;
+  float4* sab = sm4 + wid * 32;  // (a, b) per point
+  float2* scc = reinterpret_cast<float2*>(sm4 + P2M_CW * 32) + wid * 32 * (pitch + 1);  // conj(w) a per point
+  float2* pw = scc + 32;         // [32][pitch]: w^k per point
   const int b = chunk_box[c];
   const int l = blev[b];
   const float rinv = lo.rinv[l];
   const int bb = b - first2, c0 = cstart[bb], nc = cstart[bb + 1] - c0;
   const int i0 = pt0[b] + (c - c0) * EB_CHUNK;
   const int cnt = min(pt1[b], i0 + EB_CHUNK) - i0;
-  {
-    // two threads per point: even and odd powers
-    const int sp = tid >> 1, h = tid & 1;
-    if (sp < cnt) {
-      const int i = i0 + sp;
-      const int lam = plev[i], sh = lam - l;
-      const float f = __int_as_float((127 - sh) << 23);  // 2^-sh
-      const unsigned long long kl = keys[i] >> (2 * (EB_KEY_LEVELS - lam));
-      const unsigned int ix = compact2d(kl), iy = compact2d(kl >> 1);
-      const float4 wv = wa[i];
-      const float gx = fmaf((float)ix + 0.5f, f, -((float)(ix >> sh) + 0.5f));
-      const float gy = fmaf((float)iy + 0.5f, f, -((float)(iy >> sh) + 0.5f));
-      const float2 w = make_float2(fmaf(wv.x, f, gx), fmaf(wv.y, f, gy));
-      if (h == 0) {
-        const float2 ah = cscale<float>(qa[i], rinv);
-        sc[sp] = ah;
-        if (E == 2) {
-          sc[EB_CHUNK + sp] = cscale<float>(qb[i], rinv);
-          sc[2 * EB_CHUNK + sp] = cmul<float>(cconj<float>(w), ah);
-        }
-      }
-      const float2 w2 = cmul<float>(w, w);
-      float2 cur = h ? w : make_float2(1.f, 0.f);
-      float2* row = pw + sp * ps;
-      for (int j = h; j < p; j += 2) {
-        row[j] = cur;
-        cur = cmul<float>(cur, w2);
-      }
-    }
-  }
-  __syncthreads();
-  {
-    const int half = tid >> 6, s0 = half * 32, s1 = min(cnt, s0 + 32);
-    for (int o = tid & 63; o < nacc; o += 64) {
-      const int which = o / p, k = o - which * p;
-      const float2* scw = sc + which * EB_CHUNK;
-      float2 acc = make_float2(0.f, 0.f);
-      for (int s2 = s0; s2 < s1; ++s2) cfma<float>(acc, scw[s2], pw[s2 * ps + k]);
-      red[half * nacc + o] = acc;
-    }
-  }
-  __syncthreads();
   // a box of one chunk gets its multipole directly; otherwise the chunk's part goes to
   // mpart and the box's last chunk to finish adds the parts in chunk order
   float2* dst = nc == 1 ? mpole + (size_t)b * nout : mpart + (size_t)c * nout;
-  for (int o = tid; o < nout; o += 128) {
-    const int e = o / p, k = o - e * p;
-    float2 v = cadd<float>(red[o], red[nacc + o]);
-    if (E == 2 && e == 1 && k >= 1) {
-      const float2 cm = cadd<float>(red[2 * p + k - 1], red[nacc + 2 * p + k - 1]);
-      crfma<float>(v, (float)k, cm);
+  float2 last = make_float2(0.f, 0.f);  // C of the order below this round's
+  for (int k0 = 0; k0 < p; k0 += 32) {  // a lane per order
+    const int kw = min(32, p - k0), k = min(lane, kw - 1);
+    float2 A = make_float2(0.f, 0.f), B = A, C = A;
+    for (int s0 = 0; s0 < cnt; s0 += 32) {
+      const int ns = min(32, cnt - s0);
+      if (s0 > 0 || k0 > 0) __syncwarp();  // the previous points are consumed
+      if (lane < ns) {
+        const int i = i0 + s0 + lane;
+        const int lam = plev[i], sh = lam - l;
+        const float f = __int_as_float((127 - sh) << 23);  // 2^-sh
+        const unsigned long long kl = keys[i] >> (2 * (EB_KEY_LEVELS - lam));
+        const unsigned int ix = compact2d(kl), iy = compact2d(kl >> 1);
+        const float4 wv = wa[i];
+        const float gx = fmaf((float)ix + 0.5f, f, -((float)(ix >> sh) + 0.5f));
+        const float gy = fmaf((float)iy + 0.5f, f, -((float)(iy >> sh) + 0.5f));
+        const float2 w = make_float2(fmaf(wv.x, f, gx), fmaf(wv.y, f, gy));
+        const float2 ah = cscale<float>(qa[i], rinv);
+        if (E == 2) {
+          const float2 bh = cscale<float>(qb[i], rinv);
+          sab[lane] = make_float4(ah.x, ah.y, bh.x, bh.y);
+          scc[lane] = cmul<float>(cconj<float>(w), ah);
+        } else {
+          scc[lane] = ah;
+        }
+        // two chains: even and odd powers
+        float2* row = pw + lane * pitch;
+        const float2 w2 = cmul<float>(w, w);
+        float2 ev = k0 == 0 ? make_float2(1.f, 0.f) : cpow_int<float>(w, k0), od = cmul<float>(ev, w);
+        for (int j = 0; j < kw; j += 2) {
+          row[j] = ev;
+          if (j + 1 < kw) row[j + 1] = od;
+          ev = cmul<float>(ev, w2);
+          od = cmul<float>(od, w2);
+        }
+      }
+      __syncwarp();
+#pragma unroll 4
+      for (int s = 0; s < ns; ++s) {
+        const float2 v = pw[s * pitch + k];
+        if (E == 2) {
+          const float4 ab = sab[s];
+          cfma<float>(A, make_float2(ab.x, ab.y), v);
+          cfma<float>(B, make_float2(ab.z, ab.w), v);
+          cfma<float>(C, scc[s], v);
+        } else {
+          cfma<float>(A, scc[s], v);
+        }
+      }
     }
-    dst[o] = make_float2(-v.x, -v.y);
+    if (lane < kw) dst[k0 + lane] = make_float2(-A.x, -A.y);
+    if (E == 2) {
+      float2 cm = make_float2(__shfl_up_sync(0xffffffffu, C.x, 1), __shfl_up_sync(0xffffffffu, C.y, 1));
+      if (lane == 0) cm = last;
+      last = make_float2(__shfl_sync(0xffffffffu, C.x, 31), __shfl_sync(0xffffffffu, C.y, 31));
+      crfma<float>(B, (float)(k0 + lane), cm);
+      if (lane < kw) dst[p + k0 + lane] = make_float2(-B.x, -B.y);
+    }
   }
-  if (nc == 1) return;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) s_last = atomicAdd(&cdone[bb], 1) == nc - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  for (int o = tid; o < nout; o += 128) {
-    float2 acc = __ldcg(&mpart[(size_t)c0 * nout + o]);
-    for (int cc = c0 + 1; cc < c0 + nc; ++cc) acc = cadd<float>(acc, __ldcg(&mpart[(size_t)cc * nout + o]));
-    mpole[(size_t)b * nout + o] = acc;
+  if (nc > 1) p2m_finish(lane, nc, nout, mpart + (size_t)c0 * nout, cdone + bb, mpole + (size_t)b * nout);
+}
+
+// The same for the default order P (20), a lane per point: its terms -a w^k and
+// -(b w + k conj(w) a) w^(k-1) of every order in registers (of two points for a chunk of
+// more than 32), and one sum over the lanes through shared memory at the end. A power read
+// from shared memory costs its bytes for every lane that gets them (two cycles of an SM a
+// warp and 8 bytes), more than the multiply-adds that it feeds; here a chunk moves 320 bytes
+// a lane once. Measured (E = 2): 64 x 512 (six levels, all from the points) 16.5 -> 10.4 us
+// (13.4 with k_p2m_chunks); 73 us for 524,288 nodes, as that one.
+template <int E, int P>
+__global__ void __launch_bounds__(32 * P2M_CW, 4) k_p2m_points(LevOff lo, int nchunk, int first2,
+                                                    const unsigned char* __restrict__ blev,
+                                                    const unsigned char* __restrict__ plev,
+                                                    const int* __restrict__ chunk_box,
+                                                    const int* __restrict__ cstart,
+                                                    const unsigned long long* __restrict__ keys,
+                                                    const int* __restrict__ pt0, const int* __restrict__ pt1,
+                                                    const float4* __restrict__ wa, const float2* __restrict__ qa,
+                                                    const float2* __restrict__ qb,
+                                                    float2* __restrict__ mpart, int* __restrict__ cdone,
+                                                    float2* __restrict__ mpole) {
+  constexpr int NF = 2 * E * P, PITCH = 36;  // floats of a chunk; row pitch (16-byte reads without conflicts)
+  __shared__ float4 sm[P2M_CW][NF * PITCH / 4];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c = blockIdx.x * P2M_CW + wid;
+  if (c >= nchunk) return;
+  const int b = chunk_box[c];
+  const int l = blev[b];
+  const float rinv = lo.rinv[l];
+  const int bb = b - first2, c0 = cstart[bb], nc = cstart[bb + 1] - c0;
+  const int i0 = pt0[b] + (c - c0) * EB_CHUNK, i1 = min(pt1[b], i0 + EB_CHUNK);
+  float2 A[P], S[E == 2 ? P : 1];
+#pragma unroll
+  for (int k = 0; k < P; ++k) A[k] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < (E == 2 ? P : 1); ++k) S[k] = make_float2(0.f, 0.f);
+  for (int i = i0 + lane; i < i1; i += 32) {
+    const int lam = plev[i], sh = lam - l;
+    const float f = __int_as_float((127 - sh) << 23);  // 2^-sh
+    const unsigned long long kl = keys[i] >> (2 * (EB_KEY_LEVELS - lam));
+    const unsigned int ix = compact2d(kl), iy = compact2d(kl >> 1);
+    const float4 wv = wa[i];
+    const float gx = fmaf((float)ix + 0.5f, f, -((float)(ix >> sh) + 0.5f));
+    const float gy = fmaf((float)iy + 0.5f, f, -((float)(iy >> sh) + 0.5f));
+    const float2 w = make_float2(fmaf(wv.x, f, gx), fmaf(wv.y, f, gy));
+    const float2 q = cscale<float>(qa[i], -rinv);
+    float2 bw = make_float2(0.f, 0.f), cq = bw, pw = make_float2(1.f, 0.f);
+    A[0] = cadd<float>(A[0], q);
+    if (E == 2) {
+      const float2 qs = cscale<float>(qb[i], -rinv);
+      S[0] = cadd<float>(S[0], qs);
+      bw = cmul<float>(qs, w);
+      cq = cmul<float>(cconj<float>(w), q);
+    }
+#pragma unroll
+    for (int k = 1; k < P; ++k) {
+      if (E == 2) {
+        float2 t = bw;
+        crfma<float>(t, (float)k, cq);
+        cfma<float>(S[E == 2 ? k : 0], t, pw);
+      }
+      pw = cmul<float>(pw, w);
+      cfma<float>(A[k], q, pw);
+    }
   }
-  if (tid == 0) cdone[bb] = 0;
+  float* row = reinterpret_cast<float*>(sm[wid]) + lane;
+#pragma unroll
+  for (int k = 0; k < P; ++k) {
+    row[2 * k * PITCH] = A[k].x;
+    row[(2 * k + 1) * PITCH] = A[k].y;
+    if (E == 2) {
+      row[(2 * P + 2 * k) * PITCH] = S[E == 2 ? k : 0].x;
+      row[(2 * P + 2 * k + 1) * PITCH] = S[E == 2 ? k : 0].y;
+    }
+  }
+  __syncwarp();
+  // a box of one chunk gets its multipole directly; otherwise the chunk's part goes to
+  // mpart and the box's last chunk to finish adds the parts in chunk order
+  constexpr int nout = E * P;
+  float* dst = reinterpret_cast<float*>(nc == 1 ? mpole + (size_t)b * nout : mpart + (size_t)c * nout);
+#pragma unroll
+  for (int o0 = 0; o0 < NF; o0 += 32) {
+    const int o = o0 + lane;
+    if (o < NF) {
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        const float4 v = sm[wid][o * (PITCH / 4) + x];
+        t.x += v.x;
+        t.y += v.y;
+        t.z += v.z;
+        t.w += v.w;
+      }
+      dst[o] = (t.x + t.y) + (t.z + t.w);
+    }
+  }
+  if (nc > 1) p2m_finish(lane, nc, nout, mpart + (size_t)c0 * nout, cdone + bb, mpole + (size_t)b * nout);
 }
 
 // M2M into the boxes of one level from their children (FP32 coarse levels): all
@@ -1796,12 +2176,25 @@ __global__ void __launch_bounds__(128) k_far_df(int ngroup, const int* __restric
 // leaf and of its nearest ancestors (at most EB_FAR_LEVELS boxes, the coarsest holding
 // the L2L-accumulated expansion of the levels above) are staged in shared memory, and
 // each expansion is evaluated directly about its own centre at every target (the sum
-// equals L2P of the L2L-accumulated leaf expansion). Thread slice sl of 128 / EB_NTILE
-// takes every slice-th level, and every slice-th box of the leaf's W list, whose
-// multipoles are evaluated at the targets (M2P). Adds the near-field sums of k_near32
-// and applies the post-processing.
+// equals L2P of the L2L-accumulated leaf expansion). Each half-warp takes one level, and
+// every EB_FAR_LEVELS-th box of the leaf's W list, whose multipoles are evaluated at the
+// targets (M2P). Adds the near-field sums of k_near32 and applies the post-processing.
+//
+// Its Horner steps bound it (12 multiply-adds an order, level and target of E = 2). A lane
+// holds two targets of the tile and takes them through packed multiply-adds, with each
+// coefficient staged twice (x, x, y, y): 8 instructions an order for 32 targets of two
+// levels, where a lane per target and warps that took every fourth of six levels had 28.
+// Measured (E = 2): 1,048,576 nodes 227 -> 183 us, 64 x 512 10.8 -> 9.1 us.
+constexpr int FAR_THREADS = 16 * EB_FAR_LEVELS;
+
+__device__ __forceinline__ void chorner2(f32x2& ax, f32x2& ay, f32x2 ux, f32x2 uy, f32x2 nuy, f32x2 cx, f32x2 cy) {
+  const f32x2 x = fma2(ax, ux, fma2(ay, nuy, cx));
+  ay = fma2(ax, uy, fma2(ay, ux, cy));
+  ax = x;
+}
+
 template <int E>
-__global__ void __launch_bounds__(128) k_far32(const int4* __restrict__ tiles, const int* __restrict__ leaves,
+__global__ void __launch_bounds__(FAR_THREADS) k_far32(const int4* __restrict__ tiles, const int* __restrict__ leaves,
                                                const unsigned long long* __restrict__ bkey,
                                                const unsigned char* __restrict__ blev,
                                                const int* __restrict__ anc, const int* __restrict__ wstart,
@@ -1812,37 +2205,71 @@ __global__ void __launch_bounds__(128) k_far32(const int4* __restrict__ tiles, c
                                                const float2* __restrict__ mpole,
                                                double2* __restrict__ out, EbPost post,
                                                const double2* __restrict__ nearbuf) {
-  constexpr int T = EB_NTILE, NS = 128 / T;
-  extern __shared__ float2 sloc[];  // [nf][E][p + 1]
+  constexpr int T = EB_NTILE, NS = EB_FAR_LEVELS;
+  static_assert(T == 32, "two targets per lane of a half-warp");
+  extern __shared__ float4 sloc[];  // [nf][p + 1][E]: a coefficient as (x, x, y, y)
   __shared__ float2 sred[NS][T];
   const int4 tl = tiles[blockIdx.x];
   const int leaf = tl.x, b = leaves[leaf];
-  const int tid = threadIdx.x, tt = tid % T, sl = tid / T;
-  const int i = tl.y + tt;
-  const bool act = i < tl.z;
-  const int ii = act ? i : tl.y;
+  const int tid = threadIdx.x, tt = tid & 15, sl = tid >> 4;
+  const int i0 = tl.y + tt, i1 = i0 + 16;
+  const bool two = tl.z - tl.y > 16;  // the tile's second half holds targets
   const int ldl = p + 1, nco = E * ldl;
-  const int* fb = anc + (size_t)leaf * EB_FAR_LEVELS;
-  int nf = 0;
-  while (nf < EB_FAR_LEVELS && fb[nf] >= 0) ++nf;
-  for (int idx = tid; idx < nf * nco; idx += 128) {
-    const int q = idx / nco, o = idx - q * nco;
-    sloc[idx] = local[(size_t)fb[q] * nco + o];
+  const int box = anc[(size_t)leaf * EB_FAR_LEVELS + sl];  // this half-warp's
+  if (box >= 0) {
+    const float2* lc = local + (size_t)box * nco;
+    for (int m = tt; m < ldl; m += 16)
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const float2 v = lc[e * ldl + m];
+        sloc[sl * nco + m * E + e] = make_float4(v.x, v.x, v.y, v.y);
+      }
   }
-  __syncthreads();
-  float fx = 0.f, fy = 0.f;
   const unsigned long long kb = bkey[b];
   const unsigned int ix = compact2d(kb), iy = compact2d(kb >> 1);
-  const float4 wv = wa[ii];
-  // With u the leaf-scaled offset, the offset scaled to the ancestor sh levels up is
-  //   u 2^-sh + (i + 1/2) 2^-sh - (i >> sh) - 1/2   (i the leaf's grid index),
+  const float4 w0 = wa[i0 < tl.z ? i0 : tl.y], w1 = wa[i1 < tl.z ? i1 : tl.y];
+  float2 f0 = make_float2(0.f, 0.f), f1 = f0;
+  __syncwarp();
+  // With u the leaf-scaled offset, the offset scaled to the ancestor sl levels up is
+  //   u 2^-sl + (i + 1/2) 2^-sl - (i >> sl) - 1/2   (i the leaf's grid index),
   // whose constant part is exact in FP32 (i < 2^20).
-  for (int sh = sl; sh < nf; sh += NS) {
-    const float f = __int_as_float((127 - sh) << 23);  // 2^-sh
-    const float gx = fmaf((float)ix + 0.5f, f, -((float)(ix >> sh) + 0.5f));
-    const float gy = fmaf((float)iy + 0.5f, f, -((float)(iy >> sh) + 0.5f));
-    const float2 u = make_float2(fmaf(wv.x, f, gx), fmaf(wv.y, f, gy));
-    l2p_range<float, E>(sloc + sh * nco, p, 0, ldl, u, s, fx, fy);
+  if (box >= 0) {
+    const float f = __int_as_float((127 - sl) << 23);  // 2^-sl
+    const float gx = fmaf((float)ix + 0.5f, f, -((float)(ix >> sl) + 0.5f));
+    const float gy = fmaf((float)iy + 0.5f, f, -((float)(iy >> sl) + 0.5f));
+    const f32x2 ff = pk2(f, f), gx2 = pk2(gx, gx), gy2 = pk2(gy, gy);
+    const f32x2 ux = fma2(pk2(w0.x, w1.x), ff, gx2), uy = fma2(pk2(w0.y, w1.y), ff, gy2);
+    const f32x2 nuy = mul2(uy, pk2(-1.f, -1.f));
+    const ulonglong2* lb = reinterpret_cast<const ulonglong2*>(sloc + sl * nco);
+    ulonglong2 c = lb[p * E];
+    f32x2 phx = c.x, phy = c.y, dx = 0, dy = 0, psx = 0, psy = 0;
+    if (E == 2) {
+      c = lb[p * E + 1];
+      psx = c.x;
+      psy = c.y;
+    }
+#pragma unroll 4
+    for (int m = p - 1; m >= 0; --m) {
+      if (E == 2) chorner2(dx, dy, ux, uy, nuy, phx, phy);
+      c = lb[m * E];
+      chorner2(phx, phy, ux, uy, nuy, c.x, c.y);
+      if (E == 2) {
+        c = lb[m * E + 1];
+        chorner2(psx, psy, ux, uy, nuy, c.x, c.y);
+      }
+    }
+    f32x2 gx_, gy_;
+    if (E == 2) {  // phi + s (u conj(phi') + conj(psi))
+      const f32x2 ss = pk2(s, s), ns = pk2(-s, -s);
+      gx_ = fma2(ss, fma2(ux, dx, fma2(uy, dy, psx)), phx);
+      gy_ = fma2(ns, fma2(ux, dy, fma2(nuy, dx, psy)), phy);
+    } else {
+      gx_ = mul2(phx, pk2(-1.f, -1.f));
+      gy_ = mul2(phy, pk2(-1.f, -1.f));
+    }
+    const float2 vx = upk2(gx_), vy = upk2(gy_);
+    f0 = make_float2(vx.x, vy.x);
+    f1 = make_float2(vx.y, vy.y);
   }
   // W list (boxes below the leaf's level): the target's offset in the box's units is
   // u 2^ds + (c_leaf - c_box) / r_box, the high part of u first, so that the cancelling
@@ -1854,17 +2281,24 @@ __global__ void __launch_bounds__(128) k_far32(const int4* __restrict__ tiles, c
     const int ds = blev[w] - lt;
     const float f = pow2f(ds);
     const float dx = box_delta((int)ix, (int)compact2d(kw), ds), dy = box_delta((int)iy, (int)compact2d(kw >> 1), ds);
-    const float2 u = make_float2(fmaf(wv.z, f, fmaf(wv.x, f, dx)), fmaf(wv.w, f, fmaf(wv.y, f, dy)));
-    m2p_eval<float, E>(mpole + (size_t)w * E * p, p, u, s, fx, fy);
+    const float2* mw = mpole + (size_t)w * E * p;
+    const float2 u0 = make_float2(fmaf(w0.z, f, fmaf(w0.x, f, dx)), fmaf(w0.w, f, fmaf(w0.y, f, dy)));
+    m2p_eval<float, E>(mw, p, u0, s, f0.x, f0.y);
+    if (two) {
+      const float2 u1 = make_float2(fmaf(w1.z, f, fmaf(w1.x, f, dx)), fmaf(w1.w, f, fmaf(w1.y, f, dy)));
+      m2p_eval<float, E>(mw, p, u1, s, f1.x, f1.y);
+    }
   }
-  sred[sl][tt] = make_float2(fx, fy);
+  sred[sl][tt] = f0;
+  sred[sl][tt + 16] = f1;
   __syncthreads();
-  if (sl == 0 && act) {
-    float2 v = sred[0][tt];
+  const int i = tl.y + tid;
+  if (tid < T && i < tl.z) {
+    float2 v = sred[0][tid];
 #pragma unroll
     for (int q = 1; q < NS; ++q) {
-      v.x += sred[q][tt].x;
-      v.y += sred[q][tt].y;
+      v.x += sred[q][tid].x;
+      v.y += sred[q][tid].y;
     }
     const double2 nv = nearbuf[i];
     eb_post_store_f32(post, perm[i], make_float2(v.x + (float)nv.x, v.y + (float)nv.y), out);
@@ -1873,20 +2307,34 @@ __global__ void __launch_bounds__(128) k_far32(const int4* __restrict__ tiles, c
 
 // FP32 near field, one block per tile of up to EB_NTILE (32) targets of one leaf: the
 // sources of the leaf's U list (32 boxes at a time) are staged through shared memory in
-// slabs of NEAR_SLAB. Each thread holds two targets of the tile (lanes l and l + 16 of
-// the tile) and each half-warp takes one of 8 source slices, so every staged source is
+// slabs of NEAR_SLAB, source q of a slab beside source q + half the slab. Each thread holds
+// two targets of the tile (lanes l and l + 16 of the tile; one, if the tile has no more than
+// 16) and each half-warp takes one of 4 slices of the source pairs, so every staged pair is
 // read once per two targets (a broadcast within the half-warp). The slices are added in
 // a fixed order. The self pair needs no test: its offset is exactly zero, and with the
 // squared distance offset by 1e-36 its terms are exact zeros. Plain FP32 sums: the error
 // of the FP32 terms themselves (~1e-6 of the largest) dominates the summation error, so
 // compensated sums buy nothing. Writes the near-field sums in sorted order. Positions are
 // absolute (float hi + lo), so sources of any level are alike.
+// The issue of the pairs bounds it: two sources go through packed arithmetic at once, 17
+// instructions with the two reciprocals, where single ones with a division took 30 each.
+// A tile takes two warps: with four, the waits of its start and end weighed twice as much.
+// Measured (Stokes): the 57.1 M pairs of 524,288 nodes 112 -> 72 us, 95 us with four warps.
 #define NEAR_SLAB 256
+#define NEAR32_THREADS 64
+
+// 1 / x to an ulp for normal x (the squared distance is at least 1e-36)
+__device__ __forceinline__ float rcp32(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 template <int K>
 __device__ __forceinline__ void near_pair(const float4 hlj, const float4 c, const float4 hl, float& gx, float& gy) {
   const float dx = (hlj.x - hl.x) + (hlj.z - hl.z);
   const float dy = (hlj.y - hl.y) + (hlj.w - hl.w);
-  const float rr = __fdividef(1.0f, fmaf(dx, dx, fmaf(dy, dy, 1e-36f)));
+  const float rr = rcp32(fmaf(dx, dx, fmaf(dy, dy, 1e-36f)));
   const float ex = dx * rr, ey = dy * rr;  // conj(1/D), D = z_s - z_t
   if (K == NEAR_Q) {  // c = (q, -, -)
     gx = fmaf(-c.x, ex, fmaf(-c.y, ey, gx));
@@ -1902,29 +2350,62 @@ __device__ __forceinline__ void near_pair(const float4 hlj, const float4 c, cons
   }
 }
 
+// A target against the sources of a slab pair by pair: its negated position, and the two
+// sources' sums side by side.
+struct NearT {
+  f32x2 hx, hy, lx, ly, gx, gy;
+};
+__device__ __forceinline__ NearT near_target(float4 h) {
+  return NearT{pk2(-h.x, -h.x), pk2(-h.y, -h.y), pk2(-h.z, -h.z), pk2(-h.w, -h.w), 0, 0};
+}
+
+// The pair of near_pair for two sources: H = (x, x', y, y') of the high parts, L of the low
+// ones, C = (ax, ax', ay, ay') or (q, q'), D = (c0, c0', c1, c1').
 template <int K>
-__global__ void __launch_bounds__(128, 8) k_near32(const int4* __restrict__ tiles, const int* __restrict__ leaves,
-                                                   const int* __restrict__ pt0, const int* __restrict__ pt1,
+__device__ __forceinline__ void near_pair2(ulonglong2 H, ulonglong2 L, ulonglong2 C, ulonglong2 D, NearT& t) {
+  const f32x2 dx = add2(add2(H.x, t.hx), add2(L.x, t.lx));
+  const f32x2 dy = add2(add2(H.y, t.hy), add2(L.y, t.ly));
+  const float2 dd = upk2(fma2(dx, dx, fma2(dy, dy, pk2(1e-36f, 1e-36f))));
+  const f32x2 rr = pk2(rcp32(dd.x), rcp32(dd.y));
+  const f32x2 ex = mul2(dx, rr), ey = mul2(dy, rr);
+  if (K == NEAR_Q) {
+    const f32x2 neg = pk2(-1.f, -1.f), nex = mul2(ex, neg);
+    t.gx = fma2(C.x, nex, fma2(mul2(C.y, neg), ey, t.gx));
+    t.gy = fma2(C.x, ey, fma2(C.y, nex, t.gy));
+  } else {
+    const f32x2 v = fma2(ey, fma2(C.x, dx, mul2(C.y, dy)), D.x);
+    t.gx = fma2(ex, v, t.gx);
+    t.gy = fma2(ey, v, t.gy);
+    if (K == NEAR_VC) {
+      t.gx = fma2(mul2(ey, pk2(-1.f, -1.f)), D.y, t.gx);
+      t.gy = fma2(ex, D.y, t.gy);
+    }
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(NEAR32_THREADS, 16) k_near32(const int4* __restrict__ tiles, const int* __restrict__ pt0,
+                                                   const int* __restrict__ pt1,
                                                    const int* __restrict__ ustart, const int* __restrict__ ulist,
                                                    const float4* __restrict__ zhl,
                                                    const float2* __restrict__ qn, int plus,
                                                    double2* __restrict__ nearbuf) {
   constexpr bool ST = K != NEAR_Q;
   static_assert(EB_NTILE == 32, "two targets per thread over 16 lanes");
-  constexpr int NS = 8;
-  __shared__ float4 sz[NEAR_SLAB];
-  __shared__ float4 sp[ST ? NEAR_SLAB : 1];
-  __shared__ float2 sa[ST ? 1 : NEAR_SLAB];
+  constexpr int NS = NEAR32_THREADS / 16, NP = NEAR_SLAB / 2;
+  __shared__ float4 sh[NP], slo[NP], sc[NP];
+  __shared__ float4 sd[K == NEAR_VC ? NP : 1];
+  __shared__ float2 sd0[K == NEAR_V ? NP : 1];
   __shared__ int spre[33], sj0[32];
   __shared__ float2 sred[NS][EB_NTILE];
   const int4 tl = tiles[blockIdx.x];
   const int leaf = tl.x;
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int sl = 2 * (tid >> 5) + (lane >> 4);  // source slice 0..7
-  const int t0 = lane & 15;                       // targets t0 and t0 + 16 of the tile
+  const int tid = threadIdx.x;
+  const int sl = tid >> 4;    // source slice
+  const int t0 = tid & 15;    // targets t0 and t0 + 16 of the tile
   const int i0 = tl.y + t0, i1 = i0 + 16;
-  const float4 h0 = zhl[i0 < tl.z ? i0 : tl.y], h1 = zhl[i1 < tl.z ? i1 : tl.y];
-  float gx0 = 0.f, gy0 = 0.f, gx1 = 0.f, gy1 = 0.f;
+  const bool two = tl.z - tl.y > 16;
+  NearT a0 = near_target(zhl[i0 < tl.z ? i0 : tl.y]), a1 = near_target(zhl[i1 < tl.z ? i1 : tl.y]);
   const int ub = ustart[leaf], ue = ustart[leaf + 1];
   for (int cb = ub; cb < ue; cb += 32) {
     const int nc = min(32, ue - cb);
@@ -1949,33 +2430,61 @@ __global__ void __launch_bounds__(128, 8) k_near32(const int4* __restrict__ tile
     __syncthreads();
     const int total = spre[nc];
     for (int base = 0; base < total; base += NEAR_SLAB) {
-      const int ns = min(NEAR_SLAB, total - base);
+      const int ns = min(NEAR_SLAB, total - base), np = (ns + 1) >> 1;
       if (base > 0) __syncthreads();
-      for (int s2 = tid; s2 < ns; s2 += 128) {
-        const int gs = base + s2;
-        int lo = 0, hi = nc;  // the box k with spre[k] <= gs < spre[k + 1]
-        while (hi - lo > 1) {
-          const int mid = (lo + hi) >> 1;
-          if (spre[mid] <= gs) lo = mid;
-          else hi = mid;
+      for (int s2 = tid; s2 < np; s2 += NEAR32_THREADS) {
+        auto find = [&](int gs) {
+          int lo = 0, hi = nc;  // the box k with spre[k] <= gs < spre[k + 1]
+          while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (spre[mid] <= gs) lo = mid;
+            else hi = mid;
+          }
+          return sj0[lo] + gs - spre[lo];
+        };
+        const bool odd = s2 + np >= ns;  // no second source: the first with charges of zero
+        const int j = find(base + s2), k = odd ? j : find(base + np + s2);
+        const float4 zj = zhl[j], zk = zhl[k];
+        sh[s2] = make_float4(zj.x, zk.x, zj.y, zk.y);
+        slo[s2] = make_float4(zj.z, zk.z, zj.w, zk.w);
+        if (ST) {
+          const float4 cj = reinterpret_cast<const float4*>(qn)[j];
+          float4 ck = reinterpret_cast<const float4*>(qn)[k];
+          if (odd) ck = make_float4(0.f, 0.f, 0.f, 0.f);
+          sc[s2] = make_float4(cj.x, ck.x, cj.y, ck.y);
+          if (K == NEAR_VC) sd[s2] = make_float4(cj.z, ck.z, cj.w, ck.w);
+          else sd0[s2] = make_float2(cj.z, ck.z);
+        } else {
+          const float2 cj = qn[j];
+          float2 ck = qn[k];
+          if (odd) ck = make_float2(0.f, 0.f);
+          sc[s2] = make_float4(cj.x, ck.x, cj.y, ck.y);
         }
-        const int j = sj0[lo] + gs - spre[lo];
-        sz[s2] = zhl[j];
-        if (ST) sp[s2] = reinterpret_cast<const float4*>(qn)[j];
-        else sa[s2] = qn[j];
       }
       __syncthreads();
+      auto run = [&](auto both) {
 #pragma unroll 2
-      for (int jj = sl; jj < ns; jj += NS) {
-        const float4 hlj = sz[jj];
-        const float4 c = ST ? sp[jj] : make_float4(sa[jj].x, sa[jj].y, 0.f, 0.f);
-        near_pair<K>(hlj, c, h0, gx0, gy0);
-        near_pair<K>(hlj, c, h1, gx1, gy1);
-      }
+        for (int q = sl; q < np; q += NS) {
+          const ulonglong2 H = reinterpret_cast<const ulonglong2*>(sh)[q];
+          const ulonglong2 L = reinterpret_cast<const ulonglong2*>(slo)[q];
+          const ulonglong2 C = reinterpret_cast<const ulonglong2*>(sc)[q];
+          ulonglong2 D = make_ulonglong2(0, 0);
+          if (K == NEAR_VC) D = reinterpret_cast<const ulonglong2*>(sd)[q];
+          if (K == NEAR_V) D.x = reinterpret_cast<const f32x2*>(sd0)[q];
+          near_pair2<K>(H, L, C, D, a0);
+          if (both.value) near_pair2<K>(H, L, C, D, a1);
+        }
+      };
+      if (two) run(std::true_type());
+      else run(std::false_type());
     }
   }
-  sred[sl][t0] = make_float2(gx0, gy0);
-  sred[sl][t0 + 16] = make_float2(gx1, gy1);
+  auto sum2 = [](f32x2 v) {
+    const float2 f = upk2(v);
+    return f.x + f.y;
+  };
+  sred[sl][t0] = make_float2(sum2(a0.gx), sum2(a0.gy));
+  sred[sl][t0 + 16] = make_float2(sum2(a1.gx), sum2(a1.gy));
   __syncthreads();
   if (tid < EB_NTILE && tl.y + tid < tl.z) {
     float2 v = sred[0][tid];
@@ -2282,6 +2791,13 @@ int tables_build(EbTables& tb, int p, double tol) {
   EB_CUDA_TRY(cudaMemcpy(tb.pd.p, pd.data(), sizeof(int) * pd.size(), cudaMemcpyHostToDevice));
   EB_CUDA_TRY(cudaMemcpy(tb.epow.p, epow2.data(), sizeof(c_t<T>) * epow2.size(), cudaMemcpyHostToDevice));
   EB_CUDA_TRY(cudaMemcpy(tb.einv.p, einv.data(), sizeof(c_t<T>) * einv.size(), cudaMemcpyHostToDevice));
+  if (sizeof(T) == 4) {  // M2L's binomials with the output order innermost
+    std::vector<T> bt((size_t)p * (p + 1));
+    for (int k = 0; k < p; ++k)
+      for (int m = 0; m <= p; ++m) bt[(size_t)k * (p + 1) + m] = binom[(size_t)(m + k) * ldb + m];
+    EB_TRY(tb.binom_t.ensure(sizeof(T) * bt.size()));
+    EB_CUDA_TRY(cudaMemcpy(tb.binom_t.p, bt.data(), sizeof(T) * bt.size(), cudaMemcpyHostToDevice));
+  }
   if (sizeof(T) == 8) {
     auto split = [](double v, float& h, float& l) {
       h = (float)v;
@@ -2456,14 +2972,15 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w, bool brea
       lo.v[l] = t.lev_off[l];
       lo.rinv[l] = (float)((double)(1u << std::min(l, 30)) / t.W);
     }
-    const size_t sm = sizeof(float2) * ((size_t)EB_CHUNK * (p + 1) + (E == 2 ? 3 : 1) * (EB_CHUNK + 2 * (size_t)p));
-    k_p2m_chunks<E><<<t.nchunk, 128, sm, st>>>(lo, first2, t.blev.as<unsigned char>(), t.plev.as<unsigned char>(),
-                                              t.chunk_box.as<int>(), t.cstart.as<int>(),
-                                              t.keys.as<unsigned long long>(), t.pt0.as<int>(), t.pt1.as<int>(),
-                                              t.wdf.as<float4>(), reinterpret_cast<const float2*>(w.qa.p),
-                                              reinterpret_cast<const float2*>(w.qb.p), t.W, p,
-                                              w.mpart.as<float2>(), t.cdone.as<int>(),
-                                              reinterpret_cast<float2*>(w.mpole.p));
+    auto p2m = [&](auto kern, size_t sm, auto... order) {
+      kern<<<nblk(t.nchunk, P2M_CW), 32 * P2M_CW, sm, st>>>(
+          lo, t.nchunk, first2, t.blev.as<unsigned char>(), t.plev.as<unsigned char>(), t.chunk_box.as<int>(),
+          t.cstart.as<int>(), t.keys.as<unsigned long long>(), t.pt0.as<int>(), t.pt1.as<int>(), t.wdf.as<float4>(),
+          reinterpret_cast<const float2*>(w.qa.p), reinterpret_cast<const float2*>(w.qb.p), order...,
+          w.mpart.as<float2>(), t.cdone.as<int>(), reinterpret_cast<float2*>(w.mpole.p));
+    };
+    if (p == 20) p2m(k_p2m_points<E, 20>, 0);
+    else p2m(k_p2m_chunks<E>, p2m_smem(p), p);
     eb_count_launch(ctx);
     for (int l = lmin - 1; l >= 2; --l) {
       int nb = t.lev_off[l + 1] - t.lev_off[l];
@@ -2503,17 +3020,34 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w, bool brea
     ProfScope ps(ctx, 1, st);
     const bool fixed = sizeof(T) == 8 && p <= EB_FX_MAXP;
     const int ncoarse = coarse_boxes(t);
+    auto m2l32 = [&](int n, DevBuf& list, DevBuf& code, DevBuf& count, DevBuf& mp, int accumulate) -> int {
+      const float2* dinv = reinterpret_cast<const float2*>(tb.dinv.p);
+      const float2* m = reinterpret_cast<const float2*>(mp.p);
+      float2* out = reinterpret_cast<float2*>(w.local.p);
+      if (n < M2L32_WIDE) {
+        k_m2l_f32w<E, 20><<<std::min(n, M2L32_CTAS * ctx->nsm), 128, 0, st>>>(
+            first, n, list.as<int>(), code.as<unsigned char>(), count.as<int>(), tb.binom_t.as<float>(), dinv,
+            tb.pd.as<int>(), m, out, accumulate);
+        return EB_OK;
+      }
+      // boxes per warp: 6 have the 32 entries of a round on average, 16 in several rounds
+      // leave fewer lanes without one where there are warps enough (256 x 512: 125.0 against
+      // 143.0 us an apply; 1,024 x 1,024: 745 against 722 us)
+      const int nc = std::min(ncoarse, n), nb = n >= 256 * ctx->nsm ? 16 : 6;
+      constexpr size_t sm = sizeof(M2l32Smem<E, 20>);
+      EB_CUDA_TRY(cudaFuncSetAttribute(k_m2l_f32p<E, 20>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+      k_m2l_f32p<E, 20><<<nblk(nc + nblk(n - nc, nb), M2L32_WARPS), 32 * M2L32_WARPS, sm, st>>>(
+          first, n, nc, nb, list.as<int>(), code.as<unsigned char>(), count.as<int>(), dinv, tb.pd.as<int>(), m, out,
+          accumulate);
+      return EB_OK;
+    };
     if (nt > 0 && sizeof(T) == 4 && p == 20 && ctx->opts.m2l_tc > 0) {
       EB_TRY(eb_m2l_tc(ctx, E, first, nt, t.vlist.as<int>(), t.vcode.as<unsigned char>(), t.vcount.as<int>(),
                        reinterpret_cast<const float*>(tb.binom.p), ldb, reinterpret_cast<const float2*>(tb.dinv.p),
                        tb.pd.as<int>(), reinterpret_cast<const float2*>(w.mpole.p),
                        reinterpret_cast<float2*>(w.local.p), st));
     } else if (nt > 0 && sizeof(T) == 4 && p == 20) {
-      k_m2l_f32p<E, 20><<<nt, 128, 0, st>>>(first, t.vlist.as<int>(), t.vcode.as<unsigned char>(),
-                                            t.vcount.as<int>(), reinterpret_cast<const float*>(tb.binom.p), ldb,
-                                            reinterpret_cast<const float2*>(tb.dinv.p), tb.pd.as<int>(),
-                                            reinterpret_cast<const float2*>(w.mpole.p),
-                                            reinterpret_cast<float2*>(w.local.p), 0);
+      EB_TRY(m2l32(nt, t.vlist, t.vcode, t.vcount, w.mpole, 0));
       eb_count_launch(ctx);
     } else if (nt > 0 && fixed) {
       EB_TRY(eb_m2l_fx(ctx, E, false, first, nt, nt, ncoarse, t.vlist.as<int>(), t.vcode.as<unsigned char>(),
@@ -2531,11 +3065,7 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w, bool brea
       k_reflect<T><<<nblk((long long)nbi * p, 128), 128, 0, st>>>(first, nbi, t.bkey.as<unsigned long long>(), p,
                                                                  w.mpole.as<c_t<T>>(), w.mimg.as<c_t<T>>());
       if (sizeof(T) == 4 && p == 20)
-        k_m2l_f32p<E, 20><<<nbi, 128, 0, st>>>(first, t.ilist.as<int>(), t.icode.as<unsigned char>(),
-                                               t.icount.as<int>(), reinterpret_cast<const float*>(tb.binom.p), ldb,
-                                               reinterpret_cast<const float2*>(tb.dinv.p), tb.pd.as<int>(),
-                                               reinterpret_cast<const float2*>(w.mimg.p),
-                                               reinterpret_cast<float2*>(w.local.p), 1);
+        EB_TRY(m2l32(nbi, t.ilist, t.icode, t.icount, w.mimg, 1));
       else if (fixed)
         EB_TRY(eb_m2l_fx(ctx, E, false, first, nbi, nbi, ncoarse, t.ilist.as<int>(), t.icode.as<unsigned char>(),
                          t.icount.as<int>(), tb, w, w.mimg.p, w.local.p, 1, st));
@@ -2713,7 +3243,7 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
     } else {
       const float2* nq = E == 2 ? w.nc.as<float2>() : w.qa.as<float2>();
       auto go = [&](auto kern) {
-        kern<<<t.ntile, 128, 0, ns>>>(t.tiles.as<int4>(), t.leaves.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(),
+        kern<<<t.ntile, NEAR32_THREADS, 0, ns>>>(t.tiles.as<int4>(), t.pt0.as<int>(), t.pt1.as<int>(),
                                       t.ustart.as<int>(), t.ulist.as<int>(), t.zhl.as<float4>(), nq, plus, nb);
       };
       if (E == 1) go(k_near32<NEAR_Q>);
@@ -2756,7 +3286,7 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
     EB_TRY(w.local_df.ensure(sizeof(float4) * (size_t)(E * (tb.p + 1))));
   }
   const int far_lev = has_far ? std::min(t.L - 1, EB_FAR_LEVELS) : 0;  // far boxes per leaf, at most
-  const size_t far_sm = sizeof(float2) * (size_t)far_lev * E * (tb.p + 1);
+  const size_t far_sm = sizeof(float4) * (size_t)far_lev * E * (tb.p + 1);
   if (split) EB_CUDA_TRY(cudaStreamWaitEvent(st, ctx->ev_p2p, 0));
   if (join) EB_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
   if (!split && !f64) {
@@ -2783,7 +3313,7 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
     if (lpt == 1) go(k_far64<E, 1>);
     else go(k_far64<E, 4>);
   } else {
-    k_far32<E><<<t.ntile, 128, far_sm, st>>>(t.tiles.as<int4>(), t.leaves.as<int>(),
+    k_far32<E><<<t.ntile, FAR_THREADS, far_sm, st>>>(t.tiles.as<int4>(), t.leaves.as<int>(),
                                              t.bkey.as<unsigned long long>(), t.blev.as<unsigned char>(),
                                              t.anc.as<int>(), t.wstart.as<int>(), t.wlist.as<int>(), t.perm.as<int>(),
                                              t.wdf.as<float4>(), tb.p, (float)sign, w.local.as<float2>(),

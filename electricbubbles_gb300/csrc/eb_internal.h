@@ -157,6 +157,7 @@ struct EbTables {
   DevBuf pd;      // int[EB_NCODE]: per-offset truncation order
   DevBuf epow;    // c_t<T>[4*(p+2)]: e_q^j for the 4 child offsets (child units)
   DevBuf einv;    // c_t<T>[4*(p+2)]: e_q^-j
+  DevBuf binom_t;   // FP32 tables only: C(m+k, m) at [k*(p+1) + m] (k < p)
   // double-float copies (FP64 tables only) for the double-float M2L
   DevBuf binom_df;  // float2[(2p+2)*(2p+2)]
   DevBuf dinv_df;   // float4[EB_NCODE*(p+2)]
