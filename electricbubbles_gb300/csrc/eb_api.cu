@@ -1,4 +1,5 @@
 // C ABI of libeb_gb300: context, geometry, operator applies and the Fortran shims.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -97,29 +98,35 @@ __global__ void k_lap_constraints(const int* __restrict__ start, const double* _
   if (threadIdx.x == 0) sums[b] = s[0];
 }
 
-__global__ void k_fill_drop(int k, const int* __restrict__ start, int* __restrict__ drop_of,
-                            double* __restrict__ hpt) {
-  int b = blockIdx.x;
-  if (b >= k) return;
-  int i0 = start[b], i1 = start[b + 1];
-  double h = 2.0 * EB_PI / (double)(i1 - i0);
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+// A geometry installed in one launch: the copies of its arrays (from device memory; src
+// equal to dst where they came from the host), the nodes' drops and weights 2 pi / nd, and
+// per node the coefficients of the post-processing and the singular-sum weights. A drop a
+// row of blocks.
+struct Geom {
+  double2 *z, *dz;
+  double *dsda, *kappa;
+  double2* zk;
+};
+__global__ void __launch_bounds__(256) k_install(const int* __restrict__ start, Geom src, Geom dst, int* __restrict__ nd,
+                          int* __restrict__ drop_of, double* __restrict__ hpt, double* __restrict__ c1,
+                          double2* __restrict__ c2, double* __restrict__ d, float* __restrict__ c1f,
+                          float2* __restrict__ c2f, float* __restrict__ df, double2* __restrict__ pkw) {
+  const int b = blockIdx.x, i0 = start[b], i1 = start[b + 1];
+  const double h = 2.0 * EB_PI / (double)(i1 - i0);
+  if (blockIdx.y == 0 && threadIdx.x == 0) {
+    nd[b] = i1 - i0;
+    dst.zk[b] = src.zk[b];
+  }
+  for (int i = i0 + blockIdx.y * 256 + threadIdx.x; i < i1; i += gridDim.y * 256) {
     drop_of[i] = b;
     hpt[i] = h;
+    dst.z[i] = src.z[i];
+    dst.dz[i] = src.dz[i];
+    dst.dsda[i] = src.dsda[i];
+    dst.kappa[i] = src.kappa[i];
+    eb_post_coefs(i, src.dz, src.dsda, src.kappa, hpt, c1, c2, d, c1f, c2f, df);
+    pkw[i] = pk_weight(i, drop_of, hpt, src.z, src.dz, src.zk);
   }
-}
-
-// Per-node coefficients of the post-processing and the singular-sum weights.
-__global__ void k_post_coefs(int nbk, const double2* __restrict__ dz, const double* __restrict__ dsda,
-                             const double* __restrict__ kappa, const double* __restrict__ hpt,
-                             double* __restrict__ c1, double2* __restrict__ c2, double* __restrict__ d,
-                             float* __restrict__ c1f, float2* __restrict__ c2f, float* __restrict__ df,
-                             const int* __restrict__ drop_of, const double2* __restrict__ z,
-                             const double2* __restrict__ zk, double2* __restrict__ pkw) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nbk) return;
-  eb_post_coefs(t, dz, dsda, kappa, hpt, c1, c2, d, c1f, c2f, df);
-  pkw[t] = pk_weight(t, drop_of, hpt, z, dz, zk);
 }
 
 int copy_in(eb_ctx* ctx, DevBuf& buf, const void* src, size_t bytes, int mem) {
@@ -354,15 +361,7 @@ int eb_set_geometry(eb_ctx* ctx, int k, const int* nd, const double* z, const do
   EB_TRY(ctx->start.ensure(sizeof(int) * (k + 1)));
   EB_TRY(ctx->drop_of.ensure(sizeof(int) * nbk));
   EB_TRY(ctx->hpt.ensure(sizeof(double) * nbk));
-  EB_CUDA_TRY(cudaMemcpyAsync(ctx->nd.p, nd, sizeof(int) * k, cudaMemcpyHostToDevice, s));
   EB_CUDA_TRY(cudaMemcpyAsync(ctx->start.p, st.data(), sizeof(int) * (k + 1), cudaMemcpyHostToDevice, s));
-  EB_TRY(copy_in(ctx, ctx->z, z, sizeof(double2) * nbk, mem));
-  EB_TRY(copy_in(ctx, ctx->dz, dz, sizeof(double2) * nbk, mem));
-  EB_TRY(copy_in(ctx, ctx->dsda, dsda, sizeof(double) * nbk, mem));
-  EB_TRY(copy_in(ctx, ctx->kappa, kappa, sizeof(double) * nbk, mem));
-  EB_TRY(copy_in(ctx, ctx->zk, zk, sizeof(double2) * k, mem));
-  k_fill_drop<<<k, 256, 0, s>>>(k, ctx->start.as<int>(), ctx->drop_of.as<int>(), ctx->hpt.as<double>());
-  eb_count_launch(ctx);
   EB_TRY(ctx->pc1.ensure(sizeof(double) * nbk));
   EB_TRY(ctx->pc2.ensure(sizeof(double2) * nbk));
   EB_TRY(ctx->plap.ensure(sizeof(double) * nbk));
@@ -370,13 +369,39 @@ int eb_set_geometry(eb_ctx* ctx, int k, const int* nd, const double* z, const do
   EB_TRY(ctx->pc2f.ensure(sizeof(float2) * nbk));
   EB_TRY(ctx->plapf.ensure(sizeof(float) * nbk));
   EB_TRY(ctx->pkw.ensure(sizeof(double2) * nbk));
-  k_post_coefs<<<nblk(nbk, 256), 256, 0, s>>>(nbk, ctx->dz.as<double2>(), ctx->dsda.as<double>(),
-                                             ctx->kappa.as<double>(), ctx->hpt.as<double>(),
-                                             ctx->pc1.as<double>(), ctx->pc2.as<double2>(),
-                                             ctx->plap.as<double>(), ctx->pc1f.as<float>(),
-                                             ctx->pc2f.as<float2>(), ctx->plapf.as<float>(),
-                                             ctx->drop_of.as<int>(), ctx->z.as<double2>(),
-                                             ctx->zk.as<double2>(), ctx->pkw.as<double2>());
+  const void* src[5] = {z, dz, dsda, kappa, zk};
+  DevBuf* buf[5] = {&ctx->z, &ctx->dz, &ctx->dsda, &ctx->kappa, &ctx->zk};
+  const size_t bytes[5] = {sizeof(double2) * nbk, sizeof(double2) * nbk, sizeof(double) * nbk, sizeof(double) * nbk,
+                           sizeof(double2) * k};
+  // read in place: this device's memory, aligned for the loads (others are copied first)
+  auto readable = [&](int i) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, src[i]) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == ctx->device &&
+           (uintptr_t)src[i] % (i == 2 || i == 3 ? 8 : 16) == 0;
+  };
+  for (int i = 0; i < 5; ++i) {
+    if (mem == EB_HOST || !readable(i)) {
+      EB_TRY(copy_in(ctx, *buf[i], src[i], bytes[i], mem));
+      src[i] = buf[i]->p;
+    } else {
+      EB_TRY(buf[i]->ensure(bytes[i]));
+    }
+  }
+  auto geom = [](const void* const* a) {
+    void** q = const_cast<void**>(a);
+    return Geom{static_cast<double2*>(q[0]), static_cast<double2*>(q[1]), static_cast<double*>(q[2]),
+                static_cast<double*>(q[3]), static_cast<double2*>(q[4])};
+  };
+  const void* dst[5] = {ctx->z.p, ctx->dz.p, ctx->dsda.p, ctx->kappa.p, ctx->zk.p};
+  const int ndmax = *std::max_element(nd, nd + k);
+  k_install<<<dim3(k, std::min(nblk(ndmax, 256), 64)), 256, 0, s>>>(
+      ctx->start.as<int>(), geom(src), geom(dst), ctx->nd.as<int>(), ctx->drop_of.as<int>(), ctx->hpt.as<double>(),
+      ctx->pc1.as<double>(), ctx->pc2.as<double2>(), ctx->plap.as<double>(), ctx->pc1f.as<float>(),
+      ctx->pc2f.as<float2>(), ctx->plapf.as<float>(), ctx->pkw.as<double2>());
   eb_count_launch(ctx);
   if (ctx->nsim > 0) EB_TRY(eb_batch_install(ctx));  // a batch: nodes moved into their cells
   EB_TRY(eb_geom_tree(ctx));

@@ -50,7 +50,6 @@ struct DevBuf {
 struct EbTreeHost {
   double sq[4];            // the bounding square: W, x0, y0, 2^20 / W
   int bad;                 // 1: a non-finite coordinate; 2: a node below the wall
-  int lmax;                // deepest leaf level
   int lmin;                // the uniform floor level (no leaf above it)
   int hist[EB_KEY_LEVELS + 1];  // boxes per level (heads of existing boxes)
   int last[12];            // counts and scans of the last leaf or box (work items, lists)
@@ -122,7 +121,7 @@ struct EbTree {
   // at most EB_FAR_LEVELS of them (the coarsest one holds the accumulated locals above)
   DevBuf anc;      // int[nleaf*EB_FAR_LEVELS]
   DevBuf gcount, gstart;  // groups per leaf and their scan
-  DevBuf flags, scan, hist, bbox, partial, cubtmp, pairs;
+  DevBuf dev, bc, bbox, partial, cubtmp, pairs;  // the build's numbers, box heads per 256 points
   // FP32 direct multipoles: the boxes of levels chunk_lmin..L and the leaves above them,
   // split into chunks of EB_CHUNK points (other boxes by M2M)
   int nchunk = 0;

@@ -12,6 +12,7 @@
 // (cadap2.f:780-828: children of the parent's neighbours that are not adjacent, at most
 // 27); the leaves' U and W lists follow DALI12/DALI34 (dapif2.f:3-356) for leaves of
 // different levels.
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -55,9 +56,36 @@ __host__ __device__ __forceinline__ unsigned long long morton(unsigned int ix, u
   return spread2(ix) | (spread2(iy) << 1);
 }
 
-__global__ void k_bbox(const double2* __restrict__ z, int n, Box4* __restrict__ part,
-                       int* __restrict__ bad) {
+// The build's numbers on the device; the host reads the first part after the leaf levels
+// and `last` after the counts (one copy each).
+struct TreeDev {
+  double sq[4];                  // as in EbTreeHost, up to hist
+  int bad, lmin;
+  int hist[EB_KEY_LEVELS + 1];
+  int last[12];                  // leaves, groups, tiles, U and W entries, list error, chunks
+  int first[EB_KEY_LEVELS + 1];  // k_gather_points' histogram
+  unsigned int ticket[2];
+};
+static_assert(offsetof(TreeDev, last) == offsetof(EbTreeHost, last), "copied as one piece");
+
+// True in the block of a grid that counts itself last; it then sees what the others wrote.
+__device__ __forceinline__ bool last_block(unsigned int* ticket) {
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last;
+}
+
+__device__ void bbox_final(const Box4* part, int nb, int wall, TreeDev* T);
+
+// Bounding box per block; the last block forms the root square.
+__global__ void __launch_bounds__(256) k_bbox(const double2* __restrict__ z, int n, Box4* __restrict__ part, int wall,
+                                              int forest, Box4 given, TreeDev* T) {
   __shared__ double s[4][256];
+  int* bad = &T->bad;
   double mnx = INFINITY, mxx = -INFINITY, mny = INFINITY, mxy = -INFINITY;
   int nonfinite = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -79,17 +107,29 @@ __global__ void k_bbox(const double2* __restrict__ z, int n, Box4* __restrict__ 
     __syncthreads();
   }
   if (threadIdx.x == 0) part[blockIdx.x] = mk_box4(s[0][0], s[1][0], s[2][0], s[3][0]);
+  if (!last_block(&T->ticket[0])) return;
+  if (!forest) {
+    bbox_final(part, gridDim.x, wall, T);
+  } else if (threadIdx.x == 0) {
+    // an explicit root square (a forest of independent problems in a grid of cells)
+    T->sq[0] = given.x;
+    T->sq[1] = given.y;
+    T->sq[2] = given.z;
+    T->sq[3] = __ddiv_rn((double)(1u << EB_KEY_LEVELS), given.x);
+  }
 }
 
 // The bounding box and the root square sq = (W, x0, y0, 2^20 / W): the box's larger
 // side widened by 1e-9 relative, centred on the box (W = 1 for a single point).
-__global__ void k_bbox_final(const Box4* __restrict__ part, int nb, Box4* __restrict__ out,
-                             double* __restrict__ sq, int wall, int* __restrict__ bad) {
+__device__ void bbox_final(const Box4* part, int nb, int wall, TreeDev* T) {
   __shared__ Box4 sb[256];
+  double* sq = T->sq;
+  int* bad = &T->bad;
   Box4 r = mk_box4(INFINITY, -INFINITY, INFINITY, -INFINITY);
   for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-    Box4 p = part[i];
-    r.x = fmin(r.x, p.x); r.y = fmax(r.y, p.y); r.z = fmin(r.z, p.z); r.w = fmax(r.w, p.w);
+    const double* p = reinterpret_cast<const double*>(part + i);
+    r.x = fmin(r.x, __ldcg(p)); r.y = fmax(r.y, __ldcg(p + 1));
+    r.z = fmin(r.z, __ldcg(p + 2)); r.w = fmax(r.w, __ldcg(p + 3));
   }
   sb[threadIdx.x] = r;
   __syncthreads();
@@ -103,7 +143,6 @@ __global__ void k_bbox_final(const Box4* __restrict__ part, int nb, Box4* __rest
   }
   if (threadIdx.x != 0) return;
   r = sb[0];
-  *out = r;
   if (wall) {
     // the square [xleft, xleft + slength] x [0, slength] of the wall-bounded CADAPDR
     // (cadapdrop.f:142-145), widened by 1e-9 so that no key needs clamping
@@ -126,37 +165,161 @@ __global__ void k_bbox_final(const Box4* __restrict__ part, int nb, Box4* __rest
   sq[3] = __ddiv_rn((double)(1u << EB_KEY_LEVELS), w);
 }
 
-// An explicit root square (a forest of independent problems in a grid of cells).
-__global__ void k_set_square(double W, double x0, double y0, double* __restrict__ sq) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  sq[0] = W;
-  sq[1] = x0;
-  sq[2] = y0;
-  sq[3] = __ddiv_rn((double)(1u << EB_KEY_LEVELS), W);
+__device__ __forceinline__ unsigned long long point_key(double2 z, const double* sq) {
+  const double x0 = sq[1], y0 = sq[2], inv_cell = sq[3];
+  const double maxc = (double)((1u << EB_KEY_LEVELS) - 1);
+  double fx = floor((z.x - x0) * inv_cell), fy = floor((z.y - y0) * inv_cell);
+  fx = fmin(fmax(fx, 0.0), maxc);
+  fy = fmin(fmax(fy, 0.0), maxc);
+  return morton((unsigned int)fx, (unsigned int)fy);
 }
 
 __global__ void k_keys(const double2* __restrict__ z, int n, const double* __restrict__ sq,
                        unsigned long long* __restrict__ keys, int* __restrict__ idx) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double x0 = sq[1], y0 = sq[2], inv_cell = sq[3];
-  const double maxc = (double)((1u << EB_KEY_LEVELS) - 1);
-  double fx = floor((z[i].x - x0) * inv_cell), fy = floor((z[i].y - y0) * inv_cell);
-  fx = fmin(fmax(fx, 0.0), maxc);
-  fy = fmin(fmax(fy, 0.0), maxc);
-  keys[i] = morton((unsigned int)fx, (unsigned int)fy);
+  keys[i] = point_key(z[i], sq);
   idx[i] = i;
 }
 
-// sorted positions, also as float hi + lo pairs packed (hi.x, hi.y, lo.x, lo.y)
-__global__ void k_gather_points(const double2* __restrict__ z, const int* __restrict__ perm,
-                                int n, double2* __restrict__ zs, float4* __restrict__ zhl) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double2 p = z[perm[i]];
-  zs[i] = p;
-  float hx = (float)p.x, hy = (float)p.y;
-  zhl[i] = make_float4(hx, hy, (float)(p.x - (double)hx), (float)(p.y - (double)hy));
+// Keys and sort of up to SORT_MAX points in one launch: a stable radix sort, eight bits a
+// pass, of one cluster of 16 blocks whose shared memories hold all keys and indices (block r
+// the positions [r per, (r + 1) per)). Per pass a warp ranks its items in their order by
+// digit (match), the warps' and blocks' counts give each digit's place, and the items go to
+// the block of their new position through distributed shared memory. For tens of thousands
+// of keys a library sort's five passes are a handful of blocks each behind two launches:
+// 95 us at 32,768 points, where this takes 45 us.
+constexpr int SORT_CL = 16, SORT_BS = 1024, SORT_IPT = 4, SORT_MAX = SORT_CL * SORT_BS * SORT_IPT;
+struct SortSmem {
+  unsigned long long key[2][SORT_BS * SORT_IPT];
+  int idx[2][SORT_BS * SORT_IPT];
+  int wh[SORT_BS / 32][256];  // items of a digit per warp, then before the warp
+  int tot[256], base[256], sw[8];
+};
+__global__ void __cluster_dims__(SORT_CL, 1, 1) __launch_bounds__(SORT_BS)
+    k_sort(const double2* __restrict__ z, int n, const double* __restrict__ sq,
+           unsigned long long* __restrict__ keys, int* __restrict__ perm) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ __align__(16) unsigned char sort_smem[];
+  SortSmem& S = *reinterpret_cast<SortSmem*>(sort_smem);
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, r = (int)cl.block_rank();
+  const int per = (n + SORT_CL - 1) / SORT_CL, p0 = r * per, nr = max(0, min(n, p0 + per) - p0);
+  const int rounds = (per + SORT_BS - 1) / SORT_BS;  // of 32 items of a warp, at most SORT_IPT
+  for (int q = 0; q < rounds; ++q) {
+    const int s = (w * rounds + q) * 32 + lane;
+    if (s < nr) {
+      S.key[0][s] = point_key(z[p0 + s], sq);
+      S.idx[0][s] = p0 + s;
+    }
+  }
+  int cur = 0;
+  for (int shift = 0; shift < 2 * EB_KEY_LEVELS; shift += 8) {
+    for (int x = tid; x < SORT_BS / 32 * 256; x += SORT_BS) S.wh[0][x] = 0;
+    __syncthreads();
+    int rk[SORT_IPT];
+#pragma unroll
+    for (int q = 0; q < SORT_IPT; ++q) {
+      if (q >= rounds) break;
+      const int s = (w * rounds + q) * 32 + lane;
+      const bool in = s < nr;
+      const int d = in ? (int)(S.key[cur][s] >> shift) & 255 : 256 + lane;
+      const unsigned int m = __match_any_sync(0xffffffffu, d);
+      const int old = in ? S.wh[w][d] : 0;
+      __syncwarp();
+      rk[q] = old + __popc(m & ((1u << lane) - 1u));
+      if (in && (m >> lane) == 1u) S.wh[w][d] = rk[q] + 1;  // the highest lane of the digit
+      __syncwarp();
+    }
+    __syncthreads();
+    if (tid < 256) {
+      int run = 0;
+      for (int x = 0; x < SORT_BS / 32; ++x) {
+        const int t = S.wh[x][tid];
+        S.wh[x][tid] = run;
+        run += t;
+      }
+      S.tot[tid] = run;
+    }
+    cl.sync();
+    int all = 0, mine = 0, incl = 0;
+    if (tid < 256) {
+#pragma unroll
+      for (int x = 0; x < SORT_CL; ++x) {
+        const int t = cl.map_shared_rank(S.tot, x)[tid];
+        if (x < r) mine += t;
+        all += t;
+      }
+      incl = all;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) S.sw[w] = incl;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      int b = incl - all + mine;
+      for (int x = 0; x < w; ++x) b += S.sw[x];
+      S.base[tid] = b;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < SORT_IPT; ++q) {
+      if (q >= rounds) break;
+      const int s = (w * rounds + q) * 32 + lane;
+      if (s < nr) {
+        const unsigned long long key = S.key[cur][s];
+        const int d = (int)(key >> shift) & 255, pos = S.base[d] + S.wh[w][d] + rk[q];
+        const int to = pos / per, at = pos - to * per;
+        cl.map_shared_rank(S.key[cur ^ 1], to)[at] = key;
+        cl.map_shared_rank(S.idx[cur ^ 1], to)[at] = S.idx[cur][s];
+      }
+    }
+    cl.sync();
+    cur ^= 1;
+  }
+  for (int s = tid; s < nr; s += SORT_BS) {
+    keys[p0 + s] = S.key[cur][s];
+    perm[p0 + s] = S.idx[cur][s];
+  }
+}
+
+// Sorted positions, also as float hi + lo pairs packed (hi.x, hi.y, lo.x, lo.y), and the
+// histogram of the first level at which consecutive sorted keys fall in different boxes:
+// the occupied boxes of level l in a uniform tree number 1 + sum_{l' <= l} first[l']. The
+// last block picks the minimum leaf level from it: for one problem the shallowest level
+// whose occupied boxes hold at most `target` points on average (a uniform floor, which keeps
+// leaves of one level, and so no W lists, wherever the points are evenly spread), for a
+// forest the level of its cells.
+__global__ void __launch_bounds__(256) k_gather_points(const double2* __restrict__ z, const int* __restrict__ perm,
+                                const unsigned long long* __restrict__ keys, int n, int target, int R,
+                                double2* __restrict__ zs, float4* __restrict__ zhl, TreeDev* T) {
+  __shared__ int sh[EB_KEY_LEVELS + 1];
+  if (threadIdx.x <= EB_KEY_LEVELS) sh[threadIdx.x] = 0;
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    const double2 p = z[perm[i]];
+    zs[i] = p;
+    const float hx = (float)p.x, hy = (float)p.y;
+    zhl[i] = make_float4(hx, hy, (float)(p.x - (double)hx), (float)(p.y - (double)hy));
+    const unsigned long long x = i > 0 ? keys[i] ^ keys[i - 1] : 0ull;
+    if (x != 0) atomicAdd(&sh[EB_KEY_LEVELS - (63 - __clzll((long long)x)) / 2], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x <= EB_KEY_LEVELS && sh[threadIdx.x]) atomicAdd(&T->first[threadIdx.x], sh[threadIdx.x]);
+  if (!last_block(&T->ticket[1]) || threadIdx.x >= 32) return;
+  const int l = threadIdx.x;
+  int nb = l == 0 ? 1 : l <= EB_KEY_LEVELS ? __ldcg(&T->first[l]) : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, nb, o);
+    if (l >= o) nb += y;
+  }
+  const unsigned int ok = __ballot_sync(0xffffffffu, l <= EB_KEY_LEVELS && (double)n / nb <= (double)target);
+  if (l == 0) T->lmin = R > 0 ? R : ok ? __ffs(ok) - 1 : EB_KEY_LEVELS;
 }
 
 // The points of a direct tree in their given order, with the float hi + lo copies, and a
@@ -171,40 +334,6 @@ __global__ void k_direct_points(const double2* __restrict__ z, int n, int* __res
   zs[i] = p;
   float hx = (float)p.x, hy = (float)p.y;
   zhl[i] = make_float4(hx, hy, (float)(p.x - (double)hx), (float)(p.y - (double)hy));
-}
-
-// Histogram of the first level at which consecutive sorted keys fall in different boxes:
-// the occupied boxes of level l in a uniform tree number 1 + sum_{l' <= l} hist[l'].
-__global__ void k_level_hist(const unsigned long long* __restrict__ keys, int n, int* __restrict__ hist) {
-  __shared__ int sh[EB_KEY_LEVELS + 1];
-  for (int i = threadIdx.x; i <= EB_KEY_LEVELS; i += blockDim.x) sh[i] = 0;
-  __syncthreads();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i < n; i += gridDim.x * blockDim.x) {
-    const unsigned long long x = keys[i] ^ keys[i - 1];
-    if (x == 0) continue;
-    const int hb = 63 - __clzll((long long)x);
-    atomicAdd(&sh[EB_KEY_LEVELS - hb / 2], 1);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i <= EB_KEY_LEVELS; i += blockDim.x)
-    if (sh[i]) atomicAdd(&hist[i], sh[i]);
-}
-
-// The minimum leaf level: for one problem the shallowest level whose occupied boxes
-// hold at most `target` points on average (a uniform floor, which keeps leaves of one
-// level, and so no W lists, wherever the points are evenly spread), for a forest the
-// level of its cells.
-__global__ void k_pick_level(int n, int target, int R, const int* __restrict__ hist, int* __restrict__ lmin) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int L0 = EB_KEY_LEVELS, nb = 1;
-  for (int l = 0; l <= EB_KEY_LEVELS; ++l) {
-    if (l > 0) nb += hist[l];
-    if ((double)n / nb <= (double)target) {
-      L0 = l;
-      break;
-    }
-  }
-  *lmin = R > 0 ? R : L0;
 }
 
 // Levels shared by the keys a and b: the deepest level whose box holds both
@@ -228,20 +357,20 @@ __global__ void k_lcp_window(const unsigned long long* __restrict__ keys, int n,
 
 // Leaf level of every sorted point: one more than the deepest level whose box around the
 // point holds more than cap points, at most EB_KEY_LEVELS (coincident points), 0 when
-// n <= cap, and at least lmin (k_pick_level). Also the deepest leaf level and the number of boxes of every level l >= 1:
-// a point starts a box of level l when l <= its leaf level and its key differs from the
-// previous point's at level l.
-__global__ void k_leaf_level(const unsigned long long* __restrict__ keys, int n, int cap,
-                             const int* __restrict__ lmin_d, const unsigned char* __restrict__ lcpw,
-                             unsigned char* __restrict__ plev, int* __restrict__ lmax, int* __restrict__ hist) {
-  const int lmin = *lmin_d;
+// n <= cap, and at least lmin (k_gather_points). Also, per block of 256 points (row l of bc,
+// one entry per block), the points that start a box of level l >= 1: l is at most the
+// point's leaf level and its key differs from the previous point's at level l; row 0: the
+// points that start a leaf.
+constexpr int TREE_BS = 256;
+__global__ void __launch_bounds__(TREE_BS) k_leaf_level(const unsigned long long* __restrict__ keys, int n, int cap,
+                             const unsigned char* __restrict__ lcpw, unsigned char* __restrict__ plev,
+                             int* __restrict__ bc, const TreeDev* __restrict__ T) {
+  const int lmin = T->lmin;
   __shared__ int sh[EB_KEY_LEVELS + 1];
-  __shared__ int smax;
-  for (int i = threadIdx.x; i <= EB_KEY_LEVELS; i += blockDim.x) sh[i] = 0;
-  if (threadIdx.x == 0) smax = 0;
+  if (threadIdx.x <= EB_KEY_LEVELS) sh[threadIdx.x] = 0;
   __syncthreads();
-  int mymax = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  const int i = blockIdx.x * TREE_BS + threadIdx.x;
+  if (i < n) {
     int lam = 0;
     if (n > cap) {
       const int w0 = max(0, i - cap), w1 = min(i, n - 1 - cap);
@@ -251,59 +380,151 @@ __global__ void k_leaf_level(const unsigned long long* __restrict__ keys, int n,
     }
     lam = max(lam, lmin);
     plev[i] = (unsigned char)lam;
-    mymax = max(mymax, lam);
     const int sl = i > 0 ? shared_levels(keys[i - 1], keys[i]) : -1;
     for (int l = max(1, sl + 1); l <= lam; ++l) atomicAdd(&sh[l], 1);
+    if (sl < lam) atomicAdd(&sh[0], 1);
   }
-  atomicMax(&smax, mymax);
   __syncthreads();
-  for (int i = threadIdx.x; i <= EB_KEY_LEVELS; i += blockDim.x)
-    if (sh[i]) atomicAdd(&hist[i], sh[i]);
-  if (threadIdx.x == 0) atomicMax(lmax, smax);
+  if (threadIdx.x <= EB_KEY_LEVELS) bc[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = sh[threadIdx.x];
 }
 
-// Every level at once: flags[l*n + i] = 1 where sorted point i starts an existing box of
-// level l (l = 0..L). One exclusive scan over the concatenated rows then gives each head
-// its global box id (rows in level order: level l's ids start at lev_off[l]).
-__global__ void k_heads_all(const unsigned long long* __restrict__ keys, const unsigned char* __restrict__ plev,
-                            int n, int L, int* __restrict__ flags) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int lam = plev[i];
-  const int sl = i > 0 ? shared_levels(keys[i - 1], keys[i]) : -1;
-  for (int l = 0; l <= L; ++l) flags[(size_t)l * n + i] = (l <= lam) && (l > sl);
-}
-
-// Box key, level, first point and parent of every box; a box whose head point also starts
-// its parent is the parent's first child (a split box's points all lie in its children).
-__global__ void k_boxes_all(const unsigned long long* __restrict__ keys, int n, int L, int nbox,
-                            const int* __restrict__ flags, const int* __restrict__ scan,
-                            unsigned long long* __restrict__ bkey, unsigned char* __restrict__ blev,
-                            int* __restrict__ pt0, int* __restrict__ parent, int* __restrict__ child0) {
-  const long long tot = (long long)(L + 1) * n;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < tot;
-       idx += (long long)gridDim.x * blockDim.x) {
-    if (!flags[idx]) continue;
-    const int l = (int)(idx / n), i = (int)(idx - (long long)l * n);
-    const int b = scan[idx];
-    if (b >= nbox) continue;  // cannot happen: the flags and the level counts agree
-    bkey[b] = keys[i] >> (2 * (EB_KEY_LEVELS - l));
-    blev[b] = (unsigned char)l;
-    pt0[b] = i;
-    if (l == 0) {
-      parent[b] = -1;
-    } else {
-      const size_t up = idx - n;
-      const int P = scan[up] + flags[up] - 1;
-      parent[b] = P;
-      if (flags[up]) child0[P] = b;
+// Exclusive sums of up to six arrays, a block each; the totals go to tot.
+struct ScanJob {
+  const int* in;
+  int* out;
+  int* tot;
+  int n;
+};
+struct ScanJobs {
+  ScanJob j[6];
+};
+constexpr int SCAN_BS = 1024, SCAN_PT = 8;
+__device__ __forceinline__ void scan_array(const int* in, int* out, int n, int* tot) {
+  __shared__ int sw[32], s_run;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  if (tid == 0) s_run = 0;
+  for (int base = 0; base < n; base += SCAN_BS * SCAN_PT) {
+    const int i0 = base + tid * SCAN_PT;
+    int v[SCAN_PT], sum = 0;
+#pragma unroll
+    for (int q = 0; q < SCAN_PT; ++q) {
+      v[q] = i0 + q < n ? in[i0 + q] : 0;
+      sum += v[q];
     }
+    int x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) sw[w] = x;
+    __syncthreads();
+    if (w == 0) {
+      int y = sw[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, y, o);
+        if (lane >= o) y += u;
+      }
+      sw[lane] = y;
+    }
+    __syncthreads();
+    int run = s_run + (w > 0 ? sw[w - 1] : 0) + x - sum;
+#pragma unroll
+    for (int q = 0; q < SCAN_PT; ++q) {
+      if (i0 + q < n) out[i0 + q] = run;
+      run += v[q];
+    }
+    __syncthreads();
+    if (tid == 0) s_run += sw[31];
+    __syncthreads();
   }
+  if (tid == 0 && tot) *tot = s_run;
+}
+__global__ void __launch_bounds__(SCAN_BS) k_scan(ScanJobs jobs) {
+  const ScanJob j = jobs.j[blockIdx.x];
+  scan_array(j.in, j.out, j.n, j.tot);
+}
+// The rows of k_leaf_level's counts, in place; the totals are the boxes of each level and,
+// row 0, the leaves.
+__global__ void __launch_bounds__(SCAN_BS) k_scan_rows(int nblk, int* bc, TreeDev* T) {
+  int* row = bc + (size_t)blockIdx.x * nblk;
+  scan_array(row, row, nblk, blockIdx.x == 0 ? &T->last[0] : &T->hist[blockIdx.x]);
 }
 
 struct LevOffT {
   int v[EB_KEY_LEVELS + 3];
 };
+
+// Every box, by the point that starts it: its id is the level's offset plus the heads of the
+// level before the point (the block's from the scanned counts, the rest by ballots), so ids
+// are in level order and in point order within a level. Box key, level, first point,
+// parent and first child (the box of the next level that starts at the same point; a split
+// box's points all lie in its children). Also the leaves in point order, with the flag and
+// the exclusive count of leaf heads per point, and zeros for the counts of children and V
+// lists.
+__global__ void __launch_bounds__(TREE_BS) k_boxes(const unsigned long long* __restrict__ keys,
+                            const unsigned char* __restrict__ plev, int n, int L, LevOffT lo,
+                            const int* __restrict__ bc, unsigned long long* __restrict__ bkey,
+                            unsigned char* __restrict__ blev, int* __restrict__ pt0, int* __restrict__ parent,
+                            int* __restrict__ child0, int* __restrict__ nchild, int* __restrict__ vcount,
+                            int* __restrict__ lflag, int* __restrict__ lscan, int* __restrict__ leaves) {
+  constexpr int NW = TREE_BS / 32;
+  __shared__ int wc[EB_KEY_LEVELS + 1][NW];  // heads per warp; row 0: leaf heads
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int i = blockIdx.x * TREE_BS + tid;
+  const bool in = i < n;
+  const unsigned long long key = in ? keys[i] : 0ull;
+  const int lam = in ? plev[i] : -1;
+  const int sl = !in ? EB_KEY_LEVELS : i > 0 ? shared_levels(keys[i - 1], key) : -1;
+  const bool head = sl < lam;  // of a leaf
+  for (int l = 0; l <= L; ++l) {
+    const unsigned int m = __ballot_sync(0xffffffffu, l == 0 ? head : l <= lam && l > sl);
+    if (lane == 0) wc[l][w] = __popc(m);
+  }
+  __syncthreads();
+  auto rank = [&](int l, bool f) {  // heads before this point
+    const unsigned int m = __ballot_sync(0xffffffffu, f);
+    int r = bc[(size_t)l * gridDim.x + blockIdx.x] + __popc(m & ((1u << lane) - 1u));
+    for (int q = 0; q < w; ++q) r += wc[l][q];
+    return r;
+  };
+  int up = 0;      // the point's box of the level above, and whether the point starts it
+  bool fup = i == 0;
+  if (i == 0) {
+    bkey[0] = 0;
+    blev[0] = 0;
+    pt0[0] = 0;
+    parent[0] = -1;
+    child0[0] = -1;
+    nchild[0] = 0;
+    vcount[0] = 0;
+  }
+  for (int l = 1; l <= L; ++l) {
+    const bool f = l <= lam && l > sl;
+    const int b = lo.v[l] + rank(l, f) + (f ? 0 : -1);
+    if (f) {
+      bkey[b] = key >> (2 * (EB_KEY_LEVELS - l));
+      blev[b] = (unsigned char)l;
+      pt0[b] = i;
+      parent[b] = up;
+      child0[b] = -1;
+      nchild[b] = 0;
+      vcount[b] = 0;
+      if (fup) child0[up] = b;
+    }
+    if (l <= lam) {
+      up = b;
+      fup = f;
+    }
+  }
+  const int r = rank(0, head);
+  if (in) {
+    lflag[i] = head;
+    lscan[i] = r;
+    if (head) leaves[r] = up;
+  }
+}
 
 // Point range end of every box (binary search for the first key beyond the box's prefix)
 // and the children count of its parent.
@@ -432,27 +653,6 @@ __global__ void k_imglist(const unsigned long long* __restrict__ bkey, const uns
 }
 
 // Leaves in point order: point i starts its leaf when it heads the box of its leaf level.
-__global__ void k_leaf_heads(int n, const unsigned char* __restrict__ plev, const int* __restrict__ flags,
-                             int* __restrict__ lflag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  lflag[i] = flags[(size_t)plev[i] * n + i];
-}
-
-__global__ void k_leaf_fill(int n, const unsigned char* __restrict__ plev, const int* __restrict__ lflag,
-                            const int* __restrict__ lscan, const int* __restrict__ scan,
-                            int* __restrict__ leaves) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !lflag[i]) return;
-  leaves[lscan[i]] = scan[(size_t)plev[i] * n + i];
-}
-
-// The leaf count, from the exclusive scan of the leaf heads.
-__global__ void k_leaf_count(int n, const int* __restrict__ lflag, const int* __restrict__ lscan,
-                             int* __restrict__ nleaf) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *nleaf = lscan[n - 1] + lflag[n - 1];
-}
-
 #define EB_LIST_STACK 72
 
 // U and W lists of every leaf (DALI12 / DALI34, dapif2.f:3-356, for an adaptive tree
@@ -464,9 +664,65 @@ __global__ void k_leaf_count(int n, const int* __restrict__ lflag, const int* __
 //  * every leaf of a coarser level m adjacent to b's ancestor of level m goes to U (the
 //    dual list 4, evaluated directly: such a leaf holds at most cap points).
 // Every pair of points is then covered exactly once by U, W or a V list of a common
-// level. FILL = false counts, FILL = true writes at ustart / wstart.
+// level. FILL = false counts, FILL = true writes at ustart / wstart, each with the leaf's (and
+// box's) other work items (WorkItems).
+struct WorkItems {
+  const int *pt0, *pt1, *parent;
+  int *gcount, *tcount, *ccount;              // per leaf (nbox + 1), per box of levels >= 2 (nb2 + 1)
+  const int *gstart, *tstart, *cstart;
+  int *gleaf, *gfirst;
+  int4* tiles;
+  int *anc, *chunk_box, *cdone;
+  int nbox, cfirst, nb2, lmin, lend;
+};
+
+// Counts of thread t's work items: near-field groups of EB_GROUP targets and shared-memory
+// tiles of at most EB_NTILE of leaf t (b: its box, -1 beyond the last leaf), chunks of box t.
+__device__ __forceinline__ void count_items(const WorkItems& W, int t, int b, const unsigned char* blev,
+                                            const int* nchild) {
+  if (t <= W.nbox) {
+    const int np = b >= 0 ? W.pt1[b] - W.pt0[b] : 0;
+    W.gcount[t] = (np + EB_GROUP - 1) / EB_GROUP;
+    W.tcount[t] = (np + EB_NTILE - 1) / EB_NTILE;
+  }
+  // Chunks of the boxes whose FP32 multipoles come directly from their points: every box
+  // of the levels >= lmin and every leaf above them (coarser levels get theirs by M2M).
+  if (W.nb2 > 0 && t <= W.nb2) {
+    const int g = W.cfirst + t;
+    const bool direct = t < W.nb2 && (blev[g] >= W.lmin || nchild[g] == 0);
+    W.ccount[t] = direct ? (W.pt1[g] - W.pt0[g] + EB_CHUNK - 1) / EB_CHUNK : 0;
+    if (t < W.nb2) W.cdone[t] = 0;
+  }
+}
+
+__device__ __forceinline__ void fill_items(const WorkItems& W, int t, int b, const unsigned char* blev) {
+  if (b >= 0) {
+    const int a = W.pt0[b], nt = W.pt1[b] - a;
+    int g0 = W.gstart[t], c = W.gcount[t];
+    for (int g = 0; g < c; ++g) {
+      W.gleaf[g0 + g] = t;
+      W.gfirst[g0 + g] = a + g * EB_GROUP;
+    }
+    g0 = W.tstart[t];
+    c = W.tcount[t];
+    for (int g = 0; g < c; ++g)
+      W.tiles[g0 + g] = make_int4(t, a + (int)((long long)g * nt / c), a + (int)((long long)(g + 1) * nt / c), 0);
+    // The FP32 far field's boxes of the leaf: the leaf and its ancestors down to level
+    // max(2, min(lev, lend)), -1 beyond (levels <= lend hold the L2L-accumulated locals).
+    int up = b;
+    const int l = blev[b], lmin = max(2, min(l, W.lend));
+    for (int q = 0; q < EB_FAR_LEVELS; ++q) {
+      const int lev = l - q;
+      W.anc[(size_t)t * EB_FAR_LEVELS + q] = lev >= lmin ? up : -1;
+      if (lev > lmin) up = W.parent[up];
+    }
+  }
+  if (t < W.nb2)
+    for (int c = 0; c < W.ccount[t]; ++c) W.chunk_box[W.cstart[t] + c] = W.cfirst + t;
+}
+
 template <bool FILL>
-__global__ void k_leaf_lists(int nleaf, const int* __restrict__ nleaf_d, const int* __restrict__ leaves,
+__global__ void k_leaf_lists(WorkItems W, int nleaf, const int* __restrict__ nleaf_d, const int* __restrict__ leaves,
                              const unsigned long long* __restrict__ bkey,
                              const unsigned char* __restrict__ blev, LevOffT lo, int R,
                              const int* __restrict__ floor_d,
@@ -476,8 +732,14 @@ __global__ void k_leaf_lists(int nleaf, const int* __restrict__ nleaf_d, const i
                              int* __restrict__ ulist, int* __restrict__ wlist, int* __restrict__ err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (nleaf_d) nleaf = *nleaf_d;  // counting pass: launched for an upper bound
-  if (t >= nleaf) return;
-  const int b = leaves[t], l = blev[b];
+  const int b = t < nleaf ? leaves[t] : -1;
+  if (FILL) fill_items(W, t, b, blev);
+  else count_items(W, t, b, blev, nchild);
+  if (b < 0) {
+    if (!FILL && t <= W.nbox) ucnt[t] = wcnt[t] = 0;
+    return;
+  }
+  const int l = blev[b];
   const unsigned long long kb = bkey[b];
   const int ix = (int)compact2(kb), iy = (int)compact2(kb >> 1);
   const unsigned long long root = kb >> (2 * (l - R));  // the leaf's problem (R <= l)
@@ -572,79 +834,6 @@ __global__ void k_pair_counts(int nleaf, const int* __restrict__ leaves, const i
     atomicAdd(&out[1], vp);
     atomicAdd(&out[2], wp);
   }
-}
-
-__global__ void k_group_count(int nleaf, const int* __restrict__ nleaf_d, const int* __restrict__ leaves,
-                              const int* __restrict__ pt0, const int* __restrict__ pt1, int* __restrict__ cnt) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= *nleaf_d) return;
-  const int b = leaves[t];
-  cnt[t] = (pt1[b] - pt0[b] + EB_GROUP - 1) / EB_GROUP;
-}
-
-__global__ void k_group_fill(int nleaf, const int* __restrict__ leaves, const int* __restrict__ pt0,
-                             const int* __restrict__ cnt, const int* __restrict__ start,
-                             int* __restrict__ gleaf, int* __restrict__ gfirst) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nleaf) return;
-  const int b = leaves[t], g0 = start[t];
-  for (int g = 0; g < cnt[t]; ++g) {
-    gleaf[g0 + g] = t;
-    gfirst[g0 + g] = pt0[b] + g * EB_GROUP;
-  }
-}
-
-__global__ void k_tile_count(int nleaf, const int* __restrict__ nleaf_d, const int* __restrict__ leaves,
-                             const int* __restrict__ pt0, const int* __restrict__ pt1, int* __restrict__ cnt) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= *nleaf_d) return;
-  const int b = leaves[t];
-  cnt[t] = (pt1[b] - pt0[b] + EB_NTILE - 1) / EB_NTILE;
-}
-
-__global__ void k_tile_fill(int nleaf, const int* __restrict__ leaves, const int* __restrict__ pt0,
-                            const int* __restrict__ pt1, const int* __restrict__ cnt,
-                            const int* __restrict__ start, int4* __restrict__ tiles) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nleaf) return;
-  const int b = leaves[t];
-  const int g0 = start[t], c = cnt[t], a = pt0[b], nt = pt1[b] - a;
-  for (int g = 0; g < c; ++g)
-    tiles[g0 + g] = make_int4(t, a + (int)((long long)g * nt / c), a + (int)((long long)(g + 1) * nt / c), 0);
-}
-
-// The FP32 far field's boxes of each leaf: the leaf and its ancestors down to level
-// max(2, min(lev, lend)), -1 beyond (levels <= lend hold the L2L-accumulated locals).
-__global__ void k_far_boxes(int nleaf, const int* __restrict__ leaves, const unsigned char* __restrict__ blev,
-                            const int* __restrict__ parent, int lend, int* __restrict__ anc) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nleaf) return;
-  int a = leaves[t];
-  const int l = blev[a], lmin = max(2, min(l, lend));
-  for (int q = 0; q < EB_FAR_LEVELS; ++q) {
-    const int lev = l - q;
-    anc[(size_t)t * EB_FAR_LEVELS + q] = lev >= lmin ? a : -1;
-    if (lev > lmin) a = parent[a];
-  }
-}
-
-// Chunks of the boxes whose FP32 multipoles come directly from their points: every box
-// of the levels >= lmin and every leaf above them (coarser levels get theirs by M2M).
-__global__ void k_chunk_count(int first, int nb, int lmin, const unsigned char* __restrict__ blev,
-                              const int* __restrict__ nchild, const int* __restrict__ pt0,
-                              const int* __restrict__ pt1, int* __restrict__ cnt) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  const int g = first + b;
-  const bool direct = blev[g] >= lmin || nchild[g] == 0;
-  cnt[b] = direct ? (pt1[g] - pt0[g] + EB_CHUNK - 1) / EB_CHUNK : 0;
-}
-
-__global__ void k_chunk_fill(int first, int nb, const int* __restrict__ cnt, const int* __restrict__ start,
-                             int* __restrict__ chunk_box) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  for (int c = 0; c < cnt[b]; ++c) chunk_box[start[b] + c] = first + b;
 }
 
 inline int nblk(long long n, int bs) { return (int)((n + bs - 1) / bs); }
@@ -818,67 +1007,64 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
   if (!t.host) EB_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&t.host), sizeof(EbTreeHost)));
   EbTreeHost* H = t.host;
   t.pairs_read = false;
+  // (the whole build is a chain of small kernels, and their number and that of the copies
+  // is what it costs, about 4 us each. A solve of 64 x 512 nodes, geometry installed, spent
+  // 664 us before its first Krylov vector with 80 of them under a profiler, 288 us with
+  // these 25; without one it went from 1,897 to 1,664 us, and the Cauchy sum of 60,001 points
+  // from 1,060 to 870 us)
   // 1. bounding square, on the device
-  int nbb = std::min(nblk(n, BS), 1024);
+  const int nbb = std::min(nblk(n, BS), 1024), nb256 = nblk(n, TREE_BS);
   EB_TRY(t.partial.ensure(sizeof(Box4) * (size_t)nbb));
-  EB_TRY(t.bbox.ensure(sizeof(Box4) + sizeof(double) * 4 + sizeof(int) * 8));
-  double* sq = reinterpret_cast<double*>(t.bbox.as<char>() + sizeof(Box4));
-  int* bad = reinterpret_cast<int*>(sq + 4);
-  int* lmax_d = bad + 1;
-  int* lerr_d = bad + 2;
-  int* nleaf_d = bad + 3;
-  int* lmin_d = bad + 4;
-  EB_CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(int) * 3, st));
-  k_bbox<<<nbb, BS, 0, st>>>(z, n, t.partial.as<Box4>(), bad);
-  eb_count_launch(ctx);
-  if (root_sq) k_set_square<<<1, 32, 0, st>>>(root_sq[0], root_sq[1], root_sq[2], sq);
-  else k_bbox_final<<<1, 256, 0, st>>>(t.partial.as<Box4>(), nbb, t.bbox.as<Box4>(), sq, t.wall, bad);
+  EB_TRY(t.dev.ensure(sizeof(TreeDev)));
+  TreeDev* T = t.dev.as<TreeDev>();
+  EB_CUDA_TRY(cudaMemsetAsync(T, 0, sizeof(TreeDev), st));
+  k_bbox<<<nbb, BS, 0, st>>>(z, n, t.partial.as<Box4>(), t.wall, root_sq != nullptr,
+                             root_sq ? mk_box4(root_sq[0], root_sq[1], root_sq[2], 0.0) : Box4(), T);
   eb_count_launch(ctx);
   // 2. keys and sort (a non-finite coordinate gives clamped keys; reported below)
   EB_TRY(t.keys.ensure(sizeof(unsigned long long) * (size_t)n));
-  EB_TRY(t.keys_alt.ensure(sizeof(unsigned long long) * (size_t)n));
-  EB_TRY(t.idx_alt.ensure(sizeof(int) * (size_t)n));
   EB_TRY(t.perm.ensure(sizeof(int) * (size_t)n));
-  k_keys<<<nblk(n, BS), BS, 0, st>>>(z, n, sq, t.keys_alt.as<unsigned long long>(), t.idx_alt.as<int>());
-  eb_count_launch(ctx);
-  size_t tmp_sort = 0, tmp_scan = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, tmp_sort, t.keys_alt.as<unsigned long long>(),
-                                  t.keys.as<unsigned long long>(), t.idx_alt.as<int>(),
-                                  t.perm.as<int>(), n, 0, 2 * EB_KEY_LEVELS, st);
-  cub::DeviceScan::ExclusiveSum(nullptr, tmp_scan, t.flags.as<int>(), t.scan.as<int>(), n, st);
-  EB_TRY(t.cubtmp.ensure(std::max(tmp_sort, tmp_scan)));
-  size_t tb = t.cubtmp.bytes;
-  EB_CUDA_TRY(cub::DeviceRadixSort::SortPairs(t.cubtmp.p, tb, t.keys_alt.as<unsigned long long>(),
-                                              t.keys.as<unsigned long long>(), t.idx_alt.as<int>(),
-                                              t.perm.as<int>(), n, 0, 2 * EB_KEY_LEVELS, st));
-  eb_count_launch(ctx);
+  if (n <= SORT_MAX) {
+    EB_CUDA_TRY(cudaFuncSetAttribute(k_sort, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    EB_CUDA_TRY(cudaFuncSetAttribute(k_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem)));
+    k_sort<<<SORT_CL, SORT_BS, sizeof(SortSmem), st>>>(z, n, T->sq, t.keys.as<unsigned long long>(), t.perm.as<int>());
+    eb_count_launch(ctx);
+  } else {
+    EB_TRY(t.keys_alt.ensure(sizeof(unsigned long long) * (size_t)n));
+    EB_TRY(t.idx_alt.ensure(sizeof(int) * (size_t)n));
+    k_keys<<<nblk(n, BS), BS, 0, st>>>(z, n, T->sq, t.keys_alt.as<unsigned long long>(), t.idx_alt.as<int>());
+    eb_count_launch(ctx);
+    size_t tmp_sort = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, tmp_sort, t.keys_alt.as<unsigned long long>(),
+                                    t.keys.as<unsigned long long>(), t.idx_alt.as<int>(),
+                                    t.perm.as<int>(), n, 0, 2 * EB_KEY_LEVELS, st);
+    EB_TRY(t.cubtmp.ensure(tmp_sort));
+    size_t tb = t.cubtmp.bytes;
+    EB_CUDA_TRY(cub::DeviceRadixSort::SortPairs(t.cubtmp.p, tb, t.keys_alt.as<unsigned long long>(),
+                                                t.keys.as<unsigned long long>(), t.idx_alt.as<int>(),
+                                                t.perm.as<int>(), n, 0, 2 * EB_KEY_LEVELS, st));
+    eb_count_launch(ctx);
+  }
   const unsigned long long* keys = t.keys.as<unsigned long long>();
-  // 3. sorted positions
+  // 3. sorted positions and the uniform floor
   EB_TRY(t.zs.ensure(sizeof(double2) * (size_t)n));
   EB_TRY(t.zhl.ensure(sizeof(float4) * (size_t)n));
-  k_gather_points<<<nblk(n, BS), BS, 0, st>>>(z, t.perm.as<int>(), n, t.zs.as<double2>(), t.zhl.as<float4>());
+  k_gather_points<<<nblk(n, 256), 256, 0, st>>>(z, t.perm.as<int>(), keys, n, leaf_target, t.R, t.zs.as<double2>(),
+                                                t.zhl.as<float4>(), T);
   eb_count_launch(ctx);
   // 4. leaf level of every point, deepest level, boxes per level
   EB_TRY(t.lcpw.ensure((size_t)n));
   EB_TRY(t.plev.ensure((size_t)n));
-  EB_TRY(t.hist.ensure(sizeof(int) * (EB_KEY_LEVELS + 1)));
-  EB_CUDA_TRY(cudaMemsetAsync(t.hist.p, 0, sizeof(int) * (EB_KEY_LEVELS + 1), st));
-  k_level_hist<<<std::min(nblk(n, BS), ctx->nsm * 4), BS, 0, st>>>(keys, n, t.hist.as<int>());
-  k_pick_level<<<1, 32, 0, st>>>(n, leaf_target, t.R, t.hist.as<int>(), lmin_d);
-  EB_CUDA_TRY(cudaMemsetAsync(t.hist.p, 0, sizeof(int) * (EB_KEY_LEVELS + 1), st));
-  ctx->launches += 2;
+  EB_TRY(t.bc.ensure(sizeof(int) * (EB_KEY_LEVELS + 1) * (size_t)nb256));
   if (n > leaf_cap) {
     k_lcp_window<<<nblk(n - leaf_cap, BS), BS, 0, st>>>(keys, n, leaf_cap, t.lcpw.as<unsigned char>());
     eb_count_launch(ctx);
   }
-  k_leaf_level<<<std::min(nblk(n, BS), ctx->nsm * 8), BS, 0, st>>>(keys, n, leaf_cap, lmin_d, t.lcpw.as<unsigned char>(),
-                                                                  t.plev.as<unsigned char>(), lmax_d,
-                                                                  t.hist.as<int>());
-  eb_count_launch(ctx);
-  EB_CUDA_TRY(cudaMemcpyAsync(H->sq, sq, sizeof(H->sq), cudaMemcpyDeviceToHost, st));
-  EB_CUDA_TRY(cudaMemcpyAsync(&H->bad, bad, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
-  EB_CUDA_TRY(cudaMemcpyAsync(H->hist, t.hist.p, sizeof(H->hist), cudaMemcpyDeviceToHost, st));
-  EB_CUDA_TRY(cudaMemcpyAsync(&H->lmin, lmin_d, sizeof(int), cudaMemcpyDeviceToHost, st));
+  k_leaf_level<<<nb256, TREE_BS, 0, st>>>(keys, n, leaf_cap, t.lcpw.as<unsigned char>(), t.plev.as<unsigned char>(),
+                                          t.bc.as<int>(), T);
+  k_scan_rows<<<EB_KEY_LEVELS + 1, SCAN_BS, 0, st>>>(nb256, t.bc.as<int>(), T);
+  ctx->launches += 2;
+  EB_CUDA_TRY(cudaMemcpyAsync(H->sq, T, offsetof(TreeDev, last), cudaMemcpyDeviceToHost, st));
   EB_CUDA_TRY(cudaStreamSynchronize(st));
   if (H->bad & 1) {
     eb_set_last_error_msg("non-finite node coordinate");
@@ -891,7 +1077,8 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
   t.W = H->sq[0];
   t.x0 = H->sq[1];
   t.y0 = H->sq[2];
-  const int L = H->lmax;
+  int L = EB_KEY_LEVELS;  // the deepest leaf level: the last one with boxes
+  while (L > 0 && H->hist[L] == 0) --L;
   t.L = L;
   t.lev_off[0] = 0;
   for (int l = 0; l <= L; ++l) t.lev_off[l + 1] = t.lev_off[l] + (l == 0 ? 1 : H->hist[l]);
@@ -906,49 +1093,24 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
   EB_TRY(t.parent.ensure(sizeof(int) * NB));
   EB_TRY(t.child0.ensure(sizeof(int) * NB));
   EB_TRY(t.nchild.ensure(sizeof(int) * NB));
-  // 5. boxes of every level: heads, one scan, fill, finish
-  const size_t nflag = (size_t)(L + 1) * n;
-  EB_TRY(t.flags.ensure(sizeof(int) * nflag));
-  EB_TRY(t.scan.ensure(sizeof(int) * nflag));
-  k_heads_all<<<nblk(n, BS), BS, 0, st>>>(keys, t.plev.as<unsigned char>(), n, L, t.flags.as<int>());
-  eb_count_launch(ctx);
-  {
-    size_t need = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need, t.flags.as<int>(), t.scan.as<int>(), (int)nflag, st);
-    if (need > t.cubtmp.bytes) EB_TRY(t.cubtmp.ensure(need));
-  }
-  tb = t.cubtmp.bytes;
-  EB_CUDA_TRY(cub::DeviceScan::ExclusiveSum(t.cubtmp.p, tb, t.flags.as<int>(), t.scan.as<int>(), (int)nflag, st));
-  eb_count_launch(ctx);
-  EB_CUDA_TRY(cudaMemsetAsync(t.child0.p, 0xff, sizeof(int) * NB, st));  // -1: no children
-  EB_CUDA_TRY(cudaMemsetAsync(t.nchild.p, 0, sizeof(int) * NB, st));
-  k_boxes_all<<<std::min(nblk((long long)nflag, BS), ctx->nsm * 16), BS, 0, st>>>(
-      keys, n, L, t.nbox, t.flags.as<int>(), t.scan.as<int>(), t.bkey.as<unsigned long long>(),
-      t.blev.as<unsigned char>(), t.pt0.as<int>(), t.parent.as<int>(), t.child0.as<int>());
-  eb_count_launch(ctx);
-  k_boxes_fin<<<nblk(t.nbox, BS), BS, 0, st>>>(t.nbox, keys, n, t.bkey.as<unsigned long long>(),
-                                              t.blev.as<unsigned char>(), t.pt0.as<int>(), t.parent.as<int>(),
-                                              t.pt1.as<int>(), t.nchild.as<int>());
-  eb_count_launch(ctx);
-  LevOffT lo;
-  for (int l = 0; l < EB_KEY_LEVELS + 3; ++l) lo.v[l] = t.lev_off[std::min(l, L + 1)];
-  // 6. leaves in point order
+  // 5. boxes of every level, leaves in point order
   EB_TRY(t.lflag.ensure(sizeof(int) * (size_t)n));
   EB_TRY(t.lscan.ensure(sizeof(int) * (size_t)n));
   EB_TRY(t.leaves.ensure(sizeof(int) * NB));
-  k_leaf_heads<<<nblk(n, BS), BS, 0, st>>>(n, t.plev.as<unsigned char>(), t.flags.as<int>(), t.lflag.as<int>());
-  eb_count_launch(ctx);
-  tb = t.cubtmp.bytes;
-  EB_CUDA_TRY(cub::DeviceScan::ExclusiveSum(t.cubtmp.p, tb, t.lflag.as<int>(), t.lscan.as<int>(), n, st));
-  eb_count_launch(ctx);
-  k_leaf_fill<<<nblk(n, BS), BS, 0, st>>>(n, t.plev.as<unsigned char>(), t.lflag.as<int>(), t.lscan.as<int>(),
-                                          t.scan.as<int>(), t.leaves.as<int>());
-  eb_count_launch(ctx);
+  EB_TRY(t.vcount.ensure(sizeof(int) * NB));
+  LevOffT lo;
+  for (int l = 0; l < EB_KEY_LEVELS + 3; ++l) lo.v[l] = t.lev_off[std::min(l, L + 1)];
+  k_boxes<<<nb256, TREE_BS, 0, st>>>(keys, t.plev.as<unsigned char>(), n, L, lo, t.bc.as<int>(),
+                                     t.bkey.as<unsigned long long>(), t.blev.as<unsigned char>(), t.pt0.as<int>(),
+                                     t.parent.as<int>(), t.child0.as<int>(), t.nchild.as<int>(), t.vcount.as<int>(),
+                                     t.lflag.as<int>(), t.lscan.as<int>(), t.leaves.as<int>());
+  k_boxes_fin<<<nblk(t.nbox, BS), BS, 0, st>>>(t.nbox, keys, n, t.bkey.as<unsigned long long>(),
+                                              t.blev.as<unsigned char>(), t.pt0.as<int>(), t.parent.as<int>(),
+                                              t.pt1.as<int>(), t.nchild.as<int>());
+  ctx->launches += 2;
   // 7. V lists of every box of levels >= 2
   EB_TRY(t.vlist.ensure(sizeof(int) * NB * EB_VMAX));
   EB_TRY(t.vcode.ensure(NB * EB_VMAX));
-  EB_TRY(t.vcount.ensure(sizeof(int) * NB));
-  EB_CUDA_TRY(cudaMemsetAsync(t.vcount.p, 0, sizeof(int) * NB, st));
   if (L >= 2) {
     const int first = t.lev_off[2];
     k_vlist<<<nblk(32LL * (t.nbox - first), 128), 128, 0, st>>>(t.bkey.as<unsigned long long>(), lo, first, t.nbox, t.R,
@@ -974,69 +1136,32 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
   // EB_NTILE targets, and FP32 direct-P2M chunks of at most EB_CHUNK points of every box
   // of the chunked levels (every level up to 256K points, so that no dependent M2M
   // launches remain on the critical path; above that the EB_DIRECT_LEVELS finest).
-  // The leaf count is known on the device only: the counting kernels run over nbox
-  // threads, stop at that count and leave zeros beyond it, and the scans span nbox + 1
-  // entries, so that their last entries are the totals.
+  // The leaf count is known on the device only: the counting kernel runs over nbox + 1
+  // threads and leaves zeros beyond it, and the scans span nbox + 1 entries.
   const int NBi = t.nbox;
-  EB_TRY(t.ucnt.ensure(sizeof(int) * (NB + 1)));
-  EB_TRY(t.wcnt.ensure(sizeof(int) * (NB + 1)));
-  EB_TRY(t.ustart.ensure(sizeof(int) * (NB + 1)));
-  EB_TRY(t.wstart.ensure(sizeof(int) * (NB + 1)));
-  EB_TRY(t.tcount.ensure(sizeof(int) * (NB + 1)));
-  EB_TRY(t.tstart.ensure(sizeof(int) * (NB + 1)));
-  EB_TRY(t.gcount.ensure(sizeof(int) * (NB + 1)));
-  EB_TRY(t.gstart.ensure(sizeof(int) * (NB + 1)));
-  k_leaf_count<<<1, 32, 0, st>>>(n, t.lflag.as<int>(), t.lscan.as<int>(), nleaf_d);
-  eb_count_launch(ctx);
-  for (DevBuf* d : {&t.ucnt, &t.wcnt, &t.tcount, &t.gcount})
-    EB_CUDA_TRY(cudaMemsetAsync(d->p, 0, sizeof(int) * (NB + 1), st));
-  k_leaf_lists<false><<<nblk(NBi, 128), 128, 0, st>>>(NBi, nleaf_d, t.leaves.as<int>(), t.bkey.as<unsigned long long>(),
-                                                       t.blev.as<unsigned char>(), lo, t.R, lmin_d, t.child0.as<int>(),
-                                                       t.nchild.as<int>(), t.ucnt.as<int>(), t.wcnt.as<int>(),
-                                                       nullptr, nullptr, nullptr, nullptr, lerr_d);
-  k_group_count<<<nblk(NBi, BS), BS, 0, st>>>(NBi, nleaf_d, t.leaves.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(),
-                                              t.gcount.as<int>());
-  k_tile_count<<<nblk(NBi, BS), BS, 0, st>>>(NBi, nleaf_d, t.leaves.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(),
-                                             t.tcount.as<int>());
-  ctx->launches += 3;
-  {
-    size_t need = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need, t.ucnt.as<int>(), t.ustart.as<int>(), NBi + 1, st);
-    if (need > t.cubtmp.bytes) EB_TRY(t.cubtmp.ensure(need));
-  }
-  for (auto pr : {std::make_pair(&t.ucnt, &t.ustart), std::make_pair(&t.wcnt, &t.wstart),
-                  std::make_pair(&t.gcount, &t.gstart), std::make_pair(&t.tcount, &t.tstart)}) {
-    tb = t.cubtmp.bytes;
-    EB_CUDA_TRY(cub::DeviceScan::ExclusiveSum(t.cubtmp.p, tb, pr.first->as<int>(), pr.second->as<int>(), NBi + 1, st));
-    eb_count_launch(ctx);
-  }
-  EB_CUDA_TRY(cudaMemcpyAsync(&H->last[0], nleaf_d, sizeof(int), cudaMemcpyDeviceToHost, st));
-  EB_CUDA_TRY(cudaMemcpyAsync(&H->last[1], t.gstart.as<int>() + NBi, sizeof(int), cudaMemcpyDeviceToHost, st));
-  EB_CUDA_TRY(cudaMemcpyAsync(&H->last[2], t.tstart.as<int>() + NBi, sizeof(int), cudaMemcpyDeviceToHost, st));
-  EB_CUDA_TRY(cudaMemcpyAsync(&H->last[3], t.ustart.as<int>() + NBi, sizeof(int), cudaMemcpyDeviceToHost, st));
-  EB_CUDA_TRY(cudaMemcpyAsync(&H->last[4], t.wstart.as<int>() + NBi, sizeof(int), cudaMemcpyDeviceToHost, st));
-  EB_CUDA_TRY(cudaMemcpyAsync(&H->last[5], lerr_d, sizeof(int), cudaMemcpyDeviceToHost, st));
   t.nchunk = 0;
   t.chunk_lmin = n <= (1 << 18) ? 2 : std::max(2, L - EB_DIRECT_LEVELS + 1);
-  const int cfirst = t.lev_off[std::min(2, L + 1)], nb2 = t.nbox - cfirst;
-  if (L >= 2 && nb2 > 0) {
-    EB_TRY(t.ccount.ensure(sizeof(int) * (size_t)nb2));
-    EB_TRY(t.cstart.ensure(sizeof(int) * (size_t)(nb2 + 1)));
-    EB_TRY(t.cdone.ensure(sizeof(int) * (size_t)nb2));
-    EB_CUDA_TRY(cudaMemsetAsync(t.cdone.p, 0, sizeof(int) * (size_t)nb2, st));
-    k_chunk_count<<<nblk(nb2, BS), BS, 0, st>>>(cfirst, nb2, t.chunk_lmin, t.blev.as<unsigned char>(),
-                                                t.nchild.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(),
-                                                t.ccount.as<int>());
-    eb_count_launch(ctx);
-    size_t need = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need, t.ccount.as<int>(), t.cstart.as<int>(), nb2, st);
-    if (need > t.cubtmp.bytes) EB_TRY(t.cubtmp.ensure(need));
-    tb = t.cubtmp.bytes;
-    EB_CUDA_TRY(cub::DeviceScan::ExclusiveSum(t.cubtmp.p, tb, t.ccount.as<int>(), t.cstart.as<int>(), nb2, st));
-    eb_count_launch(ctx);
-    EB_CUDA_TRY(cudaMemcpyAsync(&H->last[6], t.ccount.as<int>() + nb2 - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    EB_CUDA_TRY(cudaMemcpyAsync(&H->last[7], t.cstart.as<int>() + nb2 - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-  }
+  const int cfirst = t.lev_off[std::min(2, L + 1)], nb2 = L >= 2 ? t.nbox - cfirst : 0;
+  for (DevBuf* d : {&t.ucnt, &t.wcnt, &t.ustart, &t.wstart, &t.tcount, &t.tstart, &t.gcount, &t.gstart})
+    EB_TRY(d->ensure(sizeof(int) * (NB + 1)));
+  for (DevBuf* d : {&t.ccount, &t.cstart, &t.cdone}) EB_TRY(d->ensure(sizeof(int) * (size_t)(nb2 + 1)));
+  WorkItems W{t.pt0.as<int>(),    t.pt1.as<int>(),    t.parent.as<int>(), t.gcount.as<int>(), t.tcount.as<int>(),
+              t.ccount.as<int>(), t.gstart.as<int>(), t.tstart.as<int>(), t.cstart.as<int>(), nullptr,
+              nullptr,            nullptr,            nullptr,            nullptr,            t.cdone.as<int>(),
+              NBi,                cfirst,             nb2,                t.chunk_lmin,       t.lend};
+  k_leaf_lists<false><<<nblk(NBi + 1, 128), 128, 0, st>>>(W, NBi, &T->last[0], t.leaves.as<int>(),
+                                                       t.bkey.as<unsigned long long>(),
+                                                       t.blev.as<unsigned char>(), lo, t.R, &T->lmin, t.child0.as<int>(),
+                                                       t.nchild.as<int>(), t.ucnt.as<int>(), t.wcnt.as<int>(),
+                                                       nullptr, nullptr, nullptr, nullptr, &T->last[5]);
+  const ScanJobs jobs{{{t.gcount.as<int>(), t.gstart.as<int>(), &T->last[1], NBi + 1},
+                       {t.tcount.as<int>(), t.tstart.as<int>(), &T->last[2], NBi + 1},
+                       {t.ucnt.as<int>(), t.ustart.as<int>(), &T->last[3], NBi + 1},
+                       {t.wcnt.as<int>(), t.wstart.as<int>(), &T->last[4], NBi + 1},
+                       {t.ccount.as<int>(), t.cstart.as<int>(), &T->last[6], nb2 + 1}}};
+  k_scan<<<nb2 > 0 ? 5 : 4, SCAN_BS, 0, st>>>(jobs);
+  ctx->launches += 2;
+  EB_CUDA_TRY(cudaMemcpyAsync(H->last, T->last, sizeof(T->last), cudaMemcpyDeviceToHost, st));
   EB_CUDA_TRY(cudaStreamSynchronize(st));
   if (H->last[5]) {
     eb_set_last_error_msg("tree build: interaction-list traversal deeper than its stack");
@@ -1051,33 +1176,24 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
   // 9. fill the lists and work items
   EB_TRY(t.ulist.ensure(sizeof(int) * (size_t)std::max<long long>(t.nu, 1)));
   EB_TRY(t.wlist.ensure(sizeof(int) * (size_t)std::max<long long>(t.nw, 1)));
-  k_leaf_lists<true><<<nblk(nl, 128), 128, 0, st>>>(nl, nullptr, t.leaves.as<int>(), t.bkey.as<unsigned long long>(),
-                                                     t.blev.as<unsigned char>(), lo, t.R, lmin_d, t.child0.as<int>(),
-                                                     t.nchild.as<int>(), nullptr, nullptr, t.ustart.as<int>(),
-                                                     t.wstart.as<int>(), t.ulist.as<int>(), t.wlist.as<int>(),
-                                                     lerr_d);
-  eb_count_launch(ctx);
   EB_TRY(t.gleaf.ensure(sizeof(int) * (size_t)t.ngroup));
   EB_TRY(t.gfirst.ensure(sizeof(int) * (size_t)t.ngroup));
-  k_group_fill<<<nblk(nl, BS), BS, 0, st>>>(nl, t.leaves.as<int>(), t.pt0.as<int>(), t.gcount.as<int>(),
-                                            t.gstart.as<int>(), t.gleaf.as<int>(), t.gfirst.as<int>());
-  eb_count_launch(ctx);
   EB_TRY(t.tiles.ensure(sizeof(int4) * (size_t)t.ntile));
-  k_tile_fill<<<nblk(nl, BS), BS, 0, st>>>(nl, t.leaves.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(),
-                                           t.tcount.as<int>(), t.tstart.as<int>(), t.tiles.as<int4>());
-  eb_count_launch(ctx);
   EB_TRY(t.anc.ensure(sizeof(int) * (size_t)nl * EB_FAR_LEVELS));
-  k_far_boxes<<<nblk(nl, BS), BS, 0, st>>>(nl, t.leaves.as<int>(), t.blev.as<unsigned char>(), t.parent.as<int>(),
-                                           t.lend, t.anc.as<int>());
+  t.nchunk = nb2 > 0 ? H->last[6] : 0;
+  EB_TRY(t.chunk_box.ensure(sizeof(int) * (size_t)std::max(t.nchunk, 1)));
+  W.gleaf = t.gleaf.as<int>();
+  W.gfirst = t.gfirst.as<int>();
+  W.tiles = t.tiles.as<int4>();
+  W.anc = t.anc.as<int>();
+  W.chunk_box = t.chunk_box.as<int>();
+  k_leaf_lists<true><<<nblk(std::max(nl, nb2), 128), 128, 0, st>>>(W, nl, nullptr, t.leaves.as<int>(),
+                                                     t.bkey.as<unsigned long long>(),
+                                                     t.blev.as<unsigned char>(), lo, t.R, &T->lmin, t.child0.as<int>(),
+                                                     t.nchild.as<int>(), nullptr, nullptr, t.ustart.as<int>(),
+                                                     t.wstart.as<int>(), t.ulist.as<int>(), t.wlist.as<int>(),
+                                                     &T->last[5]);
   eb_count_launch(ctx);
-  if (L >= 2 && nb2 > 0) {
-    t.nchunk = H->last[6] + H->last[7];
-    EB_CUDA_TRY(cudaMemcpyAsync(t.cstart.as<int>() + nb2, &t.nchunk, sizeof(int), cudaMemcpyHostToDevice, st));
-    EB_TRY(t.chunk_box.ensure(sizeof(int) * (size_t)std::max(t.nchunk, 1)));
-    k_chunk_fill<<<nblk(nb2, BS), BS, 0, st>>>(cfirst, nb2, t.ccount.as<int>(), t.cstart.as<int>(),
-                                               t.chunk_box.as<int>());
-    eb_count_launch(ctx);
-  }
   // 10. leaf-relative coordinates for the double-float kernels and the FP32 P2M / far field
   EB_TRY(t.wdf.ensure(sizeof(float4) * (size_t)n));
   EB_TRY(t.wdf_lo.ensure(sizeof(float2) * (size_t)n));
