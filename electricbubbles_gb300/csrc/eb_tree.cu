@@ -79,74 +79,81 @@ __device__ __forceinline__ bool last_block(unsigned int* ticket) {
   return s_last;
 }
 
-__device__ void bbox_final(const Box4* part, int nb, int wall, TreeDev* T);
-
-// Bounding box per block; the last block forms the root square.
-__global__ void __launch_bounds__(256) k_bbox(const double2* __restrict__ z, int n, Box4* __restrict__ part, int wall,
-                                              int forest, Box4 given, TreeDev* T) {
-  __shared__ double s[4][256];
-  int* bad = &T->bad;
-  double mnx = INFINITY, mxx = -INFINITY, mny = INFINITY, mxy = -INFINITY;
-  int nonfinite = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double2 p = z[i];
-    if (!isfinite(p.x) || !isfinite(p.y)) { nonfinite = 1; continue; }
-    mnx = fmin(mnx, p.x); mxx = fmax(mxx, p.x);
-    mny = fmin(mny, p.y); mxy = fmax(mxy, p.y);
+// Doubles as integers in their order, so that the FP64 pipe (two lanes a cycle and SM, each
+// step of a reduction 64 cycles and more) has no part in the minima and maxima.
+__device__ __forceinline__ long long ordered(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double unordered(long long b) {
+  return __longlong_as_double(b ^ ((b >> 63) & 0x7fffffffffffffffll));
+}
+struct IBox {  // (min x, -max x, min y, -max y) as ordered integers: all four by minima
+  long long v[4];
+};
+// The minima over the block (256 threads), in thread 0.
+__device__ __forceinline__ IBox box_min(IBox b) {
+  __shared__ long long s[4][8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b.v[q] = min(b.v[q], __shfl_xor_sync(0xffffffffu, b.v[q], o));
+    if (lane == 0) s[q][w] = b.v[q];
   }
-  if (nonfinite) atomicOr(bad, 1);
-  s[0][threadIdx.x] = mnx; s[1][threadIdx.x] = mxx; s[2][threadIdx.x] = mny; s[3][threadIdx.x] = mxy;
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      s[0][threadIdx.x] = fmin(s[0][threadIdx.x], s[0][threadIdx.x + o]);
-      s[1][threadIdx.x] = fmax(s[1][threadIdx.x], s[1][threadIdx.x + o]);
-      s[2][threadIdx.x] = fmin(s[2][threadIdx.x], s[2][threadIdx.x + o]);
-      s[3][threadIdx.x] = fmax(s[3][threadIdx.x], s[3][threadIdx.x + o]);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = mk_box4(s[0][0], s[1][0], s[2][0], s[3][0]);
-  if (!last_block(&T->ticket[0])) return;
-  if (!forest) {
-    bbox_final(part, gridDim.x, wall, T);
-  } else if (threadIdx.x == 0) {
-    // an explicit root square (a forest of independent problems in a grid of cells)
-    T->sq[0] = given.x;
-    T->sq[1] = given.y;
-    T->sq[2] = given.z;
-    T->sq[3] = __ddiv_rn((double)(1u << EB_KEY_LEVELS), given.x);
-  }
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int x = 1; x < 8; ++x) b.v[q] = min(b.v[q], s[q][x]);
+  __syncthreads();
+  return b;
 }
 
-// The bounding box and the root square sq = (W, x0, y0, 2^20 / W): the box's larger
-// side widened by 1e-9 relative, centred on the box (W = 1 for a single point).
-__device__ void bbox_final(const Box4* part, int nb, int wall, TreeDev* T) {
-  __shared__ Box4 sb[256];
-  double* sq = T->sq;
-  int* bad = &T->bad;
-  Box4 r = mk_box4(INFINITY, -INFINITY, INFINITY, -INFINITY);
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-    const double* p = reinterpret_cast<const double*>(part + i);
-    r.x = fmin(r.x, __ldcg(p)); r.y = fmax(r.y, __ldcg(p + 1));
-    r.z = fmin(r.z, __ldcg(p + 2)); r.w = fmax(r.w, __ldcg(p + 3));
-  }
-  sb[threadIdx.x] = r;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      const Box4 q = sb[threadIdx.x + o];
-      Box4& a = sb[threadIdx.x];
-      a.x = fmin(a.x, q.x); a.y = fmax(a.y, q.y); a.z = fmin(a.z, q.z); a.w = fmax(a.w, q.w);
+// Bounding box per block; the last block forms the root square sq = (W, x0, y0, 2^20 / W):
+// the box's larger side widened by 1e-9 relative, centred on the box (W = 1 for a single
+// point), or the given one of a forest of independent problems in a grid of cells.
+__global__ void __launch_bounds__(256) k_bbox(const double2* __restrict__ z, int n, IBox* __restrict__ part, int wall,
+                                              int forest, Box4 given, TreeDev* T) {
+  const long long inf = ordered(INFINITY);
+  IBox b{{inf, inf, inf, inf}};
+  bool nonfinite = false;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const longlong2 p = reinterpret_cast<const longlong2*>(z)[i];
+    const double x = __longlong_as_double(p.x), y = __longlong_as_double(p.y);
+    if ((~p.x & 0x7ff0000000000000ll) == 0 || (~p.y & 0x7ff0000000000000ll) == 0) {  // inf or NaN
+      nonfinite = true;
+      continue;
     }
-    __syncthreads();
+    b.v[0] = min(b.v[0], ordered(x));
+    b.v[1] = min(b.v[1], ~ordered(x));
+    b.v[2] = min(b.v[2], ordered(y));
+    b.v[3] = min(b.v[3], ~ordered(y));
   }
+  if (nonfinite) atomicOr(&T->bad, 1);
+  b = box_min(b);
+  if (threadIdx.x == 0) part[blockIdx.x] = b;
+  if (!last_block(&T->ticket[0])) return;
+  b = IBox{{inf, inf, inf, inf}};
+  for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) b.v[q] = min(b.v[q], __ldcg(&part[i].v[q]));
+  b = box_min(b);
   if (threadIdx.x != 0) return;
-  r = sb[0];
+  double* sq = T->sq;
+  if (forest) {
+    sq[0] = given.x;
+    sq[1] = given.y;
+    sq[2] = given.z;
+    sq[3] = __ddiv_rn((double)(1u << EB_KEY_LEVELS), given.x);
+    return;
+  }
+  const Box4 r = mk_box4(unordered(b.v[0]), unordered(~b.v[1]), unordered(b.v[2]), unordered(~b.v[3]));
   if (wall) {
     // the square [xleft, xleft + slength] x [0, slength] of the wall-bounded CADAPDR
     // (cadapdrop.f:142-145), widened by 1e-9 so that no key needs clamping
-    if (!(r.z >= 0.0)) atomicOr(bad, 2);
+    if (!(r.z >= 0.0)) atomicOr(&T->bad, 2);
     double w = fmax(__dadd_rn(r.y, -r.x), r.w);
     if (!(w > 0)) w = 1.0;
     w = __dmul_rn(w, 1.0 + 1e-9);
@@ -165,40 +172,40 @@ __device__ void bbox_final(const Box4* part, int nb, int wall, TreeDev* T) {
   sq[3] = __ddiv_rn((double)(1u << EB_KEY_LEVELS), w);
 }
 
-__device__ __forceinline__ unsigned long long point_key(double2 z, const double* sq) {
-  const double x0 = sq[1], y0 = sq[2], inv_cell = sq[3];
-  const double maxc = (double)((1u << EB_KEY_LEVELS) - 1);
-  double fx = floor((z.x - x0) * inv_cell), fy = floor((z.y - y0) * inv_cell);
-  fx = fmin(fmax(fx, 0.0), maxc);
-  fy = fmin(fmax(fy, 0.0), maxc);
-  return morton((unsigned int)fx, (unsigned int)fy);
-}
-
 __global__ void k_keys(const double2* __restrict__ z, int n, const double* __restrict__ sq,
                        unsigned long long* __restrict__ keys, int* __restrict__ idx) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  keys[i] = point_key(z[i], sq);
+  const double x0 = sq[1], y0 = sq[2], inv_cell = sq[3];
+  const double maxc = (double)((1u << EB_KEY_LEVELS) - 1);
+  double fx = floor((z[i].x - x0) * inv_cell), fy = floor((z[i].y - y0) * inv_cell);
+  fx = fmin(fmax(fx, 0.0), maxc);
+  fy = fmin(fmax(fy, 0.0), maxc);
+  keys[i] = morton((unsigned int)fx, (unsigned int)fy);
   idx[i] = i;
 }
 
-// Keys and sort of up to SORT_MAX points in one launch: a stable radix sort, eight bits a
-// pass, of one cluster of 16 blocks whose shared memories hold all keys and indices (block r
-// the positions [r per, (r + 1) per)). Per pass a warp ranks its items in their order by
-// digit (match), the warps' and blocks' counts give each digit's place, and the items go to
-// the block of their new position through distributed shared memory. For tens of thousands
-// of keys a library sort's five passes are a handful of blocks each behind two launches:
-// 95 us at 32,768 points, where this takes 45 us.
+// The sort of up to SORT_MAX keys in one launch: a stable radix sort, eight bits a pass, of
+// one cluster of 16 blocks whose shared memories hold all keys, each with its point's index
+// below it in one word (block r the positions [r per, (r + 1) per)). Per pass a warp ranks
+// its items in their order by digit (ballots), the block orders its items by digit in shared
+// memory, the counts of all blocks give each digit's place, and the items go on to the block
+// of their new position through distributed shared memory, neighbours of a digit side by
+// side (a remote store is paid by the segments that a warp touches). For tens of thousands of
+// keys a library sort's five passes are a handful of blocks each behind two launches: 95 us
+// at 32,768 points. Keys and indices in two arrays and scattered straight to their
+// blocks, with the keys formed on these 16 SMs as well, took 45 us, this and k_keys 31 us.
 constexpr int SORT_CL = 16, SORT_BS = 1024, SORT_IPT = 4, SORT_MAX = SORT_CL * SORT_BS * SORT_IPT;
+static_assert(2 * EB_KEY_LEVELS + 16 <= 64 && SORT_MAX <= 1 << 16, "key and index in one word");
 struct SortSmem {
-  unsigned long long key[2][SORT_BS * SORT_IPT];
-  int idx[2][SORT_BS * SORT_IPT];
-  int wh[SORT_BS / 32][256];  // items of a digit per warp, then before the warp
-  int tot[256], base[256], sw[8];
+  unsigned long long item[SORT_BS * SORT_IPT];  // this block's positions
+  unsigned long long loc[SORT_BS * SORT_IPT];   // its items by digit
+  int wh[SORT_BS / 32][256];                    // items of a digit per warp, then before the warp
+  int tot[256], lbase[256], gbase[256], sw[2][8];
 };
 __global__ void __cluster_dims__(SORT_CL, 1, 1) __launch_bounds__(SORT_BS)
-    k_sort(const double2* __restrict__ z, int n, const double* __restrict__ sq,
-           unsigned long long* __restrict__ keys, int* __restrict__ perm) {
+    k_sort(const unsigned long long* __restrict__ in, int n, unsigned long long* __restrict__ keys,
+           int* __restrict__ perm) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char sort_smem[];
@@ -206,43 +213,68 @@ __global__ void __cluster_dims__(SORT_CL, 1, 1) __launch_bounds__(SORT_BS)
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, r = (int)cl.block_rank();
   const int per = (n + SORT_CL - 1) / SORT_CL, p0 = r * per, nr = max(0, min(n, p0 + per) - p0);
   const int rounds = (per + SORT_BS - 1) / SORT_BS;  // of 32 items of a warp, at most SORT_IPT
-  for (int q = 0; q < rounds; ++q) {
+  unsigned long long v[SORT_IPT];
+#pragma unroll
+  for (int q = 0; q < SORT_IPT; ++q) {
     const int s = (w * rounds + q) * 32 + lane;
-    if (s < nr) {
-      S.key[0][s] = point_key(z[p0 + s], sq);
-      S.idx[0][s] = p0 + s;
-    }
+    v[q] = q < rounds && s < nr ? in[p0 + s] << 16 | (unsigned long long)(p0 + s) : ~0ull;
   }
-  int cur = 0;
-  for (int shift = 0; shift < 2 * EB_KEY_LEVELS; shift += 8) {
-    for (int x = tid; x < SORT_BS / 32 * 256; x += SORT_BS) S.wh[0][x] = 0;
-    __syncthreads();
+  for (int shift = 16; shift < 16 + 2 * EB_KEY_LEVELS; shift += 8) {
+    for (int x = lane; x < 256; x += 32) S.wh[w][x] = 0;
+    __syncwarp();
     int rk[SORT_IPT];
 #pragma unroll
     for (int q = 0; q < SORT_IPT; ++q) {
       if (q >= rounds) break;
-      const int s = (w * rounds + q) * 32 + lane;
-      const bool in = s < nr;
-      const int d = in ? (int)(S.key[cur][s] >> shift) & 255 : 256 + lane;
-      const unsigned int m = __match_any_sync(0xffffffffu, d);
-      const int old = in ? S.wh[w][d] : 0;
+      const bool valid = (w * rounds + q) * 32 + lane < nr;
+      const int d = (int)(v[q] >> shift) & 255;
+      unsigned int m = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const unsigned int t = __ballot_sync(0xffffffffu, (d >> b) & 1);
+        m &= (d >> b) & 1 ? t : ~t;
+      }
+      const int old = valid ? S.wh[w][d] : 0;
       __syncwarp();
       rk[q] = old + __popc(m & ((1u << lane) - 1u));
-      if (in && (m >> lane) == 1u) S.wh[w][d] = rk[q] + 1;  // the highest lane of the digit
+      if (valid && (m >> lane) == 1u) S.wh[w][d] = rk[q] + 1;  // the highest lane of the digit
       __syncwarp();
     }
     __syncthreads();
+    int tot = 0, incl = 0;
     if (tid < 256) {
-      int run = 0;
+      int c[SORT_BS / 32];
+#pragma unroll
+      for (int x = 0; x < SORT_BS / 32; ++x) c[x] = S.wh[x][tid];
+#pragma unroll
       for (int x = 0; x < SORT_BS / 32; ++x) {
-        const int t = S.wh[x][tid];
-        S.wh[x][tid] = run;
-        run += t;
+        S.wh[x][tid] = tot;
+        tot += c[x];
       }
-      S.tot[tid] = run;
+      S.tot[tid] = tot;
+      incl = tot;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) S.sw[0][w] = incl;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      int b = incl - tot;
+      for (int x = 0; x < w; ++x) b += S.sw[0][x];
+      S.lbase[tid] = b;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < SORT_IPT; ++q) {
+      if (q >= rounds) break;
+      const int d = (int)(v[q] >> shift) & 255;
+      if ((w * rounds + q) * 32 + lane < nr) S.loc[S.lbase[d] + S.wh[w][d] + rk[q]] = v[q];
     }
     cl.sync();
-    int all = 0, mine = 0, incl = 0;
+    int all = 0, mine = 0;
     if (tid < 256) {
 #pragma unroll
       for (int x = 0; x < SORT_CL; ++x) {
@@ -256,33 +288,34 @@ __global__ void __cluster_dims__(SORT_CL, 1, 1) __launch_bounds__(SORT_BS)
         const int y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
       }
-      if (lane == 31) S.sw[w] = incl;
+      if (lane == 31) S.sw[1][w] = incl;
     }
     __syncthreads();
     if (tid < 256) {
-      int b = incl - all + mine;
-      for (int x = 0; x < w; ++x) b += S.sw[x];
-      S.base[tid] = b;
+      int b = incl - all + mine - S.lbase[tid];
+      for (int x = 0; x < w; ++x) b += S.sw[1][x];
+      S.gbase[tid] = b;  // from a place in loc to the position
     }
     __syncthreads();
-#pragma unroll
-    for (int q = 0; q < SORT_IPT; ++q) {
-      if (q >= rounds) break;
-      const int s = (w * rounds + q) * 32 + lane;
-      if (s < nr) {
-        const unsigned long long key = S.key[cur][s];
-        const int d = (int)(key >> shift) & 255, pos = S.base[d] + S.wh[w][d] + rk[q];
-        const int to = pos / per, at = pos - to * per;
-        cl.map_shared_rank(S.key[cur ^ 1], to)[at] = key;
-        cl.map_shared_rank(S.idx[cur ^ 1], to)[at] = S.idx[cur][s];
-      }
+    for (int s = tid; s < nr; s += SORT_BS) {
+      const unsigned long long x = S.loc[s];
+      const int pos = s + S.gbase[(int)(x >> shift) & 255], to = pos / per;
+      cl.map_shared_rank(S.item, to)[pos - to * per] = x;
     }
     cl.sync();
-    cur ^= 1;
+#pragma unroll
+    for (int q = 0; q < SORT_IPT; ++q) {
+      const int s = (w * rounds + q) * 32 + lane;
+      v[q] = q < rounds && s < nr ? S.item[s] : ~0ull;
+    }
   }
-  for (int s = tid; s < nr; s += SORT_BS) {
-    keys[p0 + s] = S.key[cur][s];
-    perm[p0 + s] = S.idx[cur][s];
+#pragma unroll
+  for (int q = 0; q < SORT_IPT; ++q) {
+    const int s = (w * rounds + q) * 32 + lane;
+    if (q < rounds && s < nr) {
+      keys[p0 + s] = v[q] >> 16;
+      perm[p0 + s] = (int)(v[q] & 0xffff);
+    }
   }
 }
 
@@ -721,8 +754,14 @@ __device__ __forceinline__ void fill_items(const WorkItems& W, int t, int b, con
     for (int c = 0; c < W.ccount[t]; ++c) W.chunk_box[W.cstart[t] + c] = W.cfirst + t;
 }
 
+// A warp per leaf: its neighbours on its own level (tasks 0..8) and those of its ancestors
+// (eight a level, coarser levels after finer ones) go to the lanes, which look them up side
+// by side; a leaf's entries stand in the tasks' order. With a thread per leaf the chains of
+// binary searches, nine and more of some ten dependent loads, took 14 us to count and 16 us to
+// fill at 64 x 512, now 6 and 8 us.
 template <bool FILL>
-__global__ void k_leaf_lists(WorkItems W, int nleaf, const int* __restrict__ nleaf_d, const int* __restrict__ leaves,
+__global__ void __launch_bounds__(128) k_leaf_lists(WorkItems W, int nleaf, const int* __restrict__ nleaf_d,
+                             const int* __restrict__ leaves,
                              const unsigned long long* __restrict__ bkey,
                              const unsigned char* __restrict__ blev, LevOffT lo, int R,
                              const int* __restrict__ floor_d,
@@ -730,35 +769,48 @@ __global__ void k_leaf_lists(WorkItems W, int nleaf, const int* __restrict__ nle
                              int* __restrict__ ucnt, int* __restrict__ wcnt,
                              const int* __restrict__ ustart, const int* __restrict__ wstart,
                              int* __restrict__ ulist, int* __restrict__ wlist, int* __restrict__ err) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int gt = blockIdx.x * 128 + threadIdx.x, lane = threadIdx.x & 31;
   if (nleaf_d) nleaf = *nleaf_d;  // counting pass: launched for an upper bound
-  const int b = t < nleaf ? leaves[t] : -1;
-  if (FILL) fill_items(W, t, b, blev);
-  else count_items(W, t, b, blev, nchild);
-  if (b < 0) {
-    if (!FILL && t <= W.nbox) ucnt[t] = wcnt[t] = 0;
-    return;
+  // the other work items: a thread per leaf and box, the launch has 32 threads for each
+  {
+    const int b = gt < nleaf ? leaves[gt] : -1;
+    if (FILL) fill_items(W, gt, b, blev);
+    else count_items(W, gt, b, blev, nchild);
+    if (!FILL && b < 0 && gt <= W.nbox) ucnt[gt] = wcnt[gt] = 0;
   }
-  const int l = blev[b];
+  const int t = gt >> 5;
+  if (t >= nleaf) return;
+  const int b = leaves[t], l = blev[b];
   const unsigned long long kb = bkey[b];
   const int ix = (int)compact2(kb), iy = (int)compact2(kb >> 1);
   const unsigned long long root = kb >> (2 * (l - R));  // the leaf's problem (R <= l)
-  int nu = 0, nw = 0;
+  // no leaf lies above the tree's floor (every box there is split)
+  const int mstop = max(R, *floor_d), ntask = 9 + 8 * max(0, l - mstop);
+  int nu = 0, nw = 0;  // entries of the tasks before
   int* uo = FILL ? ulist + ustart[t] : nullptr;
   int* wo = FILL ? wlist + wstart[t] : nullptr;
-  int stack[EB_LIST_STACK];
-  const int side = 1 << l;
-  for (int dy = -1; dy <= 1; ++dy) {
-    for (int dx = -1; dx <= 1; ++dx) {
-      const int sx = ix + dx, sy = iy + dy;
-      if (sx < 0 || sy < 0 || sx >= side || sy >= side) continue;
-      const int C = find_box(bkey, lo.v[l], lo.v[l + 1] - lo.v[l], morton((unsigned)sx, (unsigned)sy));
-      if (C < 0 || (bkey[C] >> (2 * (l - R))) != root) continue;
-      if (nchild[C] == 0) {
-        if (FILL) uo[nu] = C;
-        ++nu;
-        continue;
+  for (int k0 = 0; k0 < ntask; k0 += 32) {
+    const int k = k0 + lane;
+    // the task's box, if it exists, belongs to the problem and (coarser levels) is a leaf
+    int C = -1;
+    bool split = false;
+    if (k < ntask) {
+      const int up = k < 9 ? 0 : 1 + (k - 9) / 8, m = l - up;
+      int q = k < 9 ? k : (k - 9) % 8;
+      if (k >= 9 && q >= 4) ++q;  // not the ancestor itself
+      const int sx = (ix >> up) + q % 3 - 1, sy = (iy >> up) + q / 3 - 1, side = 1 << m;
+      if (sx >= 0 && sy >= 0 && sx < side && sy < side) {
+        C = find_box(bkey, lo.v[m], lo.v[m + 1] - lo.v[m], morton((unsigned)sx, (unsigned)sy));
+        if (C >= 0 && (bkey[C] >> (2 * (m - R))) != root) C = -1;
+        if (C >= 0) {
+          split = nchild[C] != 0;
+          if (split && k >= 9) C = -1;
+        }
       }
+    }
+    // below a split box of the leaf's level: counted first, written with the offsets known
+    auto descend = [&](int* u, int* v, int& cu, int& cw) {
+      int stack[EB_LIST_STACK];
       int sp = 0;
       for (int c = 0; c < nchild[C]; ++c) stack[sp++] = child0[C] + c;
       while (sp > 0) {
@@ -769,36 +821,42 @@ __global__ void k_leaf_lists(WorkItems W, int nleaf, const int* __restrict__ nle
         const int x0 = ix << f, x1 = ((ix + 1) << f) - 1, y0 = iy << f, y1 = ((iy + 1) << f) - 1;
         const bool adj = jx >= x0 - 1 && jx <= x1 + 1 && jy >= y0 - 1 && jy <= y1 + 1;
         if (!adj) {
-          if (FILL) wo[nw] = D;
-          ++nw;
+          if (v) v[cw] = D;
+          ++cw;
         } else if (nchild[D] == 0) {
-          if (FILL) uo[nu] = D;
-          ++nu;
+          if (u) u[cu] = D;
+          ++cu;
         } else if (sp + nchild[D] <= EB_LIST_STACK) {
           for (int c = 0; c < nchild[D]; ++c) stack[sp++] = child0[D] + c;
         } else {
           atomicOr(err, 1);
         }
       }
-    }
-  }
-  // no leaf lies above the tree's floor (every box there is split)
-  const int mstop = max(R, *floor_d);
-  for (int m = l - 1; m >= mstop; --m) {
-    const int ax = ix >> (l - m), ay = iy >> (l - m), sm = 1 << m;
-    for (int dy = -1; dy <= 1; ++dy) {
-      for (int dx = -1; dx <= 1; ++dx) {
-        if (dx == 0 && dy == 0) continue;
-        const int sx = ax + dx, sy = ay + dy;
-        if (sx < 0 || sy < 0 || sx >= sm || sy >= sm) continue;
-        const int N = find_box(bkey, lo.v[m], lo.v[m + 1] - lo.v[m], morton((unsigned)sx, (unsigned)sy));
-        if (N < 0 || nchild[N] != 0 || (bkey[N] >> (2 * (m - R))) != root) continue;
-        if (FILL) uo[nu] = N;
-        ++nu;
+    };
+    int cu = C >= 0 && !split, cw = 0;
+    if (split && C >= 0) descend(nullptr, nullptr, cu, cw);
+    __syncwarp();
+    int eu = cu, ew = cw;  // inclusive sums over the lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, eu, o), c = __shfl_up_sync(0xffffffffu, ew, o);
+      if (lane >= o) {
+        eu += a;
+        ew += c;
       }
     }
+    if (FILL && C >= 0) {
+      if (!split) {
+        uo[nu + eu - cu] = C;
+      } else {
+        int a = 0, c = 0;
+        descend(uo + nu + eu - cu, wo + nw + ew - cw, a, c);
+      }
+    }
+    nu += __shfl_sync(0xffffffffu, eu, 31);
+    nw += __shfl_sync(0xffffffffu, ew, 31);
   }
-  if (!FILL) {
+  if (!FILL && lane == 0) {
     ucnt[t] = nu;
     wcnt[t] = nw;
   }
@@ -1014,26 +1072,26 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
   // from 1,060 to 870 us)
   // 1. bounding square, on the device
   const int nbb = std::min(nblk(n, BS), 1024), nb256 = nblk(n, TREE_BS);
-  EB_TRY(t.partial.ensure(sizeof(Box4) * (size_t)nbb));
+  EB_TRY(t.partial.ensure(sizeof(IBox) * (size_t)nbb));
   EB_TRY(t.dev.ensure(sizeof(TreeDev)));
   TreeDev* T = t.dev.as<TreeDev>();
   EB_CUDA_TRY(cudaMemsetAsync(T, 0, sizeof(TreeDev), st));
-  k_bbox<<<nbb, BS, 0, st>>>(z, n, t.partial.as<Box4>(), t.wall, root_sq != nullptr,
+  k_bbox<<<nbb, BS, 0, st>>>(z, n, t.partial.as<IBox>(), t.wall, root_sq != nullptr,
                              root_sq ? mk_box4(root_sq[0], root_sq[1], root_sq[2], 0.0) : Box4(), T);
   eb_count_launch(ctx);
   // 2. keys and sort (a non-finite coordinate gives clamped keys; reported below)
   EB_TRY(t.keys.ensure(sizeof(unsigned long long) * (size_t)n));
   EB_TRY(t.perm.ensure(sizeof(int) * (size_t)n));
+  EB_TRY(t.keys_alt.ensure(sizeof(unsigned long long) * (size_t)n));
+  EB_TRY(t.idx_alt.ensure(sizeof(int) * (size_t)n));
+  k_keys<<<nblk(n, 128), 128, 0, st>>>(z, n, T->sq, t.keys_alt.as<unsigned long long>(), t.idx_alt.as<int>());
+  eb_count_launch(ctx);
   if (n <= SORT_MAX) {
     EB_CUDA_TRY(cudaFuncSetAttribute(k_sort, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     EB_CUDA_TRY(cudaFuncSetAttribute(k_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem)));
-    k_sort<<<SORT_CL, SORT_BS, sizeof(SortSmem), st>>>(z, n, T->sq, t.keys.as<unsigned long long>(), t.perm.as<int>());
-    eb_count_launch(ctx);
+    k_sort<<<SORT_CL, SORT_BS, sizeof(SortSmem), st>>>(t.keys_alt.as<unsigned long long>(), n,
+                                                       t.keys.as<unsigned long long>(), t.perm.as<int>());
   } else {
-    EB_TRY(t.keys_alt.ensure(sizeof(unsigned long long) * (size_t)n));
-    EB_TRY(t.idx_alt.ensure(sizeof(int) * (size_t)n));
-    k_keys<<<nblk(n, BS), BS, 0, st>>>(z, n, T->sq, t.keys_alt.as<unsigned long long>(), t.idx_alt.as<int>());
-    eb_count_launch(ctx);
     size_t tmp_sort = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, tmp_sort, t.keys_alt.as<unsigned long long>(),
                                     t.keys.as<unsigned long long>(), t.idx_alt.as<int>(),
@@ -1043,8 +1101,8 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
     EB_CUDA_TRY(cub::DeviceRadixSort::SortPairs(t.cubtmp.p, tb, t.keys_alt.as<unsigned long long>(),
                                                 t.keys.as<unsigned long long>(), t.idx_alt.as<int>(),
                                                 t.perm.as<int>(), n, 0, 2 * EB_KEY_LEVELS, st));
-    eb_count_launch(ctx);
   }
+  eb_count_launch(ctx);
   const unsigned long long* keys = t.keys.as<unsigned long long>();
   // 3. sorted positions and the uniform floor
   EB_TRY(t.zs.ensure(sizeof(double2) * (size_t)n));
@@ -1149,7 +1207,7 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
               t.ccount.as<int>(), t.gstart.as<int>(), t.tstart.as<int>(), t.cstart.as<int>(), nullptr,
               nullptr,            nullptr,            nullptr,            nullptr,            t.cdone.as<int>(),
               NBi,                cfirst,             nb2,                t.chunk_lmin,       t.lend};
-  k_leaf_lists<false><<<nblk(NBi + 1, 128), 128, 0, st>>>(W, NBi, &T->last[0], t.leaves.as<int>(),
+  k_leaf_lists<false><<<nblk(32LL * NBi + 1, 128), 128, 0, st>>>(W, NBi, &T->last[0], t.leaves.as<int>(),
                                                        t.bkey.as<unsigned long long>(),
                                                        t.blev.as<unsigned char>(), lo, t.R, &T->lmin, t.child0.as<int>(),
                                                        t.nchild.as<int>(), t.ucnt.as<int>(), t.wcnt.as<int>(),
@@ -1187,7 +1245,7 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
   W.tiles = t.tiles.as<int4>();
   W.anc = t.anc.as<int>();
   W.chunk_box = t.chunk_box.as<int>();
-  k_leaf_lists<true><<<nblk(std::max(nl, nb2), 128), 128, 0, st>>>(W, nl, nullptr, t.leaves.as<int>(),
+  k_leaf_lists<true><<<nblk(std::max(32LL * nl, (long long)nb2), 128), 128, 0, st>>>(W, nl, nullptr, t.leaves.as<int>(),
                                                      t.bkey.as<unsigned long long>(),
                                                      t.blev.as<unsigned char>(), lo, t.R, &T->lmin, t.child0.as<int>(),
                                                      t.nchild.as<int>(), nullptr, nullptr, t.ustart.as<int>(),
