@@ -103,6 +103,7 @@ __global__ void k_charges_stokes(int n, const int* __restrict__ perm,
                                  const double* __restrict__ hpt, double sd,
                                  c_t<T>* __restrict__ qa, c_t<T>* __restrict__ qb,
                                  c_t<T>* __restrict__ nc, int* __restrict__ next) {
+  pdl_next();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0 && next) *next = 0;
   if (i >= n) return;
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(256) k_charges_drop(const int* __restrict__ st
                                                       const double2* __restrict__ pkw, double sd,
                                                       c_t<T>* __restrict__ nc, double2* __restrict__ za,
                                                       double* __restrict__ pk) {
+  pdl_next();
   __shared__ double red[3][8];
   const int b = blockIdx.x, i0 = start[b], i1 = start[b + 1];
   double v[3] = {0.0, 0.0, 0.0};
@@ -178,6 +180,7 @@ __global__ void k_charges_stokes_df(int n, const int* __restrict__ perm, const d
                                     const double2* __restrict__ dz, const double* __restrict__ hpt,
                                     double s, double winv, const unsigned char* __restrict__ plev,
                                     float4* __restrict__ qdf, float4* __restrict__ nc) {
+  pdl_next();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int o = perm[i];
@@ -215,6 +218,7 @@ __global__ void k_charges_cauchy_df(int n, const int* __restrict__ perm, const d
                                     const double* __restrict__ lu, const double2* __restrict__ dz,
                                     const double* __restrict__ hpt, double winv,
                                     const unsigned char* __restrict__ plev, float4* __restrict__ qdf) {
+  pdl_next();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double rinv = winv * pow2d((int)plev[i]);
@@ -227,6 +231,7 @@ __global__ void k_charges_cauchy(int n, const int* __restrict__ perm,
                                  const double2* __restrict__ q, const double* __restrict__ lu,
                                  const double2* __restrict__ dz, const double* __restrict__ hpt,
                                  c_t<T>* __restrict__ qa, int* __restrict__ next) {
+  pdl_next();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0 && next) *next = 0;
   if (i >= n) return;
@@ -332,6 +337,7 @@ __global__ void __launch_bounds__(256) k_p2m64(const int* __restrict__ leaves,
   const int grp = tid / p, k = tid - grp * p;
   double2 A = make_double2(0.0, 0.0), B = A, C = A;
   const int i0 = pt0[b], i1 = pt1[b];
+  pdl_wait();  // the charges
   const int nbat = (i1 - i0 + 31) / 32;  // batches of equal size
   for (int bt = 0; bt < nbat; ++bt) {
     const int base = i0 + bt * (i1 - i0) / nbat, cnt = i0 + (bt + 1) * (i1 - i0) / nbat - base;
@@ -437,6 +443,7 @@ __global__ void k_m2m64(int offp, int nsplit, const unsigned long long* __restri
   const int P = offp + blockIdx.x / nsplit, sp = blockIdx.x % nsplit;
   const int tid = threadIdx.x, ld = p + 2, nout = E * p;
   const int c0 = child0[P], nc = nchild[P];
+  pdl_wait();
   if (nc == 0) return;  // a leaf: its multipole comes from its points
   const double2* e0inv = einv + 3 * ld;
   const double2* e0pow = epow2 + 3 * ld;
@@ -514,6 +521,7 @@ __global__ void k_l2l64(int offp, int nsplit, const unsigned long long* __restri
   const int ldl = p + 1, ld = p + 2, nout = E * ldl, tid = threadIdx.x;
   const int P = offp + blockIdx.x / nsplit, sp = blockIdx.x % nsplit;
   const int c0 = child0[P], nc = nchild[P];
+  pdl_wait();
   if (nc == 0) return;
   // orders [ja, jb): the work of order j is p + 1 - j terms
   auto cut = [&](int i) { return i >= nsplit ? ldl : (int)(ldl * (1.f - sqrtf(1.f - (float)i / nsplit))); };
@@ -585,6 +593,7 @@ __global__ void k_l2l(int offc, const unsigned long long* __restrict__ bkey,
   const int q = quadrant(bkey[c]);
   c_t<T> eh = epow2[q * ld + 1];
   const c_t<T>* lp = local + (size_t)P * nout;
+  pdl_wait();
   for (int idx = tid; idx < nout; idx += blockDim.x) {
     int e2 = idx / ldl, m = idx - e2 * ldl;
     c_t<T> v = lp[idx];
@@ -792,6 +801,7 @@ __global__ void __launch_bounds__(128, M2L32_CTAS) k_m2l_f32w(int first, int nt,
     float2 acc[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) acc[e] = make_float2(0.f, 0.f);
+    pdl_wait();  // the multipoles
     if (ne > 0) {
       for (int c0 = 0; c0 < ne * CPE; c0 += 32) {
         const int c = c0 + lane, j = min(c / CPE, ne - 1), x = c - j * CPE;
@@ -971,6 +981,7 @@ __global__ void __launch_bounds__(32 * M2L32_WARPS, 4)
       code = vcode[x];
       pd = pdv[code];
     }
+    pdl_wait();  // the multipoles
     for (int c0 = 0; c0 < ne * CM; c0 += 32) {
       const int c = c0 + lane, j = min(c / CM, ne - 1), x = c - j * CM;
       const int sj = __shfl_sync(0xffffffffu, src, j);
@@ -1194,6 +1205,7 @@ __global__ void k_p2m_df(const int* __restrict__ leaves, const int* __restrict__
   const bool acc_thread = which < NA;
   dfacc Rx{0.f, 0.f}, Ry{0.f, 0.f};
   const int i0 = pt0[b], i1 = pt1[b];
+  pdl_wait();  // the charges
   for (int base = i0; base < i1; base += 32) {
     const int cnt = min(32, i1 - base);
     __syncthreads();
@@ -1271,6 +1283,7 @@ __global__ void k_m2m_df(int offp, const unsigned long long* __restrict__ bkey,
   float4* cr = sm4;  // [r][E*p]
   const int P = offp + blockIdx.x, tid = threadIdx.x, ld = p + 2, nout = E * p;
   const int c0 = child0[P], nc = nchild[P];
+  pdl_wait();
   if (nc == 0) return;  // a leaf: its multipole comes from its points
   // four lanes per coefficient: lane r forms c^r from the children's b (lane ci forms child ci's)
   const int o = tid >> 2, part = tid & 3;
@@ -1328,6 +1341,7 @@ __global__ void k_l2l_df(int offc, const unsigned long long* __restrict__ bkey,
   const int q = quadrant(bkey[c]);
   const cdf eh = cdf_from_float4(epow2[q * ld + 1]);
   const float4* lp = local + (size_t)P * nout;
+  pdl_wait();
   for (int idx = tid; idx < nout; idx += blockDim.x) {
     const int e2 = idx / ldl, m = idx - e2 * ldl;
     cdf v = cdf_from_float4(lp[idx]);
@@ -1432,6 +1446,7 @@ __global__ void __launch_bounds__(32 * P2M_CW) k_p2m_chunks(LevOff lo, int nchun
   const int bb = b - first2, c0 = cstart[bb], nc = cstart[bb + 1] - c0;
   const int i0 = pt0[b] + (c - c0) * EB_CHUNK;
   const int cnt = min(pt1[b], i0 + EB_CHUNK) - i0;
+  pdl_wait();  // the charges
   // a box of one chunk gets its multipole directly; otherwise the chunk's part goes to
   // mpart and the box's last chunk to finish adds the parts in chunk order
   float2* dst = nc == 1 ? mpole + (size_t)b * nout : mpart + (size_t)c * nout;
@@ -1526,6 +1541,7 @@ __global__ void __launch_bounds__(32 * P2M_CW, 4) k_p2m_points(LevOff lo, int nc
   const float rinv = lo.rinv[l];
   const int bb = b - first2, c0 = cstart[bb], nc = cstart[bb + 1] - c0;
   const int i0 = pt0[b] + (c - c0) * EB_CHUNK, i1 = min(pt1[b], i0 + EB_CHUNK);
+  pdl_wait();  // the charges
   float2 A[P], S[E == 2 ? P : 1];
 #pragma unroll
   for (int k = 0; k < P; ++k) A[k] = make_float2(0.f, 0.f);
@@ -1606,6 +1622,7 @@ __global__ void k_m2m_f32(int offp, const unsigned long long* __restrict__ bkey,
   float2* a = sm2;
   const int P = offp + blockIdx.x, tid = threadIdx.x, ld = p + 2, nout = E * p;
   const int c0 = child0[P], nc = nchild[P];
+  pdl_wait();
   if (nc == 0) return;  // a leaf: its multipole comes from its points
   for (int idx = tid; idx < nc * nout; idx += blockDim.x) {
     const int ci = idx / nout, o = idx - ci * nout;
@@ -2533,6 +2550,7 @@ template <int K>
 __global__ void __launch_bounds__(128) k_direct64(int n, const double2* __restrict__ zs,
                                                   const double2* __restrict__ q, const int* __restrict__ perm,
                                                   int plus, double2* __restrict__ out, EbPost post) {
+  pdl_wait();
   constexpr bool ST = K == NEAR_V || K == NEAR_VC;
   const int i = blockIdx.x;  // one block of 128 threads per target, the threads over the sources
   const double2 zi = zs[i];
@@ -2554,6 +2572,7 @@ template <int K>
 __global__ void __launch_bounds__(128) k_direct32(int n, const float4* __restrict__ zhl,
                                                   const float2* __restrict__ nc, const int* __restrict__ perm,
                                                   int plus, double2* __restrict__ out, EbPost post) {
+  pdl_wait();
   constexpr bool ST = K != NEAR_Q;
   const int i = blockIdx.x;
   const float4 hi = zhl[i];
@@ -2852,21 +2871,21 @@ int level_split(const eb_ctx* ctx, int nb) { return nb <= ctx->nsm ? 4 : nb <= 3
 
 // M2M into the boxes of level l, L2L out of them.
 template <int E>
-void launch_m2m64(eb_ctx* ctx, EbTree& t, EbTables& tb, int l, double2* mpole, cudaStream_t st) {
+int launch_m2m64(eb_ctx* ctx, EbTree& t, EbTables& tb, int l, double2* mpole, cudaStream_t st) {
   const int p = tb.p, nb = t.lev_off[l + 1] - t.lev_off[l], ns = level_split(ctx, nb);
   const int groups = ((E * p + 7) / 8 + ns - 1) / ns;
-  k_m2m64<E><<<nb * ns, 32 * groups, sizeof(double2) * 4 * E * p, st>>>(
-      t.lev_off[l], ns, t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
-      tb.binom.as<double>(), 2 * p + 2, tb.epow.as<double2>(), tb.einv.as<double2>(), mpole);
+  EB_CUDA_TRY(eb_launch_next(k_m2m64<E>, dim3(nb * ns), dim3(32 * groups), sizeof(double2) * 4 * E * p, st, t.lev_off[l], ns, t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
+      tb.binom.as<double>(), 2 * p + 2, tb.epow.as<double2>(), tb.einv.as<double2>(), mpole));
+  return EB_OK;
 }
 template <int E>
-void launch_l2l64(eb_ctx* ctx, EbTree& t, EbTables& tb, int l, double2* local, cudaStream_t st) {
+int launch_l2l64(eb_ctx* ctx, EbTree& t, EbTables& tb, int l, double2* local, cudaStream_t st) {
   const int p = tb.p, nb = t.lev_off[l + 1] - t.lev_off[l], ns = level_split(ctx, nb);
   // the widest range of orders is the last one
   const int ldl = p + 1, nj = ldl - (ns == 1 ? 0 : (int)(ldl * (1.f - std::sqrt(1.f / ns)))) + 1;
-  k_l2l64<E><<<nb * ns, round32(4 * (E * nj + E - 1)), sizeof(double2) * (E + 4) * (p + 1), st>>>(
-      t.lev_off[l], ns, t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
-      tb.binom.as<double>(), 2 * p + 2, tb.epow.as<double2>(), tb.einv.as<double2>(), local);
+  EB_CUDA_TRY(eb_launch_next(k_l2l64<E>, dim3(nb * ns), dim3(round32(4 * (E * nj + E - 1))), sizeof(double2) * (E + 4) * (p + 1), st, t.lev_off[l], ns, t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
+      tb.binom.as<double>(), 2 * p + 2, tb.epow.as<double2>(), tb.einv.as<double2>(), local));
+  return EB_OK;
 }
 
 // Boxes from which the double-float pipeline takes the fixed-point M2L (the rule's figures in
@@ -2897,15 +2916,14 @@ int fmm_expansions_df(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
   {
     size_t sm = sizeof(float4) * (32 * (size_t)(p + 1) + 96);
     if (sm > 48 * 1024) EB_CUDA_TRY(cudaFuncSetAttribute(k_p2m_df<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_p2m_df<E><<<t.nleaf, std::max(128, round32((E == 2 ? 3 : 1) * p)), sm, st>>>(t.leaves.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(), t.wdf.as<float4>(),
-                                          E == 2 ? w.qdf.as<float4>() : w.ncdf.as<float4>(), p, mp);
+    EB_CUDA_TRY(eb_launch_next(k_p2m_df<E>, dim3(t.nleaf), dim3(std::max(128, round32((E == 2 ? 3 : 1) * p))), sm, st, t.leaves.as<int>(), t.pt0.as<int>(), t.pt1.as<int>(), t.wdf.as<float4>(),
+                                          E == 2 ? w.qdf.as<float4>() : w.ncdf.as<float4>(), p, mp));
     eb_count_launch(ctx);
   }
   for (int l = L - 1; l >= 2; --l) {
     int nb = t.lev_off[l + 1] - t.lev_off[l];
-    k_m2m_df<E><<<nb, round32(4 * E * p), sizeof(float4) * 4 * E * p, st>>>(
-        t.lev_off[l], t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
-        tb.binom_df.as<float2>(), ldb, tb.epow_df.as<float4>(), tb.einv_df.as<float4>(), mp);
+    EB_CUDA_TRY(eb_launch_next(k_m2m_df<E>, dim3(nb), dim3(round32(4 * E * p)), sizeof(float4) * 4 * E * p, st, t.lev_off[l], t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
+        tb.binom_df.as<float2>(), ldb, tb.epow_df.as<float4>(), tb.einv_df.as<float4>(), mp));
     eb_count_launch(ctx);
   }
   {
@@ -2945,9 +2963,8 @@ int fmm_expansions_df(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
   }
   for (int l = 3; l <= L; ++l) {
     int nb = t.lev_off[l + 1] - t.lev_off[l];
-    k_l2l_df<E><<<nb, round32(4 * E * (p + 1)), sizeof(float4) * E * (p + 1), st>>>(
-          t.lev_off[l], t.bkey.as<unsigned long long>(), t.parent.as<int>(), p, tb.binom_df.as<float2>(), ldb,
-          tb.epow_df.as<float4>(), tb.einv_df.as<float4>(), lo);
+    EB_CUDA_TRY(eb_launch_next(k_l2l_df<E>, dim3(nb), dim3(round32(4 * E * (p + 1))), sizeof(float4) * E * (p + 1), st, t.lev_off[l], t.bkey.as<unsigned long long>(), t.parent.as<int>(), p, tb.binom_df.as<float2>(), ldb,
+          tb.epow_df.as<float4>(), tb.einv_df.as<float4>(), lo));
     eb_count_launch(ctx);
   }
   return EB_OK;
@@ -2975,22 +2992,21 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w, bool brea
       lo.rinv[l] = (float)((double)(1u << std::min(l, 30)) / t.W);
     }
     auto p2m = [&](auto kern, size_t sm, auto... order) {
-      kern<<<nblk(t.nchunk, P2M_CW), 32 * P2M_CW, sm, st>>>(
-          lo, t.nchunk, first2, t.blev.as<unsigned char>(), t.plev.as<unsigned char>(), t.chunk_box.as<int>(),
+      return eb_launch_next(
+          kern, dim3(nblk(t.nchunk, P2M_CW)), dim3(32 * P2M_CW), sm, st, lo, t.nchunk, first2, t.blev.as<unsigned char>(), t.plev.as<unsigned char>(), t.chunk_box.as<int>(),
           t.cstart.as<int>(), t.keys.as<unsigned long long>(), t.pt0.as<int>(), t.pt1.as<int>(), t.wdf.as<float4>(),
           reinterpret_cast<const float2*>(w.qa.p), reinterpret_cast<const float2*>(w.qb.p), order...,
           w.mpart.as<float2>(), t.cdone.as<int>(), reinterpret_cast<float2*>(w.mpole.p));
     };
-    if (p == 20) p2m(k_p2m_points<E, 20>, 0);
-    else p2m(k_p2m_chunks<E>, p2m_smem(p), p);
+    if (p == 20) EB_CUDA_TRY(p2m(k_p2m_points<E, 20>, 0));
+    else EB_CUDA_TRY(p2m(k_p2m_chunks<E>, p2m_smem(p), p));
     eb_count_launch(ctx);
     for (int l = lmin - 1; l >= 2; --l) {
       int nb = t.lev_off[l + 1] - t.lev_off[l];
       size_t sm2 = sizeof(float2) * 4 * (size_t)nout;
-      k_m2m_f32<E><<<nb, std::max(128, round32(nout)), sm2, st>>>(
-          t.lev_off[l], t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
+      EB_CUDA_TRY(eb_launch_next(k_m2m_f32<E>, dim3(nb), dim3(std::max(128, round32(nout))), sm2, st, t.lev_off[l], t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
           reinterpret_cast<const float*>(tb.binom.p), ldb, reinterpret_cast<const float2*>(tb.epow.p),
-          reinterpret_cast<const float2*>(tb.einv.p), reinterpret_cast<float2*>(w.mpole.p));
+          reinterpret_cast<const float2*>(tb.einv.p), reinterpret_cast<float2*>(w.mpole.p)));
       eb_count_launch(ctx);
     }
   } else {
@@ -2998,10 +3014,10 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w, bool brea
     auto go = [&](auto kern) -> int {
       if (sm > 48 * 1024)
         EB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-      kern<<<t.nleaf, round32(P2M_NG * p), sm, st>>>(t.leaves.as<int>(), t.bkey.as<unsigned long long>(),
+      EB_CUDA_TRY(eb_launch_next(kern, dim3(t.nleaf), dim3(round32(P2M_NG * p)), sm, st, t.leaves.as<int>(), t.bkey.as<unsigned long long>(),
                                                      t.blev.as<unsigned char>(), t.pt0.as<int>(), t.pt1.as<int>(),
                                                      t.zs.as<double2>(), w.qa.as<double2>(), w.qb.as<double2>(), t.x0,
-                                                     t.y0, t.W, 1.0 / t.W, p, w.mpole.as<double2>());
+                                                     t.y0, t.W, 1.0 / t.W, p, w.mpole.as<double2>()));
       return EB_OK;
     };
     if (E == 2 && breal) EB_TRY(go(k_p2m64<E, true>));
@@ -3009,7 +3025,7 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w, bool brea
     eb_count_launch(ctx);
     if (after_p2m) EB_TRY(after_p2m());
     for (int l = L - 1; l >= 2; --l) {
-      launch_m2m64<E>(ctx, t, tb, l, w.mpole.as<double2>(), st);
+      EB_TRY(launch_m2m64<E>(ctx, t, tb, l, w.mpole.as<double2>(), st));
       eb_count_launch(ctx);
     }
   }
@@ -3027,9 +3043,8 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w, bool brea
       const float2* m = reinterpret_cast<const float2*>(mp.p);
       float2* out = reinterpret_cast<float2*>(w.local.p);
       if (n < M2L32_WIDE) {
-        k_m2l_f32w<E, 20><<<std::min(n, M2L32_CTAS * ctx->nsm), 128, 0, st>>>(
-            first, n, list.as<int>(), code.as<unsigned char>(), count.as<int>(), tb.binom_t.as<float>(), dinv,
-            tb.pd.as<int>(), m, out, accumulate);
+        EB_CUDA_TRY(eb_launch_next(k_m2l_f32w<E, 20>, dim3(std::min(n, M2L32_CTAS * ctx->nsm)), dim3(128), 0, st, first, n, list.as<int>(), code.as<unsigned char>(), count.as<int>(), tb.binom_t.as<float>(), dinv,
+            tb.pd.as<int>(), m, out, accumulate));
         return EB_OK;
       }
       // boxes per warp: 6 have the 32 entries of a round on average, 16 in several rounds
@@ -3038,9 +3053,8 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w, bool brea
       const int nc = std::min(ncoarse, n), nb = n >= 256 * ctx->nsm ? 16 : 6;
       constexpr size_t sm = sizeof(M2l32Smem<E, 20>);
       EB_CUDA_TRY(cudaFuncSetAttribute(k_m2l_f32p<E, 20>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-      k_m2l_f32p<E, 20><<<nblk(nc + nblk(n - nc, nb), M2L32_WARPS), 32 * M2L32_WARPS, sm, st>>>(
-          first, n, nc, nb, list.as<int>(), code.as<unsigned char>(), count.as<int>(), dinv, tb.pd.as<int>(), m, out,
-          accumulate);
+      EB_CUDA_TRY(eb_launch_next(k_m2l_f32p<E, 20>, dim3(nblk(nc + nblk(n - nc, nb), M2L32_WARPS)), dim3(32 * M2L32_WARPS), sm, st, first, n, nc, nb, list.as<int>(), code.as<unsigned char>(), count.as<int>(), dinv, tb.pd.as<int>(), m, out,
+          accumulate));
       return EB_OK;
     };
     if (nt > 0 && sizeof(T) == 4 && p == 20 && ctx->opts.m2l_tc > 0) {
@@ -3088,11 +3102,10 @@ int fmm_expansions(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w, bool brea
     for (int l = 3; l <= lend; ++l) {
       int nb = t.lev_off[l + 1] - t.lev_off[l];
       if (sizeof(T) == 8)
-        launch_l2l64<E>(ctx, t, tb, l - 1, w.local.as<double2>(), st);
+        EB_TRY(launch_l2l64<E>(ctx, t, tb, l - 1, w.local.as<double2>(), st));
       else
-        k_l2l<float, E><<<nb, round32(E * (p + 1)), sizeof(float2) * E * (p + 1), st>>>(
-            t.lev_off[l], t.bkey.as<unsigned long long>(), t.parent.as<int>(), p, tb.binom.as<float>(), ldb,
-            tb.epow.as<float2>(), tb.einv.as<float2>(), w.local.as<float2>());
+        EB_CUDA_TRY(eb_launch_next(k_l2l<float, E>, dim3(nb), dim3(round32(E * (p + 1))), sizeof(float2) * E * (p + 1), st, t.lev_off[l], t.bkey.as<unsigned long long>(), t.parent.as<int>(), p, tb.binom.as<float>(), ldb,
+            tb.epow.as<float2>(), tb.einv.as<float2>(), w.local.as<float2>()));
       eb_count_launch(ctx);
     }
   }
@@ -3126,6 +3139,12 @@ int direct_run(eb_ctx* ctx, EbTree& t, bool f32, int sign, const double2* dens, 
   const int g = n;  // one block of 128 threads per target
   const int kind = near_kind<E>(sign, dz, post);
   const bool plus = sign > 0;
+  // right behind the charges, unless another stream's sums have to be waited for too
+  cudaError_t ce = cudaSuccess;
+  auto go = [&](auto kern, auto... a) {
+    if (join) kern<<<g, 128, 0, st>>>(a...);
+    else ce = eb_launch_next(kern, dim3(g), dim3(128), 0, st, a...);
+  };
   if (f32) {
     const float4* zh = t.zhl.as<float4>();
     const float2* q = E == 2 ? w.nc.as<float2>() : w.qa.as<float2>();
@@ -3141,9 +3160,9 @@ int direct_run(eb_ctx* ctx, EbTree& t, bool f32, int sign, const double2* dens, 
       k_charges_cauchy<float><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q_in, post.u, post.dz, post.hpt,
                                                             w.qa.as<float2>(), nullptr);
     if (join) EB_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
-    if (E == 1) k_direct32<NEAR_Q><<<g, 128, 0, st>>>(n, zh, q, t.perm.as<int>(), 0, out, post);
-    else if (kind == NEAR_V) k_direct32<NEAR_V><<<g, 128, 0, st>>>(n, zh, q, t.perm.as<int>(), plus, out, post);
-    else k_direct32<NEAR_VC><<<g, 128, 0, st>>>(n, zh, q, t.perm.as<int>(), plus, out, post);
+    if (E == 1) go(k_direct32<NEAR_Q>, n, zh, q, t.perm.as<int>(), 0, out, post);
+    else if (kind == NEAR_V) go(k_direct32<NEAR_V>, n, zh, q, t.perm.as<int>(), plus, out, post);
+    else go(k_direct32<NEAR_VC>, n, zh, q, t.perm.as<int>(), plus, out, post);
   } else {
     const double2* zz = t.zs.as<double2>();
     const double2* q = E == 2 ? w.nc.as<double2>() : w.qa.as<double2>();
@@ -3159,11 +3178,12 @@ int direct_run(eb_ctx* ctx, EbTree& t, bool f32, int sign, const double2* dens, 
       k_charges_cauchy<double><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q_in, post.u, post.dz, post.hpt,
                                                              w.qa.as<double2>(), nullptr);
     if (join) EB_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
-    if (kind == NEAR_Q) k_direct64<NEAR_Q><<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), 0, out, post);
-    else if (kind == NEAR_QI) k_direct64<NEAR_QI><<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), 0, out, post);
-    else if (kind == NEAR_V) k_direct64<NEAR_V><<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), plus, out, post);
-    else k_direct64<NEAR_VC><<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), plus, out, post);
+    if (kind == NEAR_Q) go(k_direct64<NEAR_Q>, n, zz, q, t.perm.as<int>(), 0, out, post);
+    else if (kind == NEAR_QI) go(k_direct64<NEAR_QI>, n, zz, q, t.perm.as<int>(), 0, out, post);
+    else if (kind == NEAR_V) go(k_direct64<NEAR_V>, n, zz, q, t.perm.as<int>(), plus, out, post);
+    else go(k_direct64<NEAR_VC>, n, zz, q, t.perm.as<int>(), plus, out, post);
   }
+  EB_CUDA_TRY(ce);
   ctx->launches += 2;
   return eb_check_launch(ctx, "direct sum");
 }

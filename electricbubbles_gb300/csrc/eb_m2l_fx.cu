@@ -145,6 +145,7 @@ __device__ __forceinline__ long long float_fix(float f, int S) {  // f 2^(61 - S
 template <int E, bool DF>
 __global__ void __launch_bounds__(128) k_m2l_fix(int first, int nb, int p, const void* __restrict__ mpole,
                                                  longlong2* __restrict__ fx, int4* __restrict__ fs) {
+  pdl_wait();
   const int wb = (blockIdx.x * 128 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (wb >= nb) return;
   const size_t b = (size_t)(first + wb), n = (size_t)E * p;
@@ -255,6 +256,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
                                                           const longlong2* __restrict__ fx,
                                                           const int4* __restrict__ fs, void* __restrict__ local,
                                                           int accumulate, int nsingle, int group) {
+  pdl_wait();
   constexpr int NE = FX_ROWS / (2 * E);  // entries of a round
   constexpr int NW = FX_TEAM / 32;
   // 256 in each digit, see store_digits
@@ -530,7 +532,7 @@ int fx_launch(eb_ctx* ctx, int first, int ntarget, int nsrc, int ncoarse, const 
   EB_TRY(w.mfix.ensure((sizeof(longlong2) * E * (size_t)p + sizeof(int4)) * (size_t)(first + nsrc)));
   longlong2* fx = w.mfix.as<longlong2>();
   int4* fs = reinterpret_cast<int4*>(fx + (size_t)(first + nsrc) * E * p);
-  k_m2l_fix<E, DF><<<(nsrc * 32 + 127) / 128, 128, 0, st>>>(first, nsrc, p, mpole, fx, fs);
+  EB_CUDA_TRY(eb_launch_next(k_m2l_fix<E, DF>, dim3((nsrc * 32 + 127) / 128), dim3(128), 0, st, first, nsrc, p, mpole, fx, fs));
   constexpr int sm = FX_ND * (2 * FX_A + FX_B) + 1024;
   EB_CUDA_TRY(cudaFuncSetAttribute(k_m2l_fx<E, DF>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   // Items of about a round's entries: single boxes on the coarse levels (their lists are
@@ -539,9 +541,9 @@ int fx_launch(eb_ctx* ctx, int first, int ntarget, int nsrc, int ncoarse, const 
   const int nsingle = std::min(ncoarse, ntarget);
   const int nitem = nsingle + (ntarget - nsingle + group - 1) / group;
   const int grid = std::min((nitem + 1) / 2, ctx->nsm);
-  k_m2l_fx<E, DF><<<grid, FX_THREADS, sm, st>>>(first, ntarget, vlist, vcode, vcount, p, reinterpret_cast<const uint4*>(tb.fxb),
+  EB_CUDA_TRY(eb_launch_next(k_m2l_fx<E, DF>, dim3(grid), dim3(FX_THREADS), sm, st, first, ntarget, vlist, vcode, vcount, p, reinterpret_cast<const uint4*>(tb.fxb),
                                                tb.fxt.as<int4>(), reinterpret_cast<const int*>(tb.fxr), tb.pd.as<int>(), fx, fs, local,
-                                               accumulate, nsingle, group);
+                                               accumulate, nsingle, group));
   ctx->launches += 2;
   return EB_OK;
 }

@@ -113,6 +113,7 @@ __device__ __forceinline__ void vtw_partials(int n, int ncol, int with_w, const 
 __global__ void k_vtw(int n, int ncol, const int* __restrict__ ncol_dev, const double* __restrict__ V,
                       size_t ldv, const double* __restrict__ w, double* __restrict__ part,
                       double* __restrict__ out, unsigned int* __restrict__ ticket, int with_w = 0) {
+  pdl_wait();
   if (ncol_dev) ncol = *ncol_dev;
   vtw_partials(n, ncol, with_w, V, ldv, w, part);
   finish_columns(gridDim.x, ncol + with_w, part, out, ticket);
@@ -158,6 +159,7 @@ __global__ void k_update_vtw(int n, int ncol, const int* __restrict__ ncol_dev, 
                              size_t ldv, const double* __restrict__ hin, double* w,
                              double* __restrict__ part, double* __restrict__ out,
                              unsigned int* __restrict__ ticket) {
+  pdl_wait();
   __shared__ double hs[128];
   if (ncol_dev) ncol = *ncol_dev;
   for (int j = threadIdx.x; j < ncol; j += blockDim.x) hs[j] = hin[j];
@@ -588,6 +590,7 @@ __global__ void k_gm_init(GmCtl* c, const double* __restrict__ hdev, cudaGraphCo
 // V[:, store_col] = xin = scale * src while the iteration continues (src may alias V).
 __global__ void k_gm_store(int n, const GmCtl* __restrict__ c, const double* src, double* V, size_t ldv,
                            double* __restrict__ xin) {
+  pdl_wait();
   if (!c->cont) return;
   const double sc = c->scale;
   double* dst = V + (size_t)c->store_col * ldv;
@@ -654,6 +657,7 @@ template <int PASSES>
 __global__ void __cluster_dims__(GM_CL, 1, 1) __launch_bounds__(GM_CL_THREADS)
     k_gm_step(int n, int ncol, double* V, size_t ldv, double* w, double* h1, double* h2, double* nw, GmCtl* c,
               double* hdev, double* __restrict__ xin, cudaGraphConditionalHandle h) {
+  pdl_wait();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   __shared__ double ws[GM_CL_THREADS];
@@ -762,7 +766,7 @@ template <int PASSES>
 int gm_step(cudaStream_t s, int n, int ncol, double* V, size_t ldv, double* w, double* h1, double* h2, double* nw,
             GmCtl* c, double* hdev, double* xin, cudaGraphConditionalHandle h) {
   EB_CUDA_TRY(cudaFuncSetAttribute(k_gm_step<PASSES>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  k_gm_step<PASSES><<<GM_CL, GM_CL_THREADS, 0, s>>>(n, ncol, V, ldv, w, h1, h2, nw, c, hdev, xin, h);
+  EB_CUDA_TRY(eb_launch_next(k_gm_step<PASSES>, dim3(GM_CL), dim3(GM_CL_THREADS), 0, s, n, ncol, V, ldv, w, h1, h2, nw, c, hdev, xin, h));
   return EB_OK;
 }
 
@@ -773,6 +777,7 @@ __global__ void k_gm_sub_arnoldi(int n, const int* __restrict__ ncol_dev, const 
                                  double* __restrict__ part, double* hdev,
                                  unsigned int* __restrict__ ticket, GmCtl* c,
                                  cudaGraphConditionalHandle h) {
+  pdl_wait();
   if (!gemv_sub(n, 0, ncol_dev, V, ldv, hcol, w, part, hdev + GM_NW, ticket)) return;
   __syncthreads();
   if (threadIdx.x < 32) gm_arnoldi_warp(c, hdev, h);
@@ -785,6 +790,7 @@ __global__ void k_gm_vtw_arnoldi(int n, const int* __restrict__ ncol_dev, const 
                                  size_t ldv, const double* __restrict__ w, double* __restrict__ part,
                                  double* hdev, unsigned int* __restrict__ ticket, GmCtl* c,
                                  cudaGraphConditionalHandle h) {
+  pdl_wait();
   const int ncol = *ncol_dev;
   vtw_partials(n, ncol, 1, V, ldv, w, part);
   if (!finish_columns(gridDim.x, ncol + 1, part, hdev + GM_H1, ticket)) return;
@@ -798,6 +804,7 @@ __global__ void k_gm_vtw_arnoldi(int n, const int* __restrict__ ncol_dev, const 
 __global__ void k_gm_sub_store(int n, const GmCtl* __restrict__ c, double* V, size_t ldv,
                                const double* __restrict__ h, const double* __restrict__ w,
                                double* __restrict__ xin) {
+  pdl_wait();
   if (!c->cont) return;
   const int col = c->store_col;  // columns 0..col-1 are read, column col written
   sub_scale_store(n, col, V, ldv, h, w, c->scale, V + (size_t)col * ldv, xin);
@@ -959,13 +966,13 @@ int build_graph(eb_ctx* ctx, GmGraph& G, int kind, op_fn op, int n, int maxl) {
     if (refine) {
       // one Gram-Schmidt pass for the inner FP32 cycle (the H2 slots stay zero), its
       // norm by Pythagoras from the same reduction, the update fused with the store
-      k_gm_vtw_arnoldi<<<nb, RBS, 0, s>>>(n, lld, V, ldv, wbuf, part, hdev, ticket, ctl, h);
-      k_gm_sub_store<<<nb, RBS, 0, s>>>(n, ctl, V, ldv, hdev + GM_H1, wbuf, xin);
+      EB_CUDA_TRY(eb_launch_next(k_gm_vtw_arnoldi, dim3(nb), dim3(RBS), 0, s, n, lld, V, ldv, wbuf, part, hdev, ticket, ctl, h));
+      EB_CUDA_TRY(eb_launch_next(k_gm_sub_store, dim3(nb), dim3(RBS), 0, s, n, ctl, V, ldv, hdev + GM_H1, wbuf, xin));
     } else {
-      k_vtw<<<nb, RBS, 0, s>>>(n, 0, lld, V, ldv, wbuf, part, hdev + GM_H1, ticket);
-      k_update_vtw<<<nb, RBS, 0, s>>>(n, 0, lld, V, ldv, hdev + GM_H1, wbuf, part, hdev + GM_H2, ticket);
-      k_gm_sub_arnoldi<<<nb, RBS, 0, s>>>(n, lld, V, ldv, hdev + GM_H2, wbuf, part, hdev, ticket, ctl, h);
-      k_gm_store<<<nb, RBS, 0, s>>>(n, ctl, wbuf, V, ldv, xin);
+      EB_CUDA_TRY(eb_launch_next(k_vtw, dim3(nb), dim3(RBS), 0, s, n, 0, lld, V, ldv, wbuf, part, hdev + GM_H1, ticket, 0));
+      EB_CUDA_TRY(eb_launch_next(k_update_vtw, dim3(nb), dim3(RBS), 0, s, n, 0, lld, V, ldv, hdev + GM_H1, wbuf, part, hdev + GM_H2, ticket));
+      EB_CUDA_TRY(eb_launch_next(k_gm_sub_arnoldi, dim3(nb), dim3(RBS), 0, s, n, lld, V, ldv, hdev + GM_H2, wbuf, part, hdev, ticket, ctl, h));
+      EB_CUDA_TRY(eb_launch_next(k_gm_store, dim3(nb), dim3(RBS), 0, s, n, ctl, wbuf, V, ldv, xin));
     }
     ctx->launches += refine ? 2 : 4;
     return eb_check_launch(ctx, "gmres graph (body)");
