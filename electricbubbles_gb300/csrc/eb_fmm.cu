@@ -1328,50 +1328,73 @@ __global__ void k_m2m_df(int offp, const unsigned long long* __restrict__ bkey,
   if (act && part == 0) mpole[(size_t)P * nout + o] = cdf_f4(cdf_mul(cdf_from_float4(epow2[3 * ld + n]), v));
 }
 
+// L2L of a level's boxes into all their children at once (see k_l2l64): the four lanes of an
+// output form the sums S_r of all children, then one child each. Measured (E = 2): a level of
+// 64 x 512 nodes 8.0 -> 5.8 us on average, of 1,024 x 1,024 100 -> 49 us.
 template <int E>
-__global__ void k_l2l_df(int offc, const unsigned long long* __restrict__ bkey,
-                         const int* __restrict__ parent, int p, const float2* __restrict__ binom,
-                         int ldb, const float4* __restrict__ epow2, const float4* __restrict__ einv,
-                         float4* __restrict__ local) {
+__global__ void k_l2l_df(int offp, const unsigned long long* __restrict__ bkey,
+                         const int* __restrict__ child0, const int* __restrict__ nchild, int p,
+                         const float2* __restrict__ binom, int ldb, const float4* __restrict__ epow2,
+                         const float4* __restrict__ einv, float4* __restrict__ local) {
   extern __shared__ float4 sm4[];
-  float4* a = sm4;
+  float4* a = sm4;                  // [E][p + 1]
+  float4* sph = a + E * (p + 1);    // [rot][p + 1]: the children's phi', for psi
+  __shared__ int s_child[4];
   const int ldl = p + 1, ld = p + 2, nout = E * ldl, tid = threadIdx.x;
-  const int c = offc + blockIdx.x;
-  const int P = parent[c];
-  const int q = quadrant(bkey[c]);
-  const cdf eh = cdf_from_float4(epow2[q * ld + 1]);
-  const float4* lp = local + (size_t)P * nout;
+  const int P = offp + blockIdx.x;
+  const int c0 = child0[P], nc = nchild[P];
   pdl_wait();
-  for (int idx = tid; idx < nout; idx += blockDim.x) {
-    const int e2 = idx / ldl, m = idx - e2 * ldl;
-    cdf v = cdf_from_float4(lp[idx]);
-    if (e2 == 1 && m < p)
-      v = cdf_add(v, cdf_mul(cdf_scale(cdf_conj(eh), (float)(m + 1)), cdf_from_float4(lp[m + 1])));
-    a[idx] = cdf_f4(cdf_mul(v, cdf_from_float4(epow2[q * ld + m])));
-  }
+  if (nc == 0) return;
+  if (tid < 4) s_child[tid] = -1;
   __syncthreads();
-  // 4 lanes per output, each summing every 4th term
+  if (tid < nc) s_child[quad_rot(quadrant(bkey[c0 + tid]))] = c0 + tid;
+  const float4* e0pow = epow2 + 3 * ld;
+  const float4* lp = local + (size_t)P * nout;
+  for (int idx = tid; idx < nout; idx += blockDim.x)
+    a[idx] = cdf_f4(cdf_mul(cdf_from_float4(lp[idx]), cdf_from_float4(e0pow[idx % ldl])));
+  __syncthreads();
   const int o = tid >> 2, part = tid & 3;
-  const bool act = o < nout;
-  const int oo = act ? o : 0;
-  const int e = oo / ldl, j = oo - e * ldl;
-  const float4* ae = a + e * ldl;
+  const bool act = o < nout, psi = act && o >= ldl;
+  const int j = !act ? p : psi ? o - ldl : o;
+  const float4* ae = a + (psi ? ldl : 0);
   dfacc sx{0.f, 0.f}, sy{0.f, 0.f};
   if (act) {
+#pragma unroll 4
     for (int m = j + part; m <= p; m += 4) {
       const float2 bm = binom[(size_t)m * ldb + j];
       cacc_rmul(sx, sy, dfl{bm.x, bm.y}, cdf_from_float4(ae[m]));
     }
   }
-  const cdf ssum = quad_merge(sx, sy);
-  if (act && part == 0) {
-    float4* lc = local + (size_t)c * nout;
-    dfacc rx{0.f, 0.f}, ry{0.f, 0.f};
-    const cdf old = cdf_from_float4(lc[o]);
-    acc_dfl(rx, old.x);
-    acc_dfl(ry, old.y);
-    cacc_mul(rx, ry, cdf_from_float4(einv[q * ld + j]), ssum);
-    lc[o] = cdf_f4(cacc_value(rx, ry));
+  // child `part` (rot): sum_r i^(rot r) S_r, S_r in the quad's lane r
+  const cdf s = cacc_value(sx, sy);
+  const int q0 = (tid & 31) & ~3;
+  cdf v{{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const cdf t{{__shfl_sync(0xffffffffu, s.x.hi, q0 + r), __shfl_sync(0xffffffffu, s.x.lo, q0 + r)},
+                {__shfl_sync(0xffffffffu, s.y.hi, q0 + r), __shfl_sync(0xffffffffu, s.y.lo, q0 + r)}};
+    const int k = (part * r) & 3;  // times i^k
+    const dfl tx = k & 1 ? t.y : t.x, ty = k & 1 ? t.x : t.y;
+    v.x = dfl_add(v.x, k == 1 || k == 2 ? dfl_neg(tx) : tx);
+    v.y = dfl_add(v.y, k >= 2 ? dfl_neg(ty) : ty);
+  }
+  v = cdf_mul(cdf_from_float4(einv[3 * ld + j]), v);
+  if (E == 2) {
+    if (act && !psi) sph[part * ldl + j] = cdf_f4(v);
+    __syncthreads();
+    if (psi && j < p) {
+      // conj(e_0 i^rot) (j + 1) phi': both parts of the conjugate are +- 1/2
+      const cdf ph = cdf_from_float4(sph[part * ldl + j + 1]);
+      const bool nx = part == 1 || part == 2, ny = part <= 1;  // its signs
+      const dfl xx = nx ? dfl_neg(ph.x) : ph.x, xy = nx ? dfl_neg(ph.y) : ph.y;
+      const dfl yx = ny ? dfl_neg(ph.x) : ph.x, yy = ny ? dfl_neg(ph.y) : ph.y;
+      v = cdf_add(v, cdf_scale(cdf{dfl_sub(xx, yy), dfl_add(xy, yx)}, 0.5f * (float)(j + 1)));
+    }
+  }
+  const int c = s_child[part];
+  if (act && c >= 0) {
+    float4* lc = local + (size_t)c * nout + o;
+    *lc = cdf_f4(cdf_add(cdf_from_float4(*lc), v));
   }
 }
 
@@ -2961,10 +2984,12 @@ int fmm_expansions_df(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
     }
     ps.done();
   }
-  for (int l = 3; l <= L; ++l) {
-    int nb = t.lev_off[l + 1] - t.lev_off[l];
-    EB_CUDA_TRY(eb_launch_next(k_l2l_df<E>, dim3(nb), dim3(round32(4 * E * (p + 1))), sizeof(float4) * E * (p + 1), st, t.lev_off[l], t.bkey.as<unsigned long long>(), t.parent.as<int>(), p, tb.binom_df.as<float2>(), ldb,
-          tb.epow_df.as<float4>(), tb.einv_df.as<float4>(), lo));
+  for (int l = 2; l < L; ++l) {
+    const int nb = t.lev_off[l + 1] - t.lev_off[l];
+    EB_CUDA_TRY(eb_launch_next(k_l2l_df<E>, dim3(nb), dim3(round32(4 * E * (p + 1))),
+                               sizeof(float4) * (E + (E == 2 ? 4 : 0)) * (p + 1), st, t.lev_off[l],
+                               t.bkey.as<unsigned long long>(), t.child0.as<int>(), t.nchild.as<int>(), p,
+                               tb.binom_df.as<float2>(), ldb, tb.epow_df.as<float4>(), tb.einv_df.as<float4>(), lo));
     eb_count_launch(ctx);
   }
   return EB_OK;
