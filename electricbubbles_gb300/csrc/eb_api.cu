@@ -144,6 +144,16 @@ int copy_in(eb_ctx* ctx, DevBuf& buf, const void* src, size_t bytes, int mem) {
 // these definitions C linkage.
 // ---------------------------------------------------------------------------------
 
+// Memory of the context's device, aligned to `align` bytes: what its kernels may read in place.
+bool eb_on_device(const eb_ctx* ctx, const void* p, size_t align) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == ctx->device && (uintptr_t)p % align == 0;
+}
+
 int eb_version(void) { return EB_GB300_VERSION; }
 
 const char* eb_status_string(int s) {
@@ -374,15 +384,7 @@ int eb_set_geometry(eb_ctx* ctx, int k, const int* nd, const double* z, const do
   const size_t bytes[5] = {sizeof(double2) * nbk, sizeof(double2) * nbk, sizeof(double) * nbk, sizeof(double) * nbk,
                            sizeof(double2) * k};
   // read in place: this device's memory, aligned for the loads (others are copied first)
-  auto readable = [&](int i) {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, src[i]) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    return at.type == cudaMemoryTypeDevice && at.device == ctx->device &&
-           (uintptr_t)src[i] % (i == 2 || i == 3 ? 8 : 16) == 0;
-  };
+  auto readable = [&](int i) { return eb_on_device(ctx, src[i], i == 2 || i == 3 ? 8 : 16); };
   for (int i = 0; i < 5; ++i) {
     if (mem == EB_HOST || !readable(i)) {
       EB_TRY(copy_in(ctx, *buf[i], src[i], bytes[i], mem));

@@ -423,6 +423,7 @@ int eb_m2l_fx(eb_ctx* ctx, int E, bool df, int first, int ntarget, int nsrc, int
 int eb_m2l_fx_tables(EbTables& tb);
 
 // api.cu: (re)build the installed geometry's tree with the current eb_opts
+bool eb_on_device(const eb_ctx* ctx, const void* p, size_t align);
 int eb_geom_tree(eb_ctx* ctx);
 
 // api.cu helpers

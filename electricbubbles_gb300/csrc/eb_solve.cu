@@ -252,6 +252,22 @@ __global__ void k_axpy(int n, double s, const double* __restrict__ a, double* __
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v[i] += s * a[i];
 }
 
+// The start of a solve in one launch: b = rhs, x = rhs (or zero, and z = b, for a refined
+// solve, whose first residual is b), the reduction ticket and the first inner tolerance.
+__global__ void k_solve_start(int n, const double* rhs, double* b, double* z, double* x, int zero_x,
+                              unsigned int* ticket, double* tol_dev, double tol) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *ticket = 0u;
+    if (zero_x) *tol_dev = tol;
+  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double v = rhs[i];
+    b[i] = v;
+    x[i] = zero_x ? 0.0 : v;
+    if (zero_x) z[i] = v;
+  }
+}
+
 typedef int (*op_fn)(eb_ctx*, const double*, double*, int);
 
 struct Gm {
@@ -1112,9 +1128,7 @@ int solve_graph(eb_ctx* ctx, int n, op_fn op, int mode, int maxl, eb_solve_info*
     inf->matvecs64 = 1 + head.lgmr;
     return EB_OK;
   }
-  double* x = ctx->gX.as<double>();
-  EB_CUDA_TRY(cudaMemsetAsync(x, 0, sizeof(double) * n, s));
-  EB_CUDA_TRY(cudaMemcpyAsync(ctx->gZ.p, ctx->gR.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+  // (k_solve_start has set x = 0, the residual to b and the first step's tolerance)
   inf->ierr = 1;
   double bnrm = 0.0;
   double err_prev = 1.0;
@@ -1159,8 +1173,6 @@ int solve_graph(eb_ctx* ctx, int n, op_fn op, int mode, int maxl, eb_solve_info*
     if (!ctx->h_spec) EB_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&ctx->h_spec), 2 * GM_HEAD));
     GmCtl* h1 = reinterpret_cast<GmCtl*>(ctx->h_spec);
     GmCtl* h2 = reinterpret_cast<GmCtl*>(ctx->h_spec + GM_HEAD);
-    const double itol = inner_tolerance(ctx, 1, err_prev);
-    EB_CUDA_TRY(cudaMemcpyAsync(ctx->gH.as<double>() + GM_TOL, &itol, sizeof(double), cudaMemcpyHostToDevice, s));
     long long b1 = 0, p1 = 0, b2 = 0, p2 = 0;
     EB_TRY(run_graph(ctx, GM_REFINE, op, n, maxl, h1, false, &b1, &p1));
     k_gm_next_tol<<<1, 32, 0, s>>>(ctx->gCtl.as<GmCtl>(), ctx->gH.as<double>() + GM_TOL, ctx->opts.inner_tol,
@@ -1180,8 +1192,10 @@ int solve_graph(eb_ctx* ctx, int n, op_fn op, int mode, int maxl, eb_solve_info*
     first = 3;
   }
   for (int outer = first; outer <= ctx->opts.max_outer; ++outer) {
-    const double itol = inner_tolerance(ctx, outer, err_prev);
-    EB_CUDA_TRY(cudaMemcpyAsync(ctx->gH.as<double>() + GM_TOL, &itol, sizeof(double), cudaMemcpyHostToDevice, s));
+    if (outer > 1) {
+      const double itol = inner_tolerance(ctx, outer, err_prev);
+      EB_CUDA_TRY(cudaMemcpyAsync(ctx->gH.as<double>() + GM_TOL, &itol, sizeof(double), cudaMemcpyHostToDevice, s));
+    }
     EB_TRY(run_graph(ctx, GM_REFINE, op, n, maxl, &head));
     bool done = false;
     EB_TRY(step_done(outer, head, &done));
@@ -1205,10 +1219,10 @@ int solve(eb_ctx* ctx, int n, op_fn op, const double* rhs, double* soln, int mod
   EB_TRY(ctx->gPart.ensure(sizeof(double) * (size_t)rmaxb(ctx) * (maxl + 2)));
   EB_TRY(ctx->gH.ensure(sizeof(double) * std::max(3 * (maxl + 2), (int)GM_HSIZE)));
   EB_TRY(ctx->gTicket.ensure(sizeof(unsigned int)));
-  EB_CUDA_TRY(cudaMemsetAsync(ctx->gTicket.p, 0, sizeof(unsigned int), s));
   g.ticket = ctx->gTicket.as<unsigned int>();
   EB_TRY(ctx->gR.ensure(sizeof(double) * n));
   EB_TRY(ctx->gX.ensure(sizeof(double) * n));
+  EB_TRY(ctx->gZ.ensure(sizeof(double) * n));
   double* b = ctx->gR.as<double>();
   double* x = ctx->gX.as<double>();
   const bool defl = op == eb_laplace_matvec_dev && ctx->opts.lap_deflate > 0;
@@ -1222,13 +1236,20 @@ int solve(eb_ctx* ctx, int n, op_fn op, const double* rhs, double* soln, int mod
   }
   // SOLVEI / SOLVE_LAPL: soln = rhs as the initial guess (stokesbubb.f:346-349); the
   // deflated solve starts from t0 = M rhs, which is x0 = rhs.
-  cudaMemcpyKind kin = mem == EB_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
+  // A refined solve starts from x = 0.
+  const bool refine = mode != EB_SOLVE_FP64;
+  if (mem == EB_HOST || !eb_on_device(ctx, rhs, sizeof(double))) {
+    EB_CUDA_TRY(cudaMemcpyAsync(b, rhs, sizeof(double) * n, mem == EB_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s));
+    rhs = b;
+  }
+  k_solve_start<<<g.nb, RBS, 0, s>>>(n, rhs, b, ctx->gZ.as<double>(), x, refine, g.ticket,
+                                     ctx->gH.as<double>() + GM_TOL, inner_tolerance(ctx, 1, 1.0));
+  eb_count_launch(ctx);
   auto init_x = [&]() -> int {
-    EB_CUDA_TRY(cudaMemcpyAsync(x, rhs, sizeof(double) * n, kin, s));
+    if (refine) return EB_OK;  // (the host-driven loop starts from zero by itself)
     if (defl) EB_TRY(deflate(ctx, x, x, 0));
     return EB_OK;
   };
-  EB_CUDA_TRY(cudaMemcpyAsync(b, rhs, sizeof(double) * n, kin, s));
   EB_TRY(init_x());
   eb_solve_info inf{};
   int st = EB_OK;
@@ -1240,6 +1261,7 @@ int solve(eb_ctx* ctx, int n, op_fn op, const double* rhs, double* soln, int mod
       ctx->opts.graphs = -1;
       inf = eb_solve_info{};
       st = EB_OK;
+      EB_CUDA_TRY(cudaMemcpyAsync(x, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
       EB_TRY(init_x());
     } else {
       inf.graph = 1;
