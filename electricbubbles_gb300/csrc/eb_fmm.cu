@@ -2569,24 +2569,87 @@ __device__ __forceinline__ void direct_block_sum(T& gx, T& gy) {
   }
 }
 
-template <int K>
+// Where the charges come from: the arrays of the charges' kernels, or from the density in place:
+// FASMVP's (with the drops' sums za and pk of k_charges_drop, formed by every block), or
+// FASMVP_LAP's. A launch costs as much as the charges of a few hundred points formed by
+// every block: an apply takes (own launch / in place) 13.8 / 12.7 us at 256 points, 16.4 / 14.4 at
+// 384, 20.5 / 22.6 at 512 (FASMVP), 13.8 / 12.2 at 512 and 14.4 / 16.4 at 640 (FASMVP_LAP).
+enum { SRC_Q = 0, SRC_STOKES = 1, SRC_LAPLACE = 2 };
+constexpr int DIRECT_STOKES = 400, DIRECT_LAPLACE = 512;  // points, at most
+
+template <int K, int SRC>
 __global__ void __launch_bounds__(128) k_direct64(int n, const double2* __restrict__ zs,
                                                   const double2* __restrict__ q, const int* __restrict__ perm,
                                                   int plus, double2* __restrict__ out, EbPost post) {
   pdl_wait();
   constexpr bool ST = K == NEAR_V || K == NEAR_VC;
+  static_assert(SRC != SRC_STOKES || K == NEAR_V, "FASMVP's charges with its sign");
   const int i = blockIdx.x;  // one block of 128 threads per target, the threads over the sources
   const double2 zi = zs[i];
   double gx = 0.0, gy = 0.0;
+  // SRC_STOKES: the sums of dens and of the singular terms over the target's drop [a0, a1),
+  // and of the latter over the drop of pinf [b0, b1)
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  int a0 = 0, a1 = 0, b0 = 0, b1 = 0;
+  if (SRC == SRC_STOKES) {
+    const int d = post.drop_of[i], d0 = post.pinf_drop ? post.pinf_drop[d] : 0;
+    a0 = post.start[d];
+    a1 = post.start[d + 1];
+    b0 = post.start[d0];
+    b1 = post.start[d0 + 1];
+  }
   for (int j = threadIdx.x; j < n; j += 128) {
-    if (j == i) continue;
-    const double2 ca = ST ? q[2 * j] : q[j], cc = ST ? q[2 * j + 1] : make_double2(0.0, 0.0);
-    near_pair64<K>(zs[j], ca, cc, zi, gx, gy);
+    double2 ca, cc = make_double2(0.0, 0.0);
+    if (SRC == SRC_Q) {
+      ca = ST ? q[2 * j] : q[j];
+      if (ST) cc = q[2 * j + 1];
+    } else if (SRC == SRC_LAPLACE) {
+      ca = cscale<double>(post.dz[j], post.u[j] * post.hpt[j]);
+    } else {
+      // (near_charge's values for s = -1: with h = 4 hpt / (2 pi), -h dens dz and the real
+      // h Re(dens) Im(dz))
+      const double2 u = post.dens[j], d = post.dz[j], kw = post.pkw[j];
+      const double h = post.hpt[j] * (2.0 / EB_PI);
+      const double2 hd = make_double2(h * d.x, h * d.y);
+      ca = make_double2(fma(u.y, hd.y, -(u.x * hd.x)), fma(-u.y, hd.x, -(u.x * hd.y)));
+      cc.x = u.x * hd.y;
+      const double t = fma(u.x, kw.x, -(u.y * kw.y));
+      if (j >= a0 && j < a1) {
+        v[0] += u.x;
+        v[1] += u.y;
+        v[2] += t;
+      }
+      if (j >= b0 && j < b1) v[3] += t;
+    }
+    if (j != i) near_pair64<K>(zs[j], ca, cc, zi, gx, gy);
+  }
+  if (SRC == SRC_STOKES) {
+    // all six sums through shared memory: 16 threads each, eight values a thread
+    __shared__ double part[6][128], tot[6];
+    part[0][threadIdx.x] = gx;
+    part[1][threadIdx.x] = gy;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) part[2 + c][threadIdx.x] = v[c];
+    __syncthreads();
+    if (threadIdx.x < 96) {
+      const double* r = part[threadIdx.x >> 4] + (threadIdx.x & 15);
+      double s = ((r[0] + r[16]) + (r[32] + r[48])) + ((r[64] + r[80]) + (r[96] + r[112]));
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if ((threadIdx.x & 15) == 0) tot[threadIdx.x >> 4] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const double h = 2.0 * EB_PI / (double)(a1 - a0);
+      eb_post_stokes(post, i, near_turn<double>(tot[0], tot[1], plus), make_double2(h * tot[2], h * tot[3]), tot[4],
+                     tot[5]);
+    }
+    return;
   }
   direct_block_sum<double>(gx, gy);
   if (threadIdx.x == 0) {
-    const double2 v = ST ? near_turn<double>(gx, gy, plus) : make_double2(gx, gy);
-    eb_post_store(post, perm[i], v, out);
+    const double2 w = ST ? near_turn<double>(gx, gy, plus) : make_double2(gx, gy);
+    eb_post_store(post, perm[i], w, out);
   }
 }
 
@@ -3191,22 +3254,49 @@ int direct_run(eb_ctx* ctx, EbTree& t, bool f32, int sign, const double2* dens, 
   } else {
     const double2* zz = t.zs.as<double2>();
     const double2* q = E == 2 ? w.nc.as<double2>() : w.qa.as<double2>();
-    if (E == 2 && post.start)
+    // in place, unless a result overwrites what another block still reads (y = x)
+    auto apart = [n](const void* a, size_t abytes, const void* b, size_t bbytes) {
+      const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+      return x + (size_t)n * abytes <= y || y + (size_t)n * bbytes <= x;
+    };
+    const void* res = post.kind == 0 ? static_cast<const void*>(out) : post.y;
+    const bool own = E == 2 ? post.start && n <= DIRECT_STOKES && apart(dens, 16, res, 16)
+                            : (q_in ? apart(q_in, 16, res, post.kind == 2 ? 8 : 16)
+                                    : n <= DIRECT_LAPLACE && apart(post.u, 8, res, post.kind == 2 ? 8 : 16));
+    if (own) {
+      // no charges' kernel (the points of a direct tree are in their given order)
+      if (q_in) q = q_in;
+      if (E == 2) {
+        post.dz = dz;
+        post.hpt = hpt;
+      }
+      ctx->launches -= 1;
+    } else if (E == 2 && post.start) {
       k_charges_drop<double><<<post.k, 256, 0, st>>>(post.start, dens, dz, hpt, post.pkw, (double)sign,
                                                      w.nc.as<double2>(), const_cast<double2*>(post.za),
                                                      const_cast<double*>(post.pk));
-    else if (E == 2)
+    } else if (E == 2) {
       k_charges_stokes<double><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), dens, dz, hpt, (double)sign,
                                                              w.qa.as<double2>(), w.qb.as<double2>(),
                                                              w.nc.as<double2>(), nullptr);
-    else
+    } else {
       k_charges_cauchy<double><<<nblk(n, 256), 256, 0, st>>>(n, t.perm.as<int>(), q_in, post.u, post.dz, post.hpt,
                                                              w.qa.as<double2>(), nullptr);
+    }
     if (join) EB_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
-    if (kind == NEAR_Q) go(k_direct64<NEAR_Q>, n, zz, q, t.perm.as<int>(), 0, out, post);
-    else if (kind == NEAR_QI) go(k_direct64<NEAR_QI>, n, zz, q, t.perm.as<int>(), 0, out, post);
-    else if (kind == NEAR_V) go(k_direct64<NEAR_V>, n, zz, q, t.perm.as<int>(), plus, out, post);
-    else go(k_direct64<NEAR_VC>, n, zz, q, t.perm.as<int>(), plus, out, post);
+    auto run = [&](auto kern) {
+      if (own || join) kern<<<g, 128, 0, st>>>(n, zz, q, t.perm.as<int>(), plus, out, post);
+      else ce = eb_launch_next(kern, dim3(g), dim3(128), 0, st, n, zz, q, t.perm.as<int>(), (int)plus, out, post);
+    };
+    if (E == 2) {
+      if (own) run(k_direct64<NEAR_V, SRC_STOKES>);
+      else if (kind == NEAR_V) run(k_direct64<NEAR_V, SRC_Q>);
+      else run(k_direct64<NEAR_VC, SRC_Q>);
+    } else {
+      const bool lap = own && !q_in;
+      if (kind == NEAR_QI) lap ? run(k_direct64<NEAR_QI, SRC_LAPLACE>) : run(k_direct64<NEAR_QI, SRC_Q>);
+      else lap ? run(k_direct64<NEAR_Q, SRC_LAPLACE>) : run(k_direct64<NEAR_Q, SRC_Q>);
+    }
   }
   EB_CUDA_TRY(ce);
   ctx->launches += 2;

@@ -76,26 +76,29 @@ __device__ __forceinline__ void eb_post_store_f32(const EbPost& P, int t, float2
 }
 
 // kind 1: identity, self and singular terms of FASMVP (stokesbubb.f:585-612) added to
-// the CADAPDR sum `stress`; kind 2: the discrete operator of FASMVP_LAP
+// the CADAPDR sum `stress`: from the drop's h sum(dens), its singular-term sum and that of
+// the drop whose pressure is pinf.
+__device__ __forceinline__ void eb_post_stokes(const EbPost& P, int t, double2 st, double2 zab, double pkd, double pk0) {
+  const double2 u = P.dens[t];
+  const double c1 = P.c1[t];
+  // zself = c1 u - c1 conj(u) n^2
+  const double2 zself = csub<double>(cscale<double>(u, c1), cmul<double>(cconj<double>(u), P.c2[t]));
+  const double pinf = -pk0, pkb = pkd + pinf;
+  const double f = -0.5 * (pinf - pkb);  // times i z
+  const double2 zz = P.z[t];
+  st.x += zself.x - f * zz.y;
+  st.y += zself.y + f * zz.x;
+  reinterpret_cast<double2*>(P.y)[t] = make_double2(u.x + zab.x + st.x, u.y + zab.y + st.y);
+}
+
+// The same with the sums in memory; kind 2: the discrete operator of FASMVP_LAP
 // (laplace.f:225-243) from the Cauchy sum cf: w = d u - Im(cf) / pi.
 __device__ __forceinline__ void eb_post_store(const EbPost& P, int t, double2 g, double2* out) {
   if (P.kind == 0) {
     out[t] = g;
   } else if (P.kind == 1) {
     const int b = P.drop_of[t];
-    const double2 u = P.dens[t];
-    const double c1 = P.c1[t];
-    // zself = c1 u - c1 conj(u) n^2
-    const double2 zself = csub<double>(cscale<double>(u, c1), cmul<double>(cconj<double>(u), P.c2[t]));
-    const double pinf = -P.pk[P.pinf_drop ? P.pinf_drop[b] : 0];
-    const double pkb = P.pk[b] + pinf;
-    const double f = -0.5 * (pinf - pkb);  // times i z
-    const double2 zz = P.z[t];
-    double2 st = g;
-    st.x += zself.x - f * zz.y;
-    st.y += zself.y + f * zz.x;
-    const double2 zab = P.za[b];
-    reinterpret_cast<double2*>(P.y)[t] = make_double2(u.x + zab.x + st.x, u.y + zab.y + st.y);
+    eb_post_stokes(P, t, g, P.za[b], P.pk[b], P.pk[P.pinf_drop ? P.pinf_drop[b] : 0]);
   } else {
     constexpr double inv_pi = 0.318309886183790671537767526745028724;
     P.y[t] = fma(P.c1[t], P.u[t], -g.y * inv_pi);
