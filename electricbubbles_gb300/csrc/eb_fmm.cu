@@ -1959,6 +1959,47 @@ __device__ __forceinline__ dfl tf_diff(float ah, float am, float al, float3 b) {
   return fast_two_sum(h.hi, __fadd_rn(h.lo, u));
 }
 
+// The near-field pair's steps without the renormalisations between them: a value's low part
+// may reach a few ulps of the high one, so the products of two low parts are kept where both
+// factors are of that kind (the Cauchy pair keeps normalized factors: its sums' errors were 2 %
+// larger without). 1,048,576 nodes: 915 -> 825 us (Stokes).
+__device__ __forceinline__ dfl dfl_mul_raw(dfl a, dfl b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = __fmaf_rn(a.hi, b.hi, -p);
+  e = __fmaf_rn(a.hi, b.lo, e);
+  return dfl{p, __fmaf_rn(a.lo, b.hi, e)};
+}
+// a b + c d
+__device__ __forceinline__ dfl dfl_dot2_raw(dfl a, dfl b, dfl c, dfl d) {
+  const dfl x = dfl_mul_raw(a, b), y = dfl_mul_raw(c, d), t = two_sum(x.hi, y.hi);
+  return dfl{t.hi, __fadd_rn(t.lo, __fadd_rn(x.lo, y.lo))};
+}
+// 1 / (x^2 + y^2): the hardware's estimate and a third-order step
+__device__ __forceinline__ dfl dfl_rcp_norm(dfl x, dfl y) {
+  const dfl d = dfl_dot2_raw(x, x, y, y);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d.hi));
+  const float t = __fmaf_rn(-d.lo, r, __fmaf_rn(-d.hi, r, 1.0f));
+  return fast_two_sum(r, __fmul_rn(r, __fmaf_rn(t, t, t)));
+}
+// a + b c, and acc += b c
+__device__ __forceinline__ dfl dfl_fma_raw(dfl a, dfl b, dfl c) {
+  const float p = __fmul_rn(b.hi, c.hi);
+  float e = __fmaf_rn(b.lo, c.lo, __fmaf_rn(b.hi, c.hi, -p));
+  e = __fmaf_rn(b.hi, c.lo, e);
+  e = __fmaf_rn(b.lo, c.hi, e);
+  const dfl t = two_sum(p, a.hi);
+  return dfl{t.hi, __fadd_rn(t.lo, __fadd_rn(e, a.lo))};
+}
+__device__ __forceinline__ void acc_prod_raw(dfacc& a, dfl x, dfl y) {
+  const float p = __fmul_rn(x.hi, y.hi);
+  float e = __fmaf_rn(x.lo, y.lo, __fmaf_rn(x.hi, y.hi, -p));
+  e = __fmaf_rn(x.hi, y.lo, e);
+  e = __fmaf_rn(x.lo, y.hi, e);
+  acc_add(a, p);
+  a.c = __fadd_rn(a.c, e);
+}
+
 // a u + c: the two products and the addend of each part summed at once
 __device__ __forceinline__ dfl dfl_dot2_add(dfl a, dfl b, dfl c, dfl d, dfl s) {  // a b + c d + s
   const float p = __fmul_rn(a.hi, b.hi), q = __fmul_rn(c.hi, d.hi);
@@ -2135,8 +2176,9 @@ __global__ void __launch_bounds__(128) k_near_df(int ngroup, const int* __restri
       const float2 jb = wb[j];
       // D / r = w_j - (w_i - offset): hi and mid parts subtracted exactly
       const dfl dx = tf_diff(ja.x, ja.z, jb.x, tx), dy = tf_diff(ja.y, ja.w, jb.y, ty);
-      const dfl rr = dfl_rcp(dfl_add(dfl_sqr(dx), dfl_sqr(dy)));
-      const dfl ex = dfl_mul(dx, rr), ey = dfl_mul(dy, rr);  // conj(1/D)
+      const dfl rr = dfl_rcp_norm(dx, dy);
+      const dfl ex = K == NEAR_Q ? dfl_mul(dx, rr) : dfl_mul_raw(dx, rr);  // conj(1/D)
+      const dfl ey = K == NEAR_Q ? dfl_mul(dy, rr) : dfl_mul_raw(dy, rr);
       if (K == NEAR_Q) {
         const cdf q = cdf_from_float4(nc[j]);  // q/(z_i - z_j) = -q/D
         acc_prod(gx, dfl_neg(q.x), ex);
@@ -2145,10 +2187,9 @@ __global__ void __launch_bounds__(128) k_near_df(int ngroup, const int* __restri
         acc_prod(gy, dfl_neg(q.y), ex);
       } else {
         const float4 a = nc[2 * (size_t)j], c = nc[2 * (size_t)j + 1];
-        const dfl m = dfl_add(dfl_mul(dfl{a.x, a.y}, dx), dfl_mul(dfl{a.z, a.w}, dy));
-        const dfl v = dfl_add(dfl{c.x, c.y}, dfl_mul(ey, m));
-        acc_prod(gx, ex, v);
-        acc_prod(gy, ey, v);
+        const dfl v = dfl_fma_raw(dfl{c.x, c.y}, ey, dfl_dot2_raw(dfl{a.x, a.y}, dx, dfl{a.z, a.w}, dy));
+        acc_prod_raw(gx, ex, v);
+        acc_prod_raw(gy, ey, v);
         if (K == NEAR_VC) {
           const dfl c1{c.z, c.w};
           acc_prod(gx, dfl_neg(ey), c1);
