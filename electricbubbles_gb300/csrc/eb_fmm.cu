@@ -22,6 +22,7 @@
 //    separation ratio needs for the requested tolerance.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <functional>
 #include <type_traits>
 #include <utility>
@@ -2884,6 +2885,14 @@ inline int round32(int n) { return (n + 31) & ~31; }
 template <typename T>
 int tables_build(EbTables& tb, int p, double tol) {
   tb.p = p;
+  std::vector<char> blob;
+  std::vector<std::pair<EbTab*, size_t>> at;
+  auto put = [&](EbTab& tab, const auto& v) {
+    const size_t o = (blob.size() + 255) & ~(size_t)255, nb = sizeof(v[0]) * v.size();
+    blob.resize(o + nb);
+    memcpy(blob.data() + o, v.data(), nb);
+    at.emplace_back(&tab, o);
+  };
   const int ldb = 2 * p + 2, ld = p + 2;
   std::vector<T> binom((size_t)ldb * ldb, (T)0);
   std::vector<double> bd((size_t)ldb * ldb, 0.0);
@@ -2927,22 +2936,16 @@ int tables_build(EbTables& tb, int p, double tol) {
       vr = nr; vi = ni;
     }
   }
-  EB_TRY(tb.binom.ensure(sizeof(T) * binom.size()));
-  EB_TRY(tb.dinv.ensure(sizeof(c_t<T>) * dinv.size()));
-  EB_TRY(tb.pd.ensure(sizeof(int) * pd.size()));
-  EB_TRY(tb.epow.ensure(sizeof(c_t<T>) * epow2.size()));
-  EB_TRY(tb.einv.ensure(sizeof(c_t<T>) * einv.size()));
-  EB_CUDA_TRY(cudaMemcpy(tb.binom.p, binom.data(), sizeof(T) * binom.size(), cudaMemcpyHostToDevice));
-  EB_CUDA_TRY(cudaMemcpy(tb.dinv.p, dinv.data(), sizeof(c_t<T>) * dinv.size(), cudaMemcpyHostToDevice));
-  EB_CUDA_TRY(cudaMemcpy(tb.pd.p, pd.data(), sizeof(int) * pd.size(), cudaMemcpyHostToDevice));
-  EB_CUDA_TRY(cudaMemcpy(tb.epow.p, epow2.data(), sizeof(c_t<T>) * epow2.size(), cudaMemcpyHostToDevice));
-  EB_CUDA_TRY(cudaMemcpy(tb.einv.p, einv.data(), sizeof(c_t<T>) * einv.size(), cudaMemcpyHostToDevice));
+  put(tb.binom, binom);
+  put(tb.dinv, dinv);
+  put(tb.pd, pd);
+  put(tb.epow, epow2);
+  put(tb.einv, einv);
   if (sizeof(T) == 4) {  // M2L's binomials with the output order innermost
     std::vector<T> bt((size_t)p * (p + 1));
     for (int k = 0; k < p; ++k)
       for (int m = 0; m <= p; ++m) bt[(size_t)k * (p + 1) + m] = binom[(size_t)(m + k) * ldb + m];
-    EB_TRY(tb.binom_t.ensure(sizeof(T) * bt.size()));
-    EB_CUDA_TRY(cudaMemcpy(tb.binom_t.p, bt.data(), sizeof(T) * bt.size(), cudaMemcpyHostToDevice));
+    put(tb.binom_t, bt);
   }
   if (sizeof(T) == 8) {
     auto split = [](double v, float& h, float& l) {
@@ -2960,15 +2963,14 @@ int tables_build(EbTables& tb, int p, double tol) {
       return o;
     };
     std::vector<float4> ddf = to_df(dinv), edf = to_df(epow2), idf = to_df(einv);
-    EB_TRY(tb.binom_df.ensure(sizeof(float2) * bdf.size()));
-    EB_TRY(tb.dinv_df.ensure(sizeof(float4) * ddf.size()));
-    EB_TRY(tb.epow_df.ensure(sizeof(float4) * edf.size()));
-    EB_TRY(tb.einv_df.ensure(sizeof(float4) * idf.size()));
-    EB_CUDA_TRY(cudaMemcpy(tb.binom_df.p, bdf.data(), sizeof(float2) * bdf.size(), cudaMemcpyHostToDevice));
-    EB_CUDA_TRY(cudaMemcpy(tb.dinv_df.p, ddf.data(), sizeof(float4) * ddf.size(), cudaMemcpyHostToDevice));
-    EB_CUDA_TRY(cudaMemcpy(tb.epow_df.p, edf.data(), sizeof(float4) * edf.size(), cudaMemcpyHostToDevice));
-    EB_CUDA_TRY(cudaMemcpy(tb.einv_df.p, idf.data(), sizeof(float4) * idf.size(), cudaMemcpyHostToDevice));
+    put(tb.binom_df, bdf);
+    put(tb.dinv_df, ddf);
+    put(tb.epow_df, edf);
+    put(tb.einv_df, idf);
   }
+  EB_TRY(tb.all.ensure(blob.size()));
+  EB_CUDA_TRY(cudaMemcpy(tb.all.p, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+  for (auto& a : at) a.first->p = static_cast<const char*>(tb.all.p) + a.second;
   return EB_OK;
 }
 

@@ -149,19 +149,26 @@ struct EbTree {
 #define EB_LEAF_CAP 96      // default maximum points per leaf
 
 // Per-precision constant tables for the translation operators.
+// All of one precision stand in one buffer, filled by one copy (sixteen allocations and copies
+// were a third of a context's creation).
+struct EbTab {
+  const void* p = nullptr;
+  template <typename T> const T* as() const { return static_cast<const T*>(p); }
+};
 struct EbTables {
   int p = 0;
-  DevBuf binom;   // T[(2p+2)*(2p+2)] binomial coefficients C(i, j) at [i*(2p+2)+j]
-  DevBuf dinv;    // c_t<T>[EB_NCODE*(p+2)]: d^-j for the offset codes
-  DevBuf pd;      // int[EB_NCODE]: per-offset truncation order
-  DevBuf epow;    // c_t<T>[4*(p+2)]: e_q^j for the 4 child offsets (child units)
-  DevBuf einv;    // c_t<T>[4*(p+2)]: e_q^-j
-  DevBuf binom_t;   // FP32 tables only: C(m+k, m) at [k*(p+1) + m] (k < p)
+  DevBuf all;
+  EbTab binom;   // T[(2p+2)*(2p+2)] binomial coefficients C(i, j) at [i*(2p+2)+j]
+  EbTab dinv;    // c_t<T>[EB_NCODE*(p+2)]: d^-j for the offset codes
+  EbTab pd;      // int[EB_NCODE]: per-offset truncation order
+  EbTab epow;    // c_t<T>[4*(p+2)]: e_q^j for the 4 child offsets (child units)
+  EbTab einv;    // c_t<T>[4*(p+2)]: e_q^-j
+  EbTab binom_t;   // FP32 tables only: C(m+k, m) at [k*(p+1) + m] (k < p)
   // double-float copies (FP64 tables only) for the double-float M2L
-  DevBuf binom_df;  // float2[(2p+2)*(2p+2)]
-  DevBuf dinv_df;   // float4[EB_NCODE*(p+2)]
-  DevBuf epow_df;   // float4[4*(p+2)]
-  DevBuf einv_df;   // float4[4*(p+2)]
+  EbTab binom_df;  // float2[(2p+2)*(2p+2)]
+  EbTab dinv_df;   // float4[EB_NCODE*(p+2)]
+  EbTab epow_df;   // float4[4*(p+2)]
+  EbTab einv_df;   // float4[4*(p+2)]
   // fixed-point M2L (FP64 tables of order <= EB_FX_MAXP): the powers (2/d)^j as limbs of
   // 2^62 fractions, then (fxb) the binomial matrix's digits and (fxr) its row scalings
   DevBuf fxt;
