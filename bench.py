@@ -363,13 +363,13 @@ def run_gpu(args, rank, world, local):
             far_flops = 8.0 * p_ord * 2 * tree["npoints"] * min(levels_l2p, 6)
             kern["k_near32<2>"] = kentry(near_ms, nn, near_pair_flops)
             kern["k_far32<2>"] = kentry(leaf_ms, nl, far_flops)
-            kern["k_m2l_f32p<2, 20>"] = kentry(m2l_ms, nm, m2l_flops)
+            kern["k_m2l_f32w<2, 20>"] = kentry(m2l_ms, nm, m2l_flops)
         elif arith == "df":
-            kern["k_leaf_df<2>"] = kentry(leaf_ms, nl, near_pair_flops + 8.0 * p_ord * 2 * tree["npoints"])
-            kern["k_m2l_df<2>"] = kentry(m2l_ms, nm, m2l_flops)
+            kern["k_near_df + k_far_df<2>"] = kentry(leaf_ms, nl, near_pair_flops + 8.0 * p_ord * 2 * tree["npoints"])
+            kern["k_m2l_fx<2> (of double-float multipoles)"] = kentry(m2l_ms, nm, m2l_flops)
         else:
-            kern["k_leaf64<2>"] = kentry(leaf_ms, nl, near_pair_flops + 8.0 * p_ord * 2 * tree["npoints"])
-            kern["k_m2l<double, 2>"] = kentry(m2l_ms, nm, m2l_flops)
+            kern["k_near64 + k_far64<2>"] = kentry(leaf_ms, nl, near_pair_flops + 8.0 * p_ord * 2 * tree["npoints"])
+            kern["k_m2l_fx<2>"] = kentry(m2l_ms, nm, m2l_flops)
     ctx_df.close()
     # the FP32 M2L on the tensor cores (tcgen05, 3xTF32) against the CUDA-core M2L
     ctx_tc = Context(device=local, graphs=graphs, m2l_tc=1)
@@ -382,13 +382,15 @@ def run_gpu(args, rank, world, local):
     ctx_tc.set_profiling(False)
     kern["k_m2l_tc<2> (tcgen05)"] = kentry(tc_ms, ntc, 2 * 8.0 * 20 * 20 * tree["v_pairs"])
     ms_tc, _, _ = timed("fp32_refined", args.steps, args.warmup, ctx_tc)
-    m2l_ab = {"k_m2l_f32p_us": 1e3 * kern["k_m2l_f32p<2, 20>"]["avg_launch_ms"],
+    m2l_ab = {"k_m2l_f32w_us": 1e3 * kern["k_m2l_f32w<2, 20>"]["avg_launch_ms"],
               "k_m2l_tc_us": 1e3 * tc_ms / max(ntc, 1),
               "refined_solves_per_s_tc": world * args.steps / (ms_tc * 1e-3),
-              "kept": "CUDA-core k_m2l_f32p (eb_opts.m2l_tc off by default)"}
+              "kept": "CUDA-core k_m2l_f32w (eb_opts.m2l_tc off by default)"}
     ctx_tc.close()
     for name, k in kern.items():
-        if name in ("k_leaf64<2>", "k_m2l<double, 2>"):
+        if "k_m2l_fx" in name:  # FP64-class results from integer and tensor-core work
+            continue
+        if name == "k_near64 + k_far64<2>":
             k["peak_tflops"] = fp64_peak
             k["frac_of_fp64_peak"] = k["achieved_tflops"] / fp64_peak
             continue
@@ -711,7 +713,7 @@ def run_gpu(args, rank, world, local):
         "accuracy": {"refined_vs_fp64_rel_l2": rel_diff, "refined_true_residual": inf32[-1]["err"]},
         "tree": tree,
         "roofline": {"kernel": "k_near32<2> (FP32 near field P2P over the U lists, 40 flop per "
-                               "target-source pair; with k_m2l_f32p<2, 20> and k_p2m_chunks<2> the largest "
+                               "target-source pair; with k_m2l_f32w<2, 20> and k_p2m_points<2, 20> the largest "
                                "kernels of the refined solve)", "bound": "fp32",
                      "achieved": dom["achieved_tflops"], "peak": fp32_peak, "unit": "TFLOP/s",
                      "frac": dom["achieved_tflops"] / fp32_peak,
