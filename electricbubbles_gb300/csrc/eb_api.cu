@@ -494,8 +494,8 @@ int eb_stokes_matvec_dev(eb_ctx* ctx, const double* x, double* y, int prec) {
   EB_TRY(ctx->pk.ensure(sizeof(double) * k));
   // the per-drop sums run on the side stream, overlapping the FMM; the leaf kernel, whose
   // fused post-processing reads them, waits for them. The direct sums' charge kernel forms
-  // them itself (EbPost::start).
-  const bool direct = ctx->tree.direct;
+  // them itself (EbPost::start), but that of EB_FP32.
+  const bool direct = ctx->tree.direct && prec != EB_FP32;
   if (!direct) {
     EB_CUDA_TRY(cudaEventRecord(ctx->ev_fork, s));
     EB_CUDA_TRY(cudaStreamWaitEvent(ctx->side_stream, ctx->ev_fork, 0));

@@ -626,7 +626,7 @@ int bg_enqueue_step(BatchWork& B, eb_op_fn op, int prec, cudaGraphConditionalHan
   k_bg_col<<<std::min(nblk(B.n, 256), 2 * ctx->nsm), 256, 0, st>>>(B.n, B.jdev, B.V, ldv, B.xin);
   eb_count_launch(ctx);
   EB_TRY(op(ctx, B.xin, B.w, prec));
-  if (prec == EB_FP32) {
+  if (prec == EB_PREC_INNER) {
     // one-pass step over work items: partial sums, then the update
     k_bg_dots1<<<B.nitem, BBS, 0, st>>>(B.jdev, B.items, B.sitem, B.V, ldv, B.w, B.ctl, B.part, B.tick, B.hbuf,
                                         B.H, B.G, B.CS, B.maxl, B.nact);
@@ -821,7 +821,7 @@ int eb_batch_solve(eb_ctx* ctx, int n, eb_op_fn op, bool stokes, const double* r
       k_bg_set_tol<<<nblk(S, 128), 128, 0, st>>>(S, B.ctl, ctx->opts.inner_tol, outer > 1 ? itol : nullptr);
       eb_count_launch(ctx);
       // the cycle's iteration count is read after this step's one wait (below)
-      EB_TRY(bg_cycle(B, op, EB_FP32, r, dd, false, skip, nullptr, 1, true));
+      EB_TRY(bg_cycle(B, op, EB_PREC_INNER, r, dd, false, skip, nullptr, 1, true));
       // x += d on the simulations that took part
       k_bg_axpy<<<S, BBS, 0, st>>>(B.seg, skip, dd, x);
       eb_count_launch(ctx);

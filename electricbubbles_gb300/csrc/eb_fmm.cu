@@ -3525,7 +3525,8 @@ int eb_fmm_apply(eb_ctx* ctx, EbTree& t, int kernel, int sign, int precision,
   if (!t.valid) return EB_ERR_NOGEOM;
   if (kernel != 0) return EB_ERR_ARG;
   const bool df = precision == EB_PREC_DF || ctx->opts.df64 > 0;
-  if (precision != EB_FP32) return fmm_run<double, 2>(ctx, t, sign, dens, dz, hpt, nullptr, out, post, join, df);
+  if (precision == EB_FP32) return eb_fp32_apply(ctx, t, sign, dens, dz, hpt, out, post, join);
+  if (precision != EB_PREC_INNER) return fmm_run<double, 2>(ctx, t, sign, dens, dz, hpt, nullptr, out, post, join, df);
   return fmm_run<float, 2>(ctx, t, sign, dens, dz, hpt, nullptr, out, post, join, false);
 }
 
@@ -3533,6 +3534,7 @@ int eb_fmm_apply_cauchy(eb_ctx* ctx, EbTree& t, int precision, const double2* q,
                         const EbPost* post) {
   if (!t.valid) return EB_ERR_NOGEOM;
   const bool df = precision == EB_PREC_DF || ctx->opts.df64 > 0;
-  if (precision != EB_FP32) return fmm_run<double, 1>(ctx, t, 0, nullptr, nullptr, nullptr, q, out, post, nullptr, df);
+  if (precision == EB_FP32) return eb_fp32_apply_cauchy(ctx, t, q, out, post);
+  if (precision != EB_PREC_INNER) return fmm_run<double, 1>(ctx, t, 0, nullptr, nullptr, nullptr, q, out, post, nullptr, df);
   return fmm_run<float, 1>(ctx, t, 0, nullptr, nullptr, nullptr, q, out, post, nullptr, false);
 }

@@ -24,6 +24,9 @@
 // double-float on the FP32 pipes whatever eb_opts.df64 says. The refined solver's FP64
 // residuals use it when eb_opts.resid_df is on.
 #define EB_PREC_DF 2
+// The FP32 operator of the refined solves' inner cycles; EB_FP32 is that of the entry points,
+// which keeps its order of additions (eb_fmm_fp32.cu).
+#define EB_PREC_INNER 3
 
 // ---------------------------------------------------------------------------------
 // Device buffer that grows on demand (never shrinks) and frees itself. Every
@@ -179,6 +182,7 @@ struct EbTables {
 
 struct EbFmmWork {
   DevBuf qa, qb;     // c_t<T>[n] sorted charges (P2M)
+  DevBuf pq, aa;     // EB_FP32 only: float2[2n], float2[n], its near-field coefficients
   DevBuf nc;         // c_t<T>[2n]: near-field coefficients of the Stokes pair
   DevBuf ncdf;       // double-float near-field data (or Cauchy charges), scaled by 1/r_leaf (float4[E n])
   DevBuf mpole_df;   // float4[nbox*E*p]: multipoles, double-float pipeline
@@ -428,6 +432,11 @@ int eb_m2l_fx(eb_ctx* ctx, int E, bool df, int first, int ntarget, int nsrc, int
               const unsigned char* vcode, const int* vcount, EbTables& tb, EbFmmWork& w, const void* mpole,
               void* local, int accumulate, cudaStream_t st);
 int eb_m2l_fx_tables(EbTables& tb);
+
+// fmm_fp32.cu: the sums for EB_FP32
+int eb_fp32_apply(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2* dz, const double* hpt,
+                  double2* out, const EbPost* post, cudaEvent_t join);
+int eb_fp32_apply_cauchy(eb_ctx* ctx, EbTree& t, const double2* q, double2* out, const EbPost* post);
 
 // api.cu: (re)build the installed geometry's tree with the current eb_opts
 bool eb_on_device(const eb_ctx* ctx, const void* p, size_t align);

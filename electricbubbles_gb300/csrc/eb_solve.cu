@@ -926,7 +926,7 @@ int build_graph(eb_ctx* ctx, GmGraph& G, int kind, op_fn op, int n, int maxl) {
   double* wbuf = ctx->gWbuf.as<double>();
   unsigned int* ticket = ctx->gTicket.as<unsigned int>();
   const bool refine = kind == GM_REFINE;
-  const int prec = refine ? EB_FP32 : EB_FP64;
+  const int prec = refine ? EB_PREC_INNER : EB_FP64;
   const double tol = refine ? ctx->opts.inner_tol : ctx->opts.gmres_tol;
   double* bb = refine ? ctx->gZ.as<double>() : ctx->gR.as<double>();  // right-hand side of the cycle
   double* xx = refine ? ctx->gD.as<double>() : ctx->gX.as<double>();  // its solution
@@ -1293,7 +1293,7 @@ int solve(eb_ctx* ctx, int n, op_fn op, const double* rhs, double* soln, int mod
       inf.outer = outer;
       int it = 0, ie = 0, nmv = 0;
       double e2 = 0;
-      st = gmres_cycle(g, op, EB_FP32, r, d, true, inner_tolerance(ctx, outer, inf.err), maxl, &it, &e2,
+      st = gmres_cycle(g, op, EB_PREC_INNER, r, d, true, inner_tolerance(ctx, outer, inf.err), maxl, &it, &e2,
                        &ie, &nmv, rnrm);
       inf.iters += it;
       inf.matvecs32 += nmv;

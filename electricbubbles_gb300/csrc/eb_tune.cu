@@ -36,9 +36,9 @@ int eb_autotune(eb_ctx* ctx, eb_tune_info* info) {
     ctx->opts.leaf64 = kCand[c][0];
     ctx->opts.leaf_cap = kCand[c][1];
     EB_TRY(eb_geom_tree(ctx));
-    for (int r = 0; r < kWarm; ++r) EB_TRY(eb_stokes_matvec_dev(ctx, x.as<double>(), y.as<double>(), EB_FP32));
+    for (int r = 0; r < kWarm; ++r) EB_TRY(eb_stokes_matvec_dev(ctx, x.as<double>(), y.as<double>(), EB_PREC_INNER));
     EB_CUDA_TRY(cudaEventRecord(ctx->ev0, s));
-    for (int r = 0; r < kReps; ++r) EB_TRY(eb_stokes_matvec_dev(ctx, x.as<double>(), y.as<double>(), EB_FP32));
+    for (int r = 0; r < kReps; ++r) EB_TRY(eb_stokes_matvec_dev(ctx, x.as<double>(), y.as<double>(), EB_PREC_INNER));
     EB_CUDA_TRY(cudaEventRecord(ctx->ev1, s));
     EB_CUDA_TRY(cudaEventSynchronize(ctx->ev1));
     float ms = 0.f;
