@@ -363,7 +363,7 @@ def run_gpu(args, rank, world, local):
             far_flops = 8.0 * p_ord * 2 * tree["npoints"] * min(levels_l2p, 6)
             kern["k_near32<2>"] = kentry(near_ms, nn, near_pair_flops)
             kern["k_far32<2>"] = kentry(leaf_ms, nl, far_flops)
-            kern["k_m2l_f32w<2, 20>"] = kentry(m2l_ms, nm, m2l_flops)
+            kern["k_m2l_f32p<2, 20>"] = kentry(m2l_ms, nm, m2l_flops)
         elif arith == "df":
             kern["k_near_df + k_far_df<2>"] = kentry(leaf_ms, nl, near_pair_flops + 8.0 * p_ord * 2 * tree["npoints"])
             kern["k_m2l_fx<2> (of double-float multipoles)"] = kentry(m2l_ms, nm, m2l_flops)
@@ -382,10 +382,10 @@ def run_gpu(args, rank, world, local):
     ctx_tc.set_profiling(False)
     kern["k_m2l_tc<2> (tcgen05)"] = kentry(tc_ms, ntc, 2 * 8.0 * 20 * 20 * tree["v_pairs"])
     ms_tc, _, _ = timed("fp32_refined", args.steps, args.warmup, ctx_tc)
-    m2l_ab = {"k_m2l_f32w_us": 1e3 * kern["k_m2l_f32w<2, 20>"]["avg_launch_ms"],
+    m2l_ab = {"k_m2l_f32p_us": 1e3 * kern["k_m2l_f32p<2, 20>"]["avg_launch_ms"],
               "k_m2l_tc_us": 1e3 * tc_ms / max(ntc, 1),
               "refined_solves_per_s_tc": world * args.steps / (ms_tc * 1e-3),
-              "kept": "CUDA-core k_m2l_f32w (eb_opts.m2l_tc off by default)"}
+              "kept": "CUDA-core k_m2l_f32p (eb_opts.m2l_tc off by default)"}
     ctx_tc.close()
     for name, k in kern.items():
         if "k_m2l_fx" in name:  # FP64-class results from integer and tensor-core work
@@ -713,8 +713,8 @@ def run_gpu(args, rank, world, local):
         "accuracy": {"refined_vs_fp64_rel_l2": rel_diff, "refined_true_residual": inf32[-1]["err"]},
         "tree": tree,
         "roofline": {"kernel": "k_near32<2> (FP32 near field P2P over the U lists, 40 flop per "
-                               "target-source pair; with k_m2l_f32w<2, 20> and k_p2m_points<2, 20> the largest "
-                               "kernels of the refined solve)", "bound": "fp32",
+                               "target-source pair; with k_m2l_f32p<2, 20> and k_p2m_chunks<2> the largest "
+                               "kernels of an FP32 apply)", "bound": "fp32",
                      "achieved": dom["achieved_tflops"], "peak": fp32_peak, "unit": "TFLOP/s",
                      "frac": dom["achieved_tflops"] / fp32_peak,
                      # DRAM bytes of one k_near32<2> launch of this workload (ncu

@@ -3,8 +3,8 @@
 // results are doubles that hold an FP32 sum, so any other order of its additions moves them
 // by some 2e-8, which a caller that compares applies sees. The refined solves' inner
 // operator (EB_PREC_INNER, eb_fmm.cu), whose rounding the FP64 residuals take out again, has
-// faster kernels: 64 x 512 nodes 45 us an apply here and 33 us there, 1,024 x 1,024
-// 1,039 and 687 us. Adding in another order here would give that speed at an error against 64
+// faster kernels: 64 x 512 nodes 57 us an apply here and 51 us there, 1,024 x 1,024
+// 1,013 and 634 us. Adding in another order here would give that speed at an error against 64
 // bits of 5.4e-8 instead of 5.3e-8 (a small direct sum), no more exact and not the same.
 #include <algorithm>
 #include <cmath>
