@@ -32,6 +32,7 @@
 
 #include "eb_df.cuh"
 #include "eb_internal.h"
+#include "eb_parts.h"
 #include "eb_post.cuh"
 
 namespace {
@@ -339,9 +340,9 @@ __global__ void __launch_bounds__(256) k_p2m64(const int* __restrict__ leaves,
   double2 A = make_double2(0.0, 0.0), B = A, C = A;
   const int i0 = pt0[b], i1 = pt1[b];
   pdl_wait();  // the charges
-  const int nbat = (i1 - i0 + 31) / 32;  // batches of equal size
-  for (int bt = 0; bt < nbat; ++bt) {
-    const int base = i0 + bt * (i1 - i0) / nbat, cnt = i0 + (bt + 1) * (i1 - i0) / nbat - base;
+  EbParts batches(i1 - i0, (i1 - i0 + 31) / 32);  // of equal size
+  while (batches.at < i1 - i0) {
+    const int base = i0 + batches.at, cnt = batches.next();
     __syncthreads();
     if (tid < cnt) {
       const int i = base + tid;
