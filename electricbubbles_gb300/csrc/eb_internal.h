@@ -179,6 +179,7 @@ struct EbTables {
 };
 #define EB_FX_K 48      // orders of the fixed-point M2L's operand tiles
 #define EB_FX_MAXP 47   // its largest expansion order (p + 1 local orders)
+#define EB_FX_WAIT (1ll << 22)  // tries of its waits
 
 struct EbFmmWork {
   DevBuf qa, qb;     // c_t<T>[n] sorted charges (P2M)
@@ -247,6 +248,7 @@ struct eb_ctx {
   EbTree tree_pv;   // tree over the 2N fine points of PVINTEV
   EbTree tree_tmp;  // tree for eb_cauchy_sum on caller points
   EbTables tab64, tab32;
+  long long fx_lock_limit[2] = {EB_FX_WAIT, EB_FX_WAIT};  // eb_fx_lock_limit
   EbFmmWork work64, work32;
 
   // operator scratch
@@ -432,6 +434,7 @@ int eb_m2l_fx(eb_ctx* ctx, int E, bool df, int first, int ntarget, int nsrc, int
               const unsigned char* vcode, const int* vcount, EbTables& tb, EbFmmWork& w, const void* mpole,
               void* local, int accumulate, cudaStream_t st);
 int eb_m2l_fx_tables(EbTables& tb);
+extern "C" int eb_fx_lock_limit(eb_ctx* ctx, int team, long long n);
 
 // fmm_fp32.cu: the sums for EB_FP32
 int eb_fp32_apply(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2* dz, const double* hpt,

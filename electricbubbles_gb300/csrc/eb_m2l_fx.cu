@@ -62,7 +62,6 @@ constexpr int FX_PITCH = FX_ROWS + 4;       // row pitch of the contributions (i
 constexpr int FX_GROUP = 8;                 // target boxes of a work item, at most
 constexpr int FX_BAD = 1 << 20;             // exponent of a box with a non-finite multipole
 constexpr int FX_EMIN = -900;               // smallest exponent of a box
-constexpr long long FX_WAIT_LIMIT = 1ll << 22;
 static_assert(EB_FX_K == 48, "the accumulators' columns and the digit layout");
 static_assert(EB_FX_K * FX_PITCH * 8 <= FX_ND * FX_A, "the contributions reuse the digits' memory");
 
@@ -255,7 +254,8 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
                                                           const int* __restrict__ pdv,
                                                           const longlong2* __restrict__ fx,
                                                           const int4* __restrict__ fs, void* __restrict__ local,
-                                                          int accumulate, int nsingle, int group) {
+                                                          int accumulate, int nsingle, int group, long long lim0,
+                                                          long long lim1) {
   pdl_wait();
   constexpr int NE = FX_ROWS / (2 * E);  // entries of a round
   constexpr int NW = FX_TEAM / 32;
@@ -266,7 +266,10 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
   __shared__ uint32_t s_taddr;
   __shared__ int sv_src[2][NE], sv_code[2][NE], sv_pd[2][NE], sv_box[2][NE], sv_exp[2][E][NE];
   __shared__ int sv_e0[2][FX_GROUP + 1], sv_E[2][E][FX_GROUP], sv_cnt[2][FX_GROUP], s_pdv[EB_NCODE];
-  __shared__ int s_fail, s_lock;
+  // s_fail: of a team (1: no tensor memory, 2: products whose end it did not see), written by its
+  // first thread before a team_sync and read by the team behind it, so that all its threads
+  // leave together; s_lock: the tensor memory is taken
+  __shared__ int s_fail[2], s_lock;
   const int team = threadIdx.x / FX_TEAM, tid = threadIdx.x - team * FX_TEAM, warp = tid >> 5, lane = tid & 31;
   int *s_src = sv_src[team], *s_code = sv_code[team], *s_pd = sv_pd[team], *s_box = sv_box[team];
   int *s_cnt = sv_cnt[team], *s_e0 = sv_e0[team], (*s_exp)[NE] = sv_exp[team], (*s_E)[FX_GROUP] = sv_E[team];
@@ -278,7 +281,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
   for (int i = threadIdx.x; i < FX_ND * FX_B / 16; i += FX_THREADS) reinterpret_cast<uint4*>(sB)[i] = bdig[i];
   for (int i = threadIdx.x; i < EB_NCODE; i += FX_THREADS) s_pdv[i] = pdv[i];
   if (threadIdx.x == 0) {
-    s_fail = 0;
+    s_fail[0] = s_fail[1] = 0;
     s_lock = 0;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[0])));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[1])));
@@ -295,6 +298,17 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t taddr = s_taddr;
   uint32_t phase = 0;
+  auto products_done = [&](uint32_t parity) {  // bounded
+    uint32_t done = 0;
+    for (long long it = 0; it < EB_FX_WAIT && !done; ++it)
+      asm volatile(
+          "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+          " selp.u32 %0, 1, 0, p;\n}\n"
+          : "=r"(done)
+          : "r"(smem_u32(&mbar[team])), "r"(parity)
+          : "memory");
+    return done != 0;
+  };
 
   // work items: the first nsingle boxes one by one, the others in groups; teams in turn
   const int nitem = nsingle + (ntarget - nsingle + group - 1) / group, step = 2 * gridDim.x;
@@ -390,9 +404,10 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
         asm volatile("fence.proxy.async.shared::cta;");
         team_sync(team);
         if (tid == 0) {
-          // the tensor memory (bounded; the other team gives it back after its reads)
+          // the tensor memory (bounded; the other team gives it back after its reads). A team
+          // whose products' end stays out keeps it.
           bool mine = false;
-          for (long long it = 0; it < FX_WAIT_LIMIT && !mine; ++it) mine = atomicCAS(&s_lock, 0, 1) == 0;
+          for (long long it = 0; it < (team ? lim1 : lim0) && !mine; ++it) mine = atomicCAS(&s_lock, 0, 1) == 0;
           __threadfence_block();
           if (mine) {
             asm volatile("tcgen05.fence::after_thread_sync;");
@@ -410,17 +425,10 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                 smem_u32(&mbar[team])));
-            uint32_t done = 0;
-            for (long long it = 0; it < FX_WAIT_LIMIT && !done; ++it)
-              asm volatile(
-                  "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                  " selp.u32 %0, 1, 0, p;\n}\n"
-                  : "=r"(done)
-                  : "r"(smem_u32(&mbar[team])), "r"(phase)
-                  : "memory");
-            mine = done != 0;
+            if (!products_done(phase)) s_fail[team] = 2;
+          } else {
+            s_fail[team] = 1;
           }
-          if (!mine) s_fail = 1;
         } else if (warp > 0 && tid - 32 < E * nbx) {
           // the common exponent of a box's entries
           const int e = (tid - 32) / nbx, bx = tid - 32 - e * nbx;
@@ -428,39 +436,36 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
           for (int j = s_e0[bx]; j < s_e0[bx + 1]; ++j) m = max(m, s_exp[e][j]);
           s_E[e][bx] = m;
         }
-        phase ^= 1u;
         team_sync(team);
-        const bool fail = *(volatile int*)&s_fail;
+        if (s_fail[team]) break;
+        phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;");
         // b_m out of the tensor memory, as integers: a warp reads the 32 rows of its quarter,
         // a part of the orders. The team then gives the tensor memory back.
         constexpr int MH = EB_FX_K / (NW / 4);
         const int row = (warp & 3) * 32 + lane, mlo = (warp >> 2) * MH;
-        if (!fail) {
-          for (int m0 = mlo; m0 < mlo + MH; m0 += 4) {
-            uint32_t v[FX_NACC][4];
+        for (int m0 = mlo; m0 < mlo + MH; m0 += 4) {
+          uint32_t v[FX_NACC][4];
 #pragma unroll
-            for (int d = 0; d < FX_NACC; ++d)
-              asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                           : "=r"(v[d][0]), "=r"(v[d][1]), "=r"(v[d][2]), "=r"(v[d][3])
-                           : "r"(taddr + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(d * EB_FX_K + m0)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;");
+          for (int d = 0; d < FX_NACC; ++d)
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(v[d][0]), "=r"(v[d][1]), "=r"(v[d][2]), "=r"(v[d][3])
+                         : "r"(taddr + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(d * EB_FX_K + m0)));
+          asm volatile("tcgen05.wait::ld.sync.aligned;");
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              int w[FX_NACC];
+          for (int q = 0; q < 4; ++q) {
+            int w[FX_NACC];
 #pragma unroll
-              for (int d = 0; d < FX_NACC; ++d) w[d] = __float2int_rn(__uint_as_float(v[d][q]));
-              // sum of w_d 2^(42 - 9 d), below 2^62 (no row of the matrix sums to 8)
-              const long long top = madw(w[0], 1 << 18, madw(w[1], 1 << 9, w[2]));
-              const long long low = madw(w[3], 1 << 15, madw(w[4], 64, (w[5] >> 3) + (w[6] >> 12)));
-              sC[(m0 + q) * FX_PITCH + row] = shl31(top, 24) + low;
-            }
+            for (int d = 0; d < FX_NACC; ++d) w[d] = __float2int_rn(__uint_as_float(v[d][q]));
+            // sum of w_d 2^(42 - 9 d), below 2^62 (no row of the matrix sums to 8)
+            const long long top = madw(w[0], 1 << 18, madw(w[1], 1 << 9, w[2]));
+            const long long low = madw(w[3], 1 << 15, madw(w[4], 64, (w[5] >> 3) + (w[6] >> 12)));
+            sC[(m0 + q) * FX_PITCH + row] = shl31(top, 24) + low;
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
         team_sync(team);
         if (tid == 0) atomicExch(&s_lock, 0);
-        if (fail) break;
         // contributions (-1)^m (2/d)^m b_m of the entries to their boxes, in place: a thread
         // per row and part of the orders reads both parts before either is replaced
         {
@@ -506,11 +511,13 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_m2l_fx(int first, int ntarget
       team_sync(team);
       b0 = b1;
     }
-    if (*(volatile int*)&s_fail) break;
+    if (s_fail[team]) break;  // (the whole team, or none: last written before the round's team_sync)
   }
+  // no tensor memory is given up under products in flight (a second wait, bounded as the first)
+  if (tid == 0 && s_fail[team] == 2) products_done(phase);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
-  if (s_fail) {
+  if (s_fail[0] | s_fail[1]) {
     // a wait ran out: mark this block's expansions non-finite
     for (int g = team * gridDim.x + blockIdx.x; g < nitem; g += step)
       for (int b = item_box(g); b < item_box(g + 1); ++b)
@@ -543,7 +550,7 @@ int fx_launch(eb_ctx* ctx, int first, int ntarget, int nsrc, int ncoarse, const 
   const int grid = std::min((nitem + 1) / 2, ctx->nsm);
   EB_CUDA_TRY(eb_launch_next(k_m2l_fx<E, DF>, dim3(grid), dim3(FX_THREADS), sm, st, first, ntarget, vlist, vcode, vcount, p, reinterpret_cast<const uint4*>(tb.fxb),
                                                tb.fxt.as<int4>(), reinterpret_cast<const int*>(tb.fxr), tb.pd.as<int>(), fx, fs, local,
-                                               accumulate, nsingle, group));
+                                               accumulate, nsingle, group, ctx->fx_lock_limit[0], ctx->fx_lock_limit[1]));
   ctx->launches += 2;
   return EB_OK;
 }
@@ -659,5 +666,13 @@ int eb_m2l_fx_tables(EbTables& tb) {
   tb.fxb = tb.fxt.as<char>() + nt;
   tb.fxr = tb.fxt.as<char>() + nt + nd;
   EB_CUDA_TRY(cudaMemcpy(tb.fxt.p, all.data(), all.size(), cudaMemcpyHostToDevice));
+  return EB_OK;
+}
+
+// For tests of the bounded wait: how often a team (0 or 1) of a block asks for the tensor memory
+// before it gives up, in the applies from now on (graphs of solves keep theirs).
+extern "C" int eb_fx_lock_limit(eb_ctx* ctx, int team, long long n) {
+  if (!ctx || team < 0 || team > 1 || n < 0) return EB_ERR_ARG;
+  ctx->fx_lock_limit[team] = n;
   return EB_OK;
 }
