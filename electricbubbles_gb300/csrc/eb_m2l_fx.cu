@@ -61,7 +61,6 @@ constexpr int FX_THREADS = 2 * FX_TEAM;
 constexpr int FX_PITCH = FX_ROWS + 4;       // row pitch of the contributions (int64)
 constexpr int FX_GROUP = 8;                 // target boxes of a work item, at most
 constexpr int FX_BAD = 1 << 20;             // exponent of a box with a non-finite multipole
-constexpr int FX_EMIN = -900;               // smallest exponent of a box
 static_assert(EB_FX_K == 48, "the accumulators' columns and the digit layout");
 static_assert(EB_FX_K * FX_PITCH * 8 <= FX_ND * FX_A, "the contributions reuse the digits' memory");
 
@@ -185,7 +184,7 @@ __global__ void __launch_bounds__(128) k_m2l_fix(int first, int nb, int p, const
   const bool bad = max(h[0], h[1]) >= (DF ? 0x7f800000u : 0x7ff00000u);
   int S[2];
 #pragma unroll
-  for (int e = 0; e < E; ++e) S[e] = max(above(h[e]), FX_EMIN);
+  for (int e = 0; e < E; ++e) S[e] = above(h[e]);  // down to -1022: zeros and subnormals too
   if (lane == 0) fs[b] = make_int4(bad ? FX_BAD : S[0], S[E - 1], max(above(hk), S[0]), 0);
   for (int o = lane; o < E * p; o += 32) {
     const int Se = E == 1 || o < p ? S[0] : S[E - 1];
@@ -196,7 +195,7 @@ __global__ void __launch_bounds__(128) k_m2l_fix(int first, int nb, int p, const
       r.y = float_fix(v.z, Se) + float_fix(v.w, Se);
     } else if (!bad) {
       const double2 v = md[o];
-      // 2^(61 - S) as two factors (S from -900 to 1024)
+      // 2^(61 - S) as two factors (S from -1022 to 1024)
       const int e1 = (61 - Se) >> 1, e2 = 61 - Se - e1;
       const double f1 = __hiloint2double((1023 + e1) << 20, 0), f2 = __hiloint2double((1023 + e2) << 20, 0);
       r.x = __double2ll_rn(v.x * f1 * f2);
