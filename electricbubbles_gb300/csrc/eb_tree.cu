@@ -951,7 +951,11 @@ void DevBuf::release() {
 // (z - x0 - (i + 1/2) r) / r, the offset of a coordinate from the centre of its leaf in
 // leaf units, with both subtractions carried exactly (two-sum, two-product), so that
 // for two nodes the offsets differ by exactly (z_j - z_i)/r minus the integer index
-// offset of their leaves, up to the final rounding (about 2^-53 of a leaf side).
+// offset of their leaves, up to the final roundings (2^-54 of a leaf side each). The division
+// is a product with rinv = 1 / r and a correction by its exact remainder, so that the quotient
+// is the rounded one: the product alone would stretch the offsets, but not the index offset, by
+// the rounding of rinv (up to 2^-53), and an FP64 division is some twenty instructions on
+// a pipe of two lanes a cycle.
 __device__ __forceinline__ double leaf_offset(double z, double x0, unsigned int i, double r, double rinv) {
   double s = __dsub_rn(z, x0);
   double bb = __dsub_rn(s, z);
@@ -962,7 +966,9 @@ __device__ __forceinline__ double leaf_offset(double z, double x0, unsigned int 
   double u = __dsub_rn(s, c);
   double bb2 = __dsub_rn(u, s);
   double e3 = __dadd_rn(__dsub_rn(s, __dsub_rn(u, bb2)), __dsub_rn(-c, bb2));
-  return __dmul_rn(__dadd_rn(u, __dadd_rn(__dsub_rn(e1, e2), e3)), rinv);
+  const double a = __dadd_rn(u, __dadd_rn(__dsub_rn(e1, e2), e3));
+  const double q = __dmul_rn(a, rinv);
+  return __fma_rn(__fma_rn(-q, r, a), rinv, q);
 }
 
 // Leaf-relative node coordinates as three floats hi + mid + lo (all 53 bits of the
@@ -986,9 +992,7 @@ __global__ void __launch_bounds__(128) k_leaf_coords(int n, const int* __restric
   const int b = leaves[lscan[i] + lflag[i] - 1];  // leaf heads up to point i
   const unsigned long long k = bkey[b];
   const unsigned int ix = compact2(k), iy = compact2(k >> 1);
-  // W / 2^level, exact, and its reciprocal: every offset of the tree carries the same relative
-  // rounding of 1 / W (a change of unit), and an FP64 division is some twenty instructions on
-  // a pipe of two lanes a cycle
+  // W / 2^level, exact, and its rounded reciprocal
   const double r = W * __hiloint2double((1023 - (int)blev[b]) << 20, 0);
   const double rinv = winv * __hiloint2double((1023 + (int)blev[b]) << 20, 0);
   const double2 z = zs[i];
