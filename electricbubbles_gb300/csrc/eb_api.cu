@@ -611,6 +611,17 @@ int eb_cauchy_sum(eb_ctx* ctx, int n, const double* z, const double* q, double* 
   return EB_OK;
 }
 
+// The refined solves' inner operator by itself, for tests and per-kernel timing: FASMVP (op 0),
+// FASMVP_LAP (1) and their transposes (2, 3), x and y in device memory.
+extern "C" int eb_inner_matvec(eb_ctx* ctx, int op, const double* x, double* y) {
+  static const eb_op_fn f[4] = {eb_stokes_matvec_dev, eb_laplace_matvec_dev, eb_stokes_matvec_adj_dev,
+                                eb_laplace_matvec_adj_dev};
+  if (!ctx || !x || !y || op < 0 || op > 3) return EB_ERR_ARG;
+  if (!ctx->geom_valid) return EB_ERR_NOGEOM;
+  cudaSetDevice(ctx->device);
+  return f[op](ctx, x, y, EB_PREC_INNER);
+}
+
 // ---------------------------------------------------------------------------------
 // gfortran shims: MATVEC(N, XX, YY, NELT, IA, JA, A, ISYM) as DPIGMR calls it.
 // ---------------------------------------------------------------------------------

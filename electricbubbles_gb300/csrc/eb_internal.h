@@ -423,6 +423,7 @@ int eb_laplace_matvec_dev(eb_ctx* ctx, const double* x, double* y, int prec);
 // adjoint.cu: the transposed operators
 int eb_stokes_matvec_adj_dev(eb_ctx* ctx, const double* x, double* y, int prec);
 int eb_laplace_matvec_adj_dev(eb_ctx* ctx, const double* x, double* y, int prec);
+extern "C" int eb_inner_matvec(eb_ctx* ctx, int op, const double* x, double* y);
 
 // m2l_tc.cu: the FP32 M2L of order 20 on the tensor cores
 int eb_m2l_tc(eb_ctx* ctx, int E, int first, int ntarget, const int* vlist, const unsigned char* vcode,
