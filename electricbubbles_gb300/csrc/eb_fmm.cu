@@ -3018,10 +3018,15 @@ int launch_l2l64(eb_ctx* ctx, EbTree& t, EbTables& tb, int l, double2* local, cu
   return EB_OK;
 }
 
-// Boxes from which the double-float pipeline takes the fixed-point M2L (the rule's figures in
-// eb_m2l_fx.cu).
+// Boxes and order from which the double-float pipeline takes the fixed-point M2L (the boxes'
+// figures, at the default order, in eb_m2l_fx.cu). Its time hardly depends on the order, that of
+// k_m2l_df goes with its square: an apply takes (k_m2l_df / fixed) at orders 12, 30, 36 and 44
+// 115 / 171, 168 / 196, 203 / 204 and 224 / 214 us for 64 x 512 nodes, 2.14 / 2.91, 3.35 / 3.51, 4.20 /
+// 3.75 and 4.87 / 4.13 ms for 1,024 x 1,024 (E = 2); 1.70 / 2.00, 2.22 / 2.27, 2.85 / 2.48 and 3.22 / 2.64
+// ms for the latter with E = 1.
 template <int E>
 constexpr int FX_DF = E == 2 ? 0 : 3072;
+constexpr int FX_DF_P = 36;
 
 // Boxes of the levels 2, 3, .. of at most 384 boxes: their V lists are the long ones.
 int coarse_boxes(const EbTree& t) {
@@ -3062,7 +3067,7 @@ int fmm_expansions_df(eb_ctx* ctx, EbTree& t, EbTables& tb, EbFmmWork& w) {
     if (sm > 48 * 1024)
       EB_CUDA_TRY(cudaFuncSetAttribute(k_m2l_df<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     ProfScope ps(ctx, 1, st);
-    const bool fixed = p <= EB_FX_MAXP && nt >= FX_DF<E>;
+    const bool fixed = p >= FX_DF_P && p <= EB_FX_MAXP && nt >= FX_DF<E>;
     const int ncoarse = coarse_boxes(t);
     if (nt > 0 && fixed) {
       EB_TRY(eb_m2l_fx(ctx, E, true, first, nt, nt, ncoarse, t.vlist.as<int>(), t.vcode.as<unsigned char>(), t.vcount.as<int>(),
