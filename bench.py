@@ -18,6 +18,7 @@ value is the aggregate over ranks. `--impl reference` times the reference algori
 (the per-level CADAPDR FMM and SLATEC GMRES, restated in C) on the host cores.
 """
 import argparse
+import ctypes
 import json
 import os
 import subprocess
@@ -319,16 +320,25 @@ def run_gpu(args, rank, world, local):
     u = torch.randn(n, dtype=torch.float64, device=dev)
     y = torch.empty_like(u)
     mpts = {}
-    for prec in ("fp64", "fp32"):
+
+    def op_apply(c, prec, x, out):  # "inner": the refined solves' inner operator by itself
+        if prec != "inner":
+            c.fasmvp(x, prec, out=out)
+            return
+        st = c._lib.eb_inner_matvec(c._h, 0, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(out.data_ptr()))
+        if st != 0:
+            raise RuntimeError("eb_inner_matvec: status %d" % st)
+
+    for prec in ("fp64", "fp32", "inner"):
         for _ in range(3):
-            ctx.fasmvp(u, prec, out=y)
+            op_apply(ctx, prec, u, y)
         reps = 10
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         tot = 0.0
         for _ in range(reps):
             flush.zero_()
             e0.record(stream)
-            ctx.fasmvp(u, prec, out=y)
+            op_apply(ctx, prec, u, y)
             e1.record(stream)
             torch.cuda.synchronize()
             tot += e0.elapsed_time(e1)
@@ -336,7 +346,10 @@ def run_gpu(args, rank, world, local):
 
     # per-kernel live CUDA-event timing of the near-field (P2P + L2P) and M2L kernels of
     # both operator precisions; algorithmic flops per launch from the tree actually built:
-    # 40 per near-field pair, 8 p e per point per level of L2P, 2 * 8 p^2 per M2L pair
+    # 23 per near-field pair as the kernels form it (two differences, the squared distance, a
+    # reciprocal, conj(1/D), one real factor, two multiply-adds; 40 for the entry points' FP32
+    # pair, whose terms are formed as written), 8 p e per point per level of L2P, 2 * 8 p^2 per
+    # M2L pair. The refined solves' inner operator is applied by itself (eb_inner_matvec).
     tree = ctx.tree_info()
     fp64_peak = ctx.measure_fp64_peak()
     fp32_peak = ctx.measure_fp32_peak()
@@ -347,23 +360,29 @@ def run_gpu(args, rank, world, local):
         return {"avg_launch_ms": ms / nl, "flops_per_launch": flops,
                 "achieved_tflops": flops / (ms / nl * 1e-3) / 1e12}
 
-    near_pair_flops = 40.0 * tree["u_pairs"]
-    for c, prec, p_ord, arith in ((ctx, "fp32", 20, "fp32"), (ctx_df, "fp64", 44, "df"),
+    near_pair_flops = 23.0 * tree["u_pairs"]
+    for c, prec, p_ord, arith in ((ctx, "inner", 20, "inner"), (ctx, "fp32", 20, "fp32"), (ctx_df, "fp64", 44, "df"),
                                   (ctx, "fp64", 44, "native")):
         c.set_profiling(True)
         for _ in range(10):
-            c.fasmvp(u, prec, out=y)
+            op_apply(c, prec, u, y)
         nl, leaf_ms = c.kernel_time(0)
         nm, m2l_ms = c.kernel_time(1)
         nn, near_ms = c.kernel_time(2)
         c.set_profiling(False)
         m2l_flops = 2 * 8.0 * p_ord * p_ord * tree["v_pairs"]
-        if arith == "fp32":
+        m2l32 = "k_m2l_f32w<2, 20>" if tree["nboxes"] < 8192 else "k_m2l_f32p<2, 20>"
+        if arith in ("inner", "fp32"):
             # the far field evaluates the locals of min(levels - 1, 6) levels at every node
             far_flops = 8.0 * p_ord * 2 * tree["npoints"] * min(levels_l2p, 6)
-            kern["k_near32<2>"] = kentry(near_ms, nn, near_pair_flops)
-            kern["k_far32<2>"] = kentry(leaf_ms, nl, far_flops)
-            kern["k_m2l_f32p<2, 20>"] = kentry(m2l_ms, nm, m2l_flops)
+            if arith == "inner":
+                kern["k_near32<NEAR_V>"] = kentry(near_ms, nn, near_pair_flops)
+                kern["k_far32<2>"] = kentry(leaf_ms, nl, far_flops)
+                kern[m2l32] = kentry(m2l_ms, nm, m2l_flops)
+            else:  # the entry points' own kernels
+                kern["ep::k_near32<2>"] = kentry(near_ms, nn, 40.0 * tree["u_pairs"])
+                kern["ep::k_far32<2>"] = kentry(leaf_ms, nl, far_flops)
+                kern["ep::k_m2l_f32p<2, 20>"] = kentry(m2l_ms, nm, m2l_flops)
         elif arith == "df":
             kern["k_near_df + k_far_df<2>"] = kentry(leaf_ms, nl, near_pair_flops + 8.0 * p_ord * 2 * tree["npoints"])
             kern["k_m2l_fx<2> (of double-float multipoles)"] = kentry(m2l_ms, nm, m2l_flops)
@@ -377,15 +396,15 @@ def run_gpu(args, rank, world, local):
     ctx_tc.extractdat(cfg.nd, cfg.rku())
     ctx_tc.set_profiling(True)
     for _ in range(10):
-        ctx_tc.fasmvp(u, "fp32", out=y)
+        op_apply(ctx_tc, "inner", u, y)
     ntc, tc_ms = ctx_tc.kernel_time(1)
     ctx_tc.set_profiling(False)
     kern["k_m2l_tc<2> (tcgen05)"] = kentry(tc_ms, ntc, 2 * 8.0 * 20 * 20 * tree["v_pairs"])
     ms_tc, _, _ = timed("fp32_refined", args.steps, args.warmup, ctx_tc)
-    m2l_ab = {"k_m2l_f32p_us": 1e3 * kern["k_m2l_f32p<2, 20>"]["avg_launch_ms"],
+    m2l_ab = {"cuda_core_kernel": m2l32, "cuda_core_us": 1e3 * kern[m2l32]["avg_launch_ms"],
               "k_m2l_tc_us": 1e3 * tc_ms / max(ntc, 1),
               "refined_solves_per_s_tc": world * args.steps / (ms_tc * 1e-3),
-              "kept": "CUDA-core k_m2l_f32p (eb_opts.m2l_tc off by default)"}
+              "kept": "the CUDA-core kernel (eb_opts.m2l_tc off by default)"}
     ctx_tc.close()
     for name, k in kern.items():
         if "k_m2l_fx" in name:  # FP64-class results from integer and tensor-core work
@@ -399,7 +418,7 @@ def run_gpu(args, rank, world, local):
         if "df" in name:
             # double-float kernels do FP64-class arithmetic on the FP32 pipes
             k["frac_of_fp64_peak"] = k["achieved_tflops"] / fp64_peak
-    dom = kern["k_near32<2>"]
+    dom = kern["k_near32<NEAR_V>"]
 
     # end to end through the C ABI with host buffers: geometry + rhs in, solution out
     zh = torch.from_numpy(np.ascontiguousarray(geo["z"]).view(np.float64).copy()).pin_memory()
@@ -411,7 +430,6 @@ def run_gpu(args, rank, world, local):
     xh = torch.empty_like(rhh).pin_memory()
     lib, h = ctx._lib, ctx._h
     nd = np.ascontiguousarray(cfg.nd, dtype=np.int32)
-    import ctypes
     from electricbubbles_gb300._lib import SolveInfo, check
 
     def e2e_step():
@@ -605,12 +623,12 @@ def run_gpu(args, rank, world, local):
     yb = torch.empty_like(ub)
     large = {"workload": "large_drops_1024x1024", "nodes": big.nbk, "tree": ctx.tree_info()}
     ea, eb_ = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    for prec in ("fp64", "fp32"):
-        ctx.fasmvp(ub, prec, out=yb)
+    for prec in ("fp64", "fp32", "inner"):
+        op_apply(ctx, prec, ub, yb)
         torch.cuda.synchronize()
         ea.record(stream)
         for _ in range(3):
-            ctx.fasmvp(ub, prec, out=yb)
+            op_apply(ctx, prec, ub, yb)
         eb_.record(stream)
         torch.cuda.synchronize()
         large["fmm_mpts_per_s_" + prec] = big.nbk / (ea.elapsed_time(eb_) / 3 * 1e-3) / 1e6
@@ -618,19 +636,21 @@ def run_gpu(args, rank, world, local):
     # the near field runs on the main stream) against the FP32 peak: where the 64 x 512
     # kernels are latency-bound, these fill the GPU
     btree = large["tree"]
-    ctx.set_profiling(True)
-    for _ in range(3):
-        ctx.fasmvp(ub, "fp32", out=yb)
-    nl, leaf_ms = ctx.kernel_time(0)
-    nm, m2l_ms = ctx.kernel_time(1)
-    nn, near_ms = ctx.kernel_time(2)
-    ctx.set_profiling(False)
-    bkern = {"k_near32<2>": kentry(near_ms, nn, 40.0 * btree["u_pairs"]),
-             "k_far32<2>": kentry(leaf_ms, nl, 8.0 * 20 * 2 * btree["npoints"] * min(max(btree["levels"] - 1, 1), 6)),
-             "k_m2l_f32p<2, 20>": kentry(m2l_ms, nm, 2 * 8.0 * 20 * 20 * btree["v_pairs"])}
-    for v in bkern.values():
-        v["frac_of_fp32_peak"] = v["achieved_tflops"] / fp32_peak
-    large["kernels_fp32"] = bkern
+    bfar = 8.0 * 20 * 2 * btree["npoints"] * min(max(btree["levels"] - 1, 1), 6)
+    for prec, pre, near, per_pair in (("inner", "", "k_near32<NEAR_V>", 23.0), ("fp32", "ep::", "k_near32<2>", 40.0)):
+        ctx.set_profiling(True)
+        for _ in range(3):
+            op_apply(ctx, prec, ub, yb)
+        nl, leaf_ms = ctx.kernel_time(0)
+        nm, m2l_ms = ctx.kernel_time(1)
+        nn, near_ms = ctx.kernel_time(2)
+        ctx.set_profiling(False)
+        bkern = {pre + near: kentry(near_ms, nn, per_pair * btree["u_pairs"]),
+                 pre + "k_far32<2>": kentry(leaf_ms, nl, bfar),
+                 pre + "k_m2l_f32p<2, 20>": kentry(m2l_ms, nm, 2 * 8.0 * 20 * 20 * btree["v_pairs"])}
+        for v in bkern.values():
+            v["frac_of_fp32_peak"] = v["achieved_tflops"] / fp32_peak
+        large["kernels_" + prec] = bkern
     rb = torch.from_numpy(surface_tension_rhs(gb["dz"], gb["dsda"])).to(dev)
     xb = torch.empty_like(rb)
     for mode in ("fp64", "fp32_refined"):
@@ -712,9 +732,8 @@ def run_gpu(args, rank, world, local):
         "solve_info": {"fp64": inf64[-1], "fp32_refined": inf32[-1]},
         "accuracy": {"refined_vs_fp64_rel_l2": rel_diff, "refined_true_residual": inf32[-1]["err"]},
         "tree": tree,
-        "roofline": {"kernel": "k_near32<2> (FP32 near field P2P over the U lists, 40 flop per "
-                               "target-source pair; with k_m2l_f32p<2, 20> and k_p2m_chunks<2> the largest "
-                               "kernels of an FP32 apply)", "bound": "fp32",
+        "roofline": {"kernel": "k_near32<NEAR_V> (FP32 near field P2P over the U lists of the refined solve's "
+                               "inner operator, 23 flop per target-source pair)", "bound": "fp32",
                      "achieved": dom["achieved_tflops"], "peak": fp32_peak, "unit": "TFLOP/s",
                      "frac": dom["achieved_tflops"] / fp32_peak,
                      # DRAM bytes of one k_near32<2> launch of this workload (ncu

@@ -1167,7 +1167,7 @@ __global__ void __launch_bounds__(128) k_m2l_df(int first, const int* __restrict
 }
 
 // ---------------------------------------------------------------------------------
-// The P2M of the double-float pipeline (its M2M and L2L are the FP64 kernels above).
+// The P2M, M2M and L2L of the double-float pipeline.
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ cdf cdf_conj(cdf a) { return cdf{a.x, dfl_neg(a.y)}; }
 __device__ __forceinline__ cdf cdf_scale(cdf a, float f) { return cdf{dfl_mul_f(a.x, f), dfl_mul_f(a.y, f)}; }
@@ -1928,7 +1928,7 @@ __global__ void __launch_bounds__(128) k_far64(int n, const int* __restrict__ lf
 }
 
 // ---------------------------------------------------------------------------------
-// FP64-accurate leaf evaluation in double-float arithmetic (the same sums as k_leaf64,
+// FP64-accurate leaf evaluation in double-float arithmetic (the sums of k_near64 and k_far64,
 // about 2^-47 relative per operation, several times faster on GB300's FP32 pipes).
 // Offsets are leaf-relative: for target i in leaf b and source j in neighbour b',
 // (z_j - z_i)/r = w_j - (w_i - (b' - b)), exact up to the double-float rounding of w;
@@ -2587,8 +2587,8 @@ __global__ void __launch_bounds__(NEAR32_THREADS, 16) k_near32(const int4* __res
 // (sorted order) and its fused post-processing; one block of 128 threads per target, the
 // threads over the sources, their partial sums added in a fixed order (direct_block_sum). On a few hundred points the
 // FMM's chain of about a dozen dependent launches, each on a handful of SMs, costs far
-// more than all N^2 pairs: an FP64 pair is ~35 FP64 instructions, so 1,024 points take
-// ~60 us of the GPU's FP64 rate. The sums are exact up to rounding (no truncation).
+// more than all N^2 pairs: an FP64 pair is 14 FP64 instructions, so 1,024 points take
+// 25 us of the GPU's FP64 rate. The sums are exact up to rounding (no truncation).
 // ---------------------------------------------------------------------------------
 // The sum of a block's partial sums, in thread 0 (warp butterflies, then the warps in
 // order through shared memory).

@@ -15,6 +15,7 @@
 #include "eb_post.cuh"
 
 namespace {
+namespace ep {  // the entry points' kernels: a name of their own beside the inner operator's
 
 __device__ __forceinline__ unsigned int compact2d(unsigned long long x) {
   x &= 0x5555555555555555ull;
@@ -794,8 +795,7 @@ __global__ void __launch_bounds__(128, 8) k_near32(const int4* __restrict__ tile
 // (sorted order) and its fused post-processing; one block of 128 threads per target, the
 // threads over the sources, their partial sums added in a fixed order (direct_block_sum). On a few hundred points the
 // FMM's chain of about a dozen dependent launches, each on a handful of SMs, costs far
-// more than all N^2 pairs: an FP64 pair is ~35 FP64 instructions, so 1,024 points take
-// ~60 us of the GPU's FP64 rate. The sums are exact up to rounding (no truncation).
+// more than all N^2 pairs. The sums are exact up to rounding (no truncation).
 // ---------------------------------------------------------------------------------
 // The sum of a block's partial sums, in thread 0 (warp butterflies, then the warps in
 // order through shared memory).
@@ -1187,13 +1187,14 @@ int run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2* dz
   return eb_check_launch(ctx, "fmm apply");
 }
 
+}  // namespace ep
 }  // namespace
 
 int eb_fp32_apply(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2* dz, const double* hpt,
                   double2* out, const EbPost* post, cudaEvent_t join) {
-  return run<2>(ctx, t, sign, dens, dz, hpt, nullptr, out, post, join);
+  return ep::run<2>(ctx, t, sign, dens, dz, hpt, nullptr, out, post, join);
 }
 
 int eb_fp32_apply_cauchy(eb_ctx* ctx, EbTree& t, const double2* q, double2* out, const EbPost* post) {
-  return run<1>(ctx, t, 0, nullptr, nullptr, nullptr, q, out, post, nullptr);
+  return ep::run<1>(ctx, t, 0, nullptr, nullptr, nullptr, q, out, post, nullptr);
 }

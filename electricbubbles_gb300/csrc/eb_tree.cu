@@ -685,7 +685,6 @@ __global__ void k_imglist(const unsigned long long* __restrict__ bkey, const uns
   icount[gid] = cnt;
 }
 
-// Leaves in point order: point i starts its leaf when it heads the box of its leaf level.
 #define EB_LIST_STACK 72
 
 // U and W lists of every leaf (DALI12 / DALI34, dapif2.f:3-356, for an adaptive tree
@@ -1073,9 +1072,9 @@ int eb_tree_build(eb_ctx* ctx, EbTree& t, const double2* z, int n, int leaf_targ
   t.pairs_read = false;
   // (the whole build is a chain of small kernels, and their number and that of the copies
   // is what it costs, about 4 us each. A solve of 64 x 512 nodes, geometry installed, spent
-  // 664 us before its first Krylov vector with 80 of them under a profiler, 288 us with
-  // these 25; without one it went from 1,897 to 1,664 us, and the Cauchy sum of 60,001 points
-  // from 1,060 to 870 us)
+  // 664 us before its first Krylov vector with 80 of them under a profiler, 288 us with 25, of
+  // which the build's are 14 kernels, a memset and two readbacks; without one it went from 1,897
+  // to 1,664 us, and the Cauchy sum of 60,001 points from 1,060 to 870 us)
   // 1. bounding square, on the device
   const int nbb = std::min(nblk(n, BS), 1024), nb256 = nblk(n, TREE_BS);
   EB_TRY(t.partial.ensure(sizeof(IBox) * (size_t)nbb));
