@@ -1765,19 +1765,24 @@ __device__ __forceinline__ void m2p_eval(const c_t<T>* M, int p, c_t<T> u, T s, 
   }
 }
 
-// FP64 near field, one block per tile of up to EB_NTILE targets of one leaf. GB300 issues
+// FP64 near field, one block per half tile, up to 16 targets of one leaf. GB300 issues
 // two FP64 lanes a cycle and SM, so that the kernel is bound by FP64 instructions, and a
 // lane without a pair costs as much as one with: the block's threads are dealt as
-// (slice, target) with as many slices of the sources as fit, 128 / T for a tile of T
-// targets (87 % of the lanes busy at T = 28, where 32-target tiles with fixed slices have
-// 77 % on average). Sources are staged through shared memory in slabs; a warp reads two or
-// three of them at once (broadcasts). The slices are added in a fixed order; the sums go
+// (slice, target) with as many slices of the sources as fit, 128 / T for T targets. Sources
+// are staged through shared memory in slabs; a warp reads two to five of them at once
+// (broadcasts). The slices are added in a fixed order; the sums go
 // to nearbuf (sorted order), so that the near field runs beside the expansion passes. It
-// does so with NEAR64_CTAS blocks per SM that draw tiles from a counter (zeroed by the
+// does so with NEAR64_CTAS blocks per SM that draw half tiles from a counter (zeroed by the
 // charges' kernel): eight warps keep the FP64 pipe busy, while as many blocks as fit left
 // the expansion passes, which share the pipe warp by warp, a seventh of it and the
 // fixed-point M2L no shared memory.
-// Measured: 3.25 ms for the 110.6 M pairs of 1,048,576 nodes (82 % of the FP64 issue rate
+// Half tiles, because the blocks' work differs: among points spread over decades a leaf beside a
+// dense part has thousands of sources where others have hundreds, and a block with a whole tile
+// of it runs on when the others are done. 12,000 such points with 400 a leaf 3.3 -> 2.4 ms a Cauchy
+// sum (3.1 with a warp per 8 targets reading from global memory), with 200 a leaf 2.8 -> 1.6 (2.5);
+// evenly spread ones 0.31 -> 0.31 ms, 30,000 of them 0.54 -> 0.50. Quarter tiles gain
+// little more there and cost evenly spread points 4 to 10 %.
+// Measured with whole tiles: 3.25 ms for the 110.6 M pairs of 1,048,576 nodes (82 % of the FP64 issue rate
 // at 14 instructions a pair), 149 us for the 4.0 M of 64 x 512; with a warp per 8 targets
 // reading every source from global memory and the longer pair, near and far field
 // together took 9.76 ms and 392 us (now, with the far field below, 5.7 ms and 233 us).
@@ -1797,9 +1802,16 @@ __global__ void __launch_bounds__(128) k_near64(int ntile, int* __restrict__ nex
   for (;;) {
     if (tid == 0) s_tile = atomicAdd(next, 1);
     __syncthreads();
-    const int tile = s_tile;
-    if (tile >= ntile) return;
-    const int4 tl = tiles[tile];
+    const int item = s_tile;
+    if (item >= 2 * ntile) return;
+    int4 tl = tiles[item >> 1];
+    const int mid = tl.y + ((tl.z - tl.y + 1) >> 1);
+    if (item & 1) tl.y = mid;
+    else tl.z = mid;
+    if (tl.y == tl.z) {  // the second half of a single target
+      __syncthreads();
+      continue;
+    }
     const int T = tl.z - tl.y, nsl = 128 / T;
     const int sl = tid / T, i = tl.y + tid - sl * T;
     const double2 zi = zs[i];
@@ -3418,7 +3430,7 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
     } else if (f64) {
       const double2* nq = E == 2 ? w.nc.as<double2>() : w.qa.as<double2>();
       auto go = [&](auto kern) {
-        kern<<<std::min(t.ntile, NEAR64_CTAS * ctx->nsm), 128, 0, ns>>>(
+        kern<<<std::min(2 * t.ntile, NEAR64_CTAS * ctx->nsm), 128, 0, ns>>>(
             t.ntile, next, t.tiles.as<int4>(), t.pt0.as<int>(), t.pt1.as<int>(), t.ustart.as<int>(),
             t.ulist.as<int>(), t.zs.as<double2>(), nq, plus, nb);
       };
