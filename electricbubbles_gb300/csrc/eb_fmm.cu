@@ -1765,30 +1765,34 @@ __device__ __forceinline__ void m2p_eval(const c_t<T>* M, int p, c_t<T> u, T s, 
   }
 }
 
-// FP64 near field, one block per half tile, up to 16 targets of one leaf. GB300 issues
+// FP64 near field, one block per tile of up to EB_NTILE targets of one leaf. GB300 issues
 // two FP64 lanes a cycle and SM, so that the kernel is bound by FP64 instructions, and a
 // lane without a pair costs as much as one with: the block's threads are dealt as
-// (slice, target) with as many slices of the sources as fit, 128 / T for T targets. Sources
-// are staged through shared memory in slabs; a warp reads two to five of them at once
-// (broadcasts). The slices are added in a fixed order; the sums go
+// (slice, target) with as many slices of the sources as fit, 128 / T for a tile of T
+// targets (87 % of the lanes busy at T = 28, where 32-target tiles with fixed slices have
+// 77 % on average). Sources are staged through shared memory in slabs; a warp reads two to five
+// of them at once (broadcasts). The slices are added in a fixed order; the sums go
 // to nearbuf (sorted order), so that the near field runs beside the expansion passes. It
-// does so with NEAR64_CTAS blocks per SM that draw half tiles from a counter (zeroed by the
+// does so with NEAR64_CTAS blocks per SM that draw tiles from a counter (zeroed by the
 // charges' kernel): eight warps keep the FP64 pipe busy, while as many blocks as fit left
 // the expansion passes, which share the pipe warp by warp, a seventh of it and the
 // fixed-point M2L no shared memory.
-// Half tiles, because the blocks' work differs: among points spread over decades a leaf beside a
-// dense part has thousands of sources where others have hundreds, and a block with a whole tile
-// of it runs on when the others are done. 12,000 such points with 400 a leaf 3.3 -> 2.4 ms a Cauchy
-// sum (3.1 with a warp per 8 targets reading from global memory), with 200 a leaf 2.8 -> 1.6 (2.5);
-// evenly spread ones 0.31 -> 0.31 ms, 30,000 of them 0.54 -> 0.50. Quarter tiles gain
-// little more there and cost evenly spread points 4 to 10 %.
-// Measured with whole tiles: 3.25 ms for the 110.6 M pairs of 1,048,576 nodes (82 % of the FP64 issue rate
+// Measured: 3.25 ms for the 110.6 M pairs of 1,048,576 nodes (82 % of the FP64 issue rate
 // at 14 instructions a pair), 149 us for the 4.0 M of 64 x 512; with a warp per 8 targets
 // reading every source from global memory and the longer pair, near and far field
 // together took 9.76 ms and 392 us (now, with the far field below, 5.7 ms and 233 us).
+// HALF: a block takes half a tile. Among points spread over decades (trees with many W lists: from
+// an entry per 8 leaves on) a leaf beside a dense part has thousands of sources where others have
+// hundreds, and a block with a whole tile of it runs on when the others are done: 12,000 such
+// points 1.4 -> 0.8 ms a Cauchy sum, with 200 and 400 a leaf 2.8 -> 1.6 and 3.3 -> 2.4 ms (2.5 and 3.1 with
+// the warp per 8 targets). And with NEAR64_HALF sources a target on average (leaves of hundreds of
+// points), where 126 lanes busy instead of 112 pay for staging every slab twice: 12,000 even
+// points with 400 a leaf 0.94 -> 0.80 ms, 200,001 11.0 -> 9.4 (10.0 with the warp per 8 targets). On the
+// other even trees half tiles take from 6 % less (64 x 1,024) to 7 % more (1,300 x 1,024).
 #define NEAR64_SLAB 128
 #define NEAR64_CTAS 4
-template <int K>
+#define NEAR64_HALF 1024
+template <int K, bool HALF>
 __global__ void __launch_bounds__(128) k_near64(int ntile, int* __restrict__ next,
                                                 const int4* __restrict__ tiles, const int* __restrict__ pt0,
                                                 const int* __restrict__ pt1, const int* __restrict__ ustart,
@@ -1803,14 +1807,16 @@ __global__ void __launch_bounds__(128) k_near64(int ntile, int* __restrict__ nex
     if (tid == 0) s_tile = atomicAdd(next, 1);
     __syncthreads();
     const int item = s_tile;
-    if (item >= 2 * ntile) return;
-    int4 tl = tiles[item >> 1];
-    const int mid = tl.y + ((tl.z - tl.y + 1) >> 1);
-    if (item & 1) tl.y = mid;
-    else tl.z = mid;
-    if (tl.y == tl.z) {  // the second half of a single target
-      __syncthreads();
-      continue;
+    if (item >= (HALF ? 2 * ntile : ntile)) return;
+    int4 tl = tiles[HALF ? item >> 1 : item];
+    if (HALF) {
+      const int mid = tl.y + ((tl.z - tl.y + 1) >> 1);
+      if (item & 1) tl.y = mid;
+      else tl.z = mid;
+      if (tl.y == tl.z) {  // the second half of a single target
+        __syncthreads();
+        continue;
+      }
     }
     const int T = tl.z - tl.y, nsl = 128 / T;
     const int sl = tid / T, i = tl.y + tid - sl * T;
@@ -3429,15 +3435,17 @@ int fmm_run(eb_ctx* ctx, EbTree& t, int sign, const double2* dens, const double2
       else go(k_near_df<NEAR_VC>);
     } else if (f64) {
       const double2* nq = E == 2 ? w.nc.as<double2>() : w.qa.as<double2>();
-      auto go = [&](auto kern) {
-        kern<<<std::min(2 * t.ntile, NEAR64_CTAS * ctx->nsm), 128, 0, ns>>>(
+      // many W lists, or many sources a target on average: see the kernel
+      const bool half = t.nw >= (t.nleaf + 7) / 8 || (double)t.nu / t.nleaf * t.n / t.nleaf >= NEAR64_HALF;
+      auto go = [&](auto whole, auto halves) {
+        (half ? halves : whole)<<<std::min(half ? 2 * t.ntile : t.ntile, NEAR64_CTAS * ctx->nsm), 128, 0, ns>>>(
             t.ntile, next, t.tiles.as<int4>(), t.pt0.as<int>(), t.pt1.as<int>(), t.ustart.as<int>(),
             t.ulist.as<int>(), t.zs.as<double2>(), nq, plus, nb);
       };
-      if (kind == NEAR_Q) go(k_near64<NEAR_Q>);
-      else if (kind == NEAR_QI) go(k_near64<NEAR_QI>);
-      else if (kind == NEAR_V) go(k_near64<NEAR_V>);
-      else go(k_near64<NEAR_VC>);
+      if (kind == NEAR_Q) go(k_near64<NEAR_Q, false>, k_near64<NEAR_Q, true>);
+      else if (kind == NEAR_QI) go(k_near64<NEAR_QI, false>, k_near64<NEAR_QI, true>);
+      else if (kind == NEAR_V) go(k_near64<NEAR_V, false>, k_near64<NEAR_V, true>);
+      else go(k_near64<NEAR_VC, false>, k_near64<NEAR_VC, true>);
     } else {
       const float2* nq = E == 2 ? w.nc.as<float2>() : w.qa.as<float2>();
       auto go = [&](auto kern) {
