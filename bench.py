@@ -736,9 +736,9 @@ def run_gpu(args, rank, world, local):
                                "inner operator, 23 flop per target-source pair)", "bound": "fp32",
                      "achieved": dom["achieved_tflops"], "peak": fp32_peak, "unit": "TFLOP/s",
                      "frac": dom["achieved_tflops"] / fp32_peak,
-                     # DRAM bytes of one k_near32<2> launch of this workload (ncu
-                     # dram__bytes_read.sum + dram__bytes_write.sum: 1,381,632 + 0)
-                     "traffic": 1381632 if WORKLOAD == "many_drops_64x512" else None,
+                     # DRAM bytes of one launch of it on this workload (ncu dram__bytes_read.sum +
+                     # dram__bytes_write.sum: 1,120,512 + 0)
+                     "traffic": 1120512 if WORKLOAD == "many_drops_64x512" else None,
                      "traffic_unit": "bytes per launch (ncu capture of this workload)",
                      "peak_source": "measured in-run FP32 FMA chain (MEASURED_PEAKS.json has no FP32 "
                                     "CUDA-core figure)",

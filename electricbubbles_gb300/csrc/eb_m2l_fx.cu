@@ -22,7 +22,9 @@
 //    accumulators of 48 tensor-memory columns;
 //  * the entries of a target box are added as 64-bit integers with one exponent (the same
 //    result in any order) and become double or double-float once per box.
-// Errors of the sums against direct sums are those of the FP64 kernel (k_m2l) or smaller.
+// Errors of the sums against direct sums are those of the FP64 kernel (k_m2l) or smaller (a
+// single small coefficient of a high order keeps fewer bits than in FP64: all are held to the
+// largest of their entry).
 //
 // What bounds it is the issue of the integer work before and after the products. One block
 // per SM (its accumulators fill the tensor memory) of two teams of 16 warps, each with

@@ -973,7 +973,8 @@ __device__ __forceinline__ double leaf_offset(double z, double x0, unsigned int 
 // Leaf-relative node coordinates as three floats hi + mid + lo (all 53 bits of the
 // double offset), for the double-float near field: wa = (x.hi, y.hi, x.mid, y.mid),
 // wb = (x.lo, y.lo). (hi, mid) alone is a double-float. One thread per point: with a block
-// per leaf, most of its lanes idle, 1,048,576 nodes took 212 us, now 112.
+// per leaf, most of its lanes idle, 1,048,576 nodes took 212 us, now 121 (112 without the
+// quotients' correction).
 __device__ __forceinline__ void split3(double w, float& hi, float& mid, float& lo) {
   hi = __double2float_rn(w);
   double r1 = w - (double)hi;
